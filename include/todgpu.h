@@ -38,11 +38,12 @@ extern "C" {
 /* Flags (todgpu_gather_args.flags). */
 #define TODGPU_FLAG_NO_TABLES 1 /* ignore ring_table: evaluate every stencil ring and spin-2
                                    angle directly (same results, slower) */
-#define TODGPU_FLAG_NO_BEAM_STAGE 2 /* read the beam from global memory even when the launch
-                                       could hold it in shared memory (same results) */
-#define TODGPU_FLAG_WIDE_CTAS 4 /* launch 256-thread CTAs even where the spin-2 table asked
-                                   for (tab_slots) fits 128-thread CTAs at 8 per SM
-                                   (same results) */
+#define TODGPU_FLAG_NO_BEAM_STAGE 2 /* accepted and without effect: every launch reads the beam
+                                       from global memory */
+#define TODGPU_FLAG_WIDE_CTAS 4 /* launch 256-thread CTAs even where 128-thread CTAs would keep
+                                   as many threads on an SM (same results) */
+#define TODGPU_FLAG_BEAM_PLANAR 8 /* vec_orig is planar, (3, S): neighbouring threads read
+                                     neighbouring elements (same results; gather calls only) */
 
 /* Element types. */
 #define TODGPU_F32 0
@@ -115,18 +116,17 @@ typedef struct todgpu_gather_args {
   int64_t tod_stride;
   unsigned long long *err_count; /* optional */
   int32_t flags;         /* TODGPU_FLAG_* */
-  int32_t tab_slots;     /* spin-2 table slots per sample in shared memory (with a
-                            ring table and Q, U): 0 keeps the default of 2048 float64
-                            / 4096 float32 pairs and 192 window rings; a footprint's
-                            worth (about 1.05 (3.06 reach^2 nside^2 + 9 reach nside
-                            + 12) + 32) also sizes the window-ring header (for a disc
-                            of tab_slots / 3.2 pixels; 128-thread CTAs reserve 80
-                            rings) and leaves the rest of the SM's memory to L1; up
-                            to about 1500 float64 / 1900 float32 pairs the call runs
-                            128-thread CTAs, 8 per SM.
-                            Capped to what the kernel's CTAs per SM can share.  A
-                            sample whose footprint needs more evaluates its spin-2
-                            angles directly (same results).  Must be >= 0. */
+  int32_t tab_slots;     /* slots of a sample's value table in shared memory (with a ring
+                            table): one per map pixel of its footprint, holding the
+                            components with Q and U turned (24 bytes for three float64
+                            components, 12 for three float32 ones).  0 keeps the default
+                            of 2048 (float32: 4096) slots and 192 window rings; a
+                            footprint's worth (about 1.03 (3.06 x^2 + 13.2 x + 12) + 8 for
+                            a beam of radius x / nside) also sizes the window's rings, and
+                            the smaller the table the more samples an SM works on.  A
+                            request beyond shared memory makes no table.  A sample whose
+                            footprint needs more than the table evaluates its pixels
+                            directly (same results).  Must be >= 0. */
   const void *ring_table;/* optional: table built by todgpu_ring_table_build for this
                             nside; NULL evaluates ring data and spin-2 angles directly */
   const void *theta;     /* (B,) boresight colatitude (TODGPU_ANGLES) */
@@ -142,16 +142,15 @@ typedef struct todgpu_gather_args {
  * Replaces tod_bilinear._gather_accum_fused_jit (tod_bilinear.py:205-477)
  * and tod_nearest._gather_accum_nearest_jit (tod_nearest.py:21-158).
  * vec_orig must be aligned to its element size and beam_vals to 4 bytes;
- * S is at most 2^29.  When the beam fits in shared memory beside the spin-2
- * table, every CTA copies it there once per launch with bulk copies. */
+ * S is at most 2^29.  Beams of more than 16384 pixels run in passes of 1024
+ * consecutive pixels, each with its own footprint: order such a beam so that
+ * neighbours on the sky follow each other. */
 int todgpu_gather_accum(const todgpu_gather_args *args, void *stream);
 
-/* Number of bounded waits of the gather kernels (the beam's bulk copies into
- * shared memory) that ran out since the library was loaded: 0 in a healthy
- * run.  A CTA whose wait ran out copies the beam with plain loads instead,
- * so its results stay correct; the call's err_count, when given, counts it
- * too.  Reading it synchronises the device; -1 on a CUDA error.  No
- * counterpart in the reference. */
+/* Number of bounded waits of the gather kernels that ran out since the library
+ * was loaded: always 0, as they wait on nothing but their own CTA's barriers.
+ * Synchronises the device; -1 on a CUDA error.  No counterpart in the
+ * reference. */
 int64_t todgpu_gather_wait_timeouts(void);
 
 /* Many jobs in one persistent launch: jobs[0 .. njobs) (a host array) are

@@ -24,8 +24,8 @@ import torch
 
 from . import _native
 from ._device import require_cuda, stream_handle, to_device
-from .kernels import (_map_tensor, _ncomp, _row_stride, _set_map, beam_order, beam_reach, pointing_buffers,
-                      pointing_params, ring_table, table_slots_for)
+from .kernels import (_map_tensor, _ncomp, _row_stride, _set_map, beam_order, beam_reach, planar_beam,
+                      pointing_buffers, pointing_params, ring_table, table_slots_for)
 
 
 class DetectorBatch:
@@ -51,7 +51,7 @@ class DetectorBatch:
             # pixels in the gather's preferred order (neighbours on the sky next to
             # each other; only the order of the pixel sums changes)
             order = torch.from_numpy(beam_order(d["vec_orig"])).to(dev)
-            vec = to_device(d["vec_orig"], np.float64).reshape(-1, 3)[order].contiguous()
+            vec = planar_beam(to_device(d["vec_orig"], np.float64).reshape(-1, 3)[order])[0]
             self.vec.append(vec)
             self.beam.append(to_device(d["beam_vals"], np.float32).reshape(-1)[order].contiguous())
             ang = [to_device(d[k], np.float32).reshape(-1) for k in ("theta", "phi", "psi")]
@@ -106,7 +106,7 @@ class DetectorBatch:
             a.beam_vals = bv.data_ptr()
             a.tod = out.data_ptr()
             a.tod_stride = _row_stride(out)
-            a.flags = self.flags
+            a.flags = self.flags | planar_beam(vec)[1]
             a.ring_table = None if self.tables[j] is None else self.tables[j].data_ptr()
             a.tab_slots = table_slots_for(self.tables[j], self.nside)
         return arr

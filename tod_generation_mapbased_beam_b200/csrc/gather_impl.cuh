@@ -3,29 +3,27 @@
 // instantiate them (gather_map_*.cu, one per map element type) and by the C
 // ABI (tod_api.cu).
 //
-// Work decomposition ("footprint" kernel): a persistent grid of CTAs (128
-// threads, 8 per SM, when the sample's spin-2 table fits an eighth of an SM's
-// shared memory; else 256 threads, 3-4 per SM) walks the samples; a CTA takes
-// one sample at a time and
-//   1. rotates the beam's centre direction with the sample's rotation to get
-//      the footprint centre, and derives the window of RING rings the
-//      footprint (beam radius + stencil reach) can touch;
-//   2. tabulates per window ring (in shared memory) the ring layout, ring z,
-//      acos(ring z) and sqrt(1 - z^2), and the longitude range of ring pixels
-//      inside the footprint;
-//   3. tabulates cos 2d / sin 2d of the spin-2 frame rotation for every ring
-//      pixel in the footprint once (a stencil pixel is shared by ~16 (beam
-//      pixel, neighbour) pairs of a sample);
-//   4. strides its threads over the beam pixels: rotate -> atan2/clamp ->
-//      RING stencil (ring data from the window) -> spin-2 (from the table) ->
-//      gather -> FP64 accumulate;
-//   5. reduces the per-lane sums (256 summation lanes in either CTA shape) in
-//      a fixed order and adds them into tod[c, b] (one writer per sample: no
-//      atomics, bit-reproducible runs, the same TOD in both shapes).
-// Table values are produced by the same functions on the same inputs as
-// direct evaluation, so they are bit-identical to it; any lookup outside the
-// window (or a footprint too large for the tables) falls back to direct
-// evaluation.  The window therefore only decides speed, never results.
+// Work decomposition ("footprint" kernel): a persistent grid of CTAs (128 or
+// 256 threads) walks the samples; a CTA takes one sample
+// at a time and
+//   1. has its rotation, footprint centre and range of RING rings prepared, for
+//      eight samples at a time by eight lanes of one warp (prepare_sample);
+//   2. lays out the window of rings the footprint (beam radius + stencil
+//      reach) can touch, each ring's stretch of the footprint disc and the
+//      ring in the sample's own longitude frame (footprint_window);
+//   3. evaluates the map once per footprint pixel into shared memory: I, and Q
+//      and U turned into the boresight's frame (fill_table; a map pixel is
+//      shared by ~10 (beam pixel, neighbour) pairs of a sample);
+//   4. strides its threads over the beam pixels: rotation into the frame ->
+//      longitude by a short series -> ring and in-ring position from the window
+//      -> weighted sum of four table entries (bilinear_table) or the nearest
+//      one (nearest_window);
+//   5. reduces the per-lane sums (256 summation lanes in either CTA shape) in a
+//      fixed order and adds them into tod[c, b] (one writer per sample: no
+//      atomics, bit-reproducible runs, the same TOD in every shape).
+// A pixel that the window or the table does not hold takes bilinear_direct /
+// nearest_exact, which do the same operations on the same values without
+// them: windows and tables only decide speed, never results.
 //
 // Compiled with -fmad=false: the pixel decisions and the FP64 accumulation
 // reproduce the reference's uncontracted arithmetic.
@@ -49,21 +47,29 @@
 
 namespace todgpu {
 
-constexpr int kRingCap = 192;   // rings per footprint window
-constexpr int kTabCapDefault = 2048;  // spin-2 table slots per sample (32 KB)
+constexpr int kRingCap = 192;   // rings per footprint window, at most
+constexpr int kTabCapDefault = 2048;  // table slots per sample when the caller asks for none
 constexpr long long kMaxNside = 16384;
-constexpr int kNTStatic = 256;  // threads of the reach kernel of the built-in table
 // Summation lanes of the gather: the beam pixels of a sample are summed in
-// kSumLanes strided partial sums (then per warp of lanes, then over those in
-// order), whatever the CTA's thread count, so CTAs of 128 and 256 threads
-// give the same TOD bit for bit.
+// this many strided partial sums, combined in a fixed order whatever the CTA's
+// thread count, so CTAs of 128 and 256 threads give the same TOD bit for bit.
 constexpr int kSumLanes = 256;
-// The narrow CTA shape (128 threads, 8 per SM) and the window rings its table
-// header always reserves, so that the table's offset is a compile-time constant
-// of that shape (the wide shape sizes its header per launch).
-constexpr int kNTNarrow = 128;
-constexpr int kMinbNarrow = 8;
-constexpr int kRingCapNarrow = 80;
+// Registers per thread and the threads that then fit an SM (in CTAs of 128).
+// Measured at 64 / 72 / 80 / 96: the 30' float64 beam 2.59 / 2.57 / 2.59 / 2.65
+// ms, detectors over a float32 map 4.69 / 4.51 / 4.44 / 5.2 ms, packed float32
+// records 1.91 / 1.97 / 1.94 / 2.5 ms: the pixel loops spill a few registers
+// below 72, and above it too few warps are left.
+constexpr int kRegs = 72;
+constexpr int kThreadsSM = 65536 / kRegs / 128 * 128;
+
+// Bytes of a window's rings and their slot ends.
+__host__ __device__ constexpr size_t window_bytes(int ring_cap) {
+  return (84 * (size_t)ring_cap + 15) & ~size_t(15);
+}
+// Bytes of the slot -> ring index of a table (one entry per 32 slots).
+__host__ __device__ constexpr size_t ring_of_bytes(int tab_cap) {
+  return (2 * ((size_t)tab_cap / 32 + 1) + 15) & ~size_t(15);
+}
 
 // Message of the calling thread's last failure (defined in tod_api.cu).
 extern thread_local std::string g_last_error;
@@ -80,7 +86,7 @@ inline int cuda_fail(cudaError_t e, const char* what) {
 struct KArgs {
   long long nside, npix, B, S;
   int C, c_q, c_u;
-  int tab_cap;               // spin-2 table slots in shared memory
+  int tab_cap;               // table slots in shared memory
   int tab_req;               // slots the caller asks for (0: default)
   const void* ring_table;    // RingRec[4 nside] or nullptr
   const void* vec;
@@ -103,10 +109,10 @@ struct KArgs {
   double* tod;
   long long tod_stride;
   unsigned long long* err;
-  int flags_stage;           // the caller allows staging the beam in shared memory
-  int beam_stage;            // the launch made room for the beam in shared memory
-  int flags_wide;            // the caller asks for 256-thread CTAs
-  int ring_cap;              // window rings the launch's table header holds
+  int flags_wide;            // the caller asks for CTAs of at least 256 threads
+  int ring_cap;              // window rings the launch has room for
+  int vec_ss;                // beam vectors: component i of pixel s at vec[s vec_ss + i vec_si]
+  long long vec_si;
 };
 
 // Pointing modes of the per-sample rotation.
@@ -296,40 +302,6 @@ __device__ __forceinline__ void load_boresight(const KArgs& a, const SampleRot& 
   boresight_from_fields<PM>(a, rot, GlobalFields<PM>{a, b}, z, sth, phi);
 }
 
-struct PackF32;
-struct PackBF16;
-struct PackF64;
-template <typename MapT>
-__device__ __forceinline__ float4 load_rec(const KArgs& a, long long p);
-__device__ __forceinline__ float rec_at(const float4& r, int c);
-
-template <typename MapT>
-__device__ __forceinline__ double map_at(const KArgs& a, int c, long long p) {
-  if constexpr (std::is_same<MapT, PackF32>::value || std::is_same<MapT, PackBF16>::value)
-    return (double)rec_at(load_rec<MapT>(a, p), c);
-  else if constexpr (std::is_same<MapT, PackF64>::value)
-    return __ldg(static_cast<const double*>(a.map) + 4 * p + c);
-  else
-    return (double)__ldg(static_cast<const MapT*>(a.map) + (long long)c * a.map_stride + p);
-}
-
-// mp[c, p] * bv with the nearest kernel's typing (tod_nearest.py:146, :158):
-// a float32 map element times the float32 weight is a float32 product.
-template <typename MapT>
-__device__ __forceinline__ double map_x_beam(const KArgs& a, int c, long long p, float bv) {
-  if constexpr (std::is_same<MapT, PackF32>::value || std::is_same<MapT, PackBF16>::value) {
-    return (double)(rec_at(load_rec<MapT>(a, p), c) * bv);
-  } else if constexpr (std::is_same<MapT, PackF64>::value) {
-    return __ldg(static_cast<const double*>(a.map) + 4 * p + c) * (double)bv;
-  } else {
-    const MapT m = __ldg(static_cast<const MapT*>(a.map) + (long long)c * a.map_stride + p);
-    if constexpr (sizeof(MapT) == 4)
-      return (double)(m * bv);
-    else
-      return m * (double)bv;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Map element types.  Planar float/double maps are the reference's
 // mp_stacked (C, N); the precision form packs a pixel's components into one
@@ -348,45 +320,27 @@ struct PackF64 {};
 template <typename MapT>
 struct MapTraits {
   static constexpr bool packed = false;
-  using Tab = double2;
 };
 template <>
 struct MapTraits<PackF32> {
   static constexpr bool packed = true;
-  using Tab = float2;
 };
 template <>
 struct MapTraits<PackBF16> {
   static constexpr bool packed = true;
-  using Tab = float2;
 };
 
 __device__ __forceinline__ float bf16_lo(unsigned v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(unsigned v) { return __uint_as_float(v & 0xffff0000u); }
 
 template <typename MapT>
-__device__ __forceinline__ float4 load_rec(const KArgs& a, long long p) {
+__device__ __forceinline__ float4 load_rec(const void* map, long long p) {
   if constexpr (std::is_same<MapT, PackF32>::value) {
-    return __ldg(static_cast<const float4*>(a.map) + p);
+    return __ldg(static_cast<const float4*>(map) + p);
   } else {
-    const uint2 r = __ldg(static_cast<const uint2*>(a.map) + p);
+    const uint2 r = __ldg(static_cast<const uint2*>(map) + p);
     return make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
   }
-}
-
-__device__ __forceinline__ float rec_at(const float4& r, int c) {
-  return c == 0 ? r.x : (c == 1 ? r.y : (c == 2 ? r.z : r.w));
-}
-
-template <typename TabT>
-__device__ __forceinline__ TabT make_tab(double c, double s);
-template <>
-__device__ __forceinline__ double2 make_tab<double2>(double c, double s) {
-  return make_double2(c, s);
-}
-template <>
-__device__ __forceinline__ float2 make_tab<float2>(double c, double s) {
-  return make_float2((float)c, (float)s);
 }
 
 // Per-thread accumulators: float64 (parity path) or float32 with Kahan
@@ -415,13 +369,10 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // ---------------------------------------------------------------------------
-// Ring table (global memory, built once per nside and footprint reach) and
-// the per-sample spin-2 table (shared memory).
+// Ring table (global memory, built once per nside and footprint reach).
 // ---------------------------------------------------------------------------
 
-// One RING ring.  Record 0 is a header: z = nside, ta = reach [rad].  The
-// fields come in 16-byte pairs in the order the stencil reads them: {z, sth},
-// {phi0, dphi}, {ta, inv_dta}, {first32, n, inv_dphi}.
+// One RING ring.  Record 0 is a header: z = nside, ta = reach [rad].
 struct __align__(16) RingRec {
   double z;         // ring centre z
   double sth;       // sqrt(max(0, 1 - z^2))
@@ -433,12 +384,31 @@ struct __align__(16) RingRec {
   int n;            // pixels in the ring
   double inv_dphi;  // 1 / dphi, correctly rounded
   long long first;  // first pixel index
-  int cap;          // spin-2 table slots reserved for this ring
+  int cap;          // table slots reserved for this ring
   int unused;
 };
 static_assert(sizeof(RingRec) == 80, "RingRec must be 80 bytes");
 static_assert(offsetof(RingRec, phi0) == 16 && offsetof(RingRec, ta) == 32 && offsetof(RingRec, first32) == 48,
               "RingRec pairs must sit on 16-byte boundaries");
+
+// The geometry of ring ir (all fields but cap), the values the ring table holds.
+__device__ __forceinline__ RingRec make_ring(long long nside, long long ir) {
+  const RingInfo ri = hp_ring_info(nside, ir, 12 * nside * nside);
+  RingRec r;
+  r.z = hp_ring_z(nside, ir);
+  r.ta = acos(r.z);
+  r.sth = sqrt(max0(1.0 - r.z * r.z));
+  r.phi0 = ri.phi0;
+  r.dphi = ri.dphi;
+  r.first = ri.first;
+  r.first32 = (int)ri.first;
+  r.n = (int)ri.n;
+  r.inv_dphi = 1.0 / ri.dphi;
+  r.inv_dta = ir < 4 * nside - 1 ? 1.0 / (acos(hp_ring_z(nside, ir + 1)) - r.ta) : 0.0;
+  r.cap = 0;
+  r.unused = 0;
+  return r;
+}
 
 // Ring provider backed by the global ring table.
 struct TableRings {
@@ -457,113 +427,80 @@ struct TableRings {
   __device__ __forceinline__ double sth(long long ir, const RingData&) const { return __ldg(&t[ir].sth); }
 };
 
-// Per-sample spin-2 table: window ring r (ring ir_lo + r) has ring[r] =
-// {off, iplo, cap, 0}: slots [off, off + cap) hold cos 2d / sin 2d of its
-// in-ring pixels iplo, iplo + 1, ... (mod n).  hdr = {ir_lo in 32 bits, window
-// rings (0: no table for this sample), filled slots, 0}.
-// A launch reserves ring[0 .. KArgs::ring_cap) (at least 1: ring_win reads
-// ring[0] for a sample without a window; at most kRingCap); the table's slots
-// follow at spin2_header_bytes(ring_cap).
-struct Spin2Tab {
-  int4 hdr;
-  long long ir_lo;
-  long long unused;
-  int4 ring[kRingCap];
-};
-static_assert(offsetof(Spin2Tab, ring) == 32 && sizeof(int4) == 16, "Spin2Tab layout");
-__host__ __device__ constexpr size_t spin2_header_bytes(int ring_cap) { return 32 + 16 * (size_t)ring_cap; }
+// ---------------------------------------------------------------------------
+// Per-sample state in shared memory.
+// ---------------------------------------------------------------------------
 
-struct Bore {
-  double z, sth, phi;
-};
-
-// One sample's rotation and boresight in shared memory, written by one thread
-// and read by all: the roll about the boresight p (cos/sin psi and 1 - cos
-// psi), the recentring about axis k (float64 form with 1 - cos a; for float32
-// parameters the reference's float32 inputs, and 1 - (double) cos a), and the
-// boresight (z, sin theta, phi) of the spin-2 angle.  Pairs sit on 16-byte
-// boundaries for 16-byte shared loads.
+// One sample, prepared by one thread for all.  The bilinear path works in the
+// sample's frame: longitudes are measured from phi_u, the longitude of the
+// rotated beam centre u, so a beam pixel's longitude is a small angle (an
+// arctangent series of six terms) and every stencil position a small number
+// relative to its ring's own origin.  m maps a beam vector (float64
+// parameters: the vector itself; reference float32 parameters: the vector
+// after the reference's float32-typed recentring) to (x, y, z) of that frame:
+// longitude phi_u + atan2(y, x), z the sky's.
 struct __align__(16) SampleBlock {
-  double px, py, pz, cp, sp, omp;
-  double kx, ky, kz, ca, sa, oma;
-  float fkx, fky, fkz, fca, fsa, fpad0, fpad1, fpad2;
-  double bz, bsth, bphi, bpad;
+  double m[9];
+  double oma;                                                // 1 - cos a
+  float fkx, fky, fkz, fca, fsa, fpad0, fpad1, fpad2;        // reference float32 recentring
+  double bz, bsth, bdl;                                      // boresight: z, sin theta, longitude - phi_u in [-pi, pi]
+  double phi_u, theta_u;                                     // rotated beam centre
+  int ir_lo, nr;                                             // window rings (nr = 0: none)
+  double cu, su;                                             // cos, sin of theta_u
 };
-static_assert(sizeof(SampleBlock) == 160, "SampleBlock layout");
+static_assert(sizeof(SampleBlock) == 176 && offsetof(SampleBlock, cu) == 160 && offsetof(SampleBlock, fkx) == 80, "SampleBlock layout");
 
-// A sample's pointing fields in shared memory, brought there by cp.async one
-// sample ahead (field i at byte 4 i for the reference float32 parameters, at
-// byte 8 i otherwise).
-struct __align__(16) RawFields {
-  unsigned long long v[12];
-};
-
-template <int PM>
-struct SharedFields {
-  const KArgs& a;
-  const RawFields& raw;
-  __device__ __forceinline__ auto operator()(int i) const {
-    if constexpr (PM == kParamsRef32)
-      return reinterpret_cast<const float*>(raw.v)[i];
-    else if constexpr (PM == kAngles)
-      return a.angles_f32 ? (double)reinterpret_cast<const float*>(raw.v)[2 * i]
-                          : reinterpret_cast<const double*>(raw.v)[i];
-    else
-      return reinterpret_cast<const double*>(raw.v)[i];
-  }
+// The reference's own two-step rotation (k, a; p, psi), for the nearest
+// rule's exact path.
+struct ExactBlock {
+  double px, py, pz, cp, sp;
+  double kx, ky, kz, ca, sa;
 };
 
-// Lane `lane` of one warp starts the copy of field `lane` of sample b into raw
-// (cp.async, this GPU's memory); every lane commits its group.
-template <int PM>
-__device__ __forceinline__ void prefetch_fields(const KArgs& a, long long b, RawFields& raw, int lane) {
-  if (lane < field_count<PM>()) {
-    const void* src = field_ptr<PM>(a, b, lane);
-    if (src != nullptr) {
-      const unsigned dst =
-          (unsigned)__cvta_generic_to_shared(reinterpret_cast<unsigned char*>(raw.v) + (PM == kParamsRef32 ? 4 : 8) * lane);
-      if (field_bytes<PM>(a) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-      else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-    }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+// Samples prepared together, one lane each: the preparation is a serial chain
+// of some 500 float64 operations, so sixteen lanes of one warp run it side by
+// side.
+constexpr int kPrep = 16;
+
+// One ring of a sample's window: the ring in the sample's frame (origin k0 +
+// f0 in units of pixels: the longitude phi_u lies f0 past pixel k0), its
+// stretch of the footprint and its geometry.  The stretch is the cnt pixels
+// from -(cnt - 1) / 2 about k0; pixel j (relative to k0) has table slot base +
+// j; slots = base << 16 | cnt - 1 (both below 65536 where a table is used).
+// 80 bytes: 16-byte reads of eight neighbouring rings fall on different
+// banks.  The pixel loop reads 36 bytes of the ring above and 20 of the one
+// below (28 and 12 in the belt): every 4 bytes a lane reads cost a
+// shared-memory wavefront.
+struct __align__(16) RingWin {
+  double f0, inv_dphi;
+  double rta, inv_dta;  // acos(z) - theta_u; 1 / (acos(z of the next ring) - acos(z))
+  double z, sth;
+  long long first;
+  double dphi;
+  unsigned slots;
+  int k0, n, pad;
+};
+static_assert(sizeof(RingWin) == 80 && offsetof(RingWin, rta) == 16 && offsetof(RingWin, z) == 32 &&
+                  offsetof(RingWin, first) == 48 && offsetof(RingWin, slots) == 64,
+              "RingWin layout");
+
+// Table slot of pixel j; true when pixels j .. j + count - 1 all have one.
+__device__ __forceinline__ bool slot_of(unsigned slots, int j, int count, int& slot) {
+  const int top = (int)(slots & 0xffffu);
+  slot = (int)(slots >> 16) + j;
+  return (unsigned)(j + (top >> 1)) < (unsigned)(top + 2 - count);
 }
 
-// One thread fills a sample's block from its fields (got: GlobalFields or
-// SharedFields); out of line, so that its registers stay out of the pixel loop.
-template <int PM, class Get>
-__device__ __noinline__ void write_block(const KArgs& a, Get got, bool has_qu, SampleBlock& sb) {
-  const SampleRot r = rot_from_fields<PM>(a, got);
-  sb.px = r.px;
-  sb.py = r.py;
-  sb.pz = r.pz;
-  sb.cp = r.cp;
-  sb.sp = r.sp;
-  sb.omp = 1.0 - r.cp;
-  sb.kx = r.kx;
-  sb.ky = r.ky;
-  sb.kz = r.kz;
-  sb.ca = r.ca;
-  sb.sa = r.sa;
-  if constexpr (PM == kParamsRef32) {
-    sb.fkx = r.fkx;
-    sb.fky = r.fky;
-    sb.fkz = r.fkz;
-    sb.fca = r.fca;
-    sb.fsa = r.fsa;
-    sb.oma = 1.0 - (double)r.fca;
-  } else {
-    sb.oma = 1.0 - r.ca;
-  }
-  if (has_qu) {
-    double z, sth, phi;
-    boresight_from_fields<PM>(a, r, got, z, sth, phi);
-    sb.bz = z;
-    sb.bsth = sth;
-    sb.bphi = phi;
-  }
+// The window's header: x first ring, y rings that have a next ring in the
+// window (0: no window), z table slots (0: no table).
+struct Bore {
+  double z, sth;
+};
+
+// Longitude of the boresight less that of pixel j (relative to k0) of a ring
+// whose origin is f0.
+__device__ __forceinline__ double pixel_dphi(double bdl, double f0, int j, double dphi) {
+  return fma(f0 - (double)j, dphi, bdl);
 }
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -571,142 +508,383 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)_
 // Shared-memory loads that stay inside the pixel loop (the values are the
 // same for every pixel of a sample; loading them per pixel keeps them out of
 // the registers the evaluation needs).
-__device__ __forceinline__ double2 lds_d2(const void* p) {
+__device__ __forceinline__ double2 lds_d2(unsigned p) {
   double2 v;
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(smem_u32(p)));
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(p));
   return v;
 }
-__device__ __forceinline__ double lds_d1(const void* p) {
+__device__ __forceinline__ double lds_d1(unsigned p) {
   double v;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(smem_u32(p)));
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(p));
   return v;
 }
-__device__ __forceinline__ float4 lds_f4(const void* p) {
+__device__ __forceinline__ float4 lds_f4(unsigned p) {
   float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(smem_u32(p)));
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p));
   return v;
 }
-__device__ __forceinline__ int4 lds_i4(const void* p) {
-  int4 v;
-  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(smem_u32(p)));
+__device__ __forceinline__ unsigned lds_u1(unsigned p) {
+  unsigned v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p));
   return v;
 }
 
-__device__ __forceinline__ Bore block_bore(const SampleBlock* sb) {
-  const double2 zs = lds_d2(&sb->bz);
-  return Bore{zs.x, zs.y, lds_d1(&sb->bphi)};
+// ---------------------------------------------------------------------------
+// Elementary functions of small arguments.
+// ---------------------------------------------------------------------------
+
+constexpr double kNearTan = 0.125;  // largest |tan| / angle of the series below
+
+// y / x for x > 0 finite: hardware reciprocal estimate, one Newton step and a
+// residual correction (Markstein, IBM J. Res. Dev. 34(1), 1990).
+__device__ __forceinline__ double div_near(double y, double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  const double q = y * r;
+  return fma(fma(-x, q, y), r, q);
 }
 
-// Rotated beam pixel with the sample's block: the operations of rot_ref32
-// (float32 parameters, float32 beam vector) or rot_f64 (float64), with 1 - cos a
-// and 1 - cos psi taken from the block (the same values).
-__device__ __forceinline__ void rotate_block(const SampleBlock* sb, float vx, float vy, float vz, double& ox,
-                                             double& oy, double& oz) {
-  const float4 fk = lds_f4(&sb->fkx);  // fkx, fky, fkz, fca
-  const float fsa = lds_f4(&sb->fsa).x;
-  const double oma = lds_d2(&sb->sa).y;
-  const float dkv = fk.x * vx + fk.y * vy + fk.z * vz;
-  const float ax = vx * fk.w + (fk.y * vz - fk.z * vy) * fsa;
-  const float ay = vy * fk.w + (fk.z * vx - fk.x * vz) * fsa;
-  const float az = vz * fk.w + (fk.x * vy - fk.y * vx) * fsa;
-  const double rx = (double)ax + (double)(fk.x * dkv) * oma;
-  const double ry = (double)ay + (double)(fk.y * dkv) * oma;
-  const double rz = (double)az + (double)(fk.z * dkv) * oma;
-  const double2 pxy = lds_d2(&sb->px), pzc = lds_d2(&sb->pz), so = lds_d2(&sb->sp);
-  const double dpr = pxy.x * rx + pxy.y * ry + pzc.x * rz;
-  ox = rx * pzc.y + (pxy.y * rz - pzc.x * ry) * so.x + pxy.x * dpr * so.y;
-  oy = ry * pzc.y + (pzc.x * rx - pxy.x * rz) * so.x + pxy.y * dpr * so.y;
-  oz = rz * pzc.y + (pxy.x * ry - pxy.y * rx) * so.x + pzc.x * dpr * so.y;
-}
-__device__ __forceinline__ void rotate_block(const SampleBlock* sb, double vx, double vy, double vz, double& ox,
-                                             double& oy, double& oz) {
-  const double2 kxy = lds_d2(&sb->kx), kzc = lds_d2(&sb->kz), sao = lds_d2(&sb->sa);
-  const double dkv = kxy.x * vx + kxy.y * vy + kzc.x * vz;
-  const double rx = vx * kzc.y + (kxy.y * vz - kzc.x * vy) * sao.x + kxy.x * dkv * sao.y;
-  const double ry = vy * kzc.y + (kzc.x * vx - kxy.x * vz) * sao.x + kxy.y * dkv * sao.y;
-  const double rz = vz * kzc.y + (kxy.x * vy - kxy.y * vx) * sao.x + kzc.x * dkv * sao.y;
-  const double2 pxy = lds_d2(&sb->px), pzc = lds_d2(&sb->pz), so = lds_d2(&sb->sp);
-  const double dpr = pxy.x * rx + pxy.y * ry + pzc.x * rz;
-  ox = rx * pzc.y + (pxy.y * rz - pzc.x * ry) * so.x + pxy.x * dpr * so.y;
-  oy = ry * pzc.y + (pzc.x * rx - pxy.x * rz) * so.x + pxy.y * dpr * so.y;
-  oz = rz * pzc.y + (pxy.x * ry - pxy.y * rx) * so.x + pzc.x * dpr * so.y;
+// sqrt(s) for s > 0: reciprocal square-root estimate and Goldschmidt's
+// iteration with a residual correction (same reference).
+__device__ __forceinline__ double sqrt_near(double s) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  double g = s * y, h = 0.5 * y;
+  const double r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  return fma(fma(-g, g, s), h, g);
 }
 
-// The float64 form of the block's rotation applied to a float64 vector (the
-// footprint centre; the operations of rot_f64).
-__device__ __forceinline__ void rotate_block_f64(const SampleBlock& sb, double vx, double vy, double vz, double& ox,
-                                                 double& oy, double& oz) {
-  const double dkv = sb.kx * vx + sb.ky * vy + sb.kz * vz;
-  const double rx = vx * sb.ca + (sb.ky * vz - sb.kz * vy) * sb.sa + sb.kx * dkv * sb.oma;
-  const double ry = vy * sb.ca + (sb.kz * vx - sb.kx * vz) * sb.sa + sb.ky * dkv * sb.oma;
-  const double rz = vz * sb.ca + (sb.kx * vy - sb.ky * vx) * sb.sa + sb.kz * dkv * sb.oma;
-  const double dpr = sb.px * rx + sb.py * ry + sb.pz * rz;
-  ox = rx * sb.cp + (sb.py * rz - sb.pz * ry) * sb.sp + sb.px * dpr * sb.omp;
-  oy = ry * sb.cp + (sb.pz * rx - sb.px * rz) * sb.sp + sb.py * dpr * sb.omp;
-  oz = rz * sb.cp + (sb.px * ry - sb.py * rx) * sb.sp + sb.pz * dpr * sb.omp;
+// atan(t) for |t| <= kNearTan: Taylor series through t^15 (the first term left
+// out, t^17 / 17, is below 3e-17 there).
+__device__ __forceinline__ double atan_near(double t) {
+  const double w = t * t;
+  double p = fma(w, -1.0 / 15.0, 1.0 / 13.0);
+  p = fma(w, p, -1.0 / 11.0);
+  p = fma(w, p, 1.0 / 9.0);
+  p = fma(w, p, -1.0 / 7.0);
+  p = fma(w, p, 1.0 / 5.0);
+  p = fma(w, p, -1.0 / 3.0);
+  return fma(t * w, p, t);
 }
 
-template <typename TabT>
-__device__ __forceinline__ void spin2_lookup(const Spin2Tab& w, const TabT* tab, long long ring, long long ip,
-                                             long long n, double zn, double phin, const Bore& bo, double& c2d,
-                                             double& s2d) {
-  // ip is the pixel's in-ring index and n its ring's length; the spill case
-  // (ip == n) and anything outside the window use direct evaluation.
-  const long long r = ring - w.ir_lo;
-  if ((unsigned long long)r < (unsigned long long)w.hdr.y && (unsigned long long)ip < (unsigned long long)n) {
-    const int4 wr = w.ring[r];
-    long long j = ip - wr.y;
-    if (j < 0) j += n;
-    if (j >= 0 && j < wr.z) {
-      const TabT v = tab[wr.x + j];
-      c2d = (double)v.x;
-      s2d = (double)v.y;
-      return;
+// sin and cos of |x| <= kNearTan by their Taylor series (terms left out below
+// 2e-17 relative).
+__device__ __forceinline__ void sincos_near(double x, double& s, double& c) {
+  const double w = x * x;
+  double p = fma(w, 1.0 / 362880.0, -1.0 / 5040.0);
+  p = fma(w, p, 1.0 / 120.0);
+  p = fma(w, p, -1.0 / 6.0);
+  s = fma(x * w, p, x);
+  double q = fma(w, -1.0 / 3628800.0, 1.0 / 40320.0);
+  q = fma(w, q, -1.0 / 720.0);
+  q = fma(w, q, 1.0 / 24.0);
+  q = fma(w, q, -0.5);
+  c = fma(w, q, 1.0);
+}
+
+// Longitude of (x, y) in the sample's frame.
+// x > 0 and |t| < kNearTan for t = y / x by div_near, on the high words (a t
+// that is not finite -- x zero, denormal, infinite or NaN -- fails).
+__device__ __forceinline__ bool lon_is_near(double x, double t) {
+  return __double2hiint(x) >= 0 && (__double2hiint(t) & 0x7fffffff) < 0x3fc00000;
+}
+__device__ __forceinline__ double frame_lon(double x, double y) {
+  const double t = div_near(y, x);
+  return lon_is_near(x, t) ? atan_near(t) : atan2(y, x);
+}
+
+// cos 2d / sin 2d of the frame rotation between a pixel centre and the
+// boresight for longitudes up to kNearTan apart (false beyond: spin2_far).
+// Reference float32 parameters: the haversine form of spin2_c2s2 (the
+// reference forms the boresight's sin theta from a float32 square, so its z
+// and sin theta disagree by 6e-8, and only the same
+// form of N and D gives the same angle).  Float64 pointing: the same ratio
+// N / D with the common factor 2h divided out,
+//   N : D = (z + z_b) sin dphi : sin theta sin theta_b + (1 + z z_b) cos dphi,
+// half the operations and well conditioned (D is near 2 for a nearby pixel).
+template <int PM>
+__device__ __forceinline__ bool spin2_small(double z, double sth, double dphi, const Bore& bo, double& c2d,
+                                            double& s2d) {
+  if ((__double2hiint(dphi) & 0x7fffffff) >= 0x3fc00000) return false;  // |dphi| >= kNearTan
+  double N, D;
+  if constexpr (PM == kParamsRef32) {
+    if (dphi == 0.0 && bo.sth == sth && bo.z == z) {
+      c2d = 1.0;
+      s2d = 0.0;
+      return true;
+    }
+    double sh, ch;
+    sincos_near(dphi * 0.5, sh, ch);
+    const double sin_dphi = 2.0 * ch * sh;
+    const double sh2 = sh * sh;
+    const double cos_dphi = fma(-2.0, sh2, 1.0);
+    const double dz = bo.z - z, ds = bo.sth - sth;
+    const double st2 = 0.25 * fma(dz, dz, ds * ds);
+    const double S = sth * bo.sth, S2 = S * sh2;
+    N = 2.0 * sin_dphi * ((bo.z + z) * (st2 + S2));
+    const double q = 4.0 * st2;
+    D = fma(q - q * st2, cos_dphi, fma(S * sin_dphi, sin_dphi, -4.0 * (bo.z * z) * (S2 * sh2)));
+  } else {
+    double s, c;
+    sincos_near(dphi, s, c);
+    N = s * (bo.z + z);
+    D = fma(fma(bo.z, z, 1.0), c, sth * bo.sth);
+  }
+  const double n2 = N * N;
+  const double u = div_near(1.0, fma(D, D, n2));
+  c2d = fma(D, D, -n2) * u;
+  s2d = 2.0 * N * D * u;
+  return true;
+}
+static __device__ __noinline__ double2 spin2_far(double z, double sth, double dphi, double bz, double bsth) {
+  double2 r;
+  spin2_c2s2(z, sth, 0.0, bz, bsth, dphi, r.x, r.y);
+  return r;
+}
+
+// Position of the frame's origin longitude on a ring: phi_u lies f0 in [0, 1)
+// pixels past pixel k0 (mod the ring's length).
+__device__ __forceinline__ void ring_origin(double phi_u, double phi0, double dphi, double inv_dphi, int& k0,
+                                            double& f0) {
+  const double x = phi_u - phi0;
+  const double k = floor(x * inv_dphi);
+  f0 = fma(-k, dphi, x) * inv_dphi;
+  k0 = (int)k;
+}
+
+// ---------------------------------------------------------------------------
+// Per-sample preparation (one lane per sample, out of line).
+// ---------------------------------------------------------------------------
+
+// 3 x 3 matrix of r -> r cos t + (k x r) sin t + k (k . r) (1 - cos t).
+__device__ __forceinline__ void rodrigues_matrix(double x, double y, double z, double c, double s, double omc,
+                                                 double* m) {
+  const double ox = omc * x, oy = omc * y, oz = omc * z;
+  m[0] = fma(ox, x, c);
+  m[1] = fma(ox, y, -(s * z));
+  m[2] = fma(ox, z, s * y);
+  m[3] = fma(oy, x, s * z);
+  m[4] = fma(oy, y, c);
+  m[5] = fma(oy, z, -(s * x));
+  m[6] = fma(oz, x, -(s * y));
+  m[7] = fma(oz, y, s * x);
+  m[8] = fma(oz, z, c);
+}
+
+template <int PM>
+__device__ __noinline__ void prepare_sample(const KArgs& a, long long b, bool has_qu, double cx, double cy, double cz,
+                                            double rbeam, bool window, double polar, SampleBlock& sb,
+                                            ExactBlock* eb) {
+  const GlobalFields<PM> got{a, b};
+  const SampleRot r = rot_from_fields<PM>(a, got);
+  if (eb != nullptr) {
+    eb->px = r.px;
+    eb->py = r.py;
+    eb->pz = r.pz;
+    eb->cp = r.cp;
+    eb->sp = r.sp;
+    eb->kx = r.kx;
+    eb->ky = r.ky;
+    eb->kz = r.kz;
+    eb->ca = r.ca;
+    eb->sa = r.sa;
+  }
+  const double omp = 1.0 - r.cp, oma = 1.0 - r.ca;
+  sb.oma = oma;
+  if constexpr (PM == kParamsRef32) {
+    sb.fkx = r.fkx;
+    sb.fky = r.fky;
+    sb.fkz = r.fkz;
+    sb.fca = r.fca;
+    sb.fsa = r.fsa;
+  }
+  double bphi = 0.0;
+  if (has_qu) {
+    double z, sth;
+    boresight_from_fields<PM>(a, r, got, z, sth, bphi);
+    sb.bz = z;
+    sb.bsth = sth;
+  }
+  double A[9], M[9];
+  rodrigues_matrix(r.px, r.py, r.pz, r.cp, r.sp, omp, A);
+  rodrigues_matrix(r.kx, r.ky, r.kz, r.ca, r.sa, oma, M);
+  double ux, uy, uz;
+  {
+    const double wx = fma(M[0], cx, fma(M[1], cy, M[2] * cz));
+    const double wy = fma(M[3], cx, fma(M[4], cy, M[5] * cz));
+    const double wz = fma(M[6], cx, fma(M[7], cy, M[8] * cz));
+    ux = fma(A[0], wx, fma(A[1], wy, A[2] * wz));
+    uy = fma(A[3], wx, fma(A[4], wy, A[5] * wz));
+    uz = fma(A[6], wx, fma(A[7], wy, A[8] * wz));
+  }
+  double phi_u = atan2(uy, ux);
+  if (phi_u < 0.0) phi_u += kTwoPi;
+  double s, c;
+  sincos(phi_u, &s, &c);
+  // rows of the roll turned by -phi_u about z, then times the recentring
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double a0 = A[j], a1 = A[3 + j];
+    A[j] = fma(c, a0, s * a1);
+    A[3 + j] = fma(c, a1, -(s * a0));
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      sb.m[3 * i + j] = PM == kParamsRef32
+                            ? A[3 * i + j]
+                            : fma(A[3 * i], M[j], fma(A[3 * i + 1], M[3 + j], A[3 * i + 2] * M[6 + j]));
+  sb.phi_u = phi_u;
+  double bdl = bphi - phi_u;
+  if (bdl > kPi)
+    bdl -= kTwoPi;
+  else if (bdl < -kPi)
+    bdl += kTwoPi;
+  sb.bdl = bdl;
+  const double theta_u = acos(clamp1(uz));
+  sb.theta_u = theta_u;
+  sincos(theta_u, &sb.su, &sb.cu);
+  int ir_lo = 0, nr = 0;
+  const double th_lo = theta_u - rbeam, th_hi = theta_u + rbeam;
+  if (window && isfinite(phi_u) && isfinite(uz) && th_lo >= polar && th_hi <= kPi - polar) {
+    long long lo = th_lo <= 0.0 ? 1 : hp_ring_above(a.nside, cos(th_lo));
+    long long hi = th_hi >= kPi ? 4 * a.nside - 1 : hp_ring_above(a.nside, cos(th_hi)) + 1;
+    lo = max(lo, 1LL);
+    hi = min(hi, 4 * a.nside - 1);
+    if (hi >= lo && hi - lo + 1 <= a.ring_cap) {
+      ir_lo = (int)lo;
+      nr = (int)(hi - lo + 1);
     }
   }
-  const double sth_n = sqrt(max0(1.0 - zn * zn));
-  spin2_c2s2(zn, sth_n, phin, bo.z, bo.sth, bo.phi, c2d, s2d);
+  sb.ir_lo = ir_lo;
+  sb.nr = nr;
 }
 
-// Beam centre direction (normalised mean of the beam vectors) and the
-// largest angle between it and any beam vector; block-wide, once per CTA.
-template <int PM, int NT>
-__device__ void beam_extent(const KArgs& a, double* s_red, double& cx, double& cy, double& cz, double& radius) {
-  constexpr int NW = NT / 32;
+// Two beam pixels (or one) in the sample's frame.  The rotation is read from
+// shared memory for every pair: held in registers (18, and 7 more for the
+// reference typing) it left room for a third fewer warps.
+template <int N>
+__device__ __forceinline__ void to_frame(unsigned sb, const double (&v)[N][3], double* x, double* y, double* z) {
+  const double2 m0 = lds_d2(sb), m1 = lds_d2(sb + 16);
+#pragma unroll
+  for (int k = 0; k < N; ++k) x[k] = fma(m0.x, v[k][0], fma(m0.y, v[k][1], m1.x * v[k][2]));
+  const double2 m2 = lds_d2(sb + 32);
+#pragma unroll
+  for (int k = 0; k < N; ++k) y[k] = fma(m1.y, v[k][0], fma(m2.x, v[k][1], m2.y * v[k][2]));
+  const double2 m3 = lds_d2(sb + 48);
+  const double m8 = lds_d1(sb + 64);
+#pragma unroll
+  for (int k = 0; k < N; ++k) z[k] = fma(m3.x, v[k][0], fma(m3.y, v[k][1], m8 * v[k][2]));
+}
+template <int N>
+__device__ __forceinline__ void rotate_frame(unsigned sb, const double* const* vec, const int (&at)[N], double* x,
+                                             double* y, double* z) {
+  double v[N][3];
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[k][i] = __ldg(vec[i] + at[k]);
+  to_frame<N>(sb, v, x, y, z);
+}
+// Reference typing: the recentring's products and sums are float32, as in
+// rot_ref32 (the same bits), the roll and the frame float64.
+template <int N>
+__device__ __forceinline__ void rotate_frame(unsigned sb, const float* const* vec, const int (&at)[N], double* x,
+                                             double* y, double* z) {
+  double v[N][3];
+  const float4 fk = lds_f4(sb + 80);  // fkx, fky, fkz, fca
+  const float fsa = __uint_as_float(lds_u1(sb + 96));
+  const double oma = lds_d1(sb + 72);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const float vx = __ldg(vec[0] + at[k]), vy = __ldg(vec[1] + at[k]), vz = __ldg(vec[2] + at[k]);
+    const float dkv = fk.x * vx + fk.y * vy + fk.z * vz;
+    const float ax = vx * fk.w + (fk.y * vz - fk.z * vy) * fsa;
+    const float ay = vy * fk.w + (fk.z * vx - fk.x * vz) * fsa;
+    const float az = vz * fk.w + (fk.x * vy - fk.y * vx) * fsa;
+    v[k][0] = (double)ax + (double)(fk.x * dkv) * oma;
+    v[k][1] = (double)ay + (double)(fk.y * dkv) * oma;
+    v[k][2] = (double)az + (double)(fk.z * dkv) * oma;
+  }
+  to_frame<N>(sb, v, x, y, z);
+}
+
+// The reference's own rotation of a beam pixel (rot_ref32 / rot_f64).
+__device__ __forceinline__ void rotate_exact(const SampleBlock* sb, const ExactBlock* eb, float vx, float vy, float vz,
+                                             double& ox, double& oy, double& oz) {
+  SampleRot r;
+  r.px = eb->px;
+  r.py = eb->py;
+  r.pz = eb->pz;
+  r.cp = eb->cp;
+  r.sp = eb->sp;
+  r.fkx = sb->fkx;
+  r.fky = sb->fky;
+  r.fkz = sb->fkz;
+  r.fca = sb->fca;
+  r.fsa = sb->fsa;
+  rot_ref32(r, vx, vy, vz, ox, oy, oz);
+}
+__device__ __forceinline__ void rotate_exact(const SampleBlock*, const ExactBlock* eb, double vx, double vy, double vz,
+                                             double& ox, double& oy, double& oz) {
+  SampleRot r;
+  r.px = eb->px;
+  r.py = eb->py;
+  r.pz = eb->pz;
+  r.cp = eb->cp;
+  r.sp = eb->sp;
+  r.kx = eb->kx;
+  r.ky = eb->ky;
+  r.kz = eb->kz;
+  r.ca = eb->ca;
+  r.sa = eb->sa;
+  rot_f64(r, vx, vy, vz, ox, oy, oz);
+}
+
+// Beam centre direction (normalised mean of the beam vectors [s0, s1)) and the
+// largest angle between it and any of them; by the whole CTA.  The mean is
+// summed by the first 128 threads whatever the CTA's size, so that every CTA
+// shape measures longitudes in the same frame, bit for bit.
+constexpr int kMeanLanes = 128;
+template <int PM>
+__device__ void beam_extent(const KArgs& a, int s0, int s1, double* s_red, double& cx, double& cy, double& cz,
+                            double& radius) {
+  using VecT = typename std::conditional<PM == kParamsRef32, float, double>::type;
+  const VecT* vec = static_cast<const VecT*>(a.vec);
+  const long long si = a.vec_si;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, NT = blockDim.x;
   double sx = 0.0, sy = 0.0, sz = 0.0;
-  for (long long s = threadIdx.x; s < a.S; s += NT) {
-    if constexpr (PM != kParamsRef32) {
-      const double* v = static_cast<const double*>(a.vec) + 3 * s;
-      sx += v[0];
-      sy += v[1];
-      sz += v[2];
-    } else {
-      const float* v = static_cast<const float*>(a.vec) + 3 * s;
+  __syncthreads();  // earlier users of s_red are done
+  if (tid < kMeanLanes) {
+#pragma unroll 4
+    for (int s = s0 + tid; s < s1; s += kMeanLanes) {
+      const VecT* v = vec + (long long)s * a.vec_ss;
       sx += (double)v[0];
-      sy += (double)v[1];
-      sz += (double)v[2];
+      sy += (double)v[si];
+      sz += (double)v[2 * si];
     }
-  }
-  sx = warp_sum(sx);
-  sy = warp_sum(sy);
-  sz = warp_sum(sz);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    s_red[warp * 4 + 0] = sx;
-    s_red[warp * 4 + 1] = sy;
-    s_red[warp * 4 + 2] = sz;
+    sx = warp_sum(sx);
+    sy = warp_sum(sy);
+    sz = warp_sum(sz);
+    if (lane == 0) {
+      s_red[warp * 4 + 0] = sx;
+      s_red[warp * 4 + 1] = sy;
+      s_red[warp * 4 + 2] = sz;
+    }
   }
   __syncthreads();
   sx = sy = sz = 0.0;
-  for (int i = 0; i < NW; ++i) {
+  for (int i = 0; i < kMeanLanes / 32; ++i) {
     sx += s_red[i * 4 + 0];
     sy += s_red[i * 4 + 1];
     sz += s_red[i * 4 + 2];
   }
   const double nrm = sqrt(sx * sx + sy * sy + sz * sz);
-  if (nrm > 0.0) {
+  if (nrm > 0.0 && nrm < 1e300) {
     cx = sx / nrm;
     cy = sy / nrm;
     cz = sz / nrm;
@@ -716,19 +894,10 @@ __device__ void beam_extent(const KArgs& a, double* s_red, double& cx, double& c
     cz = 1.0;
   }
   double mind = 1.0;
-  for (long long s = threadIdx.x; s < a.S; s += NT) {
-    double vx, vy, vz;
-    if constexpr (PM != kParamsRef32) {
-      const double* v = static_cast<const double*>(a.vec) + 3 * s;
-      vx = v[0];
-      vy = v[1];
-      vz = v[2];
-    } else {
-      const float* v = static_cast<const float*>(a.vec) + 3 * s;
-      vx = v[0];
-      vy = v[1];
-      vz = v[2];
-    }
+#pragma unroll 4
+  for (int s = s0 + tid; s < s1; s += NT) {
+    const VecT* v = vec + (long long)s * a.vec_ss;
+    const double vx = v[0], vy = v[si], vz = v[2 * si];
     const double vn = sqrt(vx * vx + vy * vy + vz * vz);
     const double d = vn > 0.0 ? (vx * cx + vy * cy + vz * cz) / vn : -1.0;
     mind = fmin(mind, d);
@@ -739,313 +908,419 @@ __device__ void beam_extent(const KArgs& a, double* s_red, double& cx, double& c
   if (lane == 0) s_red[warp] = mind;
   __syncthreads();
   mind = 1.0;
-  for (int i = 0; i < NW; ++i) mind = fmin(mind, s_red[i]);
+  for (int i = 0; i < NT / 32; ++i) mind = fmin(mind, s_red[i]);
   __syncthreads();
   radius = acos(clamp1(mind));
 }
 
 // ---------------------------------------------------------------------------
-// The beam in shared memory.  When the launch leaves room after the spin-2
-// table, each CTA copies its job's beam (pixel vectors and weights, in the
-// caller's layout) there once with bulk copies (cp.async.bulk, 1-D, this
-// GPU's memory, no multicast) on an mbarrier, the unaligned ends of the two
-// arrays with plain loads, and the pixel loop reads it from shared memory.
-// Every wait is bounded: a wait that runs out is counted in
-// g_gather_wait_timeouts (and in the call's error counter), the CTA copies the
-// beam with plain loads instead and waits, again bounded, for the bulk copies
-// it started before going on.
-// ---------------------------------------------------------------------------
-
-constexpr int kStageWaitLimit = 1 << 20;
-__device__ unsigned long long g_gather_wait_timeouts;
-
-// Shared-memory bytes of a staged beam of S pixels with vector elements of
-// vec_elem bytes: each array rounded up to 16 bytes, plus 16 for the offset
-// that keeps a shared copy congruent to its global source modulo 16.
-__host__ __device__ constexpr size_t beam_stage_bytes(long long S, size_t vec_elem) {
-  return (((size_t)(3 * S) * vec_elem + 15) / 16) * 16 + 16 + (((size_t)S * 4 + 15) / 16) * 16 + 16;
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
-  unsigned done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-               : "=r"(done)
-               : "r"(bar), "r"(parity)
-               : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity) {
-  for (int it = 0; it < kStageWaitLimit; ++it)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
-// One array of `count` elements of T at global `src` into shared memory at
-// `region` (16-byte aligned); returns the shared copy's element 0.  Thread 0
-// issues the bulk copy of the 16-byte aligned middle (its bytes are added to
-// `tx`); every thread copies its share of the ends.
-template <typename T, int NT>
-__device__ __forceinline__ T* stage_array(const T* src, long long count, unsigned char* region, unsigned bar,
-                                          unsigned& tx, bool issue) {
-  const unsigned long long g = reinterpret_cast<unsigned long long>(src);
-  const unsigned long long g_end = g + (unsigned long long)count * sizeof(T);
-  const unsigned pad = (unsigned)(g & 15u);
-  T* dst = reinterpret_cast<T*>(region + pad);
-  const unsigned long long body = (g + 15u) & ~15ull, body_end = g_end & ~15ull;
-  // elements [0, head) and [tail0, count) go by plain loads (whole elements:
-  // the source is element-aligned), [head, tail0) by the bulk copy
-  long long head = count, tail0 = count;
-  unsigned bytes = 0;
-  if (body_end > body) {
-    bytes = (unsigned)(body_end - body);
-    head = (long long)((body - g) / sizeof(T));
-    tail0 = (long long)((body_end - g) / sizeof(T));
-  }
-  if (bytes > 0 && issue && threadIdx.x == 0) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(region + pad + (body - g))),
-                 "l"(body), "r"(bytes), "r"(bar)
-                 : "memory");
-  }
-  tx += bytes;
-  const long long ends = head + (count - tail0);
-  for (long long e = threadIdx.x; e < (issue ? ends : count); e += NT) {
-    const long long i = issue ? (e < head ? e : tail0 + (e - head)) : e;
-    dst[i] = src[i];
-  }
-  return dst;
-}
-
-template <typename VecT, int NT>
-__device__ void stage_beam(const KArgs& a, unsigned char* region, unsigned long long* bar_mem, const VecT*& vsrc,
-                           const float*& bsrc) {
-  // (vsrc, bsrc: the shared copies on return)
-  const unsigned bar = smem_u32(bar_mem);
-  const long long S = a.S;
-  unsigned char* vreg = region;
-  unsigned char* breg = region + ((3 * S * sizeof(VecT) + 15) / 16) * 16 + 16;
-  __syncthreads();  // earlier users of the region (the previous job) are done
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    // order this CTA's earlier generic-proxy accesses of the region before the
-    // bulk copies' writes
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  __syncthreads();
-  // bytes the bulk copies will deliver (the same in every thread)
-  unsigned tx = 0;
-  {
-    const unsigned long long gv = reinterpret_cast<unsigned long long>(a.vec);
-    const unsigned long long gb = reinterpret_cast<unsigned long long>(a.beam);
-    const unsigned long long ve = gv + (unsigned long long)(3 * S) * sizeof(VecT), be = gb + (unsigned long long)S * 4;
-    const unsigned long long vb = (gv + 15) & ~15ull, vbe = ve & ~15ull, bb = (gb + 15) & ~15ull, bbe = be & ~15ull;
-    tx = (unsigned)((vbe > vb ? vbe - vb : 0) + (bbe > bb ? bbe - bb : 0));
-  }
-  if (threadIdx.x == 0 && tx > 0)
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tx) : "memory");
-  unsigned tx_issued = 0;
-  VecT* sv = stage_array<VecT, NT>(static_cast<const VecT*>(a.vec), 3 * S, vreg, bar, tx_issued, true);
-  float* sbv = stage_array<float, NT>(a.beam, S, breg, bar, tx_issued, true);
-  bool ok = true;
-  if (tx > 0) ok = mbar_wait_bounded(bar, 0);
-  if (!ok) {
-    // the bulk copies did not report back in time: copy everything with plain
-    // loads (the same bytes), then give the copies in flight a last bounded wait
-    if (threadIdx.x == 0) {
-      atomicAdd(&g_gather_wait_timeouts, 1ull);
-      if (a.err != nullptr) atomicAdd(a.err, 1ull);
-    }
-    unsigned dummy = 0;
-    stage_array<VecT, NT>(static_cast<const VecT*>(a.vec), 3 * S, vreg, bar, dummy, false);
-    stage_array<float, NT>(a.beam, S, breg, bar, dummy, false);
-    mbar_wait_bounded(bar, 0);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-  vsrc = sv;
-  bsrc = sbv;
-}
-
-// One beam pixel's contribution per component: generic path (64-bit indices,
-// any ring provider, any component layout), used without a ring table and for
-// non-finite rotated vectors.  err = 1: a stencil pixel fell outside the map,
-// nothing to add.
-struct Contrib {
-  double v[4];
-  int err;
-};
-
-template <int MODE, bool HAS_QU, typename MapT, class Rings, typename TabT>
-__device__ __forceinline__ Contrib generic_terms(const KArgs& a, const SampleBlock* sb, const Rings& rings,
-                                                 const Spin2Tab& w, const TabT* tab, double vx, double vy, double vz,
-                                                 double phi_w, float bvf) {
-  Contrib out{{0.0, 0.0, 0.0, 0.0}, 0};
-  const double bv = (double)bvf;
-  const Bore bo{sb->bz, sb->bsth, sb->bphi};
-  if constexpr (MODE == TODGPU_BILINEAR) {
-    const double z = clamp1(vz);
-    // Per-neighbour terms are summed in the reference's order k = 0..3.
-    double tq = 0.0, tu = 0.0, to[4] = {0.0, 0.0, 0.0, 0.0};
-    bool ok = true;
-    hp_stencil(a.nside, z, phi_w, rings,
-               [&](int k, long long p, double wk, long long ring, long long ip, long long n, double zn,
-                   double phin) {
-                 if ((unsigned long long)p >= (unsigned long long)a.npix) {
-                   ok = false;
-                   return;
-                 }
-                 if constexpr (HAS_QU) {
-                   double c2, s2;
-                   spin2_lookup(w, tab, ring, ip, n, zn, phin, bo, c2, s2);
-                   const double q = map_at<MapT>(a, a.c_q, p);
-                   const double u = map_at<MapT>(a, a.c_u, p);
-                   const double vq = wk * fma(q, c2, u * s2);
-                   const double vu = wk * fma(u, c2, -q * s2);
-                   tq = (k == 0) ? vq : tq + vq;
-                   tu = (k == 0) ? vu : tu + vu;
-                 }
-                 for (int c = 0; c < a.C; ++c) {
-                   if (HAS_QU && (c == a.c_q || c == a.c_u)) continue;
-                   const double m = map_at<MapT>(a, c, p);
-                   to[c] = (k == 0) ? wk * m : fma(wk, m, to[c]);
-                 }
-               });
-    if (!ok) {
-      out.err = 1;
-      return out;
-    }
-    for (int c = 0; c < a.C; ++c) {
-      if (HAS_QU && c == a.c_q)
-        out.v[c] = tq * bv;
-      else if (HAS_QU && c == a.c_u)
-        out.v[c] = tu * bv;
-      else
-        out.v[c] = to[c] * bv;
-    }
-  } else {
-    const double sin_th = sqrt(max0(vx * vx + vy * vy));
-    const Nearest nb = hp_nearest(a.nside, vz, sin_th, phi_w, rings);
-    if ((unsigned long long)nb.pix >= (unsigned long long)a.npix) {
-      out.err = 1;
-      return out;
-    }
-    if constexpr (HAS_QU) {
-      double c2d, s2d;
-      spin2_lookup(w, tab, nb.ring, nb.ip, nb.n, nb.zc, nb.phic, bo, c2d, s2d);
-      const double qv = map_at<MapT>(a, a.c_q, nb.pix);
-      const double uv = map_at<MapT>(a, a.c_u, nb.pix);
-      for (int c = 0; c < a.C; ++c) {
-        if (c == a.c_q)
-          out.v[c] = fma(qv, c2d, uv * s2d) * bv;
-        else if (c == a.c_u)
-          out.v[c] = fma(uv, c2d, -qv * s2d) * bv;
-        else
-          out.v[c] = map_x_beam<MapT>(a, c, nb.pix, bvf);
-      }
-    } else {
-      for (int c = 0; c < a.C; ++c) out.v[c] = map_x_beam<MapT>(a, c, nb.pix, bvf);
-    }
-  }
-  return out;
-}
-
-// The generic path out of line, in the form that measured faster for each mode:
-// bilinear returns its terms by value (adding into the caller's accumulator
-// by reference would keep that accumulator in local memory for the whole
-// pixel loop: 15 -> 12 local loads per warp-evaluation, +1.3% on config 2);
-// nearest adds them itself (by value measured 2.7% slower there).
-template <int MODE, bool HAS_QU, typename MapT, class Rings, typename TabT>
-__device__ __noinline__ Contrib eval_generic(const KArgs& a, const SampleBlock* sb, const Rings& rings,
-                                             const Spin2Tab& w, const TabT* tab, double vx, double vy, double vz,
-                                             double phi_w, float bvf) {
-  return generic_terms<MODE, HAS_QU, MapT>(a, sb, rings, w, tab, vx, vy, vz, phi_w, bvf);
-}
-
-template <int MODE, bool HAS_QU, typename MapT, class Rings, typename TabT, class Acc>
-__device__ __noinline__ void eval_generic_into(const KArgs& a, const SampleBlock* sb, const Rings& rings,
-                                               const Spin2Tab& w, const TabT* tab, double vx, double vy, double vz,
-                                               double phi_w, float bvf, Acc& acc, unsigned long long& nerr) {
-  const Contrib r = generic_terms<MODE, HAS_QU, MapT>(a, sb, rings, w, tab, vx, vy, vz, phi_w, bvf);
-  if (r.err) {
-    ++nerr;
-  } else {
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-      if (c < a.C) acc.add(c, r.v[c]);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Fast path: finite rotated vector, ring table present, nside <= 8192 (all
-// ring and pixel indices fit 32 bits).  Same decisions and the same floating
-// point operations as the generic path, with 32-bit index arithmetic, ring
-// data from the table in 16-byte loads, a compile-time component layout and
-// the spin-2 window looked up once per ring.
+// Values of one map pixel as the accumulation uses them: every component,
+// with Q and U turned into the boresight's frame.
 // ---------------------------------------------------------------------------
 
 constexpr int kLayoutGeneric = 0;  // runtime C, c_q, c_u
 constexpr int kLayoutIQU = 1;      // C = 3, Q at 1, U at 2
 
-struct RingFast {
-  int n, first;
-  double phi0, dphi, z, ta, inv_dphi, inv_dta;
+template <int LAYOUT>
+struct Chan {
+  int C, q, u;
+  Chan() = default;
+  __device__ __forceinline__ explicit Chan(const KArgs& a) : C(a.C), q(a.c_q), u(a.c_u) {}
+};
+template <>
+struct Chan<kLayoutIQU> {
+  static constexpr int C = 3, q = 1, u = 2;
+  Chan() = default;
+  __device__ __forceinline__ explicit Chan(const KArgs&) {}
 };
 
-__device__ __forceinline__ RingFast ring_fast(const RingRec* rt, int ir) {
-  const RingRec* r = rt + ir;
-  const double2 zs = __ldg(reinterpret_cast<const double2*>(&r->z));
-  const double2 pd = __ldg(reinterpret_cast<const double2*>(&r->phi0));
-  const double2 ti = __ldg(reinterpret_cast<const double2*>(&r->ta));
-  const int4 fn = __ldg(reinterpret_cast<const int4*>(&r->first32));
-  RingFast d;
-  d.z = zs.x;
-  d.phi0 = pd.x;
-  d.dphi = pd.y;
-  d.ta = ti.x;
-  d.inv_dta = ti.y;
-  d.first = fn.x;
-  d.n = fn.y;
-  d.inv_dphi = __longlong_as_double(((long long)(unsigned)fn.w << 32) | (unsigned)fn.z);
-  return d;
+template <typename MapT>
+using ValT = typename std::conditional<MapTraits<MapT>::packed, float, double>::type;
+
+template <typename R>
+struct Vals {
+  R v[4];
+};
+
+// q turned by (c2, s2) and u turned by (c2, s2): the products of the reference
+// (tod_bilinear.py:440-470), float32 for packed float32/bfloat16 records.
+__device__ __forceinline__ double turn_q(double q, double u, double c2, double s2) { return fma(q, c2, u * s2); }
+__device__ __forceinline__ double turn_u(double q, double u, double c2, double s2) { return fma(u, c2, -q * s2); }
+__device__ __forceinline__ float turn_q(float q, float u, double c2, double s2) {
+  return fmaf(q, (float)c2, u * (float)s2);
+}
+__device__ __forceinline__ float turn_u(float q, float u, double c2, double s2) {
+  return fmaf(u, (float)c2, -q * (float)s2);
 }
 
-// The ring above also needs sin theta of its centre.
-__device__ __forceinline__ RingFast ring_fast_sth(const RingRec* rt, int ir, double& sth) {
-  const RingRec* r = rt + ir;
-  const double2 zs = __ldg(reinterpret_cast<const double2*>(&r->z));
-  const double2 pd = __ldg(reinterpret_cast<const double2*>(&r->phi0));
-  const double2 ti = __ldg(reinterpret_cast<const double2*>(&r->ta));
-  const int4 fn = __ldg(reinterpret_cast<const int4*>(&r->first32));
-  RingFast d;
-  d.z = zs.x;
-  sth = zs.y;
-  d.phi0 = pd.x;
-  d.dphi = pd.y;
-  d.ta = ti.x;
-  d.inv_dta = ti.y;
-  d.first = fn.x;
-  d.n = fn.y;
-  d.inv_dphi = __longlong_as_double(((long long)(unsigned)fn.w << 32) | (unsigned)fn.z);
-  return d;
+template <typename R>
+__device__ __forceinline__ R pick4(const R* v, int c) {
+  return c == 0 ? v[0] : (c == 1 ? v[1] : (c == 2 ? v[2] : v[3]));
 }
 
-// hp_ring_above for a finite |z| <= 1 (int() of an in-range value truncates).
-__device__ __forceinline__ int ring_above_fast(int nside, double z) {
+struct MapRef {
+  const void* map;
+  long long stride;
+};
+
+template <typename MapT, int LAYOUT>
+__device__ __forceinline__ Vals<ValT<MapT>> raw_vals(const Chan<LAYOUT>& ch, const MapRef& m, long long p) {
+  Vals<ValT<MapT>> o{{0, 0, 0, 0}};
+  if constexpr (MapTraits<MapT>::packed) {
+    const float4 r = load_rec<MapT>(m.map, p);
+    o.v[0] = r.x;
+    o.v[1] = r.y;
+    o.v[2] = r.z;
+    o.v[3] = r.w;
+  } else if constexpr (std::is_same<MapT, PackF64>::value) {
+    const double2 lo = __ldg(static_cast<const double2*>(m.map) + 2 * p);
+    o.v[0] = lo.x;
+    o.v[1] = lo.y;
+    if (ch.C > 2) {
+      const double2 hi = __ldg(static_cast<const double2*>(m.map) + 2 * p + 1);
+      o.v[2] = hi.x;
+      o.v[3] = hi.y;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (c < ch.C) o.v[c] = (double)__ldg(static_cast<const MapT*>(m.map) + (long long)c * m.stride + p);
+  }
+  return o;
+}
+
+template <typename MapT, int LAYOUT>
+__device__ __forceinline__ Vals<ValT<MapT>> turned_vals(const Chan<LAYOUT>& ch, const MapRef& m, long long p,
+                                                        double c2, double s2) {
+  using R = ValT<MapT>;
+  Vals<R> o = raw_vals<MapT, LAYOUT>(ch, m, p);
+  const R q = pick4(o.v, ch.q), u = pick4(o.v, ch.u);
+  const R tq = turn_q(q, u, c2, s2), tu = turn_u(q, u, c2, s2);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c == ch.q) o.v[c] = tq;
+    if (c == ch.u) o.v[c] = tu;
+  }
+  return o;
+}
+
+template <int PM, bool HAS_QU, typename MapT, int LAYOUT>
+__device__ __forceinline__ Vals<ValT<MapT>> pixel_vals(const Chan<LAYOUT>& ch, const MapRef& m, const Bore& bo,
+                                                       double z, double sth, double dphi, long long p) {
+  if constexpr (HAS_QU) {
+    double c2, s2;
+    if (!spin2_small<PM>(z, sth, dphi, bo, c2, s2)) {
+      const double2 r = spin2_far(z, sth, dphi, bo.z, bo.sth);
+      c2 = r.x;
+      s2 = r.y;
+    }
+    return turned_vals<MapT, LAYOUT>(ch, m, p, c2, s2);
+  } else {
+    return raw_vals<MapT, LAYOUT>(ch, m, p);
+  }
+}
+
+// The sample's value table in shared memory: slot i holds the values of one
+// footprint pixel -- packed maps components 0 and 1 as a pair, then component
+// 2 and component 3 arrays; float64 values components 0 and 1
+// as a pair (a single for C = 1), then component 2 and component 3 arrays.
+__host__ __device__ constexpr int slot_bytes(bool packed, int C) {
+  return packed ? (C <= 3 ? 12 : 16) : (C == 1 ? 8 : (C == 2 ? 16 : (C == 3 ? 24 : 32)));
+}
+
+template <typename MapT, int LAYOUT>
+struct ValTable {
+  using R = ValT<MapT>;
+  unsigned base;  // shared address
+  int cap;
+  __device__ __forceinline__ void store(const Chan<LAYOUT>& ch, int i, const Vals<R>& o) const {
+    if constexpr (MapTraits<MapT>::packed) {
+      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(base + 8u * i), "f"(o.v[0]), "f"(o.v[1]) : "memory");
+      asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + 8u * cap + 4u * i), "f"(o.v[2]) : "memory");
+      if (ch.C > 3) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + 12u * cap + 4u * i), "f"(o.v[3]) : "memory");
+    } else {
+      if (ch.C == 1) {
+        asm volatile("st.shared.f64 [%0], %1;" ::"r"(base + 8u * i), "d"(o.v[0]) : "memory");
+        return;
+      }
+      asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(base + 16u * i), "d"(o.v[0]), "d"(o.v[1]) : "memory");
+      if (ch.C > 2) asm volatile("st.shared.f64 [%0], %1;" ::"r"(base + 16u * cap + 8u * i), "d"(o.v[2]) : "memory");
+      if (ch.C > 3) asm volatile("st.shared.f64 [%0], %1;" ::"r"(base + 24u * cap + 8u * i), "d"(o.v[3]) : "memory");
+    }
+  }
+  __device__ __forceinline__ Vals<R> load(const Chan<LAYOUT>& ch, int i) const {
+    Vals<R> o{{0, 0, 0, 0}};
+    if constexpr (MapTraits<MapT>::packed) {
+      asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(o.v[0]), "=f"(o.v[1]) : "r"(base + 8u * i));
+      o.v[2] = __uint_as_float(lds_u1(base + 8u * cap + 4u * i));
+      if (ch.C > 3) o.v[3] = __uint_as_float(lds_u1(base + 12u * cap + 4u * i));
+    } else {
+      if (ch.C == 1) {
+        o.v[0] = lds_d1(base + 8u * i);
+        return o;
+      }
+      const double2 p = lds_d2(base + 16u * i);
+      o.v[0] = p.x;
+      o.v[1] = p.y;
+      if (ch.C > 2) o.v[2] = lds_d1(base + 16u * cap + 8u * i);
+      if (ch.C > 3) o.v[3] = lds_d1(base + 24u * cap + 8u * i);
+    }
+    return o;
+  }
+};
+
+// Weighted sum of the four neighbours per component, in the reference's order
+// k = 0..3; float32 (with the reference form's separate Q/U products) for
+// packed maps.
+template <typename MapT, int LAYOUT, bool HAS_QU>
+struct Mix {
+  using R = ValT<MapT>;
+  R t[4];
+  __device__ __forceinline__ void add(const Chan<LAYOUT>& ch, bool start, double wk, const Vals<R>& o) {
+    const R w = (R)wk;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c >= ch.C) break;
+      if constexpr (MapTraits<MapT>::packed) {
+        if (HAS_QU && (c == ch.q || c == ch.u)) {
+          const float x = w * o.v[c];
+          t[c] = start ? x : t[c] + x;
+          continue;
+        }
+      }
+      t[c] = start ? w * o.v[c] : fma(w, o.v[c], t[c]);
+    }
+  }
+};
+
+// What one beam pixel adds per component; err = 1: nothing (non-finite or
+// outside the map).
+struct Contrib {
+  double v[4];
+  int err;
+};
+
+template <typename MapT>
+__device__ __forceinline__ void accumulate(Acc64& acc, int c, double t, float bv) {
+  acc.v[c] = fma(t, (double)bv, acc.v[c]);
+}
+template <typename MapT>
+__device__ __forceinline__ void accumulate(AccKahan& acc, int c, float t, float bv) {
+  acc.add(c, t * bv);
+}
+
+// ---------------------------------------------------------------------------
+// Bilinear stencil.
+// ---------------------------------------------------------------------------
+
+// hp_ring_above for |z| <= 1, with the table path's square root and one fused
+// multiply-add (the weights are continuous across a ring).
+__device__ __forceinline__ long long ring_above(long long nside, double z) {
   const double az = fabs(z);
   if (az > kTwoThirds) {
-    const int ir = (int)((double)nside * sqrt(3.0 * (1.0 - az)));
-    return (z < 0.0) ? 4 * nside - ir - 1 : ir;
+    const double s = 3.0 * (1.0 - az);
+    const long long ir = s > 0.0 ? (long long)((double)nside * sqrt_near(s)) : 0;
+    return z < 0.0 ? 4 * nside - ir - 1 : ir;
   }
-  return (int)((double)nside * (2.0 - 1.5 * z));
+  return (long long)((double)nside * fma(-1.5, z, 2.0));
 }
 
-// (x + d) mod n for 0 <= x <= n, 1 <= d <= 2 and n >= 4.
-__device__ __forceinline__ int wrap_up(int x, int d, int n) {
-  const int v = x + d;
-  return v >= n ? v - n : v;
+// theta_q - theta_u of a query z from sin(theta_q - theta_u) = cos(theta_u)
+// sin(theta_q) - z sin(theta_u) and the arcsine series for angles under
+// kNearSin (the first term left out, 231/13312 d^13, is below 2e-18 there).
+constexpr double kNearSin = 0.0625;
+__device__ __forceinline__ double colat_near(double z, double cu, double su, double& d) {
+  d = fma(cu, sqrt_near((1.0 - z) * (1.0 + z)), -z * su);
+  const double d2 = d * d;
+  double p = fma(d2, 63.0 / 2816.0, 35.0 / 1152.0);
+  p = fma(d2, p, 5.0 / 112.0);
+  p = fma(d2, p, 3.0 / 40.0);
+  p = fma(d2, p, 1.0 / 6.0);
+  return fma(d * d2, p, d);
 }
+__device__ __forceinline__ bool sin_is_near(double d) { return (__double2hiint(d) & 0x7fffffff) < 0x3fb00000; }
+
+__device__ __forceinline__ RingRec ring_at(const KArgs& a, long long ir) {
+  if (a.ring_table != nullptr) {
+    const RingRec* r = static_cast<const RingRec*>(a.ring_table) + ir;
+    RingRec o;
+    o.z = __ldg(&r->z);
+    o.sth = __ldg(&r->sth);
+    o.phi0 = __ldg(&r->phi0);
+    o.dphi = __ldg(&r->dphi);
+    o.ta = __ldg(&r->ta);
+    o.inv_dta = __ldg(&r->inv_dta);
+    o.n = __ldg(&r->n);
+    o.inv_dphi = __ldg(&r->inv_dphi);
+    o.first = __ldg(&r->first);
+    return o;
+  }
+  return make_ring(a.nside, ir);
+}
+
+// One beam pixel without the sample's table: any position (poles, ring ends, longitudes far from the frame's
+// origin), every ring and pixel value evaluated here.  Out of line; the same
+// operations on the same values as the table path.
+template <int PM, bool HAS_QU, typename MapT, int LAYOUT, typename VecT>
+__device__ __noinline__ Contrib bilinear_direct(const KArgs& a, const SampleBlock* sb, const VecT* v) {
+  Contrib out{{0.0, 0.0, 0.0, 0.0}, 0};
+  double x, y, vz;
+  const VecT* const vec[3] = {v, v + a.vec_si, v + 2 * a.vec_si};
+  rotate_frame<1>(smem_u32(sb), vec, {0}, &x, &y, &vz);
+  if (!(isfinite(x) && isfinite(y) && isfinite(vz))) {
+    out.err = 1;
+    return out;
+  }
+  const Chan<LAYOUT> ch(a);
+  const Bore bo{sb->bz, sb->bsth};
+  const double z = clamp1(vz);
+  // a vector on the axis has longitude 0, as atan2(0, 0)
+  const double rel = x == 0.0 && y == 0.0 ? -sb->phi_u : frame_lon(x, y);
+  Mix<MapT, LAYOUT, HAS_QU> mix;
+  int k0;
+  double f0;
+  // ring pixel j relative to the frame's origin
+  auto visit = [&](bool start, const RingRec& r, int j, double wk) {
+    const int ip = (int)py_imod((long long)k0 + j, r.n);
+    mix.add(ch, start, wk,
+            pixel_vals<PM, HAS_QU, MapT, LAYOUT>(ch, MapRef{a.map, a.map_stride}, bo, r.z, r.sth,
+                                                 pixel_dphi(sb->bdl, f0, j, r.dphi), r.first + ip));
+  };
+  // the pixel left of the query and the fraction past it
+  auto locate = [&](const RingRec& r, double& frac) {
+    ring_origin(sb->phi_u, r.phi0, r.dphi, r.inv_dphi, k0, f0);
+    const double u = fma(rel, r.inv_dphi, f0);
+    const int j = __double2int_rd(u);
+    frac = u - (double)j;
+    return j;
+  };
+  const long long ir = ring_above(a.nside, z), last = 4 * a.nside - 1;
+  double frac, d = 0.0;
+  if (ir == 0 || ir == last) {
+    // beyond the first or last ring: its pair and the opposite pair
+    const RingRec r = ring_at(a, ir == 0 ? 1 : last);
+    const int j = locate(r, frac);
+    const double theta = acos(z);
+    if (ir == 0) {
+      const double wt = theta / r.ta;
+      const double nf = (1.0 - wt) * 0.25;
+      visit(true, r, j + 2, nf);
+      visit(false, r, j + 3, nf);
+      visit(false, r, j, (1.0 - frac) * wt + nf);
+      visit(false, r, j + 1, frac * wt + nf);
+    } else {
+      const double ws = (theta - r.ta) / (kPi - r.ta);
+      const double sf = ws * 0.25;
+      visit(true, r, j, (1.0 - frac) * (1.0 - ws) + sf);
+      visit(false, r, j + 1, frac * (1.0 - ws) + sf);
+      visit(false, r, j + 2, sf);
+      visit(false, r, j + 3, sf);
+    }
+  } else {
+    double wb;
+    {
+      const RingRec r = ring_at(a, ir);
+      double rel_th = colat_near(z, sb->cu, sb->su, d);
+      if (!sin_is_near(d)) rel_th = acos(z) - sb->theta_u;
+      wb = (rel_th - (r.ta - sb->theta_u)) * r.inv_dta;
+      const int j = locate(r, frac);
+      const double wa = 1.0 - wb;
+      visit(true, r, j, wa * (1.0 - frac));
+      visit(false, r, j + 1, wa * frac);
+    }
+    const RingRec r = ring_at(a, ir + 1);
+    const int j = locate(r, frac);
+    visit(false, r, j, wb * (1.0 - frac));
+    visit(false, r, j + 1, wb * frac);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c >= ch.C) break;
+    out.v[c] = (double)mix.t[c];
+  }
+  return out;
+}
+
+// Where a beam pixel falls in the sample's table: the slots left of it on the
+// ring above and the ring below, and the four weights.
+struct Place {
+  int ia, ib;
+  double w[4];
+};
+
+// Regions of the sky whose ring above a query is found by one formula.
+constexpr int kBelt = 0;     // all window rings within the belt |z| <= 2/3 (and of one length)
+constexpr int kAnywhere = 1;
+
+// Place of a beam pixel: false when the query is not near the frame's origin
+// in longitude, not between two rings of the window or not among their slots.
+// Straight-line code, so that two pixels' chains interleave.
+template <int REGION>
+__device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin, int nside, double cu, double su,
+                                            double belt_inv, double x, double y, double z, Place& o) {
+  const double t = div_near(y, x);
+  const double rel = atan_near(t);
+  double rc = (double)nside * fma(-1.5, z, 2.0);
+  int r;
+  if constexpr (REGION == kBelt) {
+    r = (int)rc;
+  } else {
+    const double az = fabs(z);
+    const bool cap = az > kTwoThirds;
+    const double rp = (double)nside * sqrt_near(3.0 * (1.0 - az));
+    r = (int)(cap ? rp : rc);
+    if (cap && z < 0.0) r = 4 * nside - r - 1;
+  }
+  r -= ir_lo;
+  // (|z| >= 1 or NaN gives a ring outside every window)
+  const bool in = lon_is_near(x, t) && (unsigned)r < (unsigned)nwin;
+  const unsigned ra = rings + 80u * (in ? (unsigned)r : 0u);
+  double2 f0, f1;
+  if constexpr (REGION == kBelt) {
+    f0 = make_double2(lds_d1(ra), belt_inv);
+    f1 = make_double2(lds_d1(ra + 80), belt_inv);
+  } else {
+    f0 = lds_d2(ra);
+    f1 = lds_d2(ra + 80);
+  }
+  const double ua = fma(rel, f0.y, f0.x), ub = fma(rel, f1.y, f1.x);
+  const int ja = __double2int_rd(ua), jb = __double2int_rd(ub);
+  int ia, ib;
+  const bool in_a = slot_of(lds_u1(ra + 64), ja, 2, ia), in_b = slot_of(lds_u1(ra + 144), jb, 2, ib);
+  const double xa = ua - (double)ja, xb = ub - (double)jb;
+  double d;
+  const double rel_th = colat_near(z, cu, su, d);
+  const double2 ti = lds_d2(ra + 16);
+  const double wb = (rel_th - ti.x) * ti.y;
+  const double wa = 1.0 - wb;
+  o.ia = ia;
+  o.ib = ib;
+  o.w[0] = wa * (1.0 - xa);
+  o.w[1] = wa * xa;
+  o.w[2] = wb * (1.0 - xb);
+  o.w[3] = wb * xb;
+  return in && in_a && in_b && sin_is_near(d);
+}
+
+// A placed pixel's contribution from the table.
+template <bool HAS_QU, typename MapT, int LAYOUT, class Acc>
+__device__ __forceinline__ void add_placed(const Chan<LAYOUT>& ch, const ValTable<MapT, LAYOUT>& tab, const Place& o,
+                                           float bvf, Acc& acc) {
+  Mix<MapT, LAYOUT, HAS_QU> mix;
+  mix.add(ch, true, o.w[0], tab.load(ch, o.ia));
+  mix.add(ch, false, o.w[1], tab.load(ch, o.ia + 1));
+  mix.add(ch, false, o.w[2], tab.load(ch, o.ib));
+  mix.add(ch, false, o.w[3], tab.load(ch, o.ib + 1));
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c >= ch.C) break;
+    accumulate<MapT>(acc, c, mix.t[c], bvf);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Nearest rule.
+// ---------------------------------------------------------------------------
 
 // cos(d) for |d| <= kCosSmallMax by its Taylor series through d^6 (the first
 // term left out, d^8 / 8!, is below 7e-19 there), in Horner form in d^2.
@@ -1055,879 +1330,572 @@ __device__ __forceinline__ double cos_small(double d) {
   return fma(u, fma(u, fma(u, -1.0 / 720.0, 1.0 / 24.0), -0.5), 1.0);
 }
 
-// x / d correctly rounded, from y = 1 / d correctly rounded: the quotient
-// x y and two residual corrections by Markstein's theorem (P. Markstein, IBM
-// J. Res. Dev. 34(1), 1990: with y within half an ulp of 1/d and q within
-// one ulp of x/d, the residual r = x - q d is exact under fma and
-// fma(r, y, q) is x/d rounded to nearest).  The first correction brings x y
-// (within two ulps) within one ulp, the second rounds correctly.  For finite
-// x and d whose quotient and residuals stay in the normal range -- the ring,
-// weight and longitude quotients here (|x| < 1e6, 1e-5 < |d| < 7).
-__device__ __forceinline__ double div_rn(double x, double d, double y) {
-  const double q0 = x * y;
-  const double q1 = fma(fma(-q0, d, x), y, q0);
-  return fma(fma(-q1, d, x), y, q1);
+// A component's term of the nearest mode: value x weight in float64, but a
+// float32 map's own components as a float32 product (tod_nearest.py:146, :158).
+template <bool HAS_QU, typename MapT, int LAYOUT>
+__device__ __forceinline__ double nearest_term(const Chan<LAYOUT>& ch, int c, ValT<MapT> v, float bvf) {
+  if constexpr (MapTraits<MapT>::packed) {
+    return (double)(v * bvf);
+  } else if constexpr (std::is_same<MapT, float>::value) {
+    return (HAS_QU && (c == ch.q || c == ch.u)) ? v * (double)bvf : (double)((float)v * bvf);
+  } else {
+    return v * (double)bvf;
+  }
 }
-constexpr double kInvTwoPi = 1.0 / kTwoPi;
 
-// Spin-2 window entry of one ring of the sample: {off, iplo, cap} and
-// whether the ring lies in the window.
-struct RingWin {
-  int off, iplo, cap;
-  bool in;
+// The nearest rule as the reference evaluates it: its own rotation, atan2,
+// four candidates ranked by cos().  Out of line.
+template <int PM, bool HAS_QU, typename MapT, int LAYOUT, typename VecT>
+__device__ __noinline__ Contrib nearest_exact(const KArgs& a, const SampleBlock* sb, const ExactBlock* eb, VecT v0,
+                                              VecT v1, VecT v2, float bvf) {
+  Contrib out{{0.0, 0.0, 0.0, 0.0}, 0};
+  const Chan<LAYOUT> ch(a);
+  double vx, vy, vz;
+  rotate_exact(sb, eb, v0, v1, v2, vx, vy, vz);
+  double phi_w = atan2(vy, vx);
+  if (phi_w < 0.0) phi_w += kTwoPi;
+  const double sin_th = sqrt(max0(vx * vx + vy * vy));
+  const Nearest nb =
+      a.ring_table != nullptr
+          ? hp_nearest(a.nside, vz, sin_th, phi_w, TableRings{static_cast<const RingRec*>(a.ring_table)})
+          : hp_nearest(a.nside, vz, sin_th, phi_w, DirectRingsNoAcos{a.nside, a.npix});
+  if ((unsigned long long)nb.pix >= (unsigned long long)a.npix) {
+    out.err = 1;
+    return out;
+  }
+  const Bore bo{sb->bz, sb->bsth};
+  // the boresight's longitude less the pixel's, as the window path forms it
+  double dphi = sb->phi_u + sb->bdl - nb.phic;  // (ring 0: no candidate, a non-finite query)
+  if (nb.ring > 0) {
+    const RingRec r = ring_at(a, nb.ring);
+    int k0;
+    double f0;
+    ring_origin(sb->phi_u, r.phi0, r.dphi, r.inv_dphi, k0, f0);
+    int j = (int)nb.ip - k0;
+    if (j > r.n / 2)
+      j -= r.n;
+    else if (j < -(r.n / 2))
+      j += r.n;
+    dphi = pixel_dphi(sb->bdl, f0, j, r.dphi);
+  }
+  const Vals<ValT<MapT>> o = pixel_vals<PM, HAS_QU, MapT, LAYOUT>(ch, MapRef{a.map, a.map_stride}, bo, nb.zc,
+                                                                  sqrt(max0(1.0 - nb.zc * nb.zc)), dphi, nb.pix);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c >= ch.C) break;
+    out.v[c] = nearest_term<HAS_QU, MapT, LAYOUT>(ch, c, o.v[c], bvf);
+  }
+  return out;
+}
+
+// Where a beam pixel of the nearest mode falls: window ring (its shared
+// address) and pixel relative to the ring's origin.
+//
+// On each of the two rings that bracket z, the reference's two candidates are
+// the pixels either side of the query, so the closer one is the rounded
+// position; the two rings' winners are ranked by the cosine of their angular
+// distance (cos_small).  The frame's positions differ from the reference's
+// own (rounded) ones by under 1e-14 rad and the cosines by under 1e-15, so
+// the reference picks the same pixel unless the query lies within 1e-9 of a
+// candidate boundary (of a ring's or a pixel's width) or the lead is under
+// 1e-13: then, and when anything is out of the window, false is returned and
+// the caller takes the reference's evaluation.  Straight-line code; a false
+// result still holds a valid ring.
+struct NearPlace {
+  unsigned ring;
+  int j;
 };
-
-__device__ __forceinline__ int2 lds_i2(const void* p) {
-  int2 v;
-  asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(smem_u32(p)));
-  return v;
+template <int REGION>
+__device__ __forceinline__ bool place_nearest(unsigned rings, int ir_lo, int nwin, int nside, double x, double y,
+                                              double z, NearPlace& o) {
+  constexpr double kEdge = 1e-9;
+  const double t = div_near(y, x);
+  const double rel = atan_near(t);
+  double rc = (double)nside * (2.0 - 1.5 * z);
+  bool south = false;
+  if constexpr (REGION != kBelt) {
+    const double az = fabs(z);
+    const double rp = (double)nside * sqrt_near(3.0 * (1.0 - az));
+    const bool cap = az > kTwoThirds;
+    rc = cap ? rp : rc;
+    south = cap && z < 0.0;
+  }
+  int r = (int)rc;
+  const double rf = rc - (double)r;
+  if (south) r = 4 * nside - r - 1;
+  r -= ir_lo;
+  // (|z| >= 1 or NaN gives a ring outside every window)
+  const bool in = lon_is_near(x, t) && (unsigned)r < (unsigned)nwin;
+  const unsigned ra = rings + 80u * (in ? (unsigned)r : 0u);
+  const double2 fa = lds_d2(ra), fb = lds_d2(ra + 80);
+  const double ua = fma(rel, fa.y, fa.x), ub = fma(rel, fb.y, fb.x);
+  const int ja = __double2int_rn(ua), jb = __double2int_rn(ub);
+  const double ea = ua - (double)ja, eb = ub - (double)jb;
+  const double la = ea * lds_d1(ra + 56), lb = eb * lds_d1(ra + 136);
+  const double2 za = lds_d2(ra + 32), zb = lds_d2(ra + 112);
+  const double sin_th = sqrt_near(fma(x, x, y * y));
+  const double ca = fma(sin_th * za.y, cos_small(la), z * za.x);
+  const double cb = fma(sin_th * zb.y, cos_small(lb), z * zb.x);
+  const bool b = cb > ca;
+  o.ring = ra + (b ? 80u : 0u);
+  o.j = b ? jb : ja;
+  return in && fabs(rf - 0.5) < 0.5 - kEdge && fmax(fabs(ea), fabs(eb)) < 0.5 - kEdge &&
+         fmax(fabs(la), fabs(lb)) <= kCosSmallMax && fabs(ca - cb) > 1e-13;
 }
 
-__device__ __forceinline__ RingWin ring_win(const Spin2Tab& w, const int2& hdr, int ring) {
-  const unsigned r = (unsigned)(ring - hdr.x);
-  RingWin rw;
-  rw.in = r < (unsigned)hdr.y;
-  const int4 v = lds_i4(&w.ring[rw.in ? r : 0u]);
-  rw.off = v.x;
-  rw.iplo = v.y;
-  rw.cap = v.z;
-  return rw;
+// A placed pixel's contribution: from the table, or from the map where the
+// launch has no table; false when the table does not hold the pixel.
+template <int PM, bool HAS_QU, typename MapT, int LAYOUT, class Acc>
+__device__ __forceinline__ bool add_nearest(const Chan<LAYOUT>& ch, const MapRef& map, const Bore& bo, double bdl,
+                                            const ValTable<MapT, LAYOUT>& tab, bool table, const NearPlace& o,
+                                            const float* bv, Acc& acc) {
+  Vals<ValT<MapT>> v;
+  if (HAS_QU && table) {
+    int slot;
+    if (!slot_of(lds_u1(o.ring + 64), o.j, 1, slot)) return false;
+    v = tab.load(ch, slot);
+  } else {
+    const int n = (int)lds_u1(o.ring + 72);
+    int ip = (int)lds_u1(o.ring + 68) + o.j;
+    ip += ip < 0 ? n : 0;
+    ip -= ip >= n ? n : 0;
+    const long long p = __double_as_longlong(lds_d1(o.ring + 48)) + ip;
+    if constexpr (HAS_QU) {
+      const double2 zs = lds_d2(o.ring + 32);
+      double c2, s2;
+      if (!spin2_small<PM>(zs.x, zs.y, pixel_dphi(bdl, lds_d1(o.ring), o.j, lds_d1(o.ring + 56)), bo, c2, s2))
+        return false;
+      v = turned_vals<MapT, LAYOUT>(ch, map, p, c2, s2);
+    } else {
+      v = raw_vals<MapT, LAYOUT>(ch, map, p);
+    }
+  }
+  const float bvf = __ldg(bv);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c >= ch.C) break;
+    acc.add(c, nearest_term<HAS_QU, MapT, LAYOUT>(ch, c, v.v[c], bvf));
+  }
+  return true;
 }
 
-// cos 2d / sin 2d of in-ring pixel ip (of n) from the table, or directly
-// (pixel outside the window, spill case ip == n).
-template <typename TabT>
-__device__ __forceinline__ void spin2_win(const RingWin& rw, const TabT* tab, const SampleBlock* sb, int ip, int n,
-                                          double zn, double phin, double& c2d, double& s2d) {
-  int j = ip - rw.iplo;
-  j += (j >> 31) & n;
-  if (rw.in && (unsigned)ip < (unsigned)n && (unsigned)j < (unsigned)rw.cap) {
-    const TabT v = tab[rw.off + j];
-    c2d = (double)v.x;
-    s2d = (double)v.y;
+// ---------------------------------------------------------------------------
+// One sample's window and table.
+// ---------------------------------------------------------------------------
+
+// Window of one sample, by the whole CTA: warp 0 places each ring in the
+// sample's frame, counts its slots and lays them out, the other warps copy the
+// rings' geometry.  ring_end[t] is the first slot past ring t, ring_of[i] the
+// ring that holds slot 32 i (where the fill starts its search).
+//
+// Slots per ring: pixel j of ring r is a neighbour of queries between rings r
+// - 1 and r + 1, so within d = max(0, |theta_r - theta_u| - spacing) of the
+// disc's centre at the nearest; at that colatitude theta_q the beam disc
+// (radius rbeam) reaches 2 asin(sqrt((sin^2(rbeam / 2) - sin^2(d / 2)) /
+// (sin theta_u sin theta_q))) in longitude (2% margin), H pixels, and the
+// query's two neighbours lie between -floor(f0 + H) - 1 and floor(f0 + H) + 1.
+// Near the poles the
+// ring table's reservation for any footprint of its reach is taken.  (A
+// pixel outside its ring's slots is still evaluated, directly; only the cost
+// changes.)
+template <int MODE>
+__device__ __noinline__ void footprint_window(const RingRec* rt0, const SampleBlock* sb, int nside, int tab_cap,
+                                              float rbeam, RingWin* rings, int* ring_end, unsigned short* ring_of,
+                                              int4* s_hdr) {
+  const int nr = sb->nr, ir_lo = sb->ir_lo;
+  const RingRec* rt = rt0 + ir_lo;
+  const double theta_u = sb->theta_u, phi_u = sb->phi_u;
+  if (threadIdx.x >= 32) {
+    for (int t = threadIdx.x - 32; t < nr; t += blockDim.x - 32) {
+      const RingRec* r = rt + t;
+      RingWin& w = rings[t];
+      w.inv_dphi = __ldg(&r->inv_dphi);
+      w.rta = __ldg(&r->ta) - theta_u;
+      w.z = __ldg(&r->z);
+      w.sth = __ldg(&r->sth);
+      w.inv_dta = __ldg(&r->inv_dta);
+      w.first = __ldg(&r->first);
+      w.dphi = __ldg(&r->dphi);
+      w.n = __ldg(&r->n);
+    }
     return;
   }
-  const Bore bo = block_bore(sb);
-  const double sth_n = sqrt(max0(1.0 - zn * zn));
-  spin2_c2s2(zn, sth_n, phin, bo.z, bo.sth, bo.phi, c2d, s2d);
-}
-
-// The bilinear stencil of hp_stencil with 32-bit indices; tw is in [0, n]
-// for finite phi in [0, 2 pi], so int(tw) is a plain truncation.  visit(k,
-// pixel, weight, in-ring index, ring length, ring z, pixel phi, ring window).
-template <bool HAS_QU, class Visit>
-__device__ __forceinline__ void stencil_fast(int nside, double z, double phi_w, const RingRec* rt, const Spin2Tab& w,
-                                             const int2& hdr, Visit&& visit) {
-  const int ir_above = ring_above_fast(nside, z);
-  RingWin ra_w{0, 0, 0, false};
-  if (ir_above == 0) {
-    const RingFast ra = ring_fast(rt, 1);
-    if constexpr (HAS_QU) ra_w = ring_win(w, hdr, 1);
-    const double tw = py_fmod_pos((phi_w - ra.phi0) / ra.dphi, (double)ra.n);
-    const int ip = (int)tw;
-    const double frac = tw - (double)ip;
-    const int ip2 = wrap_up(ip, 1, ra.n);
-    const int o1 = wrap_up(ip, 2, ra.n), o2 = wrap_up(ip2, 2, ra.n);
-    const double theta = acos(z);
-    const double wt = theta / ra.ta;
-    const double nf = (1.0 - wt) * 0.25;
-    visit(0, ra.first + o1, nf, o1, ra.n, ra.z, ra.phi0 + (double)o1 * ra.dphi, ra_w);
-    visit(1, ra.first + o2, nf, o2, ra.n, ra.z, ra.phi0 + (double)o2 * ra.dphi, ra_w);
-    visit(2, ra.first + ip, (1.0 - frac) * wt + nf, ip, ra.n, ra.z, ra.phi0 + (double)ip * ra.dphi, ra_w);
-    visit(3, ra.first + ip2, frac * wt + nf, ip2, ra.n, ra.z, ra.phi0 + (double)ip2 * ra.dphi, ra_w);
-  } else if (ir_above == 4 * nside - 1) {
-    const int ir_last = 4 * nside - 1;
-    const RingFast ra = ring_fast(rt, ir_last);
-    if constexpr (HAS_QU) ra_w = ring_win(w, hdr, ir_last);
-    const double tw = py_fmod_pos((phi_w - ra.phi0) / ra.dphi, (double)ra.n);
-    const int ip = (int)tw;
-    const double frac = tw - (double)ip;
-    const int ip2 = wrap_up(ip, 1, ra.n);
-    const int o1 = wrap_up(ip, 2, ra.n), o2 = wrap_up(ip2, 2, ra.n);
-    const double theta = acos(z);
-    const double ws = (theta - ra.ta) / (kPi - ra.ta);
-    const double sf = ws * 0.25;
-    visit(0, ra.first + ip, (1.0 - frac) * (1.0 - ws) + sf, ip, ra.n, ra.z, ra.phi0 + (double)ip * ra.dphi, ra_w);
-    visit(1, ra.first + ip2, frac * (1.0 - ws) + sf, ip2, ra.n, ra.z, ra.phi0 + (double)ip2 * ra.dphi, ra_w);
-    visit(2, ra.first + o1, sf, o1, ra.n, ra.z, ra.phi0 + (double)o1 * ra.dphi, ra_w);
-    visit(3, ra.first + o2, sf, o2, ra.n, ra.z, ra.phi0 + (double)o2 * ra.dphi, ra_w);
-  } else {
-    const int ir_below = ir_above + 1;
-    double sth_a;
-    const RingFast ra = ring_fast_sth(rt, ir_above, sth_a);
-    // of the ring below only its colatitude is needed before the ring above's
-    // neighbours; the rest is loaded after them
-    const double ta_b = __ldg(&rt[ir_below].ta);
-    double dta;
-    if (!dtheta_small(z, ra.z, sth_a, dta)) dta = acos(z) - ra.ta;
-    const double wb = div_rn(dta, ta_b - ra.ta, ra.inv_dta);
-    const double wa = 1.0 - wb;
-    double tw = py_fmod_pos(div_rn(phi_w - ra.phi0, ra.dphi, ra.inv_dphi), (double)ra.n);
-    const int ia = (int)tw;
-    const double fa = tw - (double)ia;
-    const int ia1 = wrap_up(ia, 1, ra.n);
-    if constexpr (HAS_QU) ra_w = ring_win(w, hdr, ir_above);
-    visit(0, ra.first + ia, wa * (1.0 - fa), ia, ra.n, ra.z, ra.phi0 + (double)ia * ra.dphi, ra_w);
-    visit(1, ra.first + ia1, wa * fa, ia1, ra.n, ra.z, ra.phi0 + (double)ia1 * ra.dphi, ra_w);
-    const RingFast rb = ring_fast(rt, ir_below);
-    tw = py_fmod_pos(div_rn(phi_w - rb.phi0, rb.dphi, rb.inv_dphi), (double)rb.n);
-    const int ib = (int)tw;
-    const double fb = tw - (double)ib;
-    const int ib1 = wrap_up(ib, 1, rb.n);
-    RingWin rb_w{0, 0, 0, false};
-    if constexpr (HAS_QU) rb_w = ring_win(w, hdr, ir_below);
-    visit(2, rb.first + ib, wb * (1.0 - fb), ib, rb.n, rb.z, rb.phi0 + (double)ib * rb.dphi, rb_w);
-    visit(3, rb.first + ib1, wb * fb, ib1, rb.n, rb.z, rb.phi0 + (double)ib1 * rb.dphi, rb_w);
-  }
-}
-
-template <int LAYOUT>
-struct Chan {
-  int C, q, u;
-  __device__ __forceinline__ explicit Chan(const KArgs& a) : C(a.C), q(a.c_q), u(a.c_u) {}
-};
-template <>
-struct Chan<kLayoutIQU> {
-  static constexpr int C = 3, q = 1, u = 2;
-  __device__ __forceinline__ explicit Chan(const KArgs&) {}
-};
-
-template <typename MapT>
-__device__ __forceinline__ double map_i(const KArgs& a, int c, int p) {
-  if constexpr (std::is_same<MapT, PackF64>::value)
-    return __ldg(static_cast<const double*>(a.map) + 4LL * p + c);
-  else
-    return (double)__ldg(static_cast<const MapT*>(a.map) + (long long)c * a.map_stride + p);
-}
-
-template <typename MapT>
-__device__ __forceinline__ double map_x_beam_i(const KArgs& a, int c, int p, float bv) {
-  if constexpr (std::is_same<MapT, PackF64>::value) {
-    return __ldg(static_cast<const double*>(a.map) + 4LL * p + c) * (double)bv;
-  } else {
-    const MapT m = __ldg(static_cast<const MapT*>(a.map) + (long long)c * a.map_stride + p);
-    if constexpr (sizeof(MapT) == 4)
-      return (double)(m * bv);
-    else
-      return m * (double)bv;
-  }
-}
-
-// A pixel's map values for the float64 bilinear path: planar maps read each
-// component where it is used; PackF64 records are read as two 16-byte loads.
-template <typename MapT>
-struct PixelVals {
-  const KArgs& a;
-  int p;
-  __device__ __forceinline__ PixelVals(const KArgs& a_, int p_) : a(a_), p(p_) {}
-  __device__ __forceinline__ double operator()(int c) const { return map_i<MapT>(a, c, p); }
-};
-template <>
-struct PixelVals<PackF64> {
-  double2 lo, hi;
-  __device__ __forceinline__ PixelVals(const KArgs& a, int p)
-      : lo(__ldg(static_cast<const double2*>(a.map) + 2LL * p)),
-        hi(__ldg(static_cast<const double2*>(a.map) + 2LL * p + 1)) {}
-  __device__ __forceinline__ double operator()(int c) const {
-    return c == 0 ? lo.x : (c == 1 ? lo.y : (c == 2 ? hi.x : hi.y));
-  }
-};
-
-// The nearest rule's ring data: n, phi0, dphi, z and sin theta of ring ir.
-struct RingNear {
-  int n, first;
-  double phi0, dphi, z, sth;
-};
-__device__ __forceinline__ RingNear ring_near(const RingRec* rt, int ir) {
-  const RingRec* r = rt + ir;
-  const double2 zs = __ldg(reinterpret_cast<const double2*>(&r->z));
-  const double2 pd = __ldg(reinterpret_cast<const double2*>(&r->phi0));
-  const int2 fn = __ldg(reinterpret_cast<const int2*>(&r->first32));
-  return RingNear{fn.y, fn.x, pd.x, pd.y, zs.x, zs.y};
-}
-
-// Per-neighbour mixing of the bilinear path, in the reference's k = 0..3 order:
-// float64 for planar maps and float64 records, float32 for packed records
-// (precision form); term(c) is what the pixel adds to component c.
-template <typename MapT, int LAYOUT, bool HAS_QU>
-struct BilinearMix {
-  static constexpr bool kPacked = MapTraits<MapT>::packed;
-  using R = typename std::conditional<kPacked, float, double>::type;
-  R tq = 0, tu = 0, to[4] = {0, 0, 0, 0};
-  __device__ __forceinline__ void visit(const KArgs& a, const Chan<LAYOUT>& ch, int k, int p, double wk, double c2,
-                                        double s2) {
-    if constexpr (kPacked) {
-      const float4 rec = load_rec<MapT>(a, p);
-      const float wf = (float)wk;
-      if constexpr (HAS_QU) {
-        const float c2f = (float)c2, s2f = (float)s2;
-        const float q = rec_at(rec, ch.q), u = rec_at(rec, ch.u);
-        const float vq = wf * fmaf(q, c2f, u * s2f);
-        const float vu = wf * fmaf(u, c2f, -q * s2f);
-        tq = (k == 0) ? vq : tq + vq;
-        tu = (k == 0) ? vu : tu + vu;
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c >= ch.C) break;
-        if (HAS_QU && (c == ch.q || c == ch.u)) continue;
-        to[c] = (k == 0) ? wf * rec_at(rec, c) : fmaf(wf, rec_at(rec, c), to[c]);
-      }
-    } else {
-      const PixelVals<MapT> pv(a, p);
-      if constexpr (HAS_QU) {
-        const double q = pv(ch.q);
-        const double u = pv(ch.u);
-        const double vq = wk * fma(q, c2, u * s2);
-        const double vu = wk * fma(u, c2, -q * s2);
-        tq = (k == 0) ? vq : tq + vq;
-        tu = (k == 0) ? vu : tu + vu;
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c >= ch.C) break;
-        if (HAS_QU && (c == ch.q || c == ch.u)) continue;
-        const double m = pv(c);
-        to[c] = (k == 0) ? wk * m : fma(wk, m, to[c]);
-      }
-    }
-  }
-  __device__ __forceinline__ double term(const Chan<LAYOUT>& ch, int c, float bvf) const {
-    if constexpr (kPacked) {
-      return (double)((HAS_QU && c == ch.q) ? tq * bvf : ((HAS_QU && c == ch.u) ? tu * bvf : to[c] * bvf));
-    } else {
-      const double bv = (double)bvf;
-      return (HAS_QU && c == ch.q) ? tq * bv : ((HAS_QU && c == ch.u) ? tu * bv : to[c] * bv);
-    }
-  }
-};
-
-// The bilinear stencil in the common case, without branches per neighbour:
-// a query between two rings away from the poles, both longitude quotients
-// inside their rings (no modulo, no spill into the next ring) and, with Q and
-// U, all four neighbours in the sample's spin-2 table.  The same operations
-// on the same values as stencil_fast + spin2_win; returns false (having added
-// nothing) when any of these does not hold, for the caller to take the full
-// path.
-template <bool HAS_QU, typename MapT, int LAYOUT, typename TabT, class Acc>
-__device__ __forceinline__ bool bilinear_lean(const KArgs& a, const RingRec* rt, const Spin2Tab& w,
-                                              const TabT* tab, const int2& hdr, double z, double phi_w, float bvf,
-                                              Acc& acc) {
-  const int nside = (int)a.nside;
-  const int ir_above = ring_above_fast(nside, z);
-  if (ir_above == 0 || ir_above == 4 * nside - 1) return false;
-  const int ir_below = ir_above + 1;
-  double sth_a;
-  const RingFast ra = ring_fast_sth(rt, ir_above, sth_a);
-  const RingFast rb = ring_fast(rt, ir_below);
-  // longitude quotients: py_fmod_pos without its fmod branch
-  const double xa = div_rn(phi_w - ra.phi0, ra.dphi, ra.inv_dphi);
-  const double xb = div_rn(phi_w - rb.phi0, rb.dphi, rb.inv_dphi);
-  const double na = (double)ra.n, nb = (double)rb.n;
-  if (!(fabs(xa) < na && fabs(xb) < nb)) return false;
-  const double twa = xa < 0.0 ? xa + na : (xa == 0.0 ? 0.0 : xa);
-  const double twb = xb < 0.0 ? xb + nb : (xb == 0.0 ? 0.0 : xb);
-  const int ia = (int)twa, ib = (int)twb;
-  if (ia >= ra.n || ib >= rb.n) return false;  // the spill into the next ring
-  const int ia1 = ia + 1 == ra.n ? 0 : ia + 1, ib1 = ib + 1 == rb.n ? 0 : ib + 1;
-  double c2[4] = {1.0, 1.0, 1.0, 1.0}, s2[4] = {0.0, 0.0, 0.0, 0.0};
-  if constexpr (HAS_QU) {
-    const RingWin wa = ring_win(w, hdr, ir_above), wb = ring_win(w, hdr, ir_below);
-    int j0 = ia - wa.iplo, j1 = ia1 - wa.iplo, j2 = ib - wb.iplo, j3 = ib1 - wb.iplo;
-    j0 += (j0 >> 31) & ra.n;
-    j1 += (j1 >> 31) & ra.n;
-    j2 += (j2 >> 31) & rb.n;
-    j3 += (j3 >> 31) & rb.n;
-    if (!(wa.in && wb.in && (unsigned)j0 < (unsigned)wa.cap && (unsigned)j1 < (unsigned)wa.cap &&
-          (unsigned)j2 < (unsigned)wb.cap && (unsigned)j3 < (unsigned)wb.cap))
-      return false;
-    const TabT t0 = tab[wa.off + j0], t1 = tab[wa.off + j1], t2 = tab[wb.off + j2], t3 = tab[wb.off + j3];
-    c2[0] = (double)t0.x;
-    s2[0] = (double)t0.y;
-    c2[1] = (double)t1.x;
-    s2[1] = (double)t1.y;
-    c2[2] = (double)t2.x;
-    s2[2] = (double)t2.y;
-    c2[3] = (double)t3.x;
-    s2[3] = (double)t3.y;
-  }
-  double dta;
-  if (!dtheta_small(z, ra.z, sth_a, dta)) dta = acos(z) - ra.ta;
-  const double wgt_b = div_rn(dta, rb.ta - ra.ta, ra.inv_dta);
-  const double wgt_a = 1.0 - wgt_b;
-  const double fa = twa - (double)ia, fb = twb - (double)ib;
-  const Chan<LAYOUT> ch(a);
-  BilinearMix<MapT, LAYOUT, HAS_QU> mix;
-  mix.visit(a, ch, 0, ra.first + ia, wgt_a * (1.0 - fa), c2[0], s2[0]);
-  mix.visit(a, ch, 1, ra.first + ia1, wgt_a * fa, c2[1], s2[1]);
-  mix.visit(a, ch, 2, rb.first + ib, wgt_b * (1.0 - fb), c2[2], s2[2]);
-  mix.visit(a, ch, 3, rb.first + ib1, wgt_b * fb, c2[3], s2[3]);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    if (c >= ch.C) break;
-    acc.add(c, mix.term(ch, c, bvf));
-  }
-  return true;
-}
-
-// The full bilinear fast path (poles, ring ends, spills, neighbours outside
-// the table), out of line, returning its terms by value.
-template <bool HAS_QU, typename MapT, int LAYOUT, typename TabT>
-__device__ __noinline__ Contrib bilinear_full(const KArgs& a, const SampleBlock* sb, const RingRec* rt,
-                                              const Spin2Tab& w, const TabT* tab, int2 hdr, double z, double phi_w,
-                                              float bvf) {
-  const Chan<LAYOUT> ch(a);
-  BilinearMix<MapT, LAYOUT, HAS_QU> mix;
-  stencil_fast<HAS_QU>((int)a.nside, z, phi_w, rt, w, hdr,
-                       [&](int k, int p, double wk, int ip, int n, double zn, double phin, const RingWin& rw) {
-                         double c2 = 1.0, s2 = 0.0;
-                         if constexpr (HAS_QU) spin2_win(rw, tab, sb, ip, n, zn, phin, c2, s2);
-                         mix.visit(a, ch, k, p, wk, c2, s2);
-                       });
-  Contrib out{{0.0, 0.0, 0.0, 0.0}, 0};
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    if (c >= ch.C) break;
-    out.v[c] = mix.term(ch, c, bvf);
-  }
-  return out;
-}
-
-// The nearest rule's full path (poles and their neighbourhood, candidates
-// more than 0.02 rad apart in longitude, near-ties, neighbours outside the
-// spin-2 table), out of line, returning its terms by value.
-template <bool HAS_QU, typename MapT, int LAYOUT, typename TabT>
-__device__ __noinline__ Contrib nearest_full(const KArgs& a, const SampleBlock* sb, const RingRec* rt,
-                                             const Spin2Tab& w, const TabT* tab, int2 hdr, double vx, double vy,
-                                             double vz, double phi_w, float bvf) {
-  constexpr bool kPacked = MapTraits<MapT>::packed;
-  const Chan<LAYOUT> ch(a);
-  const int nside = (int)a.nside;
-  const double bv = (double)bvf;
-  Contrib out{{0.0, 0.0, 0.0, 0.0}, 0};
-  // nearest: unclamped z; |z| > 1 makes the reference's ring_above NaN-based
-  // and the clamp then picks ring 1 (numba_healpy.py:62-70, tod_nearest.py:115-120)
-  const double sin_th = sqrt(max0(vx * vx + vy * vy));
-  int ir_above;
-  if (fabs(vz) <= 1.0) {
-    ir_above = ring_above_fast(nside, vz);
-    ir_above = ir_above < 1 ? 1 : (ir_above > 4 * nside - 2 ? 4 * nside - 2 : ir_above);
-  } else {
-    ir_above = 1;
-  }
-  // The four candidates: two pixels on each of rings ir_above and
-  // ir_above + 1, ranked by the cosine of their angular distance.  A first
-  // pass evaluates cos(phi_w - phic) by cos_small where the difference is at
-  // most kCosSmallMax (cos() beyond); the two differ by < 2e-15, so a lead of more
-  // than 1e-13 over the runner-up picks the pixel that ranking by cos()
-  // picks.  A closer call is ranked again by cos() itself -- the same
-  // expression, order and strict comparison -- so the pixel is always the
-  // one of ranking by cos() throughout.
-  int best_g = -1, best_ip = 0;
-  const RingNear rg0 = ring_near(rt, ir_above), rg1 = ring_near(rt, ir_above + 1);
-  {
-    double lead = -3.0, runner = -3.0;
-#pragma unroll
-    for (int g = 0; g < 2; ++g) {
-      const RingNear& r = g == 0 ? rg0 : rg1;
-      int ipb = (int)div_rn(phi_w * (double)r.n, kTwoPi, kInvTwoPi);
-      if (ipb >= r.n) ipb -= r.n;
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int ip = (t == 0) ? ipb : wrap_up(ipb, 1, r.n);
-        const double dl = phi_w - (r.phi0 + (double)ip * r.dphi);
-        const double cosd = sin_th * r.sth * (fabs(dl) <= kCosSmallMax ? cos_small(dl) : cos(dl)) + vz * r.z;
-        if (cosd > lead) {
-          runner = lead;
-          lead = cosd;
-          best_g = g;
-          best_ip = ip;
-        } else if (cosd > runner) {
-          runner = cosd;
-        }
-      }
-    }
-    if (!(lead - runner > 1e-13)) {
-      double best_cos = -2.0;
-      best_g = -1;
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        const RingNear& r = g == 0 ? rg0 : rg1;
-        int ipb = (int)(phi_w * (double)r.n / kTwoPi);
-        if (ipb >= r.n) ipb -= r.n;
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          const int ip = (t == 0) ? ipb : wrap_up(ipb, 1, r.n);
-          const double phic = r.phi0 + (double)ip * r.dphi;
-          const double cosd = sin_th * r.sth * cos(phi_w - phic) + vz * r.z;
-          if (cosd > best_cos) {
-            best_cos = cosd;
-            best_g = g;
-            best_ip = ip;
-          }
-        }
-      }
-    }
-  }
-  int best_pix = 0, best_n = 1, best_ring = 0;
-  double best_zc = 0.0, best_phic = 0.0;
-  if (best_g >= 0) {
-    const RingNear& r = best_g == 0 ? rg0 : rg1;
-    best_ring = ir_above + best_g;
-    best_n = r.n;
-    best_pix = r.first + best_ip;
-    best_zc = r.z;
-    best_phic = r.phi0 + (double)best_ip * r.dphi;
-  } else {
-    best_ip = 0;
-  }
-  RingWin rw{0, 0, 0, false};
-  if constexpr (HAS_QU) rw = ring_win(w, hdr, best_ring);
-  if constexpr (kPacked) {
-    const float4 rec = load_rec<MapT>(a, best_pix);
-    float c2f = 1.f, s2f = 0.f;
-    if constexpr (HAS_QU) {
-      double c2d, s2d;
-      spin2_win(rw, tab, sb, best_ip, best_n, best_zc, best_phic, c2d, s2d);
-      c2f = (float)c2d;
-      s2f = (float)s2d;
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c >= ch.C) break;
-      if (HAS_QU && c == ch.q)
-        out.v[c] = (double)(fmaf(rec_at(rec, ch.q), c2f, rec_at(rec, ch.u) * s2f) * bvf);
-      else if (HAS_QU && c == ch.u)
-        out.v[c] = (double)(fmaf(rec_at(rec, ch.u), c2f, -rec_at(rec, ch.q) * s2f) * bvf);
-      else
-        out.v[c] = (double)(rec_at(rec, c) * bvf);
-    }
-  } else if constexpr (HAS_QU) {
-    double c2d, s2d;
-    spin2_win(rw, tab, sb, best_ip, best_n, best_zc, best_phic, c2d, s2d);
-    const double qv = map_i<MapT>(a, ch.q, best_pix);
-    const double uv = map_i<MapT>(a, ch.u, best_pix);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c >= ch.C) break;
-      if (c == ch.q)
-        out.v[c] = (double)(fma(qv, c2d, uv * s2d) * bv);
-      else if (c == ch.u)
-        out.v[c] = (double)(fma(uv, c2d, -qv * s2d) * bv);
-      else
-        out.v[c] = (double)(map_x_beam_i<MapT>(a, c, best_pix, bvf));
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c >= ch.C) break;
-      out.v[c] = (double)(map_x_beam_i<MapT>(a, c, best_pix, bvf));
-    }
-  }
-  return out;
-}
-
-// The nearest rule in the common case, without branches: a query within the
-// rings of the map (|z| <= 1), all four candidates within kCosSmallMax of it in
-// longitude (so ranked by cos_small), a lead over the runner-up above 1e-13
-// (so no re-ranking by cos()), and with Q and U the chosen pixel in the
-// sample's spin-2 table.  The same operations on the same values as the full
-// path; returns false (having added nothing) when any of these does not hold.
-template <bool HAS_QU, typename MapT, int LAYOUT, typename TabT, class Acc>
-__device__ __forceinline__ bool nearest_lean(const KArgs& a, const RingRec* rt, const Spin2Tab& w, const TabT* tab,
-                                             const int2& hdr, double vx, double vy, double vz, double phi_w,
-                                             float bvf, Acc& acc) {
-  constexpr bool kPacked = MapTraits<MapT>::packed;
-  const int nside = (int)a.nside;
-  if (!(fabs(vz) <= 1.0)) return false;
-  const double sin_th = sqrt(max0(vx * vx + vy * vy));
-  int ir_above = ring_above_fast(nside, vz);
-  ir_above = ir_above < 1 ? 1 : (ir_above > 4 * nside - 2 ? 4 * nside - 2 : ir_above);
-  const RingNear rg0 = ring_near(rt, ir_above), rg1 = ring_near(rt, ir_above + 1);
-  int best_g = -1, best_ip = 0;
-  double lead = -3.0, runner = -3.0;
-  bool small = true;
-#pragma unroll
-  for (int g = 0; g < 2; ++g) {
-    const RingNear& r = g == 0 ? rg0 : rg1;
-    int ipb = (int)div_rn(phi_w * (double)r.n, kTwoPi, kInvTwoPi);
-    if (ipb >= r.n) ipb -= r.n;
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int ip = (t == 0) ? ipb : wrap_up(ipb, 1, r.n);
-      const double dl = phi_w - (r.phi0 + (double)ip * r.dphi);
-      small = small && fabs(dl) <= kCosSmallMax;
-      const double cosd = sin_th * r.sth * cos_small(dl) + vz * r.z;
-      if (cosd > lead) {
-        runner = lead;
-        lead = cosd;
-        best_g = g;
-        best_ip = ip;
-      } else if (cosd > runner) {
-        runner = cosd;
-      }
-    }
-  }
-  if (!(small && lead - runner > 1e-13 && best_g >= 0)) return false;
-  const RingNear& r = best_g == 0 ? rg0 : rg1;
-  const int best_pix = r.first + best_ip;
-  double c2d = 1.0, s2d = 0.0;
-  if constexpr (HAS_QU) {
-    const RingWin rw = ring_win(w, hdr, ir_above + best_g);
-    int j = best_ip - rw.iplo;
-    j += (j >> 31) & r.n;
-    if (!(rw.in && (unsigned)j < (unsigned)rw.cap)) return false;
-    const TabT v = tab[rw.off + j];
-    c2d = (double)v.x;
-    s2d = (double)v.y;
-  }
-  const Chan<LAYOUT> ch(a);
-  if constexpr (kPacked) {
-    const float4 rec = load_rec<MapT>(a, best_pix);
-    const float c2f = (float)c2d, s2f = (float)s2d;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c >= ch.C) break;
-      if (HAS_QU && c == ch.q)
-        acc.add(c, fmaf(rec_at(rec, ch.q), c2f, rec_at(rec, ch.u) * s2f) * bvf);
-      else if (HAS_QU && c == ch.u)
-        acc.add(c, fmaf(rec_at(rec, ch.u), c2f, -rec_at(rec, ch.q) * s2f) * bvf);
-      else
-        acc.add(c, rec_at(rec, c) * bvf);
-    }
-  } else if constexpr (HAS_QU) {
-    const double bv = (double)bvf;
-    const double qv = map_i<MapT>(a, ch.q, best_pix);
-    const double uv = map_i<MapT>(a, ch.u, best_pix);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c >= ch.C) break;
-      if (c == ch.q)
-        acc.add(c, fma(qv, c2d, uv * s2d) * bv);
-      else if (c == ch.u)
-        acc.add(c, fma(uv, c2d, -qv * s2d) * bv);
-      else
-        acc.add(c, map_x_beam_i<MapT>(a, c, best_pix, bvf));
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (c >= ch.C) break;
-      acc.add(c, map_x_beam_i<MapT>(a, c, best_pix, bvf));
-    }
-  }
-  return true;
-}
-
-// One beam pixel on the fast path: the branch-free common case of its mode,
-// else that mode's full path out of line.
-template <int MODE, bool HAS_QU, typename MapT, int LAYOUT, typename TabT, class Acc>
-__device__ __forceinline__ void eval_fast(const KArgs& a, const SampleBlock* sb, const RingRec* rt,
-                                          const Spin2Tab& w, const TabT* tab, double vx, double vy, double vz,
-                                          double phi_w, float bvf, Acc& acc) {
-  const Chan<LAYOUT> ch(a);
-  int2 hdr = make_int2(0, 0);  // {first window ring, window rings}
-  if constexpr (HAS_QU) hdr = lds_i2(&w.hdr);
-  if constexpr (MODE == TODGPU_BILINEAR) {
-    const double z = clamp1(vz);
-    if (!bilinear_lean<HAS_QU, MapT, LAYOUT>(a, rt, w, tab, hdr, z, phi_w, bvf, acc)) {
-      const Contrib r = bilinear_full<HAS_QU, MapT, LAYOUT>(a, sb, rt, w, tab, hdr, z, phi_w, bvf);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c >= ch.C) break;
-        acc.add(c, r.v[c]);
-      }
-    }
-  } else {
-    if (!nearest_lean<HAS_QU, MapT, LAYOUT>(a, rt, w, tab, hdr, vx, vy, vz, phi_w, bvf, acc)) {
-      const Contrib r = nearest_full<HAS_QU, MapT, LAYOUT>(a, sb, rt, w, tab, hdr, vx, vy, vz, phi_w, bvf);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c >= ch.C) break;
-        acc.add(c, r.v[c]);
-      }
-    }
-  }
-}
-
-// Flush the per-warp partial sums of sample `b` into tod (fixed order).
-template <int NW>
-__device__ __forceinline__ void flush_sample(const KArgs& a, const double* s_red, long long b) {
-  for (int c = 0; c < a.C; ++c) {
-    double v = 0.0;
-    for (int i = 0; i < NW; ++i) v += s_red[i * 4 + c];
-    a.tod[(long long)c * a.tod_stride + b] += v;
-  }
-}
-
-// Footprint window of one sample, by the kSetupThreads setup threads (warps
-// 0 and 1) together: the window rings about the footprint centre u, each
-// ring's slots and their offsets in the spin-2 table, into w.  Out of line so
-// that its registers do not weigh on the evaluation loop around it.
-constexpr int kSetupThreads = 64;
-static __device__ __noinline__ void footprint_window(const KArgs& a, const RingRec* rt, Spin2Tab& w, double ux,
-                                                     double uy, double uz, double reach) {
-  const int lane = threadIdx.x & 31;
-  const double theta_u = acos(clamp1(uz));
-  double phi_u = atan2(uy, ux);
-  if (phi_u < 0.0) phi_u += kTwoPi;
-  const double th_lo = theta_u - reach, th_hi = theta_u + reach;
-  long long ir_lo = th_lo <= 0.0 ? 1 : hp_ring_above(a.nside, cos(th_lo));
-  long long ir_hi = th_hi >= kPi ? 4 * a.nside - 1 : hp_ring_above(a.nside, cos(th_hi)) + 1;
-  ir_lo = max(ir_lo, 1LL);
-  ir_hi = min(ir_hi, 4 * a.nside - 1);
-  // a non-finite footprint centre gives an empty or invalid window: no table
-  const long long nr = ir_hi - ir_lo + 1;
-  bool fits = nr > 0 && nr <= a.ring_cap && ir_lo >= 1 && ir_hi <= 4 * a.nside - 1;
-  // Slots per window ring: the ring's stretch of the footprint disc (radius
-  // reach about (theta_u, phi_u)), at most what the ring table reserves
-  // for any footprint of that reach.  Away from the poles the disc's
-  // half-width in longitude on a ring at colatitude theta_r is
-  // sqrt(reach^2 - (theta_r - theta_u)^2) / sin theta_r to within a
-  // percent for reach < 0.05; 2% margin and the rounding up of the
-  // half-width keep every stencil pixel in.  (A pixel outside its ring's
-  // slots is still evaluated, directly; only the cost changes.)
-  const bool disc = reach < 0.05 && theta_u - reach > 0.1 && theta_u + reach < kPi - 0.1;
-  if (fits) {
-    for (int t = threadIdx.x; t < nr; t += kSetupThreads) {
-      const RingRec* r = rt + ir_lo + t;
-      const int n = __ldg(&r->n);
-      int cnt = __ldg(&r->cap);
+  const int lane = threadIdx.x;
+  const float spacing = 0.9f / (float)nside;  // the widest step between rings
+  const bool disc = theta_u - rbeam > 0.1 && theta_u + rbeam < kPi - 0.1;
+  const float hr = __sinf(0.5f * rbeam), inv_su = 1.f / (float)sb->su;
+  int carry = 0;
+  for (int b0 = 0; b0 < nr; b0 += 32) {
+    const int t = b0 + lane;
+    int own = 0;
+    if (t < nr) {
+      const RingRec* r = rt + t;
+      const double inv = __ldg(&r->inv_dphi);
+      int k0;
+      double f0;
+      ring_origin(phi_u, __ldg(&r->phi0), __ldg(&r->dphi), inv, k0, f0);
+      rings[t].f0 = f0;
+      rings[t].k0 = k0;
+      own = __ldg(&r->cap);
       if (disc) {
-        const double dth = __ldg(&r->ta) - theta_u;
-        const double h2 = reach * reach - dth * dth;
-        const int k = h2 > 0.0 ? (int)ceil(1.02 * sqrt(h2) / __ldg(&r->sth) * __ldg(&r->inv_dphi)) : 0;
-        cnt = min(cnt, 2 * k + 1);
+        const float d = fmaxf(0.f, fabsf((float)(__ldg(&r->ta) - theta_u)) - spacing);
+        const float hd = __sinf(0.5f * d);
+        const float q = fmaxf(0.f, hr * hr - hd * hd) * inv_su / ((float)__ldg(&r->sth) - spacing);
+        const float H = 2.04f * asinf(fminf(1.f, sqrtf(q))) * (float)inv;
+        own = min(own, 2 * (int)((float)f0 + H) + 3);
       }
-      int iplo = 0;
-      if (cnt < n) {
-        const double c = floor((phi_u - __ldg(&r->phi0)) / __ldg(&r->dphi));
-        iplo = (int)py_imod((long long)c - (cnt - 1) / 2, n);
-      }
-      w.ring[t].y = iplo;
-      w.ring[t].z = cnt;
     }
-  }
-  // slot offsets: exclusive prefix sum of the counts, by warp 0 once both
-  // setup warps have written theirs
-  asm volatile("bar.sync 1, %0;" ::"n"(kSetupThreads) : "memory");
-  if (threadIdx.x < 32) {
-    int carry = 0;
-    if (fits) {
-      for (int b0 = 0; b0 < (int)nr; b0 += 32) {
-        const int t = b0 + lane;
-        const int own = t < nr ? w.ring[t].z : 0;
-        int v = own;
+    int v = own;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, v, o);
-          if (lane >= o) v += y;
-        }
-        if (t < nr) w.ring[t].x = carry + v - own;
-        carry += __shfl_sync(0xffffffffu, v, 31);
-      }
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += y;
     }
-    fits = fits && carry <= a.tab_cap;
-    if (threadIdx.x == 0) {
-      w.ir_lo = ir_lo;
-      w.hdr = make_int4((int)ir_lo, fits ? (int)nr : 0, fits ? carry : 0, 0);
+    v += carry;
+    if (t < nr) {
+      const int off = v - own;
+      rings[t].slots = (unsigned)(off + (own - 1) / 2) << 16 | (unsigned)((own - 1) & 0xffff);
+      ring_end[t] = v;
+      for (int i = (off + 31) >> 5; 32 * i < v && 32 * i < tab_cap; ++i) ring_of[i] = (unsigned short)t;
     }
+    carry = __shfl_sync(0xffffffffu, v, 31);
+  }
+  const bool fits = carry <= tab_cap;
+  if (lane == 0)
+    *s_hdr = make_int4(ir_lo, (fits || MODE == TODGPU_NEAREST) && nr > 0 ? nr - 1 : 0, fits ? carry : 0, 0);
+}
+
+// Fill of the sample's value table, by the whole CTA.
+template <int PM, bool HAS_QU, typename MapT, int LAYOUT>
+__device__ __noinline__ void fill_table(const Chan<LAYOUT> ch, const MapRef map, const SampleBlock* sb,
+                                        const RingWin* rings, const int* ring_end, const unsigned short* ring_of,
+                                        int slots, const ValTable<MapT, LAYOUT> tab) {
+  const Bore bo{sb->bz, sb->bsth};
+  const double bdl = sb->bdl;
+#pragma unroll 1
+  for (int e = threadIdx.x; e < slots; e += blockDim.x) {
+    int t = ring_of[e >> 5];
+    while (e >= ring_end[t]) ++t;
+    const RingWin& w = rings[t];
+    const int j = e - (int)(w.slots >> 16), n = w.n;
+    int ip = w.k0 + j;
+    ip += ip < 0 ? n : 0;
+    ip -= ip >= n ? n : 0;
+    tab.store(ch, e, pixel_vals<PM, HAS_QU, MapT, LAYOUT>(ch, map, bo, w.z, w.sth,
+                                                          HAS_QU ? pixel_dphi(bdl, w.f0, j, w.dphi) : 0.0,
+                                                          w.first + ip));
   }
 }
+
+// What the pixel loops of a pass over the beam read, in shared memory: as a
+// parameter it went through every thread's local memory once a sample.
+template <typename MapT, int LAYOUT, typename VecT>
+struct PixelLoop {
+  const VecT* vec[3];  // component i of beam pixel s at vec[i][s ss]
+  const float* vals;
+  MapRef map;          // nearest without a table
+  unsigned rings;      // shared addresses of the window's rings and the table
+  ValTable<MapT, LAYOUT> tab;
+  int ss, n, nside;
+  Chan<LAYOUT> ch;
+};
+
+template <class Acc>
+struct LoopState {
+  Acc acc;
+  int s;
+};
+
+// Beam pixels s, s + kSumLanes, ... < n of one summation lane, as long as the
+// window and table hold them: returns the sums and the first pixel that they
+// do not hold (or one past the last).  Without calls: a call inside would
+// spill the loop's registers.  Two pixels at a time: each is a chain of some 60
+// dependent float64 operations, and two side by side hide what the warps of an
+// SM alone do not.
+//
+// Bound (30' beam, S = 1512, nside 1024, 120k samples, float64 records): 5.30 ms
+// with the map gathered and the spin-2 angle looked up per neighbour (677
+// thread instructions an evaluation, L1 at 79%), 2.47 ms now, of which the
+// table fill is 0.4 and the window 0.1; ~210 instructions an evaluation, 66 of
+// them float64, issue slots 57% and the shared-memory data path 60-70% busy:
+// leaving out 12 of 16 shared loads saved 5%, 22 of 66 float64 operations 13%.
+template <int REGION, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+__device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LAYOUT, VecT>* sp, const SampleBlock* blk,
+                                                     int ir_lo, int nwin, LoopState<Acc> st) {
+  const PixelLoop<MapT, LAYOUT, VecT> p = *sp;
+  const unsigned sb = smem_u32(blk);
+  const double cu = blk->cu, su = blk->su, belt_inv = lds_d1(p.rings + 8);
+  int s = st.s;
+  Acc acc = st.acc;
+#pragma unroll 1
+  for (; s + kSumLanes < p.n; s += 2 * kSumLanes) {
+    double x[2], y[2], z[2];
+    rotate_frame<2>(sb, p.vec, {s * p.ss, (s + kSumLanes) * p.ss}, x, y, z);
+    Place o[2];
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      ok = place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, cu, su, belt_inv, x[k], y[k], z[k], o[k]) && ok;
+    if (!ok) break;
+    add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[0], __ldg(p.vals + s), acc);
+    add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[1], __ldg(p.vals + s + kSumLanes), acc);
+  }
+  if (s < p.n) {
+    double x, y, z;
+    rotate_frame<1>(sb, p.vec, {s * p.ss}, &x, &y, &z);
+    Place o;
+    if (place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, cu, su, belt_inv, x, y, z, o)) {
+      add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o, __ldg(p.vals + s), acc);
+      s += kSumLanes;
+    }
+  }
+  st.acc = acc;
+  st.s = s;
+  return st;
+}
+
+template <int REGION, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+__device__ __forceinline__ LoopState<Acc> nearest_loop(const PixelLoop<MapT, LAYOUT, VecT>* sp, const SampleBlock* blk,
+                                                    int ir_lo, int nwin, bool table, LoopState<Acc> st) {
+  const PixelLoop<MapT, LAYOUT, VecT> p = *sp;
+  const unsigned sb = smem_u32(blk);
+  const Bore bo{blk->bz, blk->bsth};
+  const double bdl = blk->bdl;
+  int s = st.s;
+  Acc acc = st.acc;
+#pragma unroll 1
+  for (; s + kSumLanes < p.n; s += 2 * kSumLanes) {
+    double x[2], y[2], z[2];
+    rotate_frame<2>(sb, p.vec, {s * p.ss, (s + kSumLanes) * p.ss}, x, y, z);
+    NearPlace o[2];
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      ok = place_nearest<REGION>(p.rings, ir_lo, nwin, p.nside, x[k], y[k], z[k], o[k]) && ok;
+    if (!ok) break;
+    if (!add_nearest<PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o[0], p.vals + s, acc)) break;
+    if (!add_nearest<PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o[1], p.vals + s + kSumLanes,
+                                               acc)) {
+      s += kSumLanes;
+      break;
+    }
+  }
+  if (s < p.n) {
+    double x, y, z;
+    rotate_frame<1>(sb, p.vec, {s * p.ss}, &x, &y, &z);
+    NearPlace o;
+    if (place_nearest<REGION>(p.rings, ir_lo, nwin, p.nside, x, y, z, o) &&
+        add_nearest<PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o, p.vals + s, acc))
+      s += kSumLanes;
+  }
+  st.acc = acc;
+  st.s = s;
+  return st;
+}
+
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+__device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
+                                                     const int4& hdr, int nside, const LoopState<Acc>& st) {
+  // the window's rings all in the belt (rings nside to 3 nside)?
+  const bool belt = hdr.x >= nside && hdr.x + hdr.y <= 3 * nside;
+  if constexpr (MODE == TODGPU_NEAREST) {
+    const bool table = hdr.z > 0;
+    if (belt) return nearest_loop<kBelt, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, table, st);
+    return nearest_loop<kAnywhere, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, table, st);
+  } else {
+    if (belt) return bilinear_loop<kBelt, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, st);
+    return bilinear_loop<kAnywhere, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, st);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The sample loop.
+// ---------------------------------------------------------------------------
+
+// Beams of more than kBeamChunkMin pixels run in chunks of kBeamChunk consecutive
+// pixels, each with its own centre, frame, window and table: a far-sidelobe
+// beam's whole footprint holds 1e5 to 1e6 map pixels, a chunk of a beam in
+// kernels.beam_order a patch that fits shared memory.
+constexpr int kBeamChunkMin = 16384;
+constexpr int kBeamChunk = 1024;
 
 // Samples of tiles t = t_begin, t_begin + t_step, ... < t_end of one job (one
 // beam entry over one batch of samples; tile t holds samples [t tile,
-// min(B, (t + 1) tile))), by the whole CTA.  With a ring table:
-// ring data come from it and, when the entry carries Q and U, each sample's
-// footprint gets a spin-2 table in shared memory.  Without one: everything is
-// evaluated directly.  Each sample's rotation and boresight are derived by one
-// thread, one sample ahead, into a double-buffered shared block that all
-// threads read.  The beam is read from shared memory when the launch staged
-// it there (a.beam_stage), else from global memory.  All threads of the CTA
-// must call it together.
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, int NT>
+// min(B, (t + 1) tile))), by the whole CTA.  All threads of the CTA must call
+// it together.
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
 __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, long long t_step, long long tile,
-                            unsigned char* smem_raw, double* s_red) {
-  constexpr int NW = NT / 32;
-  static_assert(NT >= 2 * kSetupThreads && kSumLanes % NT == 0, "CTA of 128 or 256 threads");
-  Spin2Tab& w = *reinterpret_cast<Spin2Tab*>(smem_raw);
-  using TabT = typename MapTraits<MapT>::Tab;
+                            unsigned char* smem_raw, double* s_red, SampleBlock* s_blk, ExactBlock* s_exact,
+                            int4* s_hdr) {
   using Acc = typename std::conditional<MapTraits<MapT>::packed, AccKahan, Acc64>::type;
   using VecT = typename std::conditional<PM == kParamsRef32, float, double>::type;
-  // window rings of the table header (a.ring_cap; a constant in the narrow shape)
-  const int hdr_rings = NT == kNTNarrow ? kRingCapNarrow : a.ring_cap;
-  TabT* tab = reinterpret_cast<TabT*>(smem_raw + spin2_header_bytes(hdr_rings));
-  __shared__ SampleBlock s_blk[2];
-  __shared__ __align__(8) unsigned long long s_bar;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const RingRec* rt = static_cast<const RingRec*>(a.ring_table);
-  const bool fast = rt != nullptr && a.nside <= 8192;
-  double cx = 0.0, cy = 0.0, cz = 1.0, reach = 0.0;
-  bool use_tab = false;
-  if (rt != nullptr && HAS_QU) {
-    double rbeam;
-    beam_extent<PM, NT>(a, s_red, cx, cy, cz, rbeam);
-    // every stencil neighbour centre lies within 1.7/nside rad of the query
-    // (one ring spacing plus one pixel width; the opposite pair around a pole
-    // within twice the colatitude of ring 1); 2/nside leaves margin, plus
-    // slack for the float32 parameter rounding.  A neighbour outside the
-    // window is still evaluated correctly (directly), only slower (measured:
-    // 3/nside and 5% more slots per ring made the tables ~25% larger and
-    // config 2 ~3% slower).
-    reach = rbeam + 2.0 / (double)a.nside + 1e-5;
-    // the ring table reserves per-ring slots for footprints up to its reach
-    use_tab = reach <= __ldg(&rt[0].ta);
-  }
-  if (threadIdx.x == 0) {
-    w.hdr = make_int4(0, 0, 0, 0);
-    w.ir_lo = 0;
-  }
-  const VecT* svec = nullptr;
-  const float* sbv = nullptr;
-  const bool staged = a.beam_stage != 0;
-  if (staged) {
-    const size_t off = spin2_header_bytes(hdr_rings) + (((size_t)a.tab_cap * sizeof(TabT) + 15) & ~size_t(15));
-    stage_beam<VecT, NT>(a, smem_raw + off, &s_bar, svec, sbv);
-  }
-  // one thread derives each sample's rotation and boresight, one sample ahead:
-  // the last thread, which has the fewest beam pixels when S is not a multiple
-  // of the CTA size
-  constexpr int kRotThread = NT - 1;
-  constexpr int kRotWarp = NW - 1;
-  __shared__ RawFields s_raw;
-  if (threadIdx.x == kRotThread && t_begin < t_end)
-    write_block<PM>(a, GlobalFields<PM>{a, t_begin * tile}, HAS_QU, s_blk[0]);
-  int slot = 0;
+  const Chan<LAYOUT> ch(a);
+  const int NT = blockDim.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  RingWin* rings = reinterpret_cast<RingWin*>(smem_raw);
+  int* ring_end = reinterpret_cast<int*>(smem_raw + sizeof(RingWin) * (size_t)a.ring_cap);
+  unsigned short* ring_of = reinterpret_cast<unsigned short*>(smem_raw + window_bytes(a.ring_cap));
+  unsigned char* tab_mem = smem_raw + window_bytes(a.ring_cap) + ring_of_bytes(a.tab_cap);
+  const ValTable<MapT, LAYOUT> tab{smem_u32(tab_mem), a.tab_cap};
+  double* xchg = reinterpret_cast<double*>(tab_mem);  // lane sums of 256-thread CTAs, after the table's last use
+  using Loop = PixelLoop<MapT, LAYOUT, VecT>;
+  __shared__ __align__(16) unsigned char loop_mem[sizeof(Loop)];
+  Loop* loop = reinterpret_cast<Loop*>(loop_mem);
+  const int nside = (int)a.nside;
+  // samples of this CTA: whole tiles, but the job's last tile may be short
+  if (t_begin >= t_end) return;
+  const long long ntile = (t_end - t_begin + t_step - 1) / t_step;
+  const long long t_last = t_begin + (ntile - 1) * t_step;
+  const long long total = (ntile - 1) * tile + min(tile, a.B - t_last * tile);
   unsigned long long nerr = 0;
-  long long prev = -1;
   const int S = (int)a.S;
-  for (long long t = t_begin; t < t_end; t += t_step)
-  for (long long b = t * tile, b_stop = min(a.B, (t + 1) * tile); b < b_stop; ++b) {
-    __syncthreads();  // previous sample is done with the table, its partial sums and its block
-    const SampleBlock* sb = &s_blk[slot];
-    // the next sample: its pointing fields start on their way to shared memory
-    // now, and the last thread turns them into its block after its pixels
-    long long bn = b + 1, tn = t;
-    if (bn >= b_stop) {
-      tn = t + t_step;
-      bn = tn * tile;
+  const int step = S > kBeamChunkMin ? kBeamChunk : S;
+  for (int s0 = 0; s0 < S; s0 += step) {
+    const int s1 = min(S, s0 + step);
+    double cx, cy, cz, rbeam;
+    beam_extent<PM>(a, s0, s1, s_red, cx, cy, cz, rbeam);
+    rbeam += 1e-5;  // slack for the float32 parameter rounding
+    // the ring table reserves per-ring slots for footprints up to its reach:
+    // a stencil neighbour's centre lies within 1.7/nside rad of its query (one
+    // ring spacing plus one pixel width; the opposite pair around a pole
+    // within twice the colatitude of ring 1)
+    const bool window = a.ring_table != nullptr && (MODE == TODGPU_NEAREST || a.tab_cap > 0) &&
+                        rbeam + 2.0 / (double)a.nside <= __ldg(&static_cast<const RingRec*>(a.ring_table)[0].ta);
+    const int n = s1 - s0;
+    const VecT* vec = static_cast<const VecT*>(a.vec) + (long long)s0 * a.vec_ss;
+    const float* vals = a.beam + s0;
+    if (tid == 0) {
+      for (int k = 0; k < 3; ++k) loop->vec[k] = vec + k * a.vec_si;
+      loop->vals = vals;
+      loop->map = MapRef{a.map, a.map_stride};
+      loop->rings = smem_u32(rings);
+      loop->tab = tab;
+      loop->ss = a.vec_ss;
+      loop->n = n;
+      loop->nside = nside;
+      loop->ch = ch;
     }
-    const bool has_next = tn < t_end && bn < a.B;
-    if (warp == kRotWarp && has_next) prefetch_fields<PM>(a, bn, s_raw, lane);
-    if (prev >= 0 && threadIdx.x == 0) flush_sample<kSumLanes / 32>(a, s_red, prev);
-    if (use_tab) {
-      if (threadIdx.x < kSetupThreads) {
-        // footprint window of this sample (same values in every setup thread)
-        double ux, uy, uz;
-        rotate_block_f64(*sb, cx, cy, cz, ux, uy, uz);
-        footprint_window(a, rt, w, ux, uy, uz, reach);
+    // the nearest rule's margin on ring boundaries (nearest_window) holds away
+    // from the poles, where a ring's width in z vanishes
+    const double polar = MODE == TODGPU_NEAREST ? 0.01 : -4.0;
+    for (long long q0 = 0; q0 < total; q0 += kPrep) {
+      const int nq = (int)min((long long)kPrep, total - q0);
+      __syncthreads();  // the previous samples' blocks are no longer read
+      if (tid < nq) {
+        const long long q = q0 + tid, ti = tile == 1 ? q : q / tile;
+        prepare_sample<PM>(a, (t_begin + ti * t_step) * tile + (q - ti * tile), HAS_QU, cx, cy, cz, rbeam, window,
+                           polar, s_blk[tid], s_exact != nullptr ? s_exact + tid : nullptr);
       }
       __syncthreads();
-      const int4 hdr = w.hdr;
-      const int ntab = hdr.z, nwin = hdr.y;
-      const Bore bo{sb->bz, sb->bsth, sb->bphi};
-      for (int e = threadIdx.x; e < ntab; e += NT) {
-        int lo = 0, hi = nwin - 1;  // last window ring with off <= e
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (w.ring[mid].x <= e)
-            lo = mid;
-          else
-            hi = mid - 1;
-        }
-        const int4 wr = w.ring[lo];
-        const RingRec* r = rt + w.ir_lo + lo;
-        const int n = __ldg(&r->n);
-        int ip = wr.y + (e - wr.x);
-        if (ip >= n) ip -= n;
-        const double phin = __ldg(&r->phi0) + (double)ip * __ldg(&r->dphi);
-        double c2, s2;
-        spin2_c2s2(__ldg(&r->z), __ldg(&r->sth), phin, bo.z, bo.sth, bo.phi, c2, s2);
-        tab[e] = make_tab<TabT>(c2, s2);
-      }
-    }
-    __syncthreads();
-
-    // summation lane l (of kSumLanes) takes the beam pixels l, l + kSumLanes,
-    // ...; thread t is lane t + i NT in pass i, so the TOD does not depend on
-    // the CTA's thread count
 #pragma unroll 1
-    for (int pass = 0; pass < kSumLanes / NT; ++pass) {
-      const int sl = threadIdx.x + pass * NT;
-      Acc acc;
-      for (int s = sl; s < S; s += kSumLanes) {
-        VecT v0, v1, v2;
-        float bvf;
-        if (staged) {
-          v0 = svec[3 * s];
-          v1 = svec[3 * s + 1];
-          v2 = svec[3 * s + 2];
-          bvf = sbv[s];
-        } else {
-          const VecT* v = static_cast<const VecT*>(a.vec) + 3 * s;
-          v0 = __ldg(v);
-          v1 = __ldg(v + 1);
-          v2 = __ldg(v + 2);
-          bvf = __ldg(a.beam + s);
+      for (int i = 0; i < nq; ++i) {
+        const SampleBlock* sb = s_blk + i;
+        // the warps' sums alternate between two sets: one sample's are read
+        // while the next sample's may already be written
+        double* red = s_red + 16 * (i & 1);
+        int4 hdr = make_int4(0, 0, 0, 0);
+        if (window) {
+          footprint_window<MODE>(static_cast<const RingRec*>(a.ring_table), sb, nside, a.tab_cap, (float)rbeam, rings,
+                                 ring_end, ring_of, s_hdr);
+          __syncthreads();
+          hdr = *s_hdr;
+          if (hdr.z > 0) {
+            fill_table<PM, HAS_QU, MapT, LAYOUT>(ch, MapRef{a.map, a.map_stride}, sb, rings, ring_end, ring_of,
+                                                 hdr.z, tab);
+            __syncthreads();
+          }
         }
-        double vx, vy, vz;
-        rotate_block(sb, v0, v1, v2, vx, vy, vz);
-        double phi_w = atan2(vy, vx);
-        if (phi_w < 0.0) phi_w += kTwoPi;
-        if (fast && isfinite(vx) && isfinite(vy) && isfinite(vz)) {
-          eval_fast<MODE, HAS_QU, MapT, LAYOUT>(a, sb, rt, w, tab, vx, vy, vz, phi_w, bvf, acc);
-        } else if constexpr (MODE == TODGPU_BILINEAR) {
-          const Contrib r =
-              rt != nullptr
-                  ? eval_generic<MODE, HAS_QU, MapT>(a, sb, TableRings{rt}, w, tab, vx, vy, vz, phi_w, bvf)
-                  : eval_generic<MODE, HAS_QU, MapT>(a, sb, DirectRings{a.nside, a.npix}, w, tab, vx, vy, vz, phi_w,
-                                                     bvf);
-          if (r.err) {
-            ++nerr;
-          } else {
+        // Summation lane l (of kSumLanes) takes the beam pixels l, l +
+        // kSumLanes, ... of the pass; thread t holds lanes t and (128-thread
+        // CTAs) t + 128.  Lane sums l and l + 128 are added, then the 128
+        // sums per warp, then the four warps': the TOD does not depend on
+        // the CTA's thread count.
+        double keep[4] = {0.0, 0.0, 0.0, 0.0};
+        Acc acc;
+#pragma unroll 1
+        for (int l = tid; l < kSumLanes; l += NT) {
+          LoopState<Acc> st{Acc(), l};
+          // pixels that the window and table do not hold are evaluated here,
+          // each in its place in the sum
+          while (st.s < n) {
+            if (hdr.y > 0) st = pixel_loop<MODE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(loop, sb, hdr, nside, st);
+            if (st.s < n) {
+              const VecT* v = vec + (long long)st.s * a.vec_ss;
+              const float bvf = vals[st.s];
+              Contrib r;
+              if constexpr (MODE == TODGPU_BILINEAR)
+                r = bilinear_direct<PM, HAS_QU, MapT, LAYOUT, VecT>(a, sb, v);
+              else
+                r = nearest_exact<PM, HAS_QU, MapT, LAYOUT, VecT>(a, sb, s_exact + i, v[0], v[a.vec_si], v[2 * a.vec_si], bvf);
+              nerr += r.err;
+              if (!r.err) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                  if (c >= ch.C) break;
+                  if constexpr (MODE == TODGPU_BILINEAR)
+                    accumulate<MapT>(st.acc, c, (ValT<MapT>)r.v[c], bvf);
+                  else
+                    st.acc.add(c, r.v[c]);
+                }
+              }
+              st.s += kSumLanes;
+            }
+          }
+          acc = st.acc;
+          if (NT < kSumLanes) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) keep[c] = l == tid ? acc.total(c) : keep[c] + acc.total(c);
+          }
+        }
+        if (NT == kSumLanes) {
+          __syncthreads();  // the table is no longer read
+          if (tid >= kMeanLanes) {
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-              if (c < a.C) acc.add(c, r.v[c]);
+              if (c < ch.C) xchg[c * kMeanLanes + tid - kMeanLanes] = acc.total(c);
           }
-        } else if (rt != nullptr) {
-          eval_generic_into<MODE, HAS_QU, MapT>(a, sb, TableRings{rt}, w, tab, vx, vy, vz, phi_w, bvf, acc, nerr);
-        } else {
-          eval_generic_into<MODE, HAS_QU, MapT>(a, sb, DirectRings{a.nside, a.npix}, w, tab, vx, vy, vz, phi_w, bvf,
-                                                acc, nerr);
+          __syncthreads();
+          if (tid < kMeanLanes) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (c < ch.C) keep[c] = acc.total(c) + xchg[c * kMeanLanes + tid];
+          }
+        }
+        if (tid < kMeanLanes) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (c >= ch.C) break;
+            const double v = warp_sum(keep[c]);
+            if (lane == 0) red[warp * 4 + c] = v;
+          }
+        }
+        __syncthreads();  // the sums are written and the table, window and header free
+        if (tid < a.C) {
+          const long long q = q0 + i, ti = tile == 1 ? q : q / tile;
+          const long long b = (t_begin + ti * t_step) * tile + (q - ti * tile);
+          double v = 0.0;
+          for (int k = 0; k < kMeanLanes / 32; ++k) v += red[k * 4 + tid];
+          a.tod[(long long)tid * a.tod_stride + b] += v;
         }
       }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c >= a.C) break;
-        const double v = warp_sum(acc.total(c));
-        if (lane == 0) s_red[(sl >> 5) * 4 + c] = v;
-      }
     }
-    // the next sample's rotation into the other block (read after the next barrier)
-    if (warp == kRotWarp && has_next) {
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncwarp();
-      if (lane == 31) write_block<PM>(a, SharedFields<PM>{a, s_raw}, HAS_QU, s_blk[slot ^ 1]);
-    }
-    slot ^= 1;
-    prev = b;
   }
-  __syncthreads();
-  if (prev >= 0 && threadIdx.x == 0) flush_sample<kSumLanes / 32>(a, s_red, prev);
   if (a.err != nullptr) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) nerr += __shfl_xor_sync(0xffffffffu, nerr, o);
     if (lane == 0 && nerr) atomicAdd(a.err, nerr);
   }
-  __syncthreads();  // the partial sums, tables and blocks may be reused by the next job
+  __syncthreads();  // shared memory may be reused by the next job
 }
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) gather_accum_kernel(const KArgs a) {
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+__global__ void __maxnreg__(kRegs) gather_accum_kernel(const __grid_constant__ KArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_red[(kSumLanes / 32) * 4];
-  run_samples<MODE, HAS_QU, MapT, PM, LAYOUT, NT>(a, blockIdx.x, a.B, gridDim.x, 1, smem_raw, s_red);
+  __shared__ SampleBlock s_blk[kPrep];
+  __shared__ ExactBlock s_exact[MODE == TODGPU_NEAREST ? kPrep : 1];
+  __shared__ int4 s_hdr;
+  run_samples<MODE, HAS_QU, MapT, PM, LAYOUT>(a, blockIdx.x, a.B, gridDim.x, 1, smem_raw, s_red, s_blk,
+                                              MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
 }
 
 // Many jobs (detectors: each its own beam, pointing, output and length) in
@@ -1951,10 +1919,13 @@ struct BatchParams {
   KArgs job[kMaxBatchJobs];
 };
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) gather_batched_kernel(const __grid_constant__ BatchParams p) {
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+__global__ void __maxnreg__(kRegs) gather_batched_kernel(const __grid_constant__ BatchParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_red[(kSumLanes / 32) * 4];
+  __shared__ SampleBlock s_blk[kPrep];
+  __shared__ ExactBlock s_exact[MODE == TODGPU_NEAREST ? kPrep : 1];
+  __shared__ int4 s_hdr;
   __shared__ __align__(16) KArgs s_job;
   const long long G = gridDim.x, k = blockIdx.x;
   for (int j = 0; j < p.njobs; ++j) {
@@ -1967,7 +1938,8 @@ __global__ void __launch_bounds__(NT, MINB) gather_batched_kernel(const __grid_c
         reinterpret_cast<unsigned long long*>(&s_job)[threadIdx.x] =
             reinterpret_cast<const unsigned long long*>(&p.job[j])[threadIdx.x];
       __syncthreads();
-      run_samples<MODE, HAS_QU, MapT, PM, LAYOUT, NT>(s_job, t0, ntiles, G, p.tile, smem_raw, s_red);
+      run_samples<MODE, HAS_QU, MapT, PM, LAYOUT>(s_job, t0, ntiles, G, p.tile, smem_raw, s_red, s_blk,
+                                              MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
     }
   }
 }
@@ -1987,231 +1959,173 @@ inline int sm_count() {
   return count;
 }
 
-struct LaunchInfo {
-  int blocks_per_sm = 0;
-  size_t smem = 0;  // dynamic shared memory blocks_per_sm was computed for
-  bool configured = false;
-};
-
-// Shared memory per SM on B200 and what the driver keeps per CTA; the
-// kernels' static shared memory (partial sums, rotation slots) stays well
-// under the 2 KiB margin below.
+// Shared memory per SM on B200, what the driver keeps per CTA, and a bound of
+// the kernels' static shared memory (sample blocks, partial sums, the batched
+// job descriptor).
 constexpr size_t kSmemPerSM = 228 * 1024;
+constexpr size_t kSmemPerCTAMax = 227 * 1024;
 constexpr size_t kSmemPerCTAReserved = 1024;
-constexpr size_t kStaticSmemMargin = 2048;
-
-#ifndef TODGPU_CTA_THREADS
-#define TODGPU_CTA_THREADS 256
-#endif
-constexpr int kNT = TODGPU_CTA_THREADS;  // threads per CTA
-
-// CTAs per SM the register budget is sized for: 4 (64 registers) for the
-// nearest mode and packed maps, where the fourth CTA measured 3-5% faster; 3
-// (80 registers) for bilinear on planar maps, where it gained nothing and the
-// extra spilling doubled the local-memory write-back to DRAM.
-template <int MODE, typename MapT>
-constexpr int min_blocks() {
-#ifdef TODGPU_CTA_MINB
-  return TODGPU_CTA_MINB;
-#else
-  return (MODE == TODGPU_NEAREST || MapTraits<MapT>::packed) ? 4 : 3;
-#endif
+template <int MODE>
+constexpr size_t static_smem() {
+  return kPrep * (sizeof(SampleBlock) + (MODE == TODGPU_NEAREST ? sizeof(ExactBlock) : 0)) + 1024;
 }
 
-// Dynamic shared memory a CTA may take while MINB CTAs still fit on an SM.
-template <int MINB>
-constexpr size_t cta_smem_budget() {
-  return kSmemPerSM / MINB - kSmemPerCTAReserved - kStaticSmemMargin;
-}
-
-// Window rings a launch's table header reserves.  A request of N slots is a
-// footprint disc of at most N / 3.2 pixels (the request of kernels.table_slots
-// is 1.05 x (1.02 x 3 (r nside)^2 + 3 per ring) + 32 for a disc of radius r),
-// so r nside <= sqrt(N / 3.2), and such a disc crosses at most 3 r nside + 4
-// rings of the RING scheme (ring spacing at least 2 / (3 nside) in colatitude,
-// plus the rings either side); the default table reserves kRingCap.  The
-// header then takes 32 + 16 x rings bytes instead of 3 KiB, and the shared
-// memory left goes to L1.
+// Window rings a launch reserves.  A request of N slots is a beam disc of
+// radius r with at least 3.15 (r nside)^2 slots (kernels.footprint_slots), so r
+// nside <= sqrt(N / 3.15), and such a disc crosses at most 3 r nside + 4 rings
+// of the RING scheme (ring spacing at least 2 / (3 nside) in colatitude, plus
+// the rings either side); the default table reserves kRingCap.
 inline int ring_cap_for(int requested) {
   if (requested <= 0) return kRingCap;
-  return std::min(kRingCap, (int)std::ceil(3.0 * std::sqrt(requested / 3.2)) + 6);
-}
-
-// Spin-2 table slots of a launch: the caller's request, else 32 KiB (2048
-// float64 or 4096 float32 pairs); never more than each of MINB CTAs can hold
-// in an SM's shared memory beside the table header.
-template <typename TabT, int MINB>
-int max_table_slots(int ring_cap) {
-  return (int)((cta_smem_budget<MINB>() - spin2_header_bytes(ring_cap)) / sizeof(TabT));
+  return std::min(kRingCap, (int)std::ceil(3.0 * std::sqrt(requested / 3.15)) + 6);
 }
 constexpr size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-// Modes whose launches stage the beam in shared memory when it fits: bilinear
-// (config 2 in 256-thread CTAs: +5%; its 128-thread CTAs have no room for
-// the beam beside the table); nearest reads one stencil pixel per beam pixel
-// and gains more from the shared memory left to L1 (1% faster without).
-template <int MODE>
-constexpr bool stage_beam_mode() {
-  return MODE == TODGPU_BILINEAR;
+// Shape of a launch: threads per CTA, window rings, table slots, dynamic
+// shared memory.
+struct Shape {
+  int nt = 128, ring_cap = 1, tab_cap = 0;
+  size_t smem = 0;
+};
+
+inline int ctas_per_sm(int nt, size_t smem) {  // smem: static and dynamic
+  const size_t per = smem + kSmemPerCTAReserved;
+  return (int)std::min<size_t>(kThreadsSM / nt, kSmemPerSM / per);
 }
 
-template <typename TabT, int MINB>
-int table_slots(int requested, int ring_cap) {
-  constexpr int kCap = (int)(kTabCapDefault * sizeof(double2) / sizeof(TabT));
-  return requested > 0 ? std::min(requested, max_table_slots<TabT, MINB>(ring_cap)) : kCap;
+// What a launch asks for: the ring window and table request, slot bytes,
+// components, samples, beam pixels per pass, the fewest threads per CTA.
+struct Wants {
+  bool window = false;
+  int requested = 0, slots = 0, slot = 0, C = 1;
+  long long samples = 0, pixels = 0;
+  int min_nt = 128;
+  size_t fixed = 0;  // static shared memory
+};
+
+inline Shape choose_shape(const Wants& w) {
+  Shape best;
+  int best_threads = 0;
+  for (int nt = w.min_nt; nt <= kSumLanes; nt *= 2) {
+    Shape s;
+    s.nt = nt;
+    s.ring_cap = w.window ? ring_cap_for(w.requested) : 1;
+    const size_t xchg = nt > kMeanLanes ? sizeof(double) * kMeanLanes * (size_t)w.C : 0;
+    const size_t head = window_bytes(s.ring_cap);
+    const size_t room = kSmemPerCTAMax - w.fixed - head - 1024;
+    // a table that no CTA can hold is not made (its samples would not fit it)
+    s.tab_cap = (size_t)w.slots <= room / (w.slot + 1) ? (w.slots + 1) & ~1 : 0;
+    s.smem = align16(head + ring_of_bytes(s.tab_cap) + std::max(xchg, (size_t)w.slot * s.tab_cap));
+    const int threads = nt * ctas_per_sm(nt, s.smem + w.fixed);
+    const bool idle = w.samples * nt <= (long long)kThreadsSM * sm_count() && w.pixels >= nt;
+    if (threads > best_threads || (threads == best_threads && idle)) {
+      best = s;
+      best_threads = threads;
+    }
+  }
+  return best;
 }
 
-// Window rings of a launch's table header: fixed in the narrow shape.
-template <int NT>
-int header_rings(bool table, int requested) {
-  if (NT == kNTNarrow) return kRingCapNarrow;
-  return table ? ring_cap_for(requested) : 1;  // ring[0] is read (not used) without a window
+// Table slots of a launch (0: no value table): the caller's request, else
+// 32 KiB of the float64 or float32 pairs earlier versions kept.
+template <int MODE, bool HAS_QU, typename MapT>
+int wanted_slots(const KArgs& k) {
+  if (k.ring_table == nullptr) return 0;
+  const int req = k.tab_req > 0 && k.S <= kBeamChunkMin
+                      ? k.tab_req
+                      : (MapTraits<MapT>::packed ? 2 * kTabCapDefault : kTabCapDefault);
+  if (MODE == TODGPU_BILINEAR) return req;
+  // nearest reads one value per beam pixel: a table pays when the footprint
+  // has fewer pixels than the beam (and only for turned Q/U values)
+  return HAS_QU && req <= std::min<long long>(k.S, k.S > kBeamChunkMin ? kBeamChunk : k.S) ? req : 0;
 }
 
-// Once per kernel: allow the largest table; per launch: CTAs per SM for the
-// launch's shared memory (recomputed when it changes).
-template <int NT, typename Kern>
-int configure_launch(Kern kern, LaunchInfo& info, std::mutex& mu, size_t smem, int& blocks_per_sm) {
-  std::lock_guard<std::mutex> lock(mu);
-  if (!info.configured) {
-    // the largest dynamic shared memory a CTA of this kernel can have
-    int dev = 0, optin = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+// One job's part in what its launch asks for (the most any job does).
+template <int MODE, bool HAS_QU, typename MapT, int PM>
+void add_wants(Wants& w, const KArgs& k) {
+  const long long pixels = k.S > kBeamChunkMin ? kBeamChunk : k.S;
+  w.window = w.window || k.ring_table != nullptr;
+  w.requested = std::max(w.requested, k.tab_req);
+  w.slots = std::max(w.slots, wanted_slots<MODE, HAS_QU, MapT>(k));
+  w.slot = slot_bytes(MapTraits<MapT>::packed, k.C);
+  w.C = k.C;
+  w.fixed = static_smem<MODE>();
+  w.samples += k.B;
+  w.pixels = std::max(w.pixels, pixels);
+  w.min_nt = std::max(w.min_nt, k.flags_wide ? 256 : 128);
+}
+
+template <typename Kern>
+int allow_smem(Kern kern, std::once_flag& once, cudaError_t& state) {
+  std::call_once(once, [&] {
     cudaFuncAttributes fa;
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kern);
-    if (e != cudaSuccess) return cuda_fail(e, "kernel shared-memory attributes");
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
-    info.configured = true;
-    info.blocks_per_sm = 0;
-  }
-  if (info.blocks_per_sm == 0 || info.smem != smem) {
-    int nb = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, NT, smem);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    info.blocks_per_sm = std::max(nb, 1);
-    info.smem = smem;
-  }
-  blocks_per_sm = info.blocks_per_sm;
-  return TODGPU_OK;
+    state = cudaFuncGetAttributes(&fa, kern);
+    if (state == cudaSuccess)
+      state = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(kSmemPerCTAMax - fa.sharedSizeBytes));
+  });
+  return state == cudaSuccess ? TODGPU_OK : cuda_fail(state, "kernel shared-memory attributes");
 }
 
-// Two CTA shapes.  Wide: kNT (256) threads, min_blocks() CTAs per SM, room
-// for the default 32 KiB spin-2 table and the staged beam.  Narrow: 128
-// threads, 8 CTAs per SM at 64 registers, for launches whose requested table
-// fits an eighth of an SM's shared memory beside the shape's 80-ring header
-// (config 2: 820 slots of 16 B): with more CTAs per SM, the per-sample setup
-// and barriers of one CTA overlap the pixel loops of more others (config 2
-// bilinear +12%, nearest +7%, although the beam no longer fits beside the
-// table).  Larger footprints (config 3: 3.2k slots) keep the wide shape: in
-// the narrow one their tables would not fit and their samples would fall back
-// to direct spin-2 evaluation.  The TOD is the same bit for bit in either
-// shape (kSumLanes).
-template <typename TabT>
-bool narrow_fits(int requested) {
-  return requested > 0 && ring_cap_for(requested) <= kRingCapNarrow &&
-         requested <= max_table_slots<TabT, kMinbNarrow>(kRingCapNarrow);
-}
-
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, int NT, int MINB>
-int launch_gather_shape(KArgs k, cudaStream_t stream) {
-  auto kern = gather_accum_kernel<MODE, HAS_QU, MapT, PM, LAYOUT, NT, MINB>;
-  static LaunchInfo info;
-  static std::mutex mu;
-  using TabT = typename MapTraits<MapT>::Tab;
-  const bool tab = HAS_QU && k.ring_table != nullptr;
-  k.ring_cap = header_rings<NT>(tab, k.tab_req);
-  const int tab_cap = tab ? table_slots<TabT, MINB>(k.tab_req, k.ring_cap) : 0;
-  const size_t tab_end = spin2_header_bytes(k.ring_cap) + align16(sizeof(TabT) * (size_t)tab_cap);
-  const size_t stage = beam_stage_bytes(k.S, PM == kParamsRef32 ? sizeof(float) : sizeof(double));
-  k.beam_stage = (stage_beam_mode<MODE>() && k.flags_stage && tab_end + stage <= cta_smem_budget<MINB>()) ? 1 : 0;
-  const size_t smem = tab_end + (k.beam_stage ? stage : 0);
-  int blocks_per_sm = 0;
-  const int rc = configure_launch<NT>(kern, info, mu, smem, blocks_per_sm);
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_gather(KArgs k, cudaStream_t stream) {
+  auto kern = gather_accum_kernel<MODE, HAS_QU, MapT, PM, LAYOUT>;
+  static std::once_flag once;
+  static cudaError_t state = cudaSuccess;
+  const int rc = allow_smem(kern, once, state);
   if (rc != TODGPU_OK) return rc;
-  k.tab_cap = tab_cap;
-  const long long max_blocks = (long long)sm_count() * blocks_per_sm;
+  Wants w;
+  add_wants<MODE, HAS_QU, MapT, PM>(w, k);
+  const Shape s = choose_shape(w);
+  k.ring_cap = s.ring_cap;
+  k.tab_cap = s.tab_cap;
+  const long long max_blocks = (long long)sm_count() * ctas_per_sm(s.nt, s.smem + w.fixed);
   const int grid = (int)std::max(1LL, std::min(k.B, max_blocks));
-  kern<<<grid, NT, smem, stream>>>(k);
+  kern<<<grid, s.nt, s.smem, stream>>>(k);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "gather_accum_kernel launch");
   return TODGPU_OK;
 }
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
-int launch_gather(KArgs k, cudaStream_t stream) {
-  using TabT = typename MapTraits<MapT>::Tab;
-  if (!k.flags_wide && narrow_fits<TabT>(k.tab_req))
-    return launch_gather_shape<MODE, HAS_QU, MapT, PM, LAYOUT, kNTNarrow, kMinbNarrow>(k, stream);
-  return launch_gather_shape<MODE, HAS_QU, MapT, PM, LAYOUT, kNT, min_blocks<MODE, MapT>()>(k, stream);
-}
-
 static_assert(sizeof(BatchParams) <= 32000, "batched descriptors must fit the kernel parameter space");
-static_assert(sizeof(KArgs) % 8 == 0 && sizeof(KArgs) / 8 <= kNTNarrow, "KArgs copied as 8-byte words, one per thread");
+static_assert(sizeof(KArgs) % 8 == 0 && sizeof(KArgs) / 8 <= 128, "KArgs copied as 8-byte words, one per thread");
 
 // Batched launch: descriptors of up to kMaxBatchJobs jobs per launch, in one
-// CTA shape: narrow when every job allows it and the table size the launch
-// takes (the largest any job asks for; a job asking for the default makes it
-// the default) fits it.
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, int NT, int MINB>
-int launch_batched_shape(BatchParams& bp, bool any_table, int req, bool any_default, cudaStream_t stream) {
-  auto kern = gather_batched_kernel<MODE, HAS_QU, MapT, PM, LAYOUT, NT, MINB>;
-  static LaunchInfo info;
-  static std::mutex mu;
-  using TabT = typename MapTraits<MapT>::Tab;
-  const int ring_cap = header_rings<NT>(HAS_QU && any_table, any_default ? 0 : req);
-  const int tab_cap = (HAS_QU && any_table) ? table_slots<TabT, MINB>(any_default ? 0 : req, ring_cap) : 0;
-  const size_t tab_end = spin2_header_bytes(ring_cap) + align16(sizeof(TabT) * (size_t)tab_cap);
-  // one shared region for every job's beam: sized for the largest
-  size_t stage = 0;
-  bool want_stage = true;
-  for (int j = 0; j < bp.njobs; ++j) {
-    stage = std::max(stage, beam_stage_bytes(bp.job[j].S, PM == kParamsRef32 ? sizeof(float) : sizeof(double)));
-    want_stage = want_stage && bp.job[j].flags_stage;
-  }
-  const int staged = (stage_beam_mode<MODE>() && want_stage && tab_end + stage <= cta_smem_budget<MINB>()) ? 1 : 0;
-  const size_t smem = tab_end + (staged ? stage : 0);
-  int blocks_per_sm = 0;
-  const int rc = configure_launch<NT>(kern, info, mu, smem, blocks_per_sm);
+// CTA shape, sized for the largest table any job asks for.
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_batched(BatchParams& bp, cudaStream_t stream) {
+  auto kern = gather_batched_kernel<MODE, HAS_QU, MapT, PM, LAYOUT>;
+  static std::once_flag once;
+  static cudaError_t state = cudaSuccess;
+  const int rc = allow_smem(kern, once, state);
   if (rc != TODGPU_OK) return rc;
-  for (int j = 0; j < bp.njobs; ++j) {
-    bp.job[j].tab_cap = tab_cap;
-    bp.job[j].ring_cap = ring_cap;
-    bp.job[j].beam_stage = staged;
-  }
   const long long T = bp.tiles_before[bp.njobs];
   if (T == 0) return TODGPU_OK;
-  const long long max_blocks = (long long)sm_count() * blocks_per_sm;
+  Wants w;
+  bool any_default = false;
+  for (int j = 0; j < bp.njobs; ++j) {
+    add_wants<MODE, HAS_QU, MapT, PM>(w, bp.job[j]);
+    any_default = any_default || bp.job[j].tab_req == 0;
+  }
+  if (any_default) w.requested = 0;
+  const Shape s = choose_shape(w);
+  for (int j = 0; j < bp.njobs; ++j) {
+    bp.job[j].tab_cap = s.tab_cap;
+    bp.job[j].ring_cap = s.ring_cap;
+  }
+  const long long max_blocks = (long long)sm_count() * ctas_per_sm(s.nt, s.smem + w.fixed);
   const int grid = (int)std::max(1LL, std::min(T, max_blocks));
-  kern<<<grid, NT, smem, stream>>>(bp);
+  kern<<<grid, s.nt, s.smem, stream>>>(bp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "gather_batched_kernel launch");
   return TODGPU_OK;
 }
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
-int launch_batched(BatchParams& bp, bool any_table, cudaStream_t stream) {
-  using TabT = typename MapTraits<MapT>::Tab;
-  int req = 0;
-  bool any_default = false, any_wide = false;
-  for (int j = 0; j < bp.njobs; ++j) {
-    req = std::max(req, bp.job[j].tab_req);
-    any_default = any_default || bp.job[j].tab_req == 0;
-    any_wide = any_wide || bp.job[j].flags_wide;
-  }
-  if (!any_wide && !any_default && narrow_fits<TabT>(req))
-    return launch_batched_shape<MODE, HAS_QU, MapT, PM, LAYOUT, kNTNarrow, kMinbNarrow>(bp, any_table, req, false,
-                                                                                        stream);
-  return launch_batched_shape<MODE, HAS_QU, MapT, PM, LAYOUT, kNT, min_blocks<MODE, MapT>()>(bp, any_table, req,
-                                                                                           any_default, stream);
-}
-
 template <int MODE, typename MapT, int PM>
-int dispatch_batched_qu(BatchParams& bp, bool has_qu, bool iqu, bool any_table, cudaStream_t s) {
-  if (has_qu && iqu) return launch_batched<MODE, true, MapT, PM, kLayoutIQU>(bp, any_table, s);
-  return has_qu ? launch_batched<MODE, true, MapT, PM, kLayoutGeneric>(bp, any_table, s)
-                : launch_batched<MODE, false, MapT, PM, kLayoutGeneric>(bp, any_table, s);
+int dispatch_batched_qu(BatchParams& bp, bool has_qu, bool iqu, cudaStream_t s) {
+  if (has_qu && iqu) return launch_batched<MODE, true, MapT, PM, kLayoutIQU>(bp, s);
+  return has_qu ? launch_batched<MODE, true, MapT, PM, kLayoutGeneric>(bp, s)
+                : launch_batched<MODE, false, MapT, PM, kLayoutGeneric>(bp, s);
 }
 
 template <int MODE, typename MapT, int PM>
@@ -2231,17 +2145,17 @@ int dispatch_single_pm(const KArgs& k, bool has_qu, int params_dtype, cudaStream
 }
 
 template <int MODE, typename MapT>
-int dispatch_batched_pm(BatchParams& bp, bool has_qu, bool iqu, bool any_table, int params_dtype, cudaStream_t s) {
-  if (params_dtype == TODGPU_F32) return dispatch_batched_qu<MODE, MapT, kParamsRef32>(bp, has_qu, iqu, any_table, s);
-  if (params_dtype == TODGPU_F64) return dispatch_batched_qu<MODE, MapT, kParamsF64>(bp, has_qu, iqu, any_table, s);
-  return dispatch_batched_qu<MODE, MapT, kAngles>(bp, has_qu, iqu, any_table, s);
+int dispatch_batched_pm(BatchParams& bp, bool has_qu, bool iqu, int params_dtype, cudaStream_t s) {
+  if (params_dtype == TODGPU_F32) return dispatch_batched_qu<MODE, MapT, kParamsRef32>(bp, has_qu, iqu, s);
+  if (params_dtype == TODGPU_F64) return dispatch_batched_qu<MODE, MapT, kParamsF64>(bp, has_qu, iqu, s);
+  return dispatch_batched_qu<MODE, MapT, kAngles>(bp, has_qu, iqu, s);
 }
 
 // Entry points of the per-map-type translation units.
 #define TODGPU_DECLARE_MAP_DISPATCH(NAME)                                                                   \
   int dispatch_single_##NAME(const KArgs& k, int interp, bool has_qu, int params_dtype, cudaStream_t s);   \
-  int dispatch_batched_##NAME(BatchParams& bp, int interp, bool has_qu, bool iqu, bool any_table,          \
-                              int params_dtype, cudaStream_t s);
+  int dispatch_batched_##NAME(BatchParams& bp, int interp, bool has_qu, bool iqu, int params_dtype,        \
+                              cudaStream_t s);
 TODGPU_DECLARE_MAP_DISPATCH(f64)
 TODGPU_DECLARE_MAP_DISPATCH(f32)
 TODGPU_DECLARE_MAP_DISPATCH(pf32)
@@ -2254,11 +2168,11 @@ TODGPU_DECLARE_MAP_DISPATCH(pf64)
     return interp == TODGPU_BILINEAR ? dispatch_single_pm<TODGPU_BILINEAR, MAPT>(k, has_qu, params_dtype, s) \
                                      : dispatch_single_pm<TODGPU_NEAREST, MAPT>(k, has_qu, params_dtype, s);  \
   }                                                                                                        \
-  int dispatch_batched_##NAME(BatchParams& bp, int interp, bool has_qu, bool iqu, bool any_table,          \
-                              int params_dtype, cudaStream_t s) {                                          \
+  int dispatch_batched_##NAME(BatchParams& bp, int interp, bool has_qu, bool iqu, int params_dtype,        \
+                              cudaStream_t s) {                                                            \
     return interp == TODGPU_BILINEAR                                                                       \
-               ? dispatch_batched_pm<TODGPU_BILINEAR, MAPT>(bp, has_qu, iqu, any_table, params_dtype, s)   \
-               : dispatch_batched_pm<TODGPU_NEAREST, MAPT>(bp, has_qu, iqu, any_table, params_dtype, s);   \
+               ? dispatch_batched_pm<TODGPU_BILINEAR, MAPT>(bp, has_qu, iqu, params_dtype, s)              \
+               : dispatch_batched_pm<TODGPU_NEAREST, MAPT>(bp, has_qu, iqu, params_dtype, s);              \
   }
 
 }  // namespace todgpu

@@ -15,33 +15,20 @@ thread_local std::string g_last_error;
 // whole ring when the disc can contain the pole.
 __global__ void ring_table_kernel(long long nside, double reach, RingRec* t, bool reach_from_header) {
   const long long nrings = 4 * nside - 1;
-  const long long npix = 12 * nside * nside;
   if (reach_from_header) reach = t[0].ta;
   for (long long ir = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; ir <= nrings;
        ir += (long long)gridDim.x * blockDim.x) {
-    const RingInfo ri = hp_ring_info(nside, ir, npix);
-    RingRec r;
-    r.z = hp_ring_z(nside, ir);
-    r.ta = acos(r.z);
-    r.sth = sqrt(max0(1.0 - r.z * r.z));
-    r.phi0 = ri.phi0;
-    r.dphi = ri.dphi;
-    r.first = ri.first;
-    r.n = (int)ri.n;
-    int cap = (int)ri.n;
+    RingRec r = make_ring(nside, ir);
+    int cap = r.n;
     if (reach < r.ta && reach < kPi - r.ta) {
       const double x = sin(reach) / r.sth;
       if (x < 1.0) {
         const double half = asin(x);
-        const long long c = 2 * (long long)ceil(half / ri.dphi) + 5;
-        cap = (int)min(c, ri.n);
+        const long long c = 2 * (long long)ceil(half / r.dphi) + 5;
+        cap = (int)min(c, (long long)r.n);
       }
     }
     r.cap = cap;
-    r.unused = 0;
-    r.first32 = (int)ri.first;
-    r.inv_dphi = 1.0 / ri.dphi;
-    r.inv_dta = ir < nrings ? 1.0 / (acos(hp_ring_z(nside, ir + 1)) - r.ta) : 0.0;
     t[ir] = r;
   }
   if (!reach_from_header && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -230,10 +217,10 @@ static __device__ __align__(256) RingRec g_static_ring_table[4 * kStaticMaxNside
 // Header of a table built from the beam on the device: the footprint reach the
 // gather kernel derives from the same beam (same code, plus a hair of margin).
 template <int PM>
-__global__ void __launch_bounds__(kNTStatic) static_reach_kernel(const KArgs a, RingRec* t) {
-  __shared__ double s_red[(kNTStatic / 32) * 4];
+__global__ void __launch_bounds__(256) static_reach_kernel(const KArgs a, RingRec* t) {
+  __shared__ double s_red[64];
   double cx, cy, cz, rbeam;
-  beam_extent<PM, kNTStatic>(a, s_red, cx, cy, cz, rbeam);
+  beam_extent<PM>(a, 0, (int)a.S, s_red, cx, cy, cz, rbeam);
   if (threadIdx.x == 0) {
     RingRec h;
     h.z = (double)a.nside;
@@ -317,14 +304,14 @@ static int dispatch_types(const KArgs& k, int interp, bool has_qu, int map_dtype
   }
 }
 
-static int dispatch_batched(BatchParams& bp, int interp, bool has_qu, bool iqu, bool any_table, int map_dtype,
-                            int params_dtype, cudaStream_t s) {
+static int dispatch_batched(BatchParams& bp, int interp, bool has_qu, bool iqu, int map_dtype, int params_dtype,
+                            cudaStream_t s) {
   switch (map_dtype) {
-    case TODGPU_PACKED_F32: return dispatch_batched_pf32(bp, interp, has_qu, iqu, any_table, params_dtype, s);
-    case TODGPU_PACKED_BF16: return dispatch_batched_pbf16(bp, interp, has_qu, iqu, any_table, params_dtype, s);
-    case TODGPU_PACKED_F64: return dispatch_batched_pf64(bp, interp, has_qu, iqu, any_table, params_dtype, s);
-    case TODGPU_F32: return dispatch_batched_f32(bp, interp, has_qu, iqu, any_table, params_dtype, s);
-    default: return dispatch_batched_f64(bp, interp, has_qu, iqu, any_table, params_dtype, s);
+    case TODGPU_PACKED_F32: return dispatch_batched_pf32(bp, interp, has_qu, iqu, params_dtype, s);
+    case TODGPU_PACKED_BF16: return dispatch_batched_pbf16(bp, interp, has_qu, iqu, params_dtype, s);
+    case TODGPU_PACKED_F64: return dispatch_batched_pf64(bp, interp, has_qu, iqu, params_dtype, s);
+    case TODGPU_F32: return dispatch_batched_f32(bp, interp, has_qu, iqu, params_dtype, s);
+    default: return dispatch_batched_f64(bp, interp, has_qu, iqu, params_dtype, s);
   }
 }
 
@@ -416,10 +403,11 @@ static KArgs make_kargs(const todgpu_gather_args* a) {
   if (k.ring_table != nullptr && (((uintptr_t)k.ring_table & 15) != 0)) k.ring_table = nullptr;
   k.tab_cap = 0;
   k.tab_req = a->tab_slots;
-  k.flags_stage = (a->flags & TODGPU_FLAG_NO_BEAM_STAGE) ? 0 : 1;
-  k.beam_stage = 0;
   k.flags_wide = (a->flags & TODGPU_FLAG_WIDE_CTAS) ? 1 : 0;
   k.ring_cap = 0;
+  const bool planar = (a->flags & TODGPU_FLAG_BEAM_PLANAR) != 0;
+  k.vec_ss = planar ? 1 : 3;
+  k.vec_si = planar ? a->S : 1;
   return k;
 }
 
@@ -478,18 +466,12 @@ extern "C" int todgpu_gather_accum_static(const todgpu_gather_args* a, void* str
   const bool has_qu = (a->c_q >= 0 && a->c_u >= 0);
   if (!(a->flags & TODGPU_FLAG_NO_TABLES)) {
     // every call rebuilds the whole table (header and records) for its own
-    // nside and beam, so nothing depends on earlier contents.  Without Q and U
-    // the gather reads only the ring records (no spin-2 tables): the header
-    // then carries a zero reach.
-    if (has_qu) {
-      if (a->params_dtype == TODGPU_F32)
-        static_reach_kernel<kParamsRef32><<<1, kNTStatic, 0, s>>>(k, t);
-      else
-        static_reach_kernel<kParamsF64><<<1, kNTStatic, 0, s>>>(k, t);
-      ring_table_kernel<<<grid_for(4 * a->nside, 256), 256, 0, s>>>(a->nside, 0.0, t, true);
-    } else {
-      ring_table_kernel<<<grid_for(4 * a->nside, 256), 256, 0, s>>>(a->nside, 0.0, t, false);
-    }
+    // nside and beam, so nothing depends on earlier contents
+    if (a->params_dtype == TODGPU_F32)
+      static_reach_kernel<kParamsRef32><<<1, 256, 0, s>>>(k, t);
+    else
+      static_reach_kernel<kParamsF64><<<1, 256, 0, s>>>(k, t);
+    ring_table_kernel<<<grid_for(4 * a->nside, 256), 256, 0, s>>>(a->nside, 0.0, t, true);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "built-in ring table kernels");
     k.ring_table = t;
@@ -500,9 +482,8 @@ extern "C" int todgpu_gather_accum_static(const todgpu_gather_args* a, void* str
 }
 
 extern "C" int64_t todgpu_gather_wait_timeouts(void) {
-  unsigned long long v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_gather_wait_timeouts, sizeof(v)) != cudaSuccess) return -1;
-  return (int64_t)v;
+  // the gather kernels wait on nothing but their own CTA's barriers
+  return cudaDeviceSynchronize() == cudaSuccess ? 0 : -1;
 }
 
 extern "C" int todgpu_gather_accum_batched(const todgpu_gather_args* jobs, int32_t njobs, int64_t tile,
@@ -531,15 +512,13 @@ extern "C" int todgpu_gather_accum_batched(const todgpu_gather_args* jobs, int32
     bp.njobs = n;
     bp.tile = tile;
     bp.tiles_before[0] = 0;
-    bool any_table = false;
     for (int j = 0; j < n; ++j) {
       const todgpu_gather_args& a = jobs[first + j];
       bp.job[j] = make_kargs(&a);
-      any_table = any_table || bp.job[j].ring_table != nullptr;
       const long long ntiles = (a.S > 0) ? (a.B + tile - 1) / tile : 0;
       bp.tiles_before[j + 1] = bp.tiles_before[j] + ntiles;
     }
-    const int rc = dispatch_batched(bp, j0.interp, has_qu, iqu, any_table, j0.map_dtype, j0.params_dtype, s);
+    const int rc = dispatch_batched(bp, j0.interp, has_qu, iqu, j0.map_dtype, j0.params_dtype, s);
     if (rc != TODGPU_OK) return rc;
   }
   return TODGPU_OK;

@@ -148,17 +148,12 @@ _TABLE_REACH = {}  # data_ptr of a cached ring table -> the reach it was built f
 
 
 def table_slots(nside, reach):
-    """Spin-2 table slots a sample needs for a footprint of radius ``reach``
-    [rad] away from the poles, an upper bound of what the kernel fills: per
-    window ring the disc's stretch with 2% margin, rounded up to 2k + 1 slots
-    -- at most 1.02 x 3 (reach nside)^2 for the disc plus 3 per ring over at
-    most 3 reach nside + 4 rings -- with 5% more and 32 to spare.  The request
-    also sizes the table header (256-thread CTAs reserve window rings for a
-    disc of request / 3.2 pixels, 128-thread CTAs a fixed 80).  Shared memory beyond them is left to L1, and a
-    request of up to about 1500 slots (float64 tables; 1900 float32) lets the
-    launch run 128-thread CTAs, 8 per SM.  For a reach of 0.05 rad or more the
-    kernel reserves whole ring stretches instead of the disc, and the
-    library's default (0) is asked for."""
+    """Upper bound of the map pixels in a footprint disc of radius ``reach`` [rad]
+    away from the poles: per ring the disc's stretch with 2% margin, rounded up to
+    2k + 1 pixels -- at most 1.02 x 3 (reach nside)^2 for the disc plus 3 per ring
+    over at most 3 reach nside + 4 rings -- with 5% more and 32 to spare; 0 from
+    0.05 rad.  A generous request: the gather lays its footprints out more tightly
+    (:func:`footprint_slots`)."""
     r = float(reach)
     n = float(nside)
     if not r < 0.05:
@@ -168,13 +163,24 @@ def table_slots(nside, reach):
     return int(min(1 << 20, math.ceil(1.05 * need) + 32))
 
 
+def footprint_slots(nside, reach):
+    """Table slots of a footprint away from the poles as the gather lays it out:
+    ``reach`` [rad] is a ring table's (the beam's radius plus 3/nside), x = radius
+    times nside; per ring 2 H + 3 slots on average for a beam disc of half-width H
+    pixels, each ring taking the disc's width one ring spacing nearer its centre --
+    1.02 x 3 x^2 + 13.2 x + 12 -- with 3% more and 8 to spare (4 to 10% above what
+    footprints of x = 3 to 60 fill)."""
+    x = max(0.0, float(reach) - 3.0 / float(nside)) * float(nside)
+    return int(min(1 << 20, math.ceil(1.03 * (1.02 * 3.0 * x * x + 13.2 * x + 12.0)) + 8))
+
+
 def table_slots_for(table, nside):
-    """``table_slots`` for a table made by :func:`ring_table` (0, the
+    """``footprint_slots`` for a table made by :func:`ring_table` (0, the
     library's default, for any other table or none)."""
     if table is None:
         return 0
     reach = _TABLE_REACH.get(table.data_ptr()) if is_tensor(table) else None
-    return 0 if reach is None else table_slots(nside, reach)
+    return 0 if reach is None else footprint_slots(nside, reach)
 
 
 def ring_table(nside, reach, device=None):
@@ -194,6 +200,26 @@ def ring_table(nside, reach, device=None):
         _RING_TABLES[key] = t
         _TABLE_REACH[t.data_ptr()] = float(reach_q)
     return t
+
+
+# Evaluations (samples x beam pixels) from which a call makes its beam vectors
+# planar: the copy takes some 5 us, interleaved vectors cost the gather a tenth
+# of its time (three strided reads of 12 or 24 bytes a pixel) -- 40 us here.
+_PLANAR_EVALS = 1 << 24
+
+
+def planar_beam(vec, evals=None):
+    """(vectors, flag) for a gather of ``evals`` evaluations over a CUDA (S, 3)
+    tensor ``vec``: as they are if they are planar already (the (S, 3) view of a
+    (3, S) tensor, as ``tod_core.device_beam`` keeps them), made planar for a
+    large gather (``evals`` None: always), else interleaved.  flag is
+    ``FLAG_BEAM_PLANAR`` or 0; the vectors' data pointer goes into vec_orig."""
+    S = vec.shape[0]
+    if S > 1 and vec.stride() == (1, S):
+        return vec, _native.FLAG_BEAM_PLANAR
+    if S > 1 and (evals is None or evals >= _PLANAR_EVALS):
+        return vec.t().contiguous().t(), _native.FLAG_BEAM_PLANAR
+    return vec.contiguous(), 0
 
 
 def _row_stride(t):
@@ -315,7 +341,11 @@ def gather_accum(interp, vec_orig, axes, cos_a, sin_a, ax_pts, cos_p, sin_p, nsi
     raw = (vec_orig, axes, cos_a, sin_a, ax_pts, cos_p, sin_p)
     pdt = _param_dtype(raw)
     shapes = [(S, 3), (B, 3), (B,), (B,), (B, 3), (B,), (B,)]
-    params = [to_device(x, pdt, sh) for x, sh in zip(raw, shapes)]
+    if is_tensor(vec_orig) and vec_orig.is_cuda and tuple(vec_orig.shape) == (S, 3):
+        vec, planar = planar_beam(vec_orig, B * S)
+    else:
+        vec, planar = planar_beam(to_device(vec_orig, pdt, (S, 3)), B * S)
+    params = [vec] + [to_device(x, pdt, sh) for x, sh in zip(raw[1:], shapes[1:])]
     if dtype_of(beam_vals) != np.dtype(np.float32):
         raise TypeError("beam_vals must be float32 (the reference casts beam weights to float32)")
     beam = to_device(beam_vals, np.float32, (S,))
@@ -343,7 +373,7 @@ def gather_accum(interp, vec_orig, axes, cos_a, sin_a, ax_pts, cos_p, sin_p, nsi
     if not flags & _native.FLAG_NO_TABLES and B > 0 and S > 0:
         table = ring_table(nside, beam_reach(vec_orig, nside), params[0].device)
     args = make_args(interp, nside, B, S, C, c_q, c_u, params, pdt, bphi, beam, mp, dtod,
-                     err_count, flags, table)
+                     err_count, flags | planar, table)
     _native.check(_native.lib().todgpu_gather_accum(ctypes.byref(args), stream_handle()))
     if host_tod is not None:
         res = dtod.cpu().numpy()
@@ -450,10 +480,14 @@ def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_th
     ``precompute=False`` (and ``static_table=True``, which allocates nothing)
     derive the rotation inside the gather."""
     require_cuda()
-    vec = to_device(vec_orig, np.float64).reshape(-1, 3)
-    S = vec.shape[0]
+    if is_tensor(vec_orig) and vec_orig.is_cuda and vec_orig.dtype == torch.float64 and vec_orig.dim() == 2:
+        given = vec_orig  # (a copy or view would be another tensor to beam_reach)
+    else:
+        given = to_device(vec_orig, np.float64).reshape(-1, 3)
+    S = given.shape[0]
     adt, th, ph, ps = _angles_on_device(theta, phi, psi)
     B = th.shape[0]
+    vec, planar = planar_beam(given, B * S)
     rot = pointing_params(th, ph, ps, center_phi, center_theta) if precompute and not static_table else None
     beam = to_device(beam_vals, np.float32, (S,))
     mp = _map_tensor(mp_stacked)
@@ -485,13 +519,13 @@ def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_th
     a.tod = tod.data_ptr()
     a.tod_stride = _row_stride(tod)
     a.err_count = ptr(err_count)
-    a.flags = int(flags)
+    a.flags = int(flags) | planar
     lib = _native.lib()
     if static_table:
         _native.check(lib.todgpu_gather_accum_static(ctypes.byref(a), stream_handle()))
         return tod
     if not flags & _native.FLAG_NO_TABLES and B > 0 and S > 0:
-        table = ring_table(nside, beam_reach(vec, nside), vec.device)
+        table = ring_table(nside, beam_reach(given, nside), vec.device)
         a.ring_table = table.data_ptr()
         a.tab_slots = table_slots_for(table, nside)
     _native.check(lib.todgpu_gather_accum(ctypes.byref(a), stream_handle()))

@@ -151,7 +151,9 @@ def device_beam(vec_orig, beam_vals, vec_dtype=torch.float64):
     def make():
         v = vec.reshape(-1, 3)
         idx = torch.from_numpy(beam_order(v)).to(v.device)
-        return v[idx].contiguous(), bv.reshape(-1)[idx].contiguous()
+        # (S, 3) views of planar (3, S) vectors: neighbouring threads read
+        # neighbouring elements
+        return v[idx].t().contiguous().t(), bv.reshape(-1)[idx].contiguous()
 
     return _derived.get((vec, bv), ("beam", str(vec_dtype)), make)
 
