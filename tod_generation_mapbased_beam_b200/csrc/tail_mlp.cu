@@ -39,6 +39,7 @@ constexpr int kMaxDepth = 8;
 constexpr int kMaxOut = 4;
 constexpr int BM = 128, BN = 128, BK = 32;
 constexpr int kLd = BK + 8;  // shared-memory row stride in elements (80 B: conflict-free ldmatrix)
+constexpr int kLdT = BM + 8;  // the same for tiles kept as S[k][row] (272 B)
 constexpr int kThreads = 256;
 
 struct Dims {
@@ -185,6 +186,12 @@ __device__ __forceinline__ void ldsm_x4(unsigned addr, unsigned& r0, unsigned& r
                : "r"(addr));
 }
 
+__device__ __forceinline__ void ldsm_x4_trans(unsigned addr, unsigned& r0, unsigned& r1, unsigned& r2, unsigned& r3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(addr));
+}
+
 __device__ __forceinline__ void mma_bf16(float* c, const unsigned* a, unsigned b0, unsigned b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -209,7 +216,10 @@ __device__ __forceinline__ void load_tile(const bf16* P, long long ld, int r0, l
   }
 }
 
-// Registers -> shared tile S[row][k] (k contiguous, row stride kLd).
+// Registers -> shared tile, as it lies in memory: S[row][k] (L = 0, row stride
+// kLd) or S[k][row] (L = 1, row stride kLdT).  The transposed operands of the
+// backward products were scattered into S[row][k] two bytes at a time; they are
+// read with transposing ldmatrix instead.
 template <int L>
 __device__ __forceinline__ void store_tile(bf16* S, const uint4* reg) {
 #pragma unroll
@@ -220,17 +230,15 @@ __device__ __forceinline__ void store_tile(bf16* S, const uint4* reg) {
       *reinterpret_cast<uint4*>(S + r * kLd + kc) = reg[i];
     } else {
       const int kr = c >> 4, rc = (c & 15) * 8;
-      const bf16* v = reinterpret_cast<const bf16*>(&reg[i]);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) S[(rc + j) * kLd + kr] = v[j];
+      *reinterpret_cast<uint4*>(S + kr * kLdT + rc) = reg[i];
     }
   }
 }
 
 template <int AL, int BL, int EPI>
 __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
-  __shared__ __align__(16) bf16 As[BM * kLd];
-  __shared__ __align__(16) bf16 Bs[BN * kLd];
+  __shared__ __align__(16) bf16 As[AL == 0 ? BM * kLd : BK * kLdT];
+  __shared__ __align__(16) bf16 Bs[BL == 0 ? BN * kLd : BK * kLdT];
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const long long kb = (long long)blockIdx.z * g.K;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -264,17 +272,30 @@ __global__ void __launch_bounds__(kThreads) gemm_kernel(GemmArgs g) {
       unsigned af[4][4];
 #pragma unroll
       for (int mt = 0; mt < 4; ++mt) {
-        const int row = wm + mt * 16 + (lane & 15);
-        const int col = ks + (lane >> 4) * 8;
-        ldsm_x4(sA + (unsigned)(row * kLd + col) * 2u, af[mt][0], af[mt][1], af[mt][2], af[mt][3]);
+        if (AL == 0) {
+          const int row = wm + mt * 16 + (lane & 15);
+          const int col = ks + (lane >> 4) * 8;
+          ldsm_x4(sA + (unsigned)(row * kLd + col) * 2u, af[mt][0], af[mt][1], af[mt][2], af[mt][3]);
+        } else {  // 8 x 8 blocks (k, m): rows 0-7 / 8-15 of m, then the upper half of k
+          const int kr = ks + (lane & 7) + ((lane >> 4) << 3);
+          const int col = wm + mt * 16 + ((lane >> 3) & 1) * 8;
+          ldsm_x4_trans(sA + (unsigned)(kr * kLdT + col) * 2u, af[mt][0], af[mt][1], af[mt][2], af[mt][3]);
+        }
       }
       unsigned bfr[4][2];
 #pragma unroll
       for (int np = 0; np < 2; ++np) {
-        const int row = wn + np * 16 + (lane & 7) + ((lane >> 4) << 3);
-        const int col = ks + ((lane >> 3) & 1) * 8;
-        ldsm_x4(sB + (unsigned)(row * kLd + col) * 2u, bfr[2 * np][0], bfr[2 * np][1], bfr[2 * np + 1][0],
-                bfr[2 * np + 1][1]);
+        if (BL == 0) {
+          const int row = wn + np * 16 + (lane & 7) + ((lane >> 4) << 3);
+          const int col = ks + ((lane >> 3) & 1) * 8;
+          ldsm_x4(sB + (unsigned)(row * kLd + col) * 2u, bfr[2 * np][0], bfr[2 * np][1], bfr[2 * np + 1][0],
+                  bfr[2 * np + 1][1]);
+        } else {
+          const int kr = ks + (lane & 7) + ((lane >> 3) & 1) * 8;
+          const int col = wn + np * 16 + ((lane >> 4) << 3);
+          ldsm_x4_trans(sB + (unsigned)(kr * kLdT + col) * 2u, bfr[2 * np][0], bfr[2 * np][1], bfr[2 * np + 1][0],
+                        bfr[2 * np + 1][1]);
+        }
       }
 #pragma unroll
       for (int mt = 0; mt < 4; ++mt)
@@ -386,17 +407,32 @@ __global__ void head_bwd_kernel(const float* dy, long long M, int H, const bf16*
   }
 }
 
+// Row blocks of the sums over the batch below: at most 128 blocks of at least
+// 64 rows, `per` partial floats each within `room`.  (One block per split of the
+// weight gradients, 256 rows one after another, left most SMs idle and waited
+// for every row: 87 us for the column sums of 8192 rows, four times a step.)
+struct RowBlocks {
+  int n;
+  long long rows;
+};
+inline RowBlocks row_blocks(long long M, long long per, long long room) {
+  const long long most = std::max(1LL, std::min({128LL, M / 64, room / per}));
+  const long long rows = (M + most - 1) / most;
+  return RowBlocks{(int)((M + rows - 1) / rows), rows};
+}
+
 // Head weight/bias gradient partials over a contiguous range of rows per block:
 // part[z][o * H + k] = sum_m dy(m, o) act(m, k), part[z][O * H + o] = sum_m dy(m, o).
 template <int O>
-__global__ void head_wgrad_kernel(const float* dy, const bf16* act, long long rows_per_split, int H, float* part) {
-  const long long r0 = (long long)blockIdx.x * rows_per_split;
+__global__ void head_wgrad_kernel(const float* dy, const bf16* act, long long M, long long rows, int H, float* part) {
+  const long long r0 = (long long)blockIdx.x * rows, r1 = min(M, r0 + rows);
   float* p = part + (long long)blockIdx.x * (O * H + O);
   for (int k = threadIdx.x; k < H; k += blockDim.x) {
     float s[O];
 #pragma unroll
     for (int o = 0; o < O; ++o) s[o] = 0.0f;
-    for (long long m = r0; m < r0 + rows_per_split; ++m) {
+#pragma unroll 16
+    for (long long m = r0; m < r1; ++m) {
       const float a = __bfloat162float(act[m * H + k]);
 #pragma unroll
       for (int o = 0; o < O; ++o) s[o] += dy[m * O + o] * a;
@@ -406,18 +442,39 @@ __global__ void head_wgrad_kernel(const float* dy, const bf16* act, long long ro
   }
   if (threadIdx.x < O) {
     float s = 0.0f;
-    for (long long m = r0; m < r0 + rows_per_split; ++m) s += dy[m * O + threadIdx.x];
+#pragma unroll 16
+    for (long long m = r0; m < r1; ++m) s += dy[m * O + threadIdx.x];
     p[O * H + threadIdx.x] = s;
   }
 }
 
-// Bias gradient partials of a hidden layer: part[z][n] = sum over the split's rows of dz(m, n).
-__global__ void colsum_kernel(const bf16* dz, long long rows_per_split, int H, float* part) {
-  const long long r0 = (long long)blockIdx.x * rows_per_split;
+// Bias gradient partials of a hidden layer: part[z][n] = sum over the block's rows of dz(m, n).
+__global__ void colsum_kernel(const bf16* dz, long long M, long long rows, int H, float* part) {
+  const long long r0 = (long long)blockIdx.x * rows, r1 = min(M, r0 + rows);
   for (int n = threadIdx.x; n < H; n += blockDim.x) {
     float s = 0.0f;
-    for (long long m = r0; m < r0 + rows_per_split; ++m) s += __bfloat162float(dz[m * H + n]);
+#pragma unroll 16
+    for (long long m = r0; m < r1; ++m) s += __bfloat162float(dz[m * H + n]);
     part[(long long)blockIdx.x * H + n] = s;
+  }
+}
+
+// out[i] = sum_z part[z * count + i]: 32 columns a block, eight threads a column
+// (z = g, g + 8, ... each), their sums added in order.
+__global__ void reduce_rows_kernel(const float* part, int n, long long count, float* out) {
+  __shared__ float red[8][32];
+  const int c = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const long long i = blockIdx.x * 32LL + c;
+  float s = 0.0f;
+  if (i < count) {
+#pragma unroll 8
+    for (int z = g; z < n; z += 8) s += part[(long long)z * count + i];
+  }
+  red[g][c] = s;
+  __syncthreads();
+  if (g == 0 && i < count) {
+    for (int q = 1; q < 8; ++q) s += red[q][c];
+    out[i] = s;
   }
 }
 
@@ -426,6 +483,7 @@ __global__ void reduce_splits_kernel(const float* part, int splits, long long co
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
        i += (long long)gridDim.x * blockDim.x) {
     float s = 0.0f;
+#pragma unroll 8
     for (int z = 0; z < splits; ++z) s += part[(long long)z * count + i];
     out[i] = s;
   }
@@ -469,8 +527,8 @@ __global__ void to_bf16_kernel(const float* p, bf16* pb, long long n) {
 // its operands staged by the tensor memory accelerator (TMA):
 //   out(m, n) = silu(sum_k A(m, k) W(n, k) + bias(n)),  A (M, K), W (N, K)
 //   bf16 row-major; the sums accumulate in float32 in tensor memory (TMEM).
-// One CTA of 256 threads per 128-row tile, all N (128 or 256) columns at once
-// in N TMEM columns.  K advances in k-tiles of 32 through a ring of 4 shared-
+// One CTA of 256 threads per 128-row tile and N (128 or 256) columns, in N TMEM
+// columns.  K advances in k-tiles of 32 through a ring of 4 shared-
 // memory stages.  Lane 0 of warp 0 is the producer and the MMA issuer: it
 // starts the TMA copies of a k-tile (A: 128 x 32, W: N x 32) on the stage's
 // "full" barrier (transaction count = the stage's bytes), waits for them,
@@ -527,8 +585,8 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
 
 // TMA copies of k-tile kt (A rows m0.., all N rows of W) into stage st.
 template <int N>
-__device__ __forceinline__ void tc_produce(const CUtensorMap* ta, const CUtensorMap* tw, long long m0, int kt,
-                                           uint32_t stage_addr, uint32_t full_bar) {
+__device__ __forceinline__ void tc_produce(const CUtensorMap* ta, const CUtensorMap* tw, long long m0, int n0,
+                                           int kt, uint32_t stage_addr, uint32_t full_bar) {
   using Sh = TcShape<N>;
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"((uint32_t)Sh::STAGE), "r"(full_bar)
                : "memory");
@@ -541,7 +599,7 @@ __device__ __forceinline__ void tc_produce(const CUtensorMap* ta, const CUtensor
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
           "r"(stage_addr + (uint32_t)Sh::A_BYTES),
-      "l"(reinterpret_cast<uint64_t>(tw)), "r"(full_bar), "r"(0), "r"(0), "r"(kc)
+      "l"(reinterpret_cast<uint64_t>(tw)), "r"(full_bar), "r"(0), "r"(n0), "r"(kc)
       : "memory");
 }
 
@@ -550,6 +608,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_fwd_kernel(const __grid_co
                                                                  const __grid_constant__ CUtensorMap tma_w, int K,
                                                                  const float* bias, float* zout, bf16* aout,
                                                                  long long ldc) {
+  const int n0 = blockIdx.y * N;  // this CTA's columns of the layer
   using Sh = TcShape<N>;
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   __shared__ __align__(8) unsigned long long bars[2 * TC_STAGES + 1];  // full[S], empty[S], done
@@ -561,7 +620,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_fwd_kernel(const __grid_co
   const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(tc_smem);
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
   const uint32_t full0 = bar0, empty0 = bar0 + 8 * TC_STAGES, done = bar0 + 16 * TC_STAGES;
-  for (int i = tid; i < N; i += TC_THREADS) s_bias[i] = bias[i];
+  for (int i = tid; i < N; i += TC_THREADS) s_bias[i] = bias[n0 + i];
   if (tid == 0) {
     for (int i = 0; i < 2 * TC_STAGES + 1; ++i)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i));
@@ -585,7 +644,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_fwd_kernel(const __grid_co
       bool ok = true;
       int produced = 0, consumed = 0;  // k-tiles whose copies were started / waited for
       for (int kt = 0; kt < TC_STAGES && kt < KT; ++kt, ++produced)
-        tc_produce<N>(&tma_a, &tma_w, m0, kt, sbase + kt * Sh::STAGE, full0 + 8 * kt);
+        tc_produce<N>(&tma_a, &tma_w, m0, n0, kt, sbase + kt * Sh::STAGE, full0 + 8 * kt);
       for (int kt = 0; kt < KT && ok; ++kt) {
         const int st = kt % TC_STAGES;
         const uint32_t sa = sbase + st * Sh::STAGE, sb = sa + Sh::A_BYTES;
@@ -616,7 +675,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_fwd_kernel(const __grid_co
             ok = false;
             break;
           }
-          tc_produce<N>(&tma_a, &tma_w, m0, kr, sbase + sp * Sh::STAGE, full0 + 8 * sp);
+          tc_produce<N>(&tma_a, &tma_w, m0, n0, kr, sbase + sp * Sh::STAGE, full0 + 8 * sp);
           ++produced;
         }
       }
@@ -657,11 +716,11 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_fwd_kernel(const __grid_co
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) + s_bias[c0 + j];
       if (zout) {
-        float4* zp = reinterpret_cast<float4*>(zout + row * ldc + c0);
+        float4* zp = reinterpret_cast<float4*>(zout + row * ldc + n0 + c0);
 #pragma unroll
         for (int j = 0; j < 8; ++j) zp[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
       }
-      uint4* ap = reinterpret_cast<uint4*>(aout + row * ldc + c0);
+      uint4* ap = reinterpret_cast<uint4*>(aout + row * ldc + n0 + c0);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         __nv_bfloat162 h[4];
@@ -772,8 +831,8 @@ bool launch_tc(const GemmArgs& g, cudaStream_t s) {
   });
   if (attr != cudaSuccess) return false;
   CUtensorMap ta, tw;
-  if (!encode_operand(&ta, g.A, g.M, g.K, TC_BM) || !encode_operand(&tw, g.B, N, g.K, N)) return false;
-  gemm_tc_fwd_kernel<N><<<g.M / TC_BM, TC_THREADS, TcShape<N>::SMEM, s>>>(ta, tw, g.K, g.bias, g.zout, g.aout,
+  if (!encode_operand(&ta, g.A, g.M, g.K, TC_BM) || !encode_operand(&tw, g.B, g.N, g.K, N)) return false;
+  gemm_tc_fwd_kernel<N><<<dim3(g.M / TC_BM, g.N / N), TC_THREADS, TcShape<N>::SMEM, s>>>(ta, tw, g.K, g.bias, g.zout, g.aout,
                                                                         g.ldc);
   tc_launch_count().fetch_add(1);
   return true;
@@ -784,8 +843,10 @@ inline bool forward_tc(const GemmArgs& g, cudaStream_t s) {
   if (forward_path().load() != TODGPU_MLP_TCGEN05 || g.K % TC_BK != 0 || g.M % TC_BM != 0 || g.lda != g.K ||
       g.ldb != g.K || g.ldc != g.N)
     return false;
-  if (g.N == 256) return launch_tc<256>(g, s);
-  if (g.N == 128) return launch_tc<128>(g, s);
+  // all 256 columns in one CTA (each row tile read once), or two CTAs of 128
+  // where the row tiles alone would leave SMs idle: 8192 rows are 64 tiles
+  if (g.N == 256 && g.M / TC_BM > 100) return launch_tc<256>(g, s);
+  if (g.N == 128 || g.N == 256) return launch_tc<128>(g, s);
   return false;
 }
 
@@ -825,14 +886,18 @@ inline void head_dispatch(const Net& n, const Ws& w, long long M, const HeadOut&
   }
 }
 
+inline void reduce_rows(const float* part, int n, long long count, float* out, cudaStream_t s) {
+  reduce_rows_kernel<<<(unsigned)((count + 31) / 32), 256, 0, s>>>(part, n, count, out);
+}
+
 template <int O>
-void head_backward(const Net& n, const Ws& w, long long M, int splits, cudaStream_t s) {
+void head_backward(const Net& n, const Ws& w, long long M, cudaStream_t s) {
   const Dims& d = n.d;
   const long long last = (long long)(d.D - 1) * M * d.H;
-  const long long rows = M / splits;
-  head_wgrad_kernel<O><<<splits, 256, 0, s>>>(w.y, w.a + last, rows, d.H, w.part);
   const long long cnt = (long long)O * d.H + O;  // head W then b, contiguous in the layout
-  reduce_splits_kernel<<<grid1d(cnt, 256), 256, 0, s>>>(w.part, splits, cnt, n.grad + n.off.w[d.D]);
+  const RowBlocks b = row_blocks(M, cnt, part_floats(d, M));
+  head_wgrad_kernel<O><<<b.n, 256, 0, s>>>(w.y, w.a + last, M, b.rows, d.H, w.part);
+  reduce_rows(w.part, b.n, cnt, n.grad + n.off.w[d.D], s);
   head_bwd_kernel<O><<<grid1d(M * d.H, 256), 256, 0, s>>>(w.y, M, d.H, n.pb + n.off.w[d.D], w.z + last, w.dz);
 }
 
@@ -849,10 +914,10 @@ inline void loss_grad(const Net& n, const Ws& w, long long M, const float* targe
   loss_mean_kernel<<<1, kThreads, 0, s>>>(w.loss, M, 1.0f / (float)(M * d.O), loss_out ? loss_out : w.loss + M);
   const int splits = splits_for(M);
   switch (d.O) {
-    case 1: head_backward<1>(n, w, M, splits, s); break;
-    case 2: head_backward<2>(n, w, M, splits, s); break;
-    case 3: head_backward<3>(n, w, M, splits, s); break;
-    default: head_backward<4>(n, w, M, splits, s); break;
+    case 1: head_backward<1>(n, w, M, s); break;
+    case 2: head_backward<2>(n, w, M, s); break;
+    case 3: head_backward<3>(n, w, M, s); break;
+    default: head_backward<4>(n, w, M, s); break;
   }
   // hidden layers, last to first; dz ping-pongs between two buffers
   for (int l = d.D - 1; l >= 0; --l) {
@@ -874,8 +939,9 @@ inline void loss_grad(const Net& n, const Ws& w, long long M, const float* targe
     gemm<1, 1, EPI_PART>(g, splits, s);
     const long long cnt = (long long)d.H * K;
     reduce_splits_kernel<<<grid1d(cnt, 256), 256, 0, s>>>(w.part, splits, cnt, n.grad + n.off.w[l]);
-    colsum_kernel<<<splits, 256, 0, s>>>(dz, M / splits, d.H, w.part);
-    reduce_splits_kernel<<<grid1d(d.H, 256), 256, 0, s>>>(w.part, splits, d.H, n.grad + n.off.b[l]);
+    const RowBlocks rb = row_blocks(M, d.H, part_floats(d, M));
+    colsum_kernel<<<rb.n, 256, 0, s>>>(dz, M, rb.rows, d.H, w.part);
+    reduce_rows(w.part, rb.n, d.H, n.grad + n.off.b[l], s);
     if (l > 0) {
       // dz_prev(m, k) = (sum_n dz(m, n) W_l(n, k)) silu'(z_{l-1}(m, k))
       GemmArgs b{};
