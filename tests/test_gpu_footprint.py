@@ -16,7 +16,7 @@ import torch
 import oracle
 from tod_generation_mapbased_beam_b200 import _native
 from tod_generation_mapbased_beam_b200.kernels import (footprint_slots, gather_accum, gather_accum_angles, pack_map,
-                                                       planar_beam)
+                                                       patch_order, planar_beam)
 
 TOD_RTOL = 1e-10
 
@@ -144,15 +144,23 @@ def test_planar_vectors_give_the_same_tod(mode, dtype):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["bilinear", "nearest"])
-def test_beam_in_chunks(mode):
+@pytest.mark.parametrize("precompute", [True, False])
+def test_beam_in_chunks(mode, precompute):
     """More than 16384 beam pixels: chunks of the beam with their own centres and
-    frames, the last one ragged."""
+    frames, the last one ragged -- as jobs of their own (precompute) or one after
+    another in one launch."""
     nside, S, B = 64, 16384 + 1029, 20
     vec, bv = _disc(S, 9.0, 13)
     ang = _pointing(B, 14, "sky")
     sky = _sky(nside, 15)
-    got = _angles(INTERP[mode], vec, bv, ang, nside, sky, 1, 2)
-    assert np.array_equal(got, _angles(INTERP[mode], vec, bv, ang, nside, sky, 1, 2, _native.FLAG_NO_TABLES))
+    outs = []
+    for flags in (0, _native.FLAG_NO_TABLES):
+        tod = torch.ones((3, B), dtype=torch.float64, device="cuda")
+        gather_accum_angles(INTERP[mode], vec, *ang, 0.0, 0.0, nside, sky, bv, tod, 1, 2, flags=flags,
+                            precompute=precompute)
+        outs.append(tod.cpu().numpy())
+    assert np.array_equal(outs[0], outs[1])
+    got = outs[0] - 1.0
     ref = _oracle(mode, vec, bv, ang, nside, sky, 1, 2)
     err = np.abs(got - ref).max(axis=0) / np.abs(ref).max()
     assert np.mean(err > TOD_RTOL) <= (0.2 if mode == "nearest" else 0.0)
@@ -181,6 +189,21 @@ def test_non_finite_beam_pixels_leave_the_others_alone(mode):
         tod = torch.zeros((3, B), dtype=torch.float64, device="cuda")
         gather_accum_angles(_native.BILINEAR, bad, *ang, 0.0, 0.0, nside, sky, bv, tod, 1, 2, err_count=err)
         assert int(err.item()) == 2 * B
+
+
+def test_patch_order_makes_compact_runs():
+    """Runs of 1024 pixels of a full disc in patch_order are patches: their radius
+    stays within twice a square patch's half diagonal, 0.71 sqrt(run's share of
+    the area); every pixel appears once."""
+    S, radius = 40000, 5.0
+    vec, _ = _disc(S, radius, 21)
+    order = patch_order(vec)
+    assert np.array_equal(np.sort(order), np.arange(S))
+    half_diagonal = math.sqrt(math.pi * math.radians(radius) ** 2 * 1024 / S / 2)
+    for a in range(0, S, 1024):
+        p = vec[order[a:a + 1024]]
+        c = p.sum(axis=0) / np.linalg.norm(p.sum(axis=0))
+        assert np.arccos(np.clip((p @ c).min(), -1, 1)) <= 2 * half_diagonal
 
 
 def _ring(n, i):

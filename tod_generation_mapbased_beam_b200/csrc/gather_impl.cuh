@@ -1715,7 +1715,8 @@ __device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOU
 // Beams of more than kBeamChunkMin pixels run in chunks of kBeamChunk consecutive
 // pixels, each with its own centre, frame, window and table: a far-sidelobe
 // beam's whole footprint holds 1e5 to 1e6 map pixels, a chunk of a beam in
-// kernels.beam_order a patch that fits shared memory.
+// kernels.beam_order a patch that fits shared memory.  (Float64 sums only: the
+// order of the float32 Kahan sums is part of their result.)
 constexpr int kBeamChunkMin = 16384;
 constexpr int kBeamChunk = 1024;
 
@@ -1748,7 +1749,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
   const long long total = (ntile - 1) * tile + min(tile, a.B - t_last * tile);
   unsigned long long nerr = 0;
   const int S = (int)a.S;
-  const int step = S > kBeamChunkMin ? kBeamChunk : S;
+  const int step = S > kBeamChunkMin && !MapTraits<MapT>::packed ? kBeamChunk : S;
   for (int s0 = 0; s0 < S; s0 += step) {
     const int s1 = min(S, s0 + step);
     double cx, cy, cz, rbeam;
@@ -2031,19 +2032,20 @@ inline Shape choose_shape(const Wants& w) {
 template <int MODE, bool HAS_QU, typename MapT>
 int wanted_slots(const KArgs& k) {
   if (k.ring_table == nullptr) return 0;
-  const int req = k.tab_req > 0 && k.S <= kBeamChunkMin
+  const bool chunked = k.S > kBeamChunkMin && !MapTraits<MapT>::packed;
+  const int req = k.tab_req > 0 && !chunked
                       ? k.tab_req
                       : (MapTraits<MapT>::packed ? 2 * kTabCapDefault : kTabCapDefault);
   if (MODE == TODGPU_BILINEAR) return req;
   // nearest reads one value per beam pixel: a table pays when the footprint
   // has fewer pixels than the beam (and only for turned Q/U values)
-  return HAS_QU && req <= std::min<long long>(k.S, k.S > kBeamChunkMin ? kBeamChunk : k.S) ? req : 0;
+  return HAS_QU && req <= (chunked ? kBeamChunk : k.S) ? req : 0;
 }
 
 // One job's part in what its launch asks for (the most any job does).
 template <int MODE, bool HAS_QU, typename MapT, int PM>
 void add_wants(Wants& w, const KArgs& k) {
-  const long long pixels = k.S > kBeamChunkMin ? kBeamChunk : k.S;
+  const long long pixels = k.S > kBeamChunkMin && !MapTraits<MapT>::packed ? kBeamChunk : k.S;
   w.window = w.window || k.ring_table != nullptr;
   w.requested = std::max(w.requested, k.tab_req);
   w.slots = std::max(w.slots, wanted_slots<MODE, HAS_QU, MapT>(k));

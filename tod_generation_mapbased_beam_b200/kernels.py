@@ -89,6 +89,38 @@ def beam_reach(vec_orig, nside):
     return r
 
 
+def patch_order(vec_orig):
+    """Order of a wide beam's pixels in which every run of ``_PIECE`` is a compact
+    patch: the plane orthogonal to the beam's mean direction is halved along its
+    longer side, at a multiple of ``_PIECE`` pixels, until a part is one run.  (Runs
+    of the Morton order, and of the Hilbert curve, jump across a beam with holes:
+    of the pieces of a 10-20 degree annulus 11% and 52% fit 3000 table slots, of
+    these 87%.)
+    For beams that run in pieces (:func:`gather_accum_angles`)."""
+    v = vec_orig.detach().cpu().numpy() if is_tensor(vec_orig) else np.asarray(vec_orig)
+    v = np.asarray(v, np.float64).reshape(-1, 3)
+    if v.shape[0] <= _PIECE:
+        return np.arange(v.shape[0], dtype=np.int64)
+    # level by level, all parts at once (on the GPU where there is one)
+    dev = "cuda" if torch.cuda.is_available() else "cpu"
+    xy = torch.from_numpy(np.stack(_tangent_plane(v))).to(dev)
+    order = torch.arange(v.shape[0], device=dev)
+    lens = [v.shape[0]]
+    while max(lens) > _PIECE:
+        size = torch.tensor(lens, device=dev)
+        part = torch.repeat_interleave(torch.arange(len(lens), device=dev), size)
+        q = xy[:, order]
+        at = part.expand(2, -1)
+        blank = torch.zeros((2, len(lens)), dtype=q.dtype, device=dev)
+        wide = (blank.scatter_reduce(1, at, q, "amax", include_self=False)
+                - blank.scatter_reduce(1, at, q, "amin", include_self=False)).argmax(dim=0)
+        by = torch.argsort(torch.where(wide[part] == 0, q[0], q[1]), stable=True)
+        order = order[by[torch.argsort(part[by], stable=True)]]
+        halves = [((n + _PIECE - 1) // _PIECE // 2 * _PIECE, n) for n in lens]
+        lens = [k for m, n in halves for k in ((m, n - m) if m > 0 else (n,))]
+    return order.cpu().numpy()
+
+
 def _beam_reach(vec_orig, nside):
     v = vec_orig.detach().cpu().numpy() if is_tensor(vec_orig) else np.asarray(vec_orig)
     v = np.asarray(v, np.float64).reshape(-1, 3)
@@ -114,6 +146,18 @@ def _spread16(a):
     return a
 
 
+def _tangent_plane(v):
+    """Coordinates of unit vectors (n, 3) in the plane orthogonal to their mean."""
+    c = v.sum(axis=0)
+    nc = np.linalg.norm(c)
+    c = c / nc if nc > 0 else np.array([0.0, 0.0, 1.0])
+    a = np.zeros(3)
+    a[int(np.argmin(np.abs(c)))] = 1.0
+    e1 = np.cross(c, a)
+    e1 /= np.linalg.norm(e1)
+    return v @ e1, v @ np.cross(c, e1)
+
+
 def beam_order(vec_orig):
     """Order of a beam's pixels that puts neighbours on the sky next to each
     other: the Morton (Z) order of their coordinates in the plane orthogonal to
@@ -127,17 +171,8 @@ def beam_order(vec_orig):
     n = v.shape[0]
     if n < 2:
         return np.arange(n, dtype=np.int64)
-    c = v.sum(axis=0)
-    nc = np.linalg.norm(c)
-    c = c / nc if nc > 0 else np.array([0.0, 0.0, 1.0])
-    a = np.zeros(3)
-    a[int(np.argmin(np.abs(c)))] = 1.0
-    e1 = np.cross(c, a)
-    e1 /= np.linalg.norm(e1)
-    e2 = np.cross(c, e1)
     code = np.zeros(n, dtype=np.int64)
-    for shift, e in ((0, e1), (1, e2)):
-        x = v @ e
+    for shift, x in enumerate(_tangent_plane(v)):
         lo, hi = x.min(), x.max()
         q = np.clip(((x - lo) / max(hi - lo, 1e-300) * 65535.0).astype(np.int64), 0, 65535)
         code |= _spread16(q) << shift
@@ -169,9 +204,10 @@ def footprint_slots(nside, reach):
     times nside; per ring 2 H + 3 slots on average for a beam disc of half-width H
     pixels, each ring taking the disc's width one ring spacing nearer its centre --
     1.02 x 3 x^2 + 13.2 x + 12 -- with 3% more and 8 to spare (4 to 10% above what
-    footprints of x = 3 to 60 fill)."""
-    x = max(0.0, float(reach) - 3.0 / float(nside)) * float(nside)
-    return int(min(1 << 20, math.ceil(1.03 * (1.02 * 3.0 * x * x + 13.2 * x + 12.0)) + 8))
+    footprints of x = 3 to 60 fill).  ``reach`` may be an array."""
+    x = np.maximum(0.0, np.asarray(reach, np.float64) - 3.0 / float(nside)) * float(nside)
+    slots = np.minimum(1 << 20, np.ceil(1.03 * (1.02 * 3.0 * x * x + 13.2 * x + 12.0)) + 8)
+    return int(slots) if slots.ndim == 0 else slots.astype(np.int64)
 
 
 def table_slots_for(table, nside):
@@ -464,9 +500,74 @@ def pointing_params(theta, phi, psi, center_phi, center_theta, out=None):
     return out
 
 
+# Beams of more pixels than this run as pieces of _PIECE consecutive pixels, each
+# a job of its own of the batched gather with its own footprint.
+_PIECE_MIN = 16384
+_PIECE = 1024
+# Largest footprint a piece gets a table for: three CTAs of 256 threads share an SM up
+# to there (284k pixels of an annulus, 301 samples: 4.72 ms; 5.06 at 3000, 5.11 at
+# 4400, 6.8 at 8192, where one CTA has the SM; pieces of 512 or 2048 pixels 5.9, 6.7).
+_PIECE_SLOTS = 2600
+
+
+def piece_footprints(vec, nside):
+    """(table slots of every piece, their largest reach) of a wide beam, a CUDA (S, 3)
+    tensor: the angle from a piece's mean direction to its farthest pixel, found on
+    the device; pieces too wide for a table ask for 2 slots.  A plan that a program
+    keeps with its beam (``gather_accum_angles(pieces=...)``)."""
+    S = vec.shape[0]
+    n = (S + _PIECE - 1) // _PIECE
+    at = torch.arange(n * _PIECE, device=vec.device).clamp_(max=S - 1)
+    p = vec[at].view(n, _PIECE, 3)
+    c = torch.nn.functional.normalize(p.sum(dim=1), dim=1)
+    low = torch.einsum("nkc,nc->nk", torch.nn.functional.normalize(p, dim=2), c).amin(dim=1)
+    r = np.arccos(np.clip(low.cpu().numpy(), -1.0, 1.0))
+    r = np.where(np.isfinite(r), r, np.pi) + 3.0 / float(nside) + 2e-5
+    slots = footprint_slots(nside, r)
+    fits = slots <= _PIECE_SLOTS
+    return np.where(fits, slots, 2).astype(np.int32), float(r[fits].max()) if fits.any() else 0.0
+
+
+def _gather_pieces(args, vec, beam, nside, tod, pieces):
+    """The gather of ``args`` (all but its beam set) over a wide beam, in pieces:
+    launches of up to 96 pieces into outputs of their own, added into ``tod`` in
+    order.  A far-sidelobe beam's footprint holds 1e5 to 1e6 map pixels, a
+    piece's a patch that fits a table in shared memory; as jobs the pieces also
+    spread over the GPU where the samples alone would not.  Pieces of like
+    footprints share a launch, whose table is sized for the largest."""
+    S = vec.shape[0]
+    slots, reach = pieces if pieces is not None else piece_footprints(vec, nside)
+    flat = vec.contiguous()  # (pieces of a planar beam are not planar beams)
+    args.flags &= ~_native.FLAG_BEAM_PLANAR
+    if not args.flags & _native.FLAG_NO_TABLES and reach > 0.0:
+        args.ring_table = ring_table(nside, reach, vec.device).data_ptr()
+    elif not args.flags & _native.FLAG_NO_TABLES:
+        args.ring_table = ring_table(nside, 3.0 / float(nside), vec.device).data_ptr()
+    C, B = tod.shape
+    most = 96
+    part = torch.empty((min(most, len(slots)), C, B), dtype=torch.float64, device=vec.device)
+    size = ctypes.sizeof(_native.GatherArgs)
+    jobs = np.tile(np.frombuffer(bytes(args), np.uint8), (len(slots), 1))
+    field = lambda name, dt: np.ndarray(len(slots), dt, jobs, getattr(_native.GatherArgs, name).offset, (size,))
+    first = np.arange(len(slots), dtype=np.int64) * _PIECE
+    field("vec_orig", np.uint64)[:] = flat.data_ptr() + first * 24
+    field("beam_vals", np.uint64)[:] = beam.data_ptr() + first * 4
+    field("S", np.int64)[:] = np.minimum(_PIECE, S - first)
+    field("tab_slots", np.int32)[:] = slots
+    jobs = np.ascontiguousarray(jobs[np.argsort(slots, kind="stable")])
+    field("tod", np.uint64)[:] = part.data_ptr() + (np.arange(len(slots)) % most) * (C * B * 8)
+    field("tod_stride", np.int64)[:] = B
+    for j0 in range(0, len(slots), most):
+        n = min(most, len(slots) - j0)
+        part[:n].zero_()
+        _native.check(_native.lib().todgpu_gather_accum_batched(
+            ctypes.cast(jobs[j0:].ctypes.data, ctypes.POINTER(_native.GatherArgs)), n, 16, stream_handle()))
+        tod += part[:n].sum(dim=0)
+
+
 def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_theta, nside,
                         mp_stacked, beam_vals, tod, c_q=-1, c_u=-1, err_count=None, flags=0,
-                        static_table=False, precompute=True):
+                        static_table=False, precompute=True, pieces=None):
     """One fused launch with the pointing given as angles: every CTA derives
     the sample's rotation on the device in float64 from (theta, phi, psi) and
     the beam centre (no float32 parameter rounding).  ``tod`` must be a float64
@@ -478,7 +579,10 @@ def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_th
     sample) and runs the gather in its float64-parameter mode: the same TOD bit
     for bit, with the per-sample rotation taken off the gather's critical path.
     ``precompute=False`` (and ``static_table=True``, which allocates nothing)
-    derive the rotation inside the gather."""
+    derive the rotation inside the gather.
+
+    ``pieces``: :func:`piece_footprints` of a beam of more than 16384 pixels, for a
+    program that keeps it (found in each call otherwise)."""
     require_cuda()
     if is_tensor(vec_orig) and vec_orig.is_cuda and vec_orig.dtype == torch.float64 and vec_orig.dim() == 2:
         given = vec_orig  # (a copy or view would be another tensor to beam_reach)
@@ -521,6 +625,9 @@ def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_th
     a.err_count = ptr(err_count)
     a.flags = int(flags) | planar
     lib = _native.lib()
+    if S > _PIECE_MIN and rot is not None and B > 0 and not (isinstance(mp, PackedMap) and mp.kind != "f64"):
+        _gather_pieces(a, given, beam, nside, tod, pieces)
+        return tod
     if static_table:
         _native.check(lib.todgpu_gather_accum_static(ctypes.byref(a), stream_handle()))
         return tod

@@ -27,7 +27,7 @@ import torch
 
 from . import _native
 from ._device import require_cuda
-from .kernels import beam_order, gather_accum_angles, pack_map
+from .kernels import _PIECE_MIN, beam_order, gather_accum_angles, pack_map, patch_order, piece_footprints
 from .tailnet import TailNet
 
 _INTERP = {"bilinear": _native.BILINEAR, "nearest": _native.NEAREST}
@@ -57,25 +57,27 @@ class LearnedTailTOD:
         if sky.shape != (3, 12 * self.nside ** 2):
             raise ValueError("sky must be a (3, 12 nside^2) I/Q/U map")
         self.sky = sky
-        self.sky_main = sky if main_map == "f64" else pack_map(sky, main_map)
+        self.sky_rec = pack_map(sky, "f64")  # the same values, a pixel's components side by side
+        self.sky_main = self.sky_rec if main_map == "f64" else pack_map(sky, main_map)
         self.main_map = main_map
         self.interp = _INTERP[interp]
         self.center = (float(center[0]), float(center[1]))
         # beam pixels in the gather's preferred order (neighbours on the sky next
         # to each other; only the order of the pixel sums changes)
-        mo, to_ = beam_order(main.vec_orig), beam_order(tail.vec_orig)
+        mo, to_ = beam_order(main.vec_orig), patch_order(tail.vec_orig)
         self.main_vec = torch.as_tensor(np.asarray(main.vec_orig, np.float64)[mo], device=self.device)
         self.main_bv = torch.as_tensor(np.asarray(main.beam_vals, np.float32)[mo], device=self.device)
         self.tail_vec = torch.as_tensor(np.asarray(tail.vec_orig, np.float64)[to_], device=self.device)
         self.tail_bv = torch.as_tensor(np.asarray(tail.beam_vals, np.float32)[to_], device=self.device)
+        self.tail_pieces = piece_footprints(self.tail_vec, self.nside) if len(to_) > _PIECE_MIN else None
         self.tail_chunk = int(tail_chunk)
         self.net = None
         self.judged = None
 
     # -- plain method --------------------------------------------------------
-    def _gather(self, vec, bv, mp, theta, phi, psi, tod):
+    def _gather(self, vec, bv, mp, theta, phi, psi, tod, pieces=None):
         gather_accum_angles(self.interp, vec, theta, phi, psi, self.center[0], self.center[1], self.nside, mp, bv,
-                            tod, c_q=1, c_u=2)
+                            tod, c_q=1, c_u=2, pieces=pieces)
 
     @staticmethod
     def _dev(a, dev):
@@ -93,7 +95,8 @@ class LearnedTailTOD:
         for b0 in range(0, B, self.tail_chunk):
             b1 = min(B, b0 + self.tail_chunk)
             part = torch.zeros((3, b1 - b0), dtype=torch.float64, device=self.device)
-            self._gather(self.tail_vec, self.tail_bv, self.sky, th[b0:b1], ph[b0:b1], ps[b0:b1], part)
+            self._gather(self.tail_vec, self.tail_bv, self.sky_rec, th[b0:b1], ph[b0:b1], ps[b0:b1], part,
+                         self.tail_pieces)
             tod[:, b0:b1] += part
         return tod
 
@@ -103,7 +106,7 @@ class LearnedTailTOD:
         th, ph, ps = (self._dev(a, self.device) for a in (theta, phi, psi))
         if tod is None:
             tod = torch.zeros((3, th.numel()), dtype=torch.float64, device=self.device)
-        self._gather(self.main_vec, self.main_bv, self.sky if exact else self.sky_main, th, ph, ps, tod)
+        self._gather(self.main_vec, self.main_bv, self.sky_rec if exact else self.sky_main, th, ph, ps, tod)
         return tod
 
     def full_plain(self, theta, phi, psi):
