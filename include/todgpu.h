@@ -234,6 +234,11 @@ int todgpu_spin2(const double *z_pix, const double *sth_pix, const double *phi_p
  * (tod_bilinear.py:308, tod_nearest.py:87). */
 int todgpu_boresight_phi_host(const float *ax_pts, int64_t B, float *out, int32_t nthreads);
 
+/* HOST function: 64-bit fingerprint of `bytes` bytes of host memory, continuing
+ * from `seed`.  Position-sensitive, and any change within one 8-byte word
+ * changes it.  No counterpart in the reference. */
+uint64_t todgpu_host_hash(const void *data, size_t bytes, uint64_t seed);
+
 /* Ring table: per-ring data of the RING scheme for one nside (ring z, acos z,
  * layout) and, for footprints of angular radius up to `reach` (radians), the
  * spin-2 table slots each ring needs.  todgpu_gather_accum reads it through

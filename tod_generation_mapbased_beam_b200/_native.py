@@ -127,6 +127,8 @@ def _declare(lib):
     lib.todgpu_spin2.restype = ctypes.c_int
     lib.todgpu_boresight_phi_host.argtypes = [_p, _i64, _p, _i32]
     lib.todgpu_boresight_phi_host.restype = ctypes.c_int
+    lib.todgpu_host_hash.argtypes = [_p, ctypes.c_size_t, ctypes.c_uint64]
+    lib.todgpu_host_hash.restype = ctypes.c_uint64
     lib.todgpu_ring_table_bytes.argtypes = [_i64]
     lib.todgpu_ring_table_bytes.restype = ctypes.c_size_t
     lib.todgpu_ring_table_build.argtypes = [_i64, ctypes.c_double, _p, ctypes.c_size_t, _p]
@@ -229,7 +231,7 @@ def exported_symbols():
         "todgpu_ang2pix",
         "todgpu_pix2ang",
         "todgpu_spin2",
-        "todgpu_boresight_phi_host",
+        "todgpu_boresight_phi_host", "todgpu_host_hash",
         "todgpu_ring_table_bytes",
         "todgpu_ring_table_build",
         "todgpu_pack_map",

@@ -597,7 +597,8 @@ extern "C" int todgpu_boresight_phi_host(const float* ax_pts, int64_t B, float* 
   if (!ax_pts || !out) return fail(TODGPU_EINVAL, "NULL pointer");
   unsigned hw = std::thread::hardware_concurrency();
   int nt = nthreads > 0 ? nthreads : (int)std::max(1u, hw);
-  if (B < 65536) nt = 1;
+  // a thread costs some 20 us to start and 8192 values 90 us to compute
+  nt = (int)std::max<int64_t>(1, std::min<int64_t>(nt, B / 8192));
   auto work = [&](int64_t lo, int64_t hi) {
     for (int64_t b = lo; b < hi; ++b) out[b] = atan2f(ax_pts[3 * b + 1], ax_pts[3 * b]);
   };
@@ -613,6 +614,41 @@ extern "C" int todgpu_boresight_phi_host(const float* ax_pts, int64_t B, float* 
   }
   for (auto& th : pool) th.join();
   return TODGPU_OK;
+}
+
+// Fingerprint of host memory: eight 64-bit lanes take the words in turn, each
+// lane h <- rotl((h ^ word) K, 27) with K odd -- a bijection of h for every
+// word and of the word for every h, so a change of any one word changes its
+// lane -- and the lanes, the length and the tail bytes are folded in the same
+// way.  Eight independent multiply chains read memory at its own speed (some
+// 15 GB/s a core; zlib's CRC-32 5).
+extern "C" uint64_t todgpu_host_hash(const void* data, size_t bytes, uint64_t seed) {
+  constexpr uint64_t K = 0x9f3ac1d4b27e5865ull;
+  auto mix = [](uint64_t h, uint64_t w) {
+    const uint64_t x = (h ^ w) * K;
+    return (x << 27) | (x >> 37);
+  };
+  const unsigned char* p = static_cast<const unsigned char*>(data);
+  uint64_t h[8];
+  for (int i = 0; i < 8; ++i) h[i] = mix(seed + 0x5851f42d4c957f2dull * (uint64_t)(i + 1), (uint64_t)bytes);
+  size_t left = data != nullptr ? bytes : 0;
+  for (; left >= 64; left -= 64, p += 64) {
+    uint64_t w[8];
+    std::memcpy(w, p, 64);
+#pragma GCC unroll 8
+    for (int i = 0; i < 8; ++i) h[i] = mix(h[i], w[i]);
+  }
+  for (int i = 0; left > 0; ++i) {
+    const size_t n = std::min<size_t>(8, left);
+    uint64_t w = 0;
+    std::memcpy(&w, p, n);
+    h[i] = mix(h[i], w);
+    left -= n;
+    p += n;
+  }
+  uint64_t r = seed;
+  for (int i = 0; i < 8; ++i) r = mix(mix(r, h[i]), h[i] >> 32);
+  return r;
 }
 
 extern "C" size_t todgpu_ring_table_bytes(int64_t nside) {

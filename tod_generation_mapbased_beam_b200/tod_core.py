@@ -13,7 +13,7 @@ accumulator (tod_core.py:128) and the float32 cast of the result
 Differences, all additive:
 * map, beam vectors and weights may be torch CUDA tensors (zero copy); numpy
   inputs are uploaded once per array object and cached on the device, and
-  re-uploaded when their contents change (every call checks a CRC-32 of the
+  re-uploaded when their contents change (every call checks a fingerprint of the
   host bytes, so a buffer refilled in place is read again, as the reference
   reads its inputs on every call);
 * without ``data["mp_stacked"]`` the ``mp`` component list is stacked and
@@ -33,43 +33,41 @@ from __future__ import annotations
 
 import os
 import weakref
-import zlib
 
 import numpy as np
 import torch
 
 from . import _native
 from ._device import is_tensor, require_cuda
-from .kernels import (beam_center_angles, beam_order, boresight_phi_host, gather_accum, gather_accum_angles,
-                      pack_map)
+from .kernels import (_PIECE_MIN, beam_center_angles, beam_order, boresight_phi_host, gather_accum,
+                      gather_accum_angles, pack_map, patch_order)
 from .tod_rotations import _rotation_params, precompute_rotation_vector_batch  # noqa: F401
 
 _INTERP = {"bilinear": _native.BILINEAR, "nearest": _native.NEAREST}
 
 
-# Host arrays of a few MiB or more are fingerprinted in chunks of this many
-# bytes on the preparation thread pool.
-_FP_CHUNK = 1 << 23
+# Host arrays of more than this many bytes are fingerprinted in chunks on the
+# preparation thread pool.
+_FP_CHUNK = 1 << 20
 
 
 def _fingerprint(arr):
-    """CRC-32 of every byte of a host array (chunk by chunk, in parallel for
-    large arrays; zlib releases the GIL).  Position-sensitive, so a refill of
-    the same buffer with other or permuted values changes it."""
+    """64-bit fingerprint of every byte of a host array (``todgpu_host_hash``;
+    chunk by chunk, in parallel for large arrays: the call releases the GIL).
+    Position-sensitive, so a refill of the same buffer with other or permuted
+    values changes it."""
     a = np.ascontiguousarray(arr)
-    mv = memoryview(a.reshape(-1)).cast("B")
-    n = mv.nbytes
+    fn, p, n = _native.lib().todgpu_host_hash, a.ctypes.data, a.nbytes
     if n <= _FP_CHUNK:
-        return (a.dtype.str, a.shape, zlib.crc32(mv))
-    bounds = [(i, min(n, i + _FP_CHUNK)) for i in range(0, n, _FP_CHUNK)]
-    crcs = tuple(_pool().map(lambda b: zlib.crc32(mv[b[0]:b[1]]), bounds))
-    return (a.dtype.str, a.shape, crcs)
+        return (a.dtype.str, a.shape, fn(p, n, 0))
+    hashes = tuple(_pool().map(lambda i: fn(p + i, min(n - i, _FP_CHUNK), i), range(0, n, _FP_CHUNK)))
+    return (a.dtype.str, a.shape, hashes)
 
 
 class _UploadCache:
     """Device copies of host arrays, keyed by array identity and dropped when
     the host array is garbage-collected.  Every call checks the host array's
-    content (CRC-32 of all its bytes, see :func:`_fingerprint`) and uploads it
+    content (a fingerprint of all its bytes, see :func:`_fingerprint`) and uploads it
     again if it changed: the reference reads its inputs on every call
     (tod_core.py:121-160), so a caller that refills the same buffer in place
     gets the new values.  ``CHECK_CONTENT = False`` trusts identity alone
@@ -150,7 +148,8 @@ def device_beam(vec_orig, beam_vals, vec_dtype=torch.float64):
 
     def make():
         v = vec.reshape(-1, 3)
-        idx = torch.from_numpy(beam_order(v)).to(v.device)
+        # (a beam wide enough to run in pieces: in an order whose runs are patches)
+        idx = torch.from_numpy((patch_order if v.shape[0] > _PIECE_MIN else beam_order)(v)).to(v.device)
         # (S, 3) views of planar (3, S) vectors: neighbouring threads read
         # neighbouring elements
         return v[idx].t().contiguous().t(), bv.reshape(-1)[idx].contiguous()
@@ -231,6 +230,16 @@ def _prep_chunk(rot_vecs, phi_b, theta_b, psis_b, s0, s1, with_bore):
     return out
 
 
+def _param_views(buf, n):
+    """The fields of n samples in a buffer laid out by :func:`_prep_chunk`."""
+    views, o = [], 0
+    for w in _PIPE_WIDTHS:
+        v = buf[o:o + w * n]
+        views.append(v.view(n, 3) if w == 3 else v)
+        o += w * n
+    return views
+
+
 def _gather_pipelined(interp, nside, rot_vecs, phi_b, theta_b, psis_b, vec, bv, mpd, tod, S, c_q, c_u):
     """beam_tod_batch's gather in chunks of PIPE_CHUNK samples: parameters
     prepared on the thread pool, uploaded through two pinned staging slots on
@@ -270,11 +279,7 @@ def _gather_pipelined(interp, nside, rot_vecs, phi_b, theta_b, psis_b, vec, bv, 
                 uploaded[k] = torch.cuda.Event()
                 uploaded[k].record(up)
             comp.wait_event(uploaded[k])
-            views, o = [], 0
-            for w in _PIPE_WIDTHS:
-                v = dbuf[k][o:o + w * n]
-                views.append(v.view(n, 3) if w == 3 else v)
-                o += w * n
+            views = _param_views(dbuf[k], n)
             gather_accum(interp, vec, *views[:6], nside, mpd, bv, n, S, tod[:, s0:s1], c_q, c_u,
                          bore_phi=views[6])
             consumed[k] = torch.cuda.Event()
@@ -312,6 +317,12 @@ def beam_tod_batch(nside, mp, data, rot_vecs, phi_b, theta_b, psis_b, interp_mod
     if host_inputs and B > PIPE_CHUNK and S > 0:
         _gather_pipelined(_INTERP[interp_mode], nside, np.asarray(rot_vecs), np.asarray(phi_b),
                           np.asarray(theta_b), np.asarray(psis_b), vec, bv, mpd, tod, S, c_q, c_u)
+    elif host_inputs and B > 0 and S > 0:
+        # the parameters in one buffer and one copy (the pipeline's layout)
+        host = _prep_chunk(np.asarray(rot_vecs), np.asarray(phi_b), np.asarray(theta_b), np.asarray(psis_b), 0, B,
+                           c_q >= 0 and c_u >= 0)
+        views = _param_views(torch.from_numpy(host).to(mpd.device), B)
+        gather_accum(_INTERP[interp_mode], vec, *views[:6], nside, mpd, bv, B, S, tod, c_q, c_u, bore_phi=views[6])
     else:
         params = _rotation_params(rot_vecs, phi_b, theta_b, psis_b)
         bore_phi = boresight_phi_host(params[3]) if (c_q >= 0 and c_u >= 0) else None
