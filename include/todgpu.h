@@ -319,13 +319,13 @@ typedef struct todgpu_mlp {
  * and 256) or TODGPU_MLP_MMA_SYNC (warp-level tensor-core instructions; any
  * width, and the path the backward products always take).  Process-wide;
  * returns the previous setting.  todgpu_mlp_wait_timeouts: number of bounded
- * waits in the tcgen05 kernel that ran out since load (0 in a healthy run;
+ * waits in the tcgen05 kernels that ran out since load (0 in a healthy run;
  * reading it synchronises the device), -1 on a CUDA error. */
 #define TODGPU_MLP_TCGEN05 0
 #define TODGPU_MLP_MMA_SYNC 1
 int todgpu_mlp_set_forward_path(int32_t path);
 int64_t todgpu_mlp_wait_timeouts(void);
-/* Number of forward layers launched on the tcgen05 path since load (a layer
+/* Number of forward layers evaluated by launches on the tcgen05 path since load (a layer
  * whose shape or tensor maps do not suit it runs on mma.sync instead). */
 int64_t todgpu_mlp_tcgen05_launches(void);
 
@@ -363,8 +363,10 @@ int todgpu_mlp_train(const todgpu_mlp *net, const float *x, const float *target,
                      int64_t first_step, int64_t n_steps, int64_t total_steps, float lr_max, float lr_min, void *ws,
                      size_t ws_bytes, float *loss_per_step, void *stream);
 /* tod[rows[o] * tod_stride + b] += y_o(theta_b, phi_b, psi_b) scale[o] + shift[o]
- * for b < B, evaluated in chunks of `chunk` samples (rows, scale, shift: host
- * arrays of n_out entries). */
+ * for b < B (rows, scale, shift: host arrays of n_out entries): in one kernel
+ * on the tcgen05 path (n_freq <= 256, width 128 or 256), which keeps a copy of
+ * the weights in the workspace while it runs, else in chunks of `chunk`
+ * samples layer by layer; the results are the same. */
 int todgpu_tail_accumulate(const todgpu_mlp *net, const void *theta, const void *phi, const void *psi,
                            int32_t angles_dtype, int64_t B, const int32_t *rows, const double *scale,
                            const double *shift, double *tod, int64_t tod_stride, int64_t chunk, void *ws,

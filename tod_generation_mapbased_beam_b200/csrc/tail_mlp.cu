@@ -14,8 +14,9 @@
 // contraction accumulates in float32: the hidden layers on the tensor cores --
 // forward products on tcgen05 with TMEM accumulators and TMA-staged operands
 // (widths 128 and 256), backward products and other widths on mma.sync
-// m16n8k16 bf16 -> f32 -- the O <= 4 wide head on the CUDA cores.  Pre-activations are kept in float32 for
-// the backward pass.  Weight gradients over the batch use a fixed split of
+// m16n8k16 bf16 -> f32 -- the O <= 4 wide head on the CUDA cores.  Inference into
+// the TOD runs the whole network in one tcgen05 kernel.  Pre-activations are
+// kept in float32 for the backward pass.  Weight gradients over the batch use a fixed split of
 // the batch and a fixed-order reduction, so training is deterministic.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -111,6 +112,28 @@ inline void ws_offsets(const Dims& d, long long M, long long* off) {
 // ---------------------------------------------------------------------------
 // inputs and Fourier features
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void input_row(double theta, double phi, double psi, float* o) {
+  double st, ct, sp, cp, ss, cs;
+  sincos(theta, &st, &ct);
+  sincos(phi, &sp, &cp);
+  sincos(psi, &ss, &cs);
+  o[0] = (float)(st * cp);
+  o[1] = (float)(st * sp);
+  o[2] = (float)ct;
+  o[3] = (float)cs;
+  o[4] = (float)ss;
+  o[5] = (float)(cs * cs - ss * ss);
+  o[6] = (float)(2.0 * ss * cs);
+}
+
+// (sin, cos)(2 pi b . x), b one frequency.
+__device__ __forceinline__ void feature(const float* b, const float* x, float& s, float& c) {
+  float z = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kIn; ++k) z += b[k] * x[k];
+  sincospif(2.0f * z, &s, &c);
+}
+
 template <typename T>
 __global__ void inputs_kernel(const T* theta, const T* phi, const T* psi, long long n, long long M, float* x) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M; i += (long long)gridDim.x * blockDim.x) {
@@ -119,17 +142,7 @@ __global__ void inputs_kernel(const T* theta, const T* phi, const T* psi, long l
       for (int k = 0; k < kIn; ++k) o[k] = 0.0f;
       continue;
     }
-    double st, ct, sp, cp, ss, cs;
-    sincos((double)theta[i], &st, &ct);
-    sincos((double)phi[i], &sp, &cp);
-    sincos((double)psi[i], &ss, &cs);
-    o[0] = (float)(st * cp);
-    o[1] = (float)(st * sp);
-    o[2] = (float)ct;
-    o[3] = (float)cs;
-    o[4] = (float)ss;
-    o[5] = (float)(cs * cs - ss * ss);
-    o[6] = (float)(2.0 * ss * cs);
+    input_row((double)theta[i], (double)phi[i], (double)psi[i], o);
   }
 }
 
@@ -139,12 +152,8 @@ __global__ void features_kernel(const float* x, long long M, const float* freq, 
        t += (long long)gridDim.x * blockDim.x) {
     const long long m = t / F;
     const int j = (int)(t - m * F);
-    const float* xm = x + m * kIn;
-    const float* bj = freq + (long long)j * kIn;
-    float z = 0.0f;
-    for (int k = 0; k < kIn; ++k) z += bj[k] * xm[k];
     float s, c;
-    sincospif(2.0f * z, &s, &c);  // (sin, cos)(2 pi z)
+    feature(freq + (long long)j * kIn, x + m * kIn, s, c);
     feat[m * 2 * F + j] = __float2bfloat16(c);
     feat[m * 2 * F + F + j] = __float2bfloat16(s);
   }
@@ -175,6 +184,38 @@ struct GemmArgs {
 };
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
+
+// silu_f of eight values.  A division's own special cases put a branch between
+// every two of them, which kept the eight chains apart (34 instructions a value);
+// the denominator here is 1 + e^-v, so one test per eight values does: for
+// -60 < v < 1e30 the quotient by Markstein's method (reciprocal estimate, one
+// Newton step, one remainder correction in fma arithmetic), which is the rounded
+// quotient -- silu_f's float for every float v in the range, counted over all of
+// them, but for the sign of -0 -- and silu_f itself otherwise (infinities, NaN).
+__device__ __forceinline__ void silu8(const float* v, float* y) {
+  float lo = v[0], hi = v[0];
+  bool num = v[0] == v[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    lo = fminf(lo, v[i]);
+    hi = fmaxf(hi, v[i]);
+    num = num && v[i] == v[i];
+  }
+  if (num && lo > -60.0f && hi < 1e30f) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float d = 1.0f + expf(-v[i]);
+      float r;
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+      r = fmaf(r, fmaf(-d, r, 1.0f), r);
+      const float q = v[i] * r;
+      y[i] = fmaf(fmaf(-d, q, v[i]), r, q);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) y[i] = silu_f(v[i]);
+  }
+}
 __device__ __forceinline__ float dsilu_f(float z) {
   const float s = 1.0f / (1.0f + expf(-z));
   return s * (1.0f + z * (1.0f - s));
@@ -723,13 +764,334 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_fwd_kernel(const __grid_co
       uint4* ap = reinterpret_cast<uint4*>(aout + row * ldc + n0 + c0);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
+        float y[8];
+        silu8(v + 8 * j, y);
         __nv_bfloat162 h[4];
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
-          h[t] = __floats2bfloat162_rn(silu_f(v[8 * j + 2 * t]), silu_f(v[8 * j + 2 * t + 1]));
+        for (int t = 0; t < 4; ++t) h[t] = __floats2bfloat162_rn(y[2 * t], y[2 * t + 1]);
         ap[j] = *reinterpret_cast<const uint4*>(h);
       }
     }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(N));
+}
+
+// ---------------------------------------------------------------------------
+// The whole network for inference in one kernel: tod[rows[o], b] += y_o(pointing
+// b) scale[o] + shift[o].
+//
+// Layer by layer (the path above, kept for training and for shapes this one does
+// not take) a row's 512 features and 4 x 256 activations went through HBM six
+// times and every layer was a wave of short CTAs: 500,009 samples took 2.25 ms,
+// 15% of them in tensor-core work.  Here a persistent CTA (two per SM) takes 128
+// samples through all layers with the activations in shared memory: its 256
+// threads compute inputs and features (two threads a sample) into operand tiles,
+// one thread issues the tcgen05 products into TMEM as tiles become ready, and all
+// read the sums back, add the bias, apply SiLU and store the next layer's operand.
+// The weights stream from L2 through a ring of four 16-deep k-tiles by bulk copies
+// of 32 N bytes each, from a copy in operand order that pack_weights_kernel lays
+// down in the workspace in each call (2 us; tensor-map copies out of the row-major
+// weights move 16 bytes a row and held the products up: 1.34 ms).  What
+// is left is the arithmetic of 256 sine/cosine pairs and 1024 SiLUs a sample:
+// 43,000 instructions, 59% of the issue slots; 500,009 samples (256 frequencies,
+// 4 x 256, 3 outputs) take 1.08 ms, 85% of them outside the tensor cores.
+// Every product, sum and rounding is the layered path's, in its order, so the
+// TOD is the same bit for bit.
+//
+// Shared memory: `act` holds the sine features of layer 0 and then each layer's
+// input (K columns x 2 KB: 8-row x 16-byte core matrices, K chunks of 8 columns
+// 2 KB apart), `cosr` two 32-column tiles of cosine features, `wr` the weight ring.
+// Every wait is bounded; when one runs out the CTA stops (its remaining samples
+// are not added), waits for its copies in flight and frees its TMEM, and the
+// time-out is counted.
+// ---------------------------------------------------------------------------
+constexpr int FU_WSTAGES = 4;
+struct FusedArgs {
+  const void *theta, *phi, *psi;
+  long long B;
+  const float* freq;
+  const unsigned char* w;  // the hidden layers' k-tiles, one after the other
+  const float* bias[kMaxDepth];
+  const bf16* head_w;
+  const float* head_b;
+  int F, D;
+  HeadOut h;
+};
+
+__device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+      "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// Row-major (N, K) weights of each hidden layer to k-tiles of (2, N, 8): tile k / 16,
+// column chunk (k / 8) % 2, row, column k % 8.  One thread copies 8 columns of a row.
+struct PackArgs {
+  const bf16* w[kMaxDepth];
+  uint4* out;
+  int N, K0, D;
+};
+__global__ void pack_weights_kernel(const __grid_constant__ PackArgs a) {
+  const int c0 = a.K0 / 8, ch = a.N / 8;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;  // (chunk of 8 columns, row), rows fastest
+  if (t >= (c0 + (a.D - 1) * ch) * a.N) return;
+  const int row = t % a.N;
+  int c = t / a.N, l = 0, K = a.K0;
+  if (c >= c0) {
+    l = 1 + (c - c0) / ch;
+    c = (c - c0) % ch;
+    K = a.N;
+  }
+  a.out[t] = *reinterpret_cast<const uint4*>(a.w[l] + (long long)row * K + c * 8);
+}
+
+template <int N>
+constexpr int fused_smem(int F) {
+  return (F > N ? F : N) * 256 + 2 * 8192 + FU_WSTAGES * N * 32;
+}
+
+template <int N, int O, typename T>
+__global__ void __launch_bounds__(256, 2) tail_fused_kernel(const __grid_constant__ FusedArgs f) {
+  constexpr int kWBytes = N * 32;            // one k-tile of weights: N rows x 16 bf16
+  constexpr uint32_t kALbo = 2048, kWLbo = (N / 8) * 128;
+  constexpr uint32_t kIdesc = TcShape<N>::IDESC;
+  extern __shared__ __align__(128) unsigned char fu_smem[];
+  __shared__ __align__(8) unsigned long long bars[2 * FU_WSTAGES + 3];  // wfull, wempty, cos empty[2], done
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const uint32_t act = (uint32_t)__cvta_generic_to_shared(fu_smem);
+  const uint32_t cosr = act + (uint32_t)(f.F > N ? f.F : N) * 256u, wr = cosr + 2 * 8192;
+  const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
+  const uint32_t wfull = bar0, wempty = bar0 + 8 * FU_WSTAGES, cempty = bar0 + 16 * FU_WSTAGES, done = cempty + 16;
+  if (tid == 0) {
+    for (int i = 0; i < 2 * FU_WSTAGES + 3; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(&tmem_slot)),
+                 "r"(N));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+
+  const long long tiles = (f.B + 127) / 128;
+  const int k0_tiles = f.F / 8, kh_tiles = N / 16;  // 16-deep k-tiles of layer 0 and of the others
+  const int per_tile = k0_tiles + (f.D - 1) * kh_tiles;
+  const long long mine = (long long)blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+  const int w_total = (int)(mine * per_tile);
+
+  // thread 0: weight k-tiles started (p, the network's tile pk next) and used (g)
+  int p = 0, pk = 0, g = 0;
+  auto produce = [&]() {
+    const uint32_t st = (uint32_t)(p & (FU_WSTAGES - 1));
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;" ::"r"((uint32_t)kWBytes), "r"(wfull + 8 * st)
+                 : "memory");
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+            wr + st * kWBytes),
+        "l"(f.w + (long long)pk * kWBytes), "r"((uint32_t)kWBytes), "r"(wfull + 8 * st)
+        : "memory");
+    ++p;
+    if (++pk == per_tile) pk = 0;
+  };
+  // the next k-tile's product with the operand columns at a_addr; false: time-out
+  auto multiply = [&](uint32_t a_addr, bool first) -> bool {
+    const uint32_t st = (uint32_t)(g & (FU_WSTAGES - 1));
+    if (!tc_wait(wfull + 8 * st, (uint32_t)((g / FU_WSTAGES) & 1))) return false;
+    ++g;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tc_mma(tmem, tc_desc(a_addr, kALbo, 128), tc_desc(wr + st * kWBytes, kWLbo, 128), kIdesc, first ? 0u : 1u);
+    tc_commit(wempty + 8 * st);
+    // refill the previous k-tile's stage once its product is done
+    if (g >= 2 && p < w_total) {
+      const int u = g - 2;
+      if (!tc_wait(wempty + 8 * (u & (FU_WSTAGES - 1)), (uint32_t)((u / FU_WSTAGES) & 1))) return false;
+      produce();
+    }
+    return true;
+  };
+  if (tid == 0)
+    while (p < FU_WSTAGES && p < w_total) produce();
+
+  const int row = tid & 127, half = tid >> 7;  // features: two threads a sample
+  const uint32_t row_off = (uint32_t)(row >> 3) * 128u + (uint32_t)(row & 7) * 16u;
+  int cc = 0, lc = 0;  // cosine tiles and layers so far
+  bool bad = false, ok = true;  // this thread's waits; the CTA's, as of its last barrier
+  for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+    const long long b = t * 128 + row;
+    float x[kIn] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (b < f.B)
+      input_row((double)static_cast<const T*>(f.theta)[b], (double)static_cast<const T*>(f.phi)[b],
+                (double)static_cast<const T*>(f.psi)[b], x);
+    // layer 0: cosine tiles as they are made, then the sine tiles
+    float4 fn[kIn];
+#pragma unroll
+    for (int i = 0; i < kIn; ++i) fn[i] = __ldg(reinterpret_cast<const float4*>(f.freq + half * 16 * kIn) + i);
+    for (int kt = 0; kt < f.F / 32; ++kt, ++cc) {
+      const uint32_t st = (uint32_t)(cc & 1);
+      if (cc >= 2 && !tc_wait(cempty + 8 * st, (uint32_t)((cc / 2 - 1) & 1))) bad = true;
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q) {
+        __nv_bfloat162 cv[4], sv[4];
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {  // four frequencies (28 floats), the next four on their way
+          float4 b4[kIn];
+#pragma unroll
+          for (int i = 0; i < kIn; ++i) b4[i] = fn[i];
+          const int k = kt * 32 + half * 16 + q * 8 + 2 * j;
+          const int kn = q == 1 && j == 2 ? (kt + 1 < f.F / 32 ? k + 20 : half * 16) : k + 4;
+          const float4* fr = reinterpret_cast<const float4*>(f.freq + kn * kIn);
+#pragma unroll
+          for (int i = 0; i < kIn; ++i) fn[i] = __ldg(fr + i);
+          const float* bq = reinterpret_cast<const float*>(b4);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            float s0, c0, s1, c1;
+            feature(bq + 2 * i * kIn, x, s0, c0);
+            feature(bq + (2 * i + 1) * kIn, x, s1, c1);
+            cv[j + i] = __floats2bfloat162_rn(c0, c1);
+            sv[j + i] = __floats2bfloat162_rn(s0, s1);
+          }
+        }
+        const uint32_t chunk = (uint32_t)(half * 2 + q) * kALbo + row_off;
+        const uint4 cq = *reinterpret_cast<const uint4*>(cv), sq = *reinterpret_cast<const uint4*>(sv);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cosr + st * 8192u + chunk), "r"(cq.x), "r"(cq.y),
+                     "r"(cq.z), "r"(cq.w)
+                     : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(act + (uint32_t)kt * 4u * kALbo + chunk),
+                     "r"(sq.x), "r"(sq.y), "r"(sq.z), "r"(sq.w)
+                     : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+      if (tid == 0 && !bad) {
+        const uint32_t a = cosr + st * 8192u;
+        if (multiply(a, kt == 0) && multiply(a + 2 * kALbo, false))
+          tc_commit(cempty + 8 * st);
+        else
+          bad = true;
+      }
+    }
+    for (int l = 0; l < f.D; ++l, ++lc) {
+      if (tid == 0 && !bad) {
+        const int n = l == 0 ? k0_tiles / 2 : kh_tiles;
+        bool good = true;
+        for (int k = 0; k < n && good; ++k) good = multiply(act + (uint32_t)k * 2u * kALbo, l > 0 && k == 0);
+        if (good)
+          tc_commit(done);
+        else
+          bad = true;
+      }
+      __syncwarp();
+      if (!tc_wait(done, (uint32_t)(lc & 1))) bad = true;
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int q = warp & 3, r = q * 32 + (tid & 31);  // this thread's row of the sums
+      const uint32_t r_off = (uint32_t)(r >> 3) * 128u + (uint32_t)(r & 7) * 16u;
+      const bool last = l == f.D - 1;
+      const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
+      const int c_end = ((warp >> 2) + 1) * (N / 2);
+      // sums and biases of 16 columns, loaded one step ahead of their use
+      uint32_t vn[16];
+      float4 bn[4];
+      auto fetch = [&](int c) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15}, [%16];"
+            : "=r"(vn[0]), "=r"(vn[1]), "=r"(vn[2]), "=r"(vn[3]), "=r"(vn[4]), "=r"(vn[5]), "=r"(vn[6]),
+              "=r"(vn[7]), "=r"(vn[8]), "=r"(vn[9]), "=r"(vn[10]), "=r"(vn[11]), "=r"(vn[12]), "=r"(vn[13]),
+              "=r"(vn[14]), "=r"(vn[15])
+            : "r"(tq + (uint32_t)c));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bn[i] = __ldg(reinterpret_cast<const float4*>(f.bias[l] + c) + i);
+      };
+      fetch((warp >> 2) * (N / 2));
+#pragma unroll 1
+      for (int c0 = (warp >> 2) * (N / 2); c0 < c_end; c0 += 16) {
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[4 * i] = __uint_as_float(vn[4 * i]) + bn[i].x;
+          v[4 * i + 1] = __uint_as_float(vn[4 * i + 1]) + bn[i].y;
+          v[4 * i + 2] = __uint_as_float(vn[4 * i + 2]) + bn[i].z;
+          v[4 * i + 3] = __uint_as_float(vn[4 * i + 3]) + bn[i].w;
+        }
+        if (c0 + 16 < c_end) fetch(c0 + 16);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {  // eight columns at a time
+          const int c = c0 + 8 * j;
+          uint4 wv[O];
+          if (last)
+#pragma unroll
+            for (int o = 0; o < O; ++o)
+              wv[o] = __ldg(reinterpret_cast<const uint4*>(f.head_w + (long long)o * N + c));
+          float y[8];
+          silu8(v + 8 * j, y);
+          __nv_bfloat162 hv[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) hv[i] = __floats2bfloat162_rn(y[2 * i], y[2 * i + 1]);
+          if (!last) {
+            const uint4 a4 = *reinterpret_cast<const uint4*>(hv);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(act + (uint32_t)(c / 8) * kALbo + r_off),
+                         "r"(a4.x), "r"(a4.y), "r"(a4.z), "r"(a4.w)
+                         : "memory");
+          } else {
+            // head_kernel's partial sum of eight columns, per output
+            const bf16* a8 = reinterpret_cast<const bf16*>(hv);
+#pragma unroll
+            for (int o = 0; o < O; ++o) {
+              const bf16* w8 = reinterpret_cast<const bf16*>(&wv[o]);
+              float sum = 0.0f;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) sum += __bfloat162float(a8[i]) * __bfloat162float(w8[i]);
+              asm volatile("st.shared.f32 [%0], %1;" ::"r"(act + (uint32_t)((o * (N / 8) + c / 8) * 128 + r) * 4u),
+                           "f"(sum)
+                           : "memory");
+            }
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      ok = __syncthreads_or(bad) == 0;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!ok) break;
+    }
+    if (!ok) break;
+    // the partial sums in head_kernel's butterfly order, then the TOD
+    const long long m = t * 128 + tid;
+    if (tid < 128 && m < f.B) {
+#pragma unroll 1
+      for (int o = 0; o < O; ++o) {
+        const float* part = reinterpret_cast<const float*>(fu_smem) + o * (N / 8) * 128 + tid;
+        float s[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s[i] = N == 256 ? part[i * 128] + part[(i + (N / 16)) * 128] : part[i * 128];
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1)
+#pragma unroll
+          for (int i = 0; i < d; ++i) s[i] += s[i + d];
+        const float y = s[0] + f.head_b[o];
+        f.h.tod[f.h.rows[o] * f.h.tod_stride + m] += (double)y * f.h.scale[o] + f.h.shift[o];
+      }
+    }
+    __syncthreads();  // the sums are read: act may be overwritten
+  }
+  if (tid == 0 && !ok) {
+    atomicAdd(&g_tc_timeouts, 1u);
+    for (; g < p; ++g) tc_wait(wfull + 8 * (g & (FU_WSTAGES - 1)), (uint32_t)((g / FU_WSTAGES) & 1));
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -848,6 +1210,82 @@ inline bool forward_tc(const GemmArgs& g, cudaStream_t s) {
   if (g.N == 256 && g.M / TC_BM > 100) return launch_tc<256>(g, s);
   if (g.N == 128 || g.N == 256) return launch_tc<128>(g, s);
   return false;
+}
+
+template <int N, int O, typename T>
+bool launch_fused(const FusedArgs& f, const PackArgs& k, cudaStream_t s) {
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(tail_fused_kernel<N, O, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                fused_smem<N>(256));
+  });
+  if (attr != cudaSuccess) return false;
+  const long long tiles = (f.B + 127) / 128;
+  const int copies = (k.K0 + (k.D - 1) * N) / 8 * N;
+  pack_weights_kernel<<<(copies + 255) / 256, 256, 0, s>>>(k);
+  tail_fused_kernel<N, O, T><<<(unsigned)std::min(tiles, 2LL * sm_count()), 256, fused_smem<N>(f.F), s>>>(f);
+  tc_launch_count().fetch_add(f.D);
+  return true;
+}
+
+// The whole network on the fused path: tcgen05 selected, widths 128 and 256, up to
+// 256 frequencies (the operand of layer 0 and two CTAs must fit an SM), and
+// tiles few enough for 32-bit k-tile counters.  No lower limit on B: fused against
+// layer by layer, 1 sample 67 against 96 us, 8192 69 against 114, 38,000 141
+// against 271, 100,000 250 against 530 (4 x 256; 2 x 128: 24 against 34, 25
+// against 40, 44 against 71, 73 against 150).  false: not launched.
+template <typename T>
+bool tail_fused(const Net& n, const T* theta, const T* phi, const T* psi, long long B, const HeadOut& h,
+                void* ws, cudaStream_t s) {
+  const Dims& d = n.d;
+  if (forward_path().load() != TODGPU_MLP_TCGEN05 || B <= 0 || B > (1LL << 28) || (d.H != 128 && d.H != 256) ||
+      d.F % 32 != 0 || d.F > 256)
+    return false;
+  FusedArgs f{};
+  PackArgs k{};
+  f.theta = theta;
+  f.phi = phi;
+  f.psi = psi;
+  f.B = B;
+  f.freq = n.freq;
+  f.head_w = n.pb + n.off.w[d.D];
+  f.head_b = n.p + n.off.b[d.D];
+  f.F = d.F;
+  f.D = d.D;
+  f.h = h;
+  // 16-byte reads of frequencies, weights and biases
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (!aligned(f.head_w) || !aligned(f.freq) || !aligned(ws)) return false;
+  for (int l = 0; l < d.D; ++l) {
+    f.bias[l] = n.p + n.off.b[l];
+    k.w[l] = n.pb + n.off.w[l];
+    if (!aligned(f.bias[l]) || !aligned(k.w[l])) return false;
+  }
+  // the packed weights: from the pre-activations' region on, which with what
+  // follows it holds at least 128 rows' worth: 768 D H + 8 H F >= 2 H (2 F + (D - 1) H) bytes
+  long long off[R_COUNT + 1];
+  ws_offsets(d, 128, off);
+  if (off[R_COUNT] - off[R_Z] < 2LL * d.H * (2 * d.F + (d.D - 1) * d.H)) return false;
+  k.out = reinterpret_cast<uint4*>(static_cast<char*>(ws) + off[R_Z]);
+  k.N = d.H;
+  k.K0 = 2 * d.F;
+  k.D = d.D;
+  f.w = reinterpret_cast<const unsigned char*>(k.out);
+  if (d.H == 256) {
+    switch (d.O) {
+      case 1: return launch_fused<256, 1, T>(f, k, s);
+      case 2: return launch_fused<256, 2, T>(f, k, s);
+      case 3: return launch_fused<256, 3, T>(f, k, s);
+      default: return launch_fused<256, 4, T>(f, k, s);
+    }
+  }
+  switch (d.O) {
+    case 1: return launch_fused<128, 1, T>(f, k, s);
+    case 2: return launch_fused<128, 2, T>(f, k, s);
+    case 3: return launch_fused<128, 3, T>(f, k, s);
+    default: return launch_fused<128, 4, T>(f, k, s);
+  }
 }
 
 inline void forward_hidden(const Net& n, const Ws& w, long long M, bool keep_z, cudaStream_t s) {
@@ -1179,6 +1617,12 @@ extern "C" int todgpu_tail_accumulate(const todgpu_mlp* m, const void* theta, co
     h.scale[o] = scale[o];
     h.shift[o] = shift[o];
   }
+  const bool fused = angles_dtype == TODGPU_F32
+                         ? tail_fused(n, static_cast<const float*>(theta), static_cast<const float*>(phi),
+                                      static_cast<const float*>(psi), B, h, ws, s)
+                         : tail_fused(n, static_cast<const double*>(theta), static_cast<const double*>(phi),
+                                      static_cast<const double*>(psi), B, h, ws, s);
+  if (fused) return finish("tail accumulate");
   for (long long b0 = 0; b0 < B; b0 += chunk) {
     const long long nv = std::min<long long>(chunk, B - b0);
     const char* th = static_cast<const char*>(theta) + b0 * esz;
