@@ -447,8 +447,11 @@ struct __align__(16) SampleBlock {
   double phi_u, theta_u;                                     // rotated beam centre
   int ir_lo, nr;                                             // window rings (nr = 0: none)
   double cu, su;                                             // cos, sin of theta_u
+  double px, py, pz, cp, sp;                                 // reference float32 roll (polar_z)
 };
-static_assert(sizeof(SampleBlock) == 176 && offsetof(SampleBlock, cu) == 160 && offsetof(SampleBlock, fkx) == 80, "SampleBlock layout");
+static_assert(sizeof(SampleBlock) == 224 && offsetof(SampleBlock, cu) == 160 && offsetof(SampleBlock, px) == 176 &&
+                  offsetof(SampleBlock, fkx) == 80,
+              "SampleBlock layout");
 
 // The reference's own two-step rotation (k, a; p, psi), for the nearest
 // rule's exact path.
@@ -700,6 +703,11 @@ __device__ __noinline__ void prepare_sample(const KArgs& a, long long b, bool ha
     sb.fkz = r.fkz;
     sb.fca = r.fca;
     sb.fsa = r.fsa;
+    sb.px = r.px;
+    sb.py = r.py;
+    sb.pz = r.pz;
+    sb.cp = r.cp;
+    sb.sp = r.sp;
   }
   double bphi = 0.0;
   if (has_qu) {
@@ -792,26 +800,44 @@ __device__ __forceinline__ void rotate_frame(unsigned sb, const double* const* v
 }
 // Reference typing: the recentring's products and sums are float32, as in
 // rot_ref32 (the same bits), the roll and the frame float64.
+__device__ __forceinline__ void recentre32(unsigned sb, float vx, float vy, float vz, double* v) {
+  const float4 fk = lds_f4(sb + 80);  // fkx, fky, fkz, fca
+  const float fsa = __uint_as_float(lds_u1(sb + 96));
+  const double oma = lds_d1(sb + 72);
+  const float dkv = fk.x * vx + fk.y * vy + fk.z * vz;
+  const float ax = vx * fk.w + (fk.y * vz - fk.z * vy) * fsa;
+  const float ay = vy * fk.w + (fk.z * vx - fk.x * vz) * fsa;
+  const float az = vz * fk.w + (fk.x * vy - fk.y * vx) * fsa;
+  v[0] = (double)ax + (double)(fk.x * dkv) * oma;
+  v[1] = (double)ay + (double)(fk.y * dkv) * oma;
+  v[2] = (double)az + (double)(fk.z * dkv) * oma;
+}
 template <int N>
 __device__ __forceinline__ void rotate_frame(unsigned sb, const float* const* vec, const int (&at)[N], double* x,
                                              double* y, double* z) {
   double v[N][3];
-  const float4 fk = lds_f4(sb + 80);  // fkx, fky, fkz, fca
-  const float fsa = __uint_as_float(lds_u1(sb + 96));
-  const double oma = lds_d1(sb + 72);
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const float vx = __ldg(vec[0] + at[k]), vy = __ldg(vec[1] + at[k]), vz = __ldg(vec[2] + at[k]);
-    const float dkv = fk.x * vx + fk.y * vy + fk.z * vz;
-    const float ax = vx * fk.w + (fk.y * vz - fk.z * vy) * fsa;
-    const float ay = vy * fk.w + (fk.z * vx - fk.x * vz) * fsa;
-    const float az = vz * fk.w + (fk.x * vy - fk.y * vx) * fsa;
-    v[k][0] = (double)ax + (double)(fk.x * dkv) * oma;
-    v[k][1] = (double)ay + (double)(fk.y * dkv) * oma;
-    v[k][2] = (double)az + (double)(fk.z * dkv) * oma;
-  }
+  for (int k = 0; k < N; ++k) recentre32(sb, __ldg(vec[0] + at[k]), __ldg(vec[1] + at[k]), __ldg(vec[2] + at[k]), v[k]);
   to_frame<N>(sb, v, x, y, z);
 }
+
+// Near a pole the colatitude is ill-conditioned in z (an error of 1e-16 becomes
+// 1e-16 / sin theta, and the ring weight's 1.2 nside times that), so the
+// reference's own rounding of z shows there: with z from the matrix one random
+// pole-crossing case of twenty differed from it by more than 1e-12 (300 seeds,
+// nside 64 and 256).  Beyond |z| = kPolarZ z is therefore formed by rot_ref32's
+// operations in its order.  Float64 pointing has no such typing to follow.
+constexpr double kPolarZ = 0.9;
+__device__ __forceinline__ bool is_polar(double z) { return fabs(z) > kPolarZ; }
+__device__ __forceinline__ double polar_z(unsigned sb, const float* const* vec, int at) {
+  double v[3];
+  recentre32(sb, __ldg(vec[0] + at), __ldg(vec[1] + at), __ldg(vec[2] + at), v);
+  const double2 pxy = lds_d2(sb + 176), pzc = lds_d2(sb + 192);
+  const double sp = lds_d1(sb + 208);
+  const double dpr = pxy.x * v[0] + pxy.y * v[1] + pzc.x * v[2];
+  return v[2] * pzc.y + (pxy.x * v[1] - pxy.y * v[0]) * sp + pzc.x * dpr * (1.0 - pzc.y);
+}
+__device__ __forceinline__ double polar_z(unsigned, const double* const*, int) { return 0.0; }
 
 // The reference's own rotation of a beam pixel (rot_ref32 / rot_f64).
 __device__ __forceinline__ void rotate_exact(const SampleBlock* sb, const ExactBlock* eb, float vx, float vy, float vz,
@@ -1167,6 +1193,7 @@ __device__ __noinline__ Contrib bilinear_direct(const KArgs& a, const SampleBloc
   double x, y, vz;
   const VecT* const vec[3] = {v, v + a.vec_si, v + 2 * a.vec_si};
   rotate_frame<1>(smem_u32(sb), vec, {0}, &x, &y, &vz);
+  if (PM == kParamsRef32 && is_polar(vz)) vz = polar_z(smem_u32(sb), vec, 0);
   if (!(isfinite(x) && isfinite(y) && isfinite(vz))) {
     out.err = 1;
     return out;
@@ -1631,6 +1658,11 @@ __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LA
   for (; s + kSumLanes < p.n; s += 2 * kSumLanes) {
     double x[2], y[2], z[2];
     rotate_frame<2>(sb, p.vec, {s * p.ss, (s + kSumLanes) * p.ss}, x, y, z);
+    if (REGION != kBelt && PM == kParamsRef32 && (is_polar(z[0]) || is_polar(z[1]))) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (is_polar(z[k])) z[k] = polar_z(sb, p.vec, (s + k * kSumLanes) * p.ss);
+    }
     Place o[2];
     bool ok = true;
 #pragma unroll
@@ -1643,6 +1675,7 @@ __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LA
   if (s < p.n) {
     double x, y, z;
     rotate_frame<1>(sb, p.vec, {s * p.ss}, &x, &y, &z);
+    if (REGION != kBelt && PM == kParamsRef32 && is_polar(z)) z = polar_z(sb, p.vec, s * p.ss);
     Place o;
     if (place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, cu, su, belt_inv, x, y, z, o)) {
       add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o, __ldg(p.vals + s), acc);
