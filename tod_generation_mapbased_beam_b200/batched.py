@@ -58,10 +58,9 @@ class DetectorBatch:
             self.angles.append(ang)
             self.out.append(torch.zeros((self.C, ang[0].shape[0]), dtype=torch.float64, device=dev))
             self.centers.append(tuple(d.get("center", (0.0, 0.0))))
-            # each detector's own ring table, sized for its own beam: the per-sample
-            # spin-2 tables fill every window ring's reserved slots, so a table
-            # sized for the widest beam of the batch costs the narrower ones work
-            # (tables are cached per reach and shared between equal beams)
+            # each detector's own ring table, built for its own beam's reach: beyond
+            # it the gather evaluates every pixel directly (tables are cached per
+            # reach and shared between equal beams)
             reach = beam_reach(vec, self.nside) if (tables and vec.shape[0]) else 0.0
             self.tables.append(ring_table(self.nside, reach, dev) if reach > 0 else None)
         self.rot = [pointing_buffers(a[0].shape[0], dev) for a in self.angles] if precompute else None

@@ -7,7 +7,7 @@
 // 256 threads) walks the samples; a CTA takes one sample
 // at a time and
 //   1. has its rotation, footprint centre and range of RING rings prepared, for
-//      eight samples at a time by eight lanes of one warp (prepare_sample);
+//      sixteen samples at a time by sixteen lanes of one warp (prepare_sample);
 //   2. lays out the window of rings the footprint (beam radius + stencil
 //      reach) can touch, each ring's stretch of the footprint disc and the
 //      ring in the sample's own longitude frame (footprint_window);
@@ -181,7 +181,7 @@ __device__ __forceinline__ SampleRot rot_from_angles(const KArgs& a, long long b
 // parameters: 0-2 axes, 3 cos_a, 4 sin_a, 5-7 ax_pts, 8 cos_p, 9 sin_p, 10 the
 // boresight longitude (when given); float64 parameters: fields 0-9 as
 // doubles; angles: 0 theta, 1 phi, 2 psi.  field_ptr gives a field's address
-// (nullptr when absent), field_bytes its size.
+// (nullptr when absent).
 template <int PM>
 __device__ __forceinline__ const void* field_ptr(const KArgs& a, long long b, int i) {
   if constexpr (PM == kAngles) {
@@ -199,14 +199,6 @@ __device__ __forceinline__ const void* field_ptr(const KArgs& a, long long b, in
     if (PM == kParamsRef32 && i == 10 && a.bore_phi != nullptr) return a.bore_phi + b;
     return nullptr;
   }
-}
-template <int PM>
-__device__ __forceinline__ int field_count() {
-  return PM == kAngles ? 3 : (PM == kParamsRef32 ? 11 : 10);
-}
-template <int PM>
-__device__ __forceinline__ int field_bytes(const KArgs& a) {
-  return PM == kParamsRef32 ? 4 : (PM == kAngles && a.angles_f32 ? 4 : 8);
 }
 
 // Rotation of a sample from its fields, got(i) returning field i (float for
@@ -294,12 +286,6 @@ struct GlobalFields {
 template <int PM>
 __device__ __forceinline__ SampleRot load_rot(const KArgs& a, long long b) {
   return rot_from_fields<PM>(a, GlobalFields<PM>{a, b});
-}
-
-template <int PM>
-__device__ __forceinline__ void load_boresight(const KArgs& a, const SampleRot& rot, long long b, double& z,
-                                               double& sth, double& phi) {
-  boresight_from_fields<PM>(a, rot, GlobalFields<PM>{a, b}, z, sth, phi);
 }
 
 // ---------------------------------------------------------------------------
@@ -1753,11 +1739,29 @@ __device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOU
 constexpr int kBeamChunkMin = 16384;
 constexpr int kBeamChunk = 1024;
 
+// What a CTA keeps from sample to sample of a run besides the pixel loop's
+// state, in shared memory: in registers it was spilled, and an L1 that the tables
+// leave little of sent the reloads to L2.  The batched kernel, with its tiles
+// and jobs to keep as well, gains most: six detectors over a float32 map 4330 ->
+// 3845 us, far sidelobes in pieces 4710 -> 4480; nearest 1872 -> 1827, packed
+// float32 records 1925 -> 1905, the 30' float64 beam 2478 -> 2486.
+struct RunState {
+  long long t_begin, t_step, tile, total;  // tiles t_begin, t_begin + t_step, ...; samples in all of them
+  double cx, cy, cz, rbeam;
+  unsigned long long nerr;
+  long long b[kPrep];                      // the samples being prepared or summed
+  // sample q of the run
+  __device__ __forceinline__ long long sample(long long q) const volatile {
+    const long long n = tile, ti = n == 1 ? q : q / n;
+    return (t_begin + ti * t_step) * n + (q - ti * n);
+  }
+};
+
 // Samples of tiles t = t_begin, t_begin + t_step, ... < t_end of one job (one
 // beam entry over one batch of samples; tile t holds samples [t tile,
 // min(B, (t + 1) tile))), by the whole CTA.  All threads of the CTA must call
 // it together.
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, bool TILES>
 __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, long long t_step, long long tile,
                             unsigned char* smem_raw, double* s_red, SampleBlock* s_blk, ExactBlock* s_exact,
                             int4* s_hdr) {
@@ -1780,7 +1784,9 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
   const long long ntile = (t_end - t_begin + t_step - 1) / t_step;
   const long long t_last = t_begin + (ntile - 1) * t_step;
   const long long total = (ntile - 1) * tile + min(tile, a.B - t_last * tile);
-  unsigned long long nerr = 0;
+  __shared__ RunState run_mem;
+  volatile RunState* run = &run_mem;
+  if (tid == 0) run->nerr = 0;
   const int S = (int)a.S;
   const int step = S > kBeamChunkMin && !MapTraits<MapT>::packed ? kBeamChunk : S;
   for (int s0 = 0; s0 < S; s0 += step) {
@@ -1795,11 +1801,20 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
     const bool window = a.ring_table != nullptr && (MODE == TODGPU_NEAREST || a.tab_cap > 0) &&
                         rbeam + 2.0 / (double)a.nside <= __ldg(&static_cast<const RingRec*>(a.ring_table)[0].ta);
     const int n = s1 - s0;
-    const VecT* vec = static_cast<const VecT*>(a.vec) + (long long)s0 * a.vec_ss;
-    const float* vals = a.beam + s0;
     if (tid == 0) {
+      const VecT* vec = static_cast<const VecT*>(a.vec) + (long long)s0 * a.vec_ss;
+      if (TILES) {
+        run->t_begin = t_begin;
+        run->t_step = t_step;
+        run->tile = tile;
+        run->total = total;
+      }
+      run->cx = cx;
+      run->cy = cy;
+      run->cz = cz;
+      run->rbeam = rbeam;
       for (int k = 0; k < 3; ++k) loop->vec[k] = vec + k * a.vec_si;
-      loop->vals = vals;
+      loop->vals = a.beam + s0;
       loop->map = MapRef{a.map, a.map_stride};
       loop->rings = smem_u32(rings);
       loop->tab = tab;
@@ -1810,14 +1825,17 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
     }
     // the nearest rule's margin on ring boundaries (nearest_window) holds away
     // from the poles, where a ring's width in z vanishes
+    const float reach = (float)rbeam;
     const double polar = MODE == TODGPU_NEAREST ? 0.01 : -4.0;
-    for (long long q0 = 0; q0 < total; q0 += kPrep) {
-      const int nq = (int)min((long long)kPrep, total - q0);
-      __syncthreads();  // the previous samples' blocks are no longer read
+    for (long long q0 = 0;; q0 += kPrep) {
+      __syncthreads();  // the previous samples' blocks are no longer read; the run's state is written
+      const int nq = (int)min((long long)kPrep, (TILES ? run->total : total) - q0);
+      if (nq <= 0) break;
       if (tid < nq) {
-        const long long q = q0 + tid, ti = tile == 1 ? q : q / tile;
-        prepare_sample<PM>(a, (t_begin + ti * t_step) * tile + (q - ti * tile), HAS_QU, cx, cy, cz, rbeam, window,
-                           polar, s_blk[tid], s_exact != nullptr ? s_exact + tid : nullptr);
+        const long long b = TILES ? run->sample(q0 + tid) : t_begin + (q0 + tid) * t_step;
+        if (TILES) run->b[tid] = b;
+        prepare_sample<PM>(a, b, HAS_QU, run->cx, run->cy, run->cz, run->rbeam, window, polar, s_blk[tid],
+                           s_exact != nullptr ? s_exact + tid : nullptr);
       }
       __syncthreads();
 #pragma unroll 1
@@ -1828,7 +1846,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
         double* red = s_red + 16 * (i & 1);
         int4 hdr = make_int4(0, 0, 0, 0);
         if (window) {
-          footprint_window<MODE>(static_cast<const RingRec*>(a.ring_table), sb, nside, a.tab_cap, (float)rbeam, rings,
+          footprint_window<MODE>(static_cast<const RingRec*>(a.ring_table), sb, nside, a.tab_cap, reach, rings,
                                  ring_end, ring_of, s_hdr);
           __syncthreads();
           hdr = *s_hdr;
@@ -1853,15 +1871,16 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
           while (st.s < n) {
             if (hdr.y > 0) st = pixel_loop<MODE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(loop, sb, hdr, nside, st);
             if (st.s < n) {
-              const VecT* v = vec + (long long)st.s * a.vec_ss;
-              const float bvf = vals[st.s];
+              const VecT* v = static_cast<const VecT*>(a.vec) + (s0 + (long long)st.s) * a.vec_ss;
+              const float bvf = a.beam[s0 + st.s];
               Contrib r;
               if constexpr (MODE == TODGPU_BILINEAR)
                 r = bilinear_direct<PM, HAS_QU, MapT, LAYOUT, VecT>(a, sb, v);
               else
                 r = nearest_exact<PM, HAS_QU, MapT, LAYOUT, VecT>(a, sb, s_exact + i, v[0], v[a.vec_si], v[2 * a.vec_si], bvf);
-              nerr += r.err;
-              if (!r.err) {
+              if (r.err) {
+                atomicAdd(&run_mem.nerr, (unsigned long long)r.err);
+              } else {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                   if (c >= ch.C) break;
@@ -1904,8 +1923,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
         }
         __syncthreads();  // the sums are written and the table, window and header free
         if (tid < a.C) {
-          const long long q = q0 + i, ti = tile == 1 ? q : q / tile;
-          const long long b = (t_begin + ti * t_step) * tile + (q - ti * tile);
+          const long long b = TILES ? run->b[i] : t_begin + (q0 + i) * t_step;
           double v = 0.0;
           for (int k = 0; k < kMeanLanes / 32; ++k) v += red[k * 4 + tid];
           a.tod[(long long)tid * a.tod_stride + b] += v;
@@ -1913,12 +1931,8 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
       }
     }
   }
-  if (a.err != nullptr) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nerr += __shfl_xor_sync(0xffffffffu, nerr, o);
-    if (lane == 0 && nerr) atomicAdd(a.err, nerr);
-  }
-  __syncthreads();  // shared memory may be reused by the next job
+  __syncthreads();  // every count is in; shared memory may be reused by the next job
+  if (tid == 0 && a.err != nullptr && run->nerr) atomicAdd(a.err, run->nerr);
 }
 
 template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
@@ -1928,8 +1942,8 @@ __global__ void __maxnreg__(kRegs) gather_accum_kernel(const __grid_constant__ K
   __shared__ SampleBlock s_blk[kPrep];
   __shared__ ExactBlock s_exact[MODE == TODGPU_NEAREST ? kPrep : 1];
   __shared__ int4 s_hdr;
-  run_samples<MODE, HAS_QU, MapT, PM, LAYOUT>(a, blockIdx.x, a.B, gridDim.x, 1, smem_raw, s_red, s_blk,
-                                              MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
+  run_samples<MODE, HAS_QU, MapT, PM, LAYOUT, false>(a, blockIdx.x, a.B, gridDim.x, 1, smem_raw, s_red, s_blk,
+                                                     MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
 }
 
 // Many jobs (detectors: each its own beam, pointing, output and length) in
@@ -1972,8 +1986,8 @@ __global__ void __maxnreg__(kRegs) gather_batched_kernel(const __grid_constant__
         reinterpret_cast<unsigned long long*>(&s_job)[threadIdx.x] =
             reinterpret_cast<const unsigned long long*>(&p.job[j])[threadIdx.x];
       __syncthreads();
-      run_samples<MODE, HAS_QU, MapT, PM, LAYOUT>(s_job, t0, ntiles, G, p.tile, smem_raw, s_red, s_blk,
-                                              MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
+      run_samples<MODE, HAS_QU, MapT, PM, LAYOUT, true>(s_job, t0, ntiles, G, p.tile, smem_raw, s_red, s_blk,
+                                                        MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
     }
   }
 }

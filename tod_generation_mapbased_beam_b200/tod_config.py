@@ -17,7 +17,7 @@ ignores::
       pointing: device       # device (FP64 rotation on the GPU) | reference (host float32 prep)
       map_precision: f64     # f64 | f32 | bf16 (packed records, Kahan sums)
       chunk: 1048576         # samples per streamed chunk
-      tables: true           # per-sample spin-2 tables (false: direct evaluation)
+      tables: true           # per-sample footprint tables (false: direct evaluation)
       learned_tail:          # optional: far-sidelobe tail by the network
         enabled: false
         budget_uK: 0.1       # held-out RMS error above which the plain tail is used
