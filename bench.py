@@ -552,7 +552,7 @@ def run_ours(args, dist):
         result["parity"] = par
 
     # mixed precision forms on the same workload: packed float32 / bfloat16
-    # records, float32 spin-2 table, float32 Kahan sum, float64 decisions;
+    # records, float32 turned values, float32 Kahan sum, float64 decisions;
     # error against the FP64 oracle on a bounded subset of samples
     if not args.no_mixed:
         mixed = {}

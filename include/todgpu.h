@@ -241,7 +241,7 @@ uint64_t todgpu_host_hash(const void *data, size_t bytes, uint64_t seed);
 
 /* Ring table: per-ring data of the RING scheme for one nside (ring z, acos z,
  * layout) and, for footprints of angular radius up to `reach` (radians), the
- * spin-2 table slots each ring needs.  todgpu_gather_accum reads it through
+ * table slots each ring needs.  todgpu_gather_accum reads it through
  * args->ring_table (lookups only; it is never written by the gather).  The
  * caller allocates `todgpu_ring_table_bytes(nside)` bytes of device memory
  * (16-byte aligned) and builds it once per (nside, reach) on `stream`.  A

@@ -1628,7 +1628,7 @@ struct LoopState {
 //
 // Bound (30' beam, S = 1512, nside 1024, 120k samples, float64 records): 5.30 ms
 // with the map gathered and the spin-2 angle looked up per neighbour (677
-// thread instructions an evaluation, L1 at 79%), 2.47 ms now, of which the
+// thread instructions an evaluation, L1 at 79%), 2.52 ms now, of which the
 // table fill is 0.4 and the window 0.1; ~210 instructions an evaluation, 66 of
 // them float64, issue slots 57% and the shared-memory data path 60-70% busy:
 // leaving out 12 of 16 shared loads saved 5%, 22 of 66 float64 operations 13%.
