@@ -43,7 +43,9 @@ class LearnedTailTOD:
     """I/Q/U TOD of one beam entry (components [I, Q, U], spin-2 on) with the
     tail learned.
 
-    ``sky``: (3, 12 nside^2) float64 map (numpy or CUDA tensor).  ``main`` and
+    ``sky``: (3, 12 nside^2) float64 map (numpy or CUDA tensor; a CUDA tensor is
+    read by every float64 evaluation, the packed ``main_map`` forms when the object
+    is made).  ``main`` and
     ``tail``: beams with ``vec_orig`` (S, 3) and ``beam_vals`` (S,) in the
     beam frame centred on the pole.  ``center``: beam centre (phi, theta) of the
     angle-mode pointing.  ``main_map``: "f32" or "bf16" (packed precision form)
@@ -56,9 +58,14 @@ class LearnedTailTOD:
         sky = torch.as_tensor(sky, dtype=torch.float64, device=self.device).contiguous()
         if sky.shape != (3, 12 * self.nside ** 2):
             raise ValueError("sky must be a (3, 12 nside^2) I/Q/U map")
+        # The float64 forms read the map itself in every call: a float64 CUDA tensor is
+        # the caller's own, and a sky refilled in place (by alm2map, say, which no
+        # modification counter shows) is the one the next call sees.  Records packed
+        # here would be the old sky's; they gain nothing at nside 1024 (301 pointings of
+        # a 284,000-pixel tail: 4.81 ms planar, 4.82 in records) and 12% below (nside 256
+        # and 512), about what packing them in each call would cost.
         self.sky = sky
-        self.sky_rec = pack_map(sky, "f64")  # the same values, a pixel's components side by side
-        self.sky_main = self.sky_rec if main_map == "f64" else pack_map(sky, main_map)
+        self.sky_main = None if main_map == "f64" else pack_map(sky, main_map)
         self.main_map = main_map
         self.interp = _INTERP[interp]
         self.center = (float(center[0]), float(center[1]))
@@ -95,7 +102,7 @@ class LearnedTailTOD:
         for b0 in range(0, B, self.tail_chunk):
             b1 = min(B, b0 + self.tail_chunk)
             part = torch.zeros((3, b1 - b0), dtype=torch.float64, device=self.device)
-            self._gather(self.tail_vec, self.tail_bv, self.sky_rec, th[b0:b1], ph[b0:b1], ps[b0:b1], part,
+            self._gather(self.tail_vec, self.tail_bv, self.sky, th[b0:b1], ph[b0:b1], ps[b0:b1], part,
                          self.tail_pieces)
             tod[:, b0:b1] += part
         return tod
@@ -106,7 +113,8 @@ class LearnedTailTOD:
         th, ph, ps = (self._dev(a, self.device) for a in (theta, phi, psi))
         if tod is None:
             tod = torch.zeros((3, th.numel()), dtype=torch.float64, device=self.device)
-        self._gather(self.main_vec, self.main_bv, self.sky_rec if exact else self.sky_main, th, ph, ps, tod)
+        mp = self.sky if exact or self.sky_main is None else self.sky_main
+        self._gather(self.main_vec, self.main_bv, mp, th, ph, ps, tod)
         return tod
 
     def full_plain(self, theta, phi, psi):
