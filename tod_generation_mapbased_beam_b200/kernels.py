@@ -258,6 +258,16 @@ def planar_beam(vec, evals=None):
     return vec.contiguous(), 0
 
 
+def resident_beam(vec_orig, np_dtype, device):
+    """``vec_orig`` itself when it is a (S, 3) tensor of ``np_dtype`` on
+    ``device`` -- in any strides, for :func:`planar_beam` -- else None: anything
+    else (another GPU's tensor too) goes through ``to_device``."""
+    if (is_tensor(vec_orig) and vec_orig.device == device and dtype_of(vec_orig) == np.dtype(np_dtype)
+            and vec_orig.dim() == 2 and vec_orig.shape[1] == 3):
+        return vec_orig
+    return None
+
+
 def _row_stride(t):
     """Row stride of a (rows, n) tensor with unit column stride; a single
     row's stride is free in torch (a ``[None, :]`` view may carry 0), so it
@@ -370,17 +380,17 @@ def gather_accum(interp, vec_orig, axes, cos_a, sin_a, ax_pts, cos_p, sin_p, nsi
     ``flags``: ``_native.FLAG_NO_TABLES`` evaluates every ring quantity and
     spin-2 angle directly instead of from the per-sample footprint tables
     (identical results; for testing)."""
-    require_cuda()
+    dev = require_cuda()
     B = int(B)
     S = int(S)
     nside = int(nside)
     raw = (vec_orig, axes, cos_a, sin_a, ax_pts, cos_p, sin_p)
     pdt = _param_dtype(raw)
     shapes = [(S, 3), (B, 3), (B,), (B,), (B, 3), (B,), (B,)]
-    if is_tensor(vec_orig) and vec_orig.is_cuda and tuple(vec_orig.shape) == (S, 3):
-        vec, planar = planar_beam(vec_orig, B * S)
-    else:
-        vec, planar = planar_beam(to_device(vec_orig, pdt, (S, 3)), B * S)
+    given = resident_beam(vec_orig, pdt, dev)
+    if given is None or given.shape[0] != S:
+        given = to_device(vec_orig, pdt, (S, 3))
+    vec, planar = planar_beam(given, B * S)
     params = [vec] + [to_device(x, pdt, sh) for x, sh in zip(raw[1:], shapes[1:])]
     if dtype_of(beam_vals) != np.dtype(np.float32):
         raise TypeError("beam_vals must be float32 (the reference casts beam weights to float32)")
@@ -583,10 +593,9 @@ def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_th
 
     ``pieces``: :func:`piece_footprints` of a beam of more than 16384 pixels, for a
     program that keeps it (found in each call otherwise)."""
-    require_cuda()
-    if is_tensor(vec_orig) and vec_orig.is_cuda and vec_orig.dtype == torch.float64 and vec_orig.dim() == 2:
-        given = vec_orig  # (a copy or view would be another tensor to beam_reach)
-    else:
+    # (a copy or view of a resident beam would be another tensor to beam_reach)
+    given = resident_beam(vec_orig, np.float64, require_cuda())
+    if given is None:
         given = to_device(vec_orig, np.float64).reshape(-1, 3)
     S = given.shape[0]
     adt, th, ph, ps = _angles_on_device(theta, phi, psi)
