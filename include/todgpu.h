@@ -235,8 +235,9 @@ int todgpu_spin2(const double *z_pix, const double *sth_pix, const double *phi_p
 int todgpu_boresight_phi_host(const float *ax_pts, int64_t B, float *out, int32_t nthreads);
 
 /* HOST function: 64-bit fingerprint of `bytes` bytes of host memory, continuing
- * from `seed`.  Position-sensitive, and any change within one 8-byte word
- * changes it.  No counterpart in the reference. */
+ * from `seed`.  Position-sensitive; two buffers share it with a probability of
+ * about 2^-63 over its (fixed) keys, whatever they differ in.  Not for hostile
+ * data.  No counterpart in the reference. */
 uint64_t todgpu_host_hash(const void *data, size_t bytes, uint64_t seed);
 
 /* Ring table: per-ring data of the RING scheme for one nside (ring z, acos z,

@@ -616,39 +616,58 @@ extern "C" int todgpu_boresight_phi_host(const float* ax_pts, int64_t B, float* 
   return TODGPU_OK;
 }
 
-// Fingerprint of host memory: eight 64-bit lanes take the words in turn, each
-// lane h <- rotl((h ^ word) K, 27) with K odd -- a bijection of h for every
-// word and of the word for every h, so a change of any one word changes its
-// lane -- and the lanes, the length and the tail bytes are folded in the same
-// way.  Eight independent multiply chains read memory at its own speed (some
-// 15 GB/s a core; zlib's CRC-32 5).
+// Fingerprint of host memory: NH (Black, Halevi, Krawczyk, Krovetz, Rogaway: UMAC,
+// CRYPTO 1999) of every 512 bytes, sum over pairs of words of (w0 + k0) (w1 + k1)
+// modulo 2^128, the sums chained by two bijective steps each.  A change in a block
+// leaves its sum as it was only where the keys happen to meet the data -- a single
+// word's change if its partner plus key is 0 modulo 2^64, in general with
+// probability 2^-64 over the keys -- and a changed sum changes the result with the
+// same odds; no pattern of flipped bits cancels by itself.  (Eight multiply-and-
+// rotate lanes, kept before, passed a flip of bit 63 of a word on as a flip of bit
+// 26: that bit flipped too eight words on, and the hash was the same for any data.)
+// One 64 x 64 -> 128 bit product per 16 bytes.
+constexpr int kHashWords = 64;
+struct HashKeys {
+  uint64_t k[kHashWords];
+};
+constexpr uint64_t hash_step(uint64_t h, uint64_t w) {  // a bijection of h for every w, and of w for every h
+  uint64_t x = (h ^ w) * 0x9f3ac1d4b27e5865ull;
+  x ^= x >> 32;
+  x *= 0xd6a4c1b93f5e7283ull;
+  return x ^ (x >> 29);
+}
+constexpr HashKeys make_hash_keys() {
+  HashKeys t{};
+  uint64_t h = 0x5851f42d4c957f2dull;
+  for (int i = 0; i < kHashWords; ++i) t.k[i] = h = hash_step(h, (uint64_t)i);
+  return t;
+}
+static constexpr HashKeys kHashKeys = make_hash_keys();
+
+static uint64_t hash_block(uint64_t h, const unsigned char* p) {
+  unsigned __int128 even = 0, odd = 0;  // two chains of additions
+  for (int i = 0; i < kHashWords; i += 4) {
+    uint64_t w[4];
+    std::memcpy(w, p + 8 * i, 32);
+    even += (unsigned __int128)(w[0] + kHashKeys.k[i]) * (w[1] + kHashKeys.k[i + 1]);
+    odd += (unsigned __int128)(w[2] + kHashKeys.k[i + 2]) * (w[3] + kHashKeys.k[i + 3]);
+  }
+  even += odd;
+  return hash_step(hash_step(h, (uint64_t)even), (uint64_t)(even >> 64));
+}
+
 extern "C" uint64_t todgpu_host_hash(const void* data, size_t bytes, uint64_t seed) {
-  constexpr uint64_t K = 0x9f3ac1d4b27e5865ull;
-  auto mix = [](uint64_t h, uint64_t w) {
-    const uint64_t x = (h ^ w) * K;
-    return (x << 27) | (x >> 37);
-  };
+  constexpr size_t kBlock = 8 * kHashWords;
   const unsigned char* p = static_cast<const unsigned char*>(data);
-  uint64_t h[8];
-  for (int i = 0; i < 8; ++i) h[i] = mix(seed + 0x5851f42d4c957f2dull * (uint64_t)(i + 1), (uint64_t)bytes);
+  uint64_t h = hash_step(hash_step(kHashKeys.k[0], seed), (uint64_t)bytes);
   size_t left = data != nullptr ? bytes : 0;
-  for (; left >= 64; left -= 64, p += 64) {
-    uint64_t w[8];
-    std::memcpy(w, p, 64);
-#pragma GCC unroll 8
-    for (int i = 0; i < 8; ++i) h[i] = mix(h[i], w[i]);
+  for (; left >= kBlock; left -= kBlock, p += kBlock) h = hash_block(h, p);
+  if (left > 0) {
+    unsigned char tail[kBlock] = {};
+    std::memcpy(tail, p, left);
+    h = hash_block(h, tail);
   }
-  for (int i = 0; left > 0; ++i) {
-    const size_t n = std::min<size_t>(8, left);
-    uint64_t w = 0;
-    std::memcpy(&w, p, n);
-    h[i] = mix(h[i], w);
-    left -= n;
-    p += n;
-  }
-  uint64_t r = seed;
-  for (int i = 0; i < 8; ++i) r = mix(mix(r, h[i]), h[i] >> 32);
-  return r;
+  return h;
 }
 
 extern "C" size_t todgpu_ring_table_bytes(int64_t nside) {
