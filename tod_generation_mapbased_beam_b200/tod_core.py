@@ -217,21 +217,28 @@ def _pool():
     return _prep_pool
 
 
-def _prep_chunk(rot_vecs, phi_b, theta_b, psis_b, s0, s1, with_bore):
-    """Float32 parameters of samples [s0, s1), field after field in one buffer."""
-    params = _rotation_params(rot_vecs[s0:s1], phi_b[s0:s1], theta_b[s0:s1], psis_b[s0:s1])
-    n = s1 - s0
+def _pack_params(params, n, with_bore):
+    """Float32 parameters of n samples, field after field in one buffer."""
     out = np.empty(_PIPE_WORDS * n, np.float32)
     o = 0
     for p, w in zip(params, _PIPE_WIDTHS):
-        out[o:o + w * n] = np.asarray(p, np.float32).reshape(-1)
+        p = np.asarray(p, np.float32).reshape(-1)
+        if p.size != w * n:  # (an assignment would repeat a single value)
+            raise ValueError(f"rot_vecs, phi_b, theta_b and psis_b must hold {n} samples each")
+        out[o:o + w * n] = p
         o += w * n
     out[o:] = boresight_phi_host(params[3]) if with_bore else np.float32(0.0)
     return out
 
 
+def _prep_chunk(rot_vecs, phi_b, theta_b, psis_b, s0, s1, with_bore):
+    """Float32 parameters of samples [s0, s1), packed."""
+    return _pack_params(_rotation_params(rot_vecs[s0:s1], phi_b[s0:s1], theta_b[s0:s1], psis_b[s0:s1]), s1 - s0,
+                        with_bore)
+
+
 def _param_views(buf, n):
-    """The fields of n samples in a buffer laid out by :func:`_prep_chunk`."""
+    """The fields of n samples in a buffer laid out by :func:`_pack_params`."""
     views, o = [], 0
     for w in _PIPE_WIDTHS:
         v = buf[o:o + w * n]
@@ -319,8 +326,7 @@ def beam_tod_batch(nside, mp, data, rot_vecs, phi_b, theta_b, psis_b, interp_mod
                           np.asarray(theta_b), np.asarray(psis_b), vec, bv, mpd, tod, S, c_q, c_u)
     elif host_inputs and B > 0 and S > 0:
         # the parameters in one buffer and one copy (the pipeline's layout)
-        host = _prep_chunk(np.asarray(rot_vecs), np.asarray(phi_b), np.asarray(theta_b), np.asarray(psis_b), 0, B,
-                           c_q >= 0 and c_u >= 0)
+        host = _pack_params(_rotation_params(rot_vecs, phi_b, theta_b, psis_b), B, c_q >= 0 and c_u >= 0)
         views = _param_views(torch.from_numpy(host).to(mpd.device), B)
         gather_accum(_INTERP[interp_mode], vec, *views[:6], nside, mpd, bv, B, S, tod, c_q, c_u, bore_phi=views[6])
     else:
