@@ -23,6 +23,7 @@ from __future__ import annotations
 import ctypes
 import math
 import weakref
+from typing import NamedTuple
 
 import numpy as np
 import torch
@@ -520,11 +521,27 @@ _PIECE = 1024
 _PIECE_SLOTS = 2600
 
 
+class PiecePlan(NamedTuple):
+    """:func:`piece_footprints` of a beam of S pixels over a map of one nside."""
+
+    slots: np.ndarray  # table slots of every piece
+    reach: float       # the pieces' largest footprint [rad]
+    S: int
+    nside: int
+
+
+def _check_plan(plan, S, nside):
+    """A plan made for another beam would leave out pixels or read past the beam's."""
+    if not isinstance(plan, PiecePlan) or plan.S != S or plan.nside != int(nside) or len(plan.slots) != -(-S // _PIECE):
+        raise ValueError(f"pieces must be piece_footprints of this beam ({S} pixels) and nside {int(nside)}")
+    return plan
+
+
 def piece_footprints(vec, nside):
-    """(table slots of every piece, their largest reach) of a wide beam, a CUDA (S, 3)
-    tensor: the angle from a piece's mean direction to its farthest pixel, found on
-    the device; pieces too wide for a table ask for 2 slots.  A plan that a program
-    keeps with its beam (``gather_accum_angles(pieces=...)``)."""
+    """:class:`PiecePlan` of a wide beam, a CUDA (S, 3) tensor: the angle from a
+    piece's mean direction to its farthest pixel, found on the device; pieces too
+    wide for a table ask for 2 slots.  A plan that a program keeps with its beam
+    (``gather_accum_angles(pieces=...)``)."""
     S = vec.shape[0]
     n = (S + _PIECE - 1) // _PIECE
     at = torch.arange(n * _PIECE, device=vec.device).clamp_(max=S - 1)
@@ -535,7 +552,8 @@ def piece_footprints(vec, nside):
     r = np.where(np.isfinite(r), r, np.pi) + 3.0 / float(nside) + 2e-5
     slots = footprint_slots(nside, r)
     fits = slots <= _PIECE_SLOTS
-    return np.where(fits, slots, 2).astype(np.int32), float(r[fits].max()) if fits.any() else 0.0
+    return PiecePlan(np.where(fits, slots, 2).astype(np.int32), float(r[fits].max()) if fits.any() else 0.0, S,
+                     int(nside))
 
 
 def _gather_pieces(args, vec, beam, nside, tod, pieces):
@@ -546,7 +564,7 @@ def _gather_pieces(args, vec, beam, nside, tod, pieces):
     spread over the GPU where the samples alone would not.  Pieces of like
     footprints share a launch, whose table is sized for the largest."""
     S = vec.shape[0]
-    slots, reach = pieces if pieces is not None else piece_footprints(vec, nside)
+    slots, reach = (pieces if pieces is not None else piece_footprints(vec, nside))[:2]
     flat = vec.contiguous()  # (pieces of a planar beam are not planar beams)
     args.flags &= ~_native.FLAG_BEAM_PLANAR
     if not args.flags & _native.FLAG_NO_TABLES and reach > 0.0:
@@ -592,12 +610,15 @@ def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_th
     derive the rotation inside the gather.
 
     ``pieces``: :func:`piece_footprints` of a beam of more than 16384 pixels, for a
-    program that keeps it (found in each call otherwise)."""
+    program that keeps it (found in each call otherwise); a plan of another beam
+    size or nside is a ValueError."""
     # (a copy or view of a resident beam would be another tensor to beam_reach)
     given = resident_beam(vec_orig, np.float64, require_cuda())
     if given is None:
         given = to_device(vec_orig, np.float64).reshape(-1, 3)
     S = given.shape[0]
+    if pieces is not None:
+        _check_plan(pieces, S, nside)
     adt, th, ph, ps = _angles_on_device(theta, phi, psi)
     B = th.shape[0]
     vec, planar = planar_beam(given, B * S)
