@@ -519,6 +519,8 @@ _PIECE = 1024
 # to there (284k pixels of an annulus, 301 samples: 4.72 ms; 5.06 at 3000, 5.11 at
 # 4400, 6.8 at 8192, where one CTA has the SM; pieces of 512 or 2048 pixels 5.9, 6.7).
 _PIECE_SLOTS = 2600
+_PIECE_TILE = 16  # samples per work tile of a piece's job
+_PIECE_SCRATCH = 1 << 28  # bytes of the pieces' own outputs: 116,000 samples of 96 pieces, I, Q and U
 
 
 class PiecePlan(NamedTuple):
@@ -562,7 +564,9 @@ def _gather_pieces(args, vec, beam, nside, tod, pieces):
     order.  A far-sidelobe beam's footprint holds 1e5 to 1e6 map pixels, a
     piece's a patch that fits a table in shared memory; as jobs the pieces also
     spread over the GPU where the samples alone would not.  Pieces of like
-    footprints share a launch, whose table is sized for the largest."""
+    footprints share a launch, whose table is sized for the largest.  Long batches
+    run in blocks of samples, so the pieces' outputs stay within _PIECE_SCRATCH (the
+    sums are a sample's own: the same in any block)."""
     S = vec.shape[0]
     slots, reach = (pieces if pieces is not None else piece_footprints(vec, nside))[:2]
     flat = vec.contiguous()  # (pieces of a planar beam are not planar beams)
@@ -572,8 +576,9 @@ def _gather_pieces(args, vec, beam, nside, tod, pieces):
     elif not args.flags & _native.FLAG_NO_TABLES:
         args.ring_table = ring_table(nside, 3.0 / float(nside), vec.device).data_ptr()
     C, B = tod.shape
-    most = 96
-    part = torch.empty((min(most, len(slots)), C, B), dtype=torch.float64, device=vec.device)
+    most = min(96, len(slots))
+    block = min(B, max(_PIECE_TILE, _PIECE_SCRATCH // (most * C * 8) // _PIECE_TILE * _PIECE_TILE))
+    part = torch.empty((most, C, block), dtype=torch.float64, device=vec.device)
     size = ctypes.sizeof(_native.GatherArgs)
     jobs = np.tile(np.frombuffer(bytes(args), np.uint8), (len(slots), 1))
     field = lambda name, dt: np.ndarray(len(slots), dt, jobs, getattr(_native.GatherArgs, name).offset, (size,))
@@ -583,14 +588,21 @@ def _gather_pieces(args, vec, beam, nside, tod, pieces):
     field("S", np.int64)[:] = np.minimum(_PIECE, S - first)
     field("tab_slots", np.int32)[:] = slots
     jobs = np.ascontiguousarray(jobs[np.argsort(slots, kind="stable")])
-    field("tod", np.uint64)[:] = part.data_ptr() + (np.arange(len(slots)) % most) * (C * B * 8)
-    field("tod_stride", np.int64)[:] = B
-    for j0 in range(0, len(slots), most):
-        n = min(most, len(slots) - j0)
-        part[:n].zero_()
-        _native.check(_native.lib().todgpu_gather_accum_batched(
-            ctypes.cast(jobs[j0:].ctypes.data, ctypes.POINTER(_native.GatherArgs)), n, 16, stream_handle()))
-        tod += part[:n].sum(dim=0)
+    for b0 in range(0, B, block):
+        nb = min(block, B - b0)
+        for name in ("axes", "cos_a", "sin_a", "ax_pts", "cos_p", "sin_p"):
+            field(name, np.uint64)[:] = getattr(args, name) + 8 * b0 * (3 if name in ("axes", "ax_pts") else 1)
+        field("B", np.int64)[:] = nb
+        field("tod", np.uint64)[:] = part.data_ptr() + (np.arange(len(slots)) % most) * (C * nb * 8)
+        field("tod_stride", np.int64)[:] = nb
+        for j0 in range(0, len(slots), most):
+            n = min(most, len(slots) - j0)
+            sums = part.view(-1)[:n * C * nb].view(n, C, nb)
+            sums.zero_()
+            _native.check(_native.lib().todgpu_gather_accum_batched(
+                ctypes.cast(jobs[j0:].ctypes.data, ctypes.POINTER(_native.GatherArgs)), n, _PIECE_TILE,
+                stream_handle()))
+            tod[:, b0:b0 + nb] += sums.sum(dim=0)
 
 
 def gather_accum_angles(interp, vec_orig, theta, phi, psi, center_phi, center_theta, nside,
