@@ -429,7 +429,9 @@ struct TableRings {
 struct __align__(16) SampleBlock {
   double m[9];
   double oma;                                                // 1 - cos a
-  float fkx, fky, fkz, fca, fsa, fpad0, fpad1, fpad2;        // reference float32 recentring
+  float fkx, fky, fkz, fca, fsa;                             // reference float32 recentring
+  int wide;                                                  // the pixel loop's form is kWide
+  float fpad0, fpad1;
   double bz, bsth, bdl;                                      // boresight: z, sin theta, longitude - phi_u in [-pi, pi]
   double phi_u, theta_u;                                     // rotated beam centre
   int ir_lo, nr;                                             // window rings (nr = 0: none)
@@ -481,8 +483,7 @@ __device__ __forceinline__ bool slot_of(unsigned slots, int j, int count, int& s
   return (unsigned)(j + (top >> 1)) < (unsigned)(top + 2 - count);
 }
 
-// The window's header: x first ring, y rings that have a next ring in the
-// window (0: no window), z table slots (0: no table).
+// The boresight: z and sin theta.
 struct Bore {
   double z, sth;
 };
@@ -523,7 +524,8 @@ __device__ __forceinline__ unsigned lds_u1(unsigned p) {
 // Elementary functions of small arguments.
 // ---------------------------------------------------------------------------
 
-constexpr double kNearTan = 0.125;  // largest |tan| / angle of the series below
+constexpr double kNearTan = 0.125;   // largest |tan| / angle of the series below
+constexpr double kNearSin = 0.0625;  // largest |sin| of colat_near's
 
 // y / x for x > 0 finite: hardware reciprocal estimate, one Newton step and a
 // residual correction (Markstein, IBM J. Res. Dev. 34(1), 1990).
@@ -757,6 +759,11 @@ __device__ __noinline__ void prepare_sample(const KArgs& a, long long b, bool ha
   }
   sb.ir_lo = ir_lo;
   sb.nr = nr;
+  // where the short series end; the nearest rule's cosine holds for half a pixel of
+  // rings of 157 pixels (kCosSmallMax)
+  sb.wide = rbeam > kNearSin - 0.001 || rbeam > (kNearTan - 0.001) * sb.su ||
+            (eb != nullptr && nr > 0 && 4 * min(ir_lo, (int)(4 * a.nside) - (ir_lo + nr - 1)) < 158) ||
+            (eb != nullptr && a.nside < 40);
 }
 
 // Two beam pixels (or one) in the sample's frame.  The rotation is read from
@@ -1140,8 +1147,7 @@ __device__ __forceinline__ long long ring_above(long long nside, double z) {
 
 // theta_q - theta_u of a query z from sin(theta_q - theta_u) = cos(theta_u)
 // sin(theta_q) - z sin(theta_u) and the arcsine series for angles under
-// kNearSin (the first term left out, 231/13312 d^13, is below 2e-18 there).
-constexpr double kNearSin = 0.0625;
+// kNearSin (the first term left out, 231/13312 d^13, is below 4e-18 there).
 __device__ __forceinline__ double colat_near(double z, double cu, double su, double& d) {
   d = fma(cu, sqrt_near((1.0 - z) * (1.0 + z)), -z * su);
   const double d2 = d * d;
@@ -1262,18 +1268,39 @@ struct Place {
   double w[4];
 };
 
-// Regions of the sky whose ring above a query is found by one formula.
-constexpr int kBelt = 0;     // all window rings within the belt |z| <= 2/3 (and of one length)
+// Forms of the pixel loops, by where a sample's window lies.
+constexpr int kBelt = 0;      // all rings within the belt |z| <= 2/3 (and of one length)
 constexpr int kAnywhere = 1;
+// Footprints whose pixels are mostly beyond the short series -- wider than 3.6
+// degrees in colatitude or 7 in longitude, so near the poles too --, and for the
+// nearest rule rings of fewer than 157 pixels: the same with atan2 and acos where the
+// series end.  Without it these went through the direct evaluation after a table had
+// been filled for them: 2000 pixels of a 10 degree disc, nside 64, 10,000 samples
+// 1976 -> 518 us; nearest at nside 16, 1560 -> 427; a 30' beam within 6 degrees of the
+// pole, nside 1024, 20,000 samples 1823 -> 1010, nearest 1927 -> 1230 (calls, with
+// their host part).
+constexpr int kWide = 2;
 
 // Place of a beam pixel: false when the query is not near the frame's origin
 // in longitude, not between two rings of the window or not among their slots.
 // Straight-line code, so that two pixels' chains interleave.
 template <int REGION>
-__device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin, int nside, double cu, double su,
-                                            double belt_inv, double x, double y, double z, Place& o) {
+__device__ __forceinline__ bool frame_position(double x, double y, double& rel) {
   const double t = div_near(y, x);
-  const double rel = atan_near(t);
+  if constexpr (REGION == kWide) {
+    rel = lon_is_near(x, t) ? atan_near(t) : atan2(y, x);
+    // not finite, or on the axis: evaluated directly
+    return fabs(x) < 1e300 && fabs(y) < 1e300 && (x != 0.0 || y != 0.0);
+  } else {
+    rel = atan_near(t);
+    return lon_is_near(x, t);
+  }
+}
+template <int REGION>
+__device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin, int nside, double theta_u, double cu,
+                                            double su, double belt_inv, double x, double y, double z, Place& o) {
+  double rel;
+  const bool near = frame_position<REGION>(x, y, rel);
   double rc = (double)nside * fma(-1.5, z, 2.0);
   int r;
   if constexpr (REGION == kBelt) {
@@ -1287,7 +1314,7 @@ __device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin,
   }
   r -= ir_lo;
   // (|z| >= 1 or NaN gives a ring outside every window)
-  const bool in = lon_is_near(x, t) && (unsigned)r < (unsigned)nwin;
+  const bool in = near && (unsigned)r < (unsigned)nwin;
   const unsigned ra = rings + 80u * (in ? (unsigned)r : 0u);
   double2 f0, f1;
   if constexpr (REGION == kBelt) {
@@ -1303,7 +1330,8 @@ __device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin,
   const bool in_a = slot_of(lds_u1(ra + 64), ja, 2, ia), in_b = slot_of(lds_u1(ra + 144), jb, 2, ib);
   const double xa = ua - (double)ja, xb = ub - (double)jb;
   double d;
-  const double rel_th = colat_near(z, cu, su, d);
+  double rel_th = colat_near(z, cu, su, d);
+  if (REGION == kWide && !sin_is_near(d)) rel_th = acos(z) - theta_u;
   const double2 ti = lds_d2(ra + 16);
   const double wb = (rel_th - ti.x) * ti.y;
   const double wa = 1.0 - wb;
@@ -1313,7 +1341,7 @@ __device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin,
   o.w[1] = wa * xa;
   o.w[2] = wb * (1.0 - xb);
   o.w[3] = wb * xb;
-  return in && in_a && in_b && sin_is_near(d);
+  return in && in_a && in_b && (REGION == kWide || sin_is_near(d));
 }
 
 // A placed pixel's contribution from the table.
@@ -1357,6 +1385,11 @@ __device__ __forceinline__ double nearest_term(const Chan<LAYOUT>& ch, int c, Va
   }
 }
 
+// Pixel j of a ring of n as the one within half a turn of the frame's origin.
+__device__ __forceinline__ int near_turn(int j, int n) {
+  return j > n / 2 ? j - n : (j <= -(n / 2) ? j + n : j);
+}
+
 // The nearest rule as the reference evaluates it: its own rotation, atan2,
 // four candidates ranked by cos().  Out of line.
 template <int PM, bool HAS_QU, typename MapT, int LAYOUT, typename VecT>
@@ -1385,12 +1418,7 @@ __device__ __noinline__ Contrib nearest_exact(const KArgs& a, const SampleBlock*
     int k0;
     double f0;
     ring_origin(sb->phi_u, r.phi0, r.dphi, r.inv_dphi, k0, f0);
-    int j = (int)nb.ip - k0;
-    if (j > r.n / 2)
-      j -= r.n;
-    else if (j < -(r.n / 2))
-      j += r.n;
-    dphi = pixel_dphi(sb->bdl, f0, j, r.dphi);
+    dphi = pixel_dphi(sb->bdl, f0, near_turn((int)nb.ip - k0, r.n), r.dphi);
   }
   const Vals<ValT<MapT>> o = pixel_vals<PM, HAS_QU, MapT, LAYOUT>(ch, MapRef{a.map, a.map_stride}, bo, nb.zc,
                                                                   sqrt(max0(1.0 - nb.zc * nb.zc)), dphi, nb.pix);
@@ -1423,8 +1451,8 @@ template <int REGION>
 __device__ __forceinline__ bool place_nearest(unsigned rings, int ir_lo, int nwin, int nside, double x, double y,
                                               double z, NearPlace& o) {
   constexpr double kEdge = 1e-9;
-  const double t = div_near(y, x);
-  const double rel = atan_near(t);
+  double rel;
+  const bool near = frame_position<REGION>(x, y, rel);
   double rc = (double)nside * (2.0 - 1.5 * z);
   bool south = false;
   if constexpr (REGION != kBelt) {
@@ -1439,7 +1467,7 @@ __device__ __forceinline__ bool place_nearest(unsigned rings, int ir_lo, int nwi
   if (south) r = 4 * nside - r - 1;
   r -= ir_lo;
   // (|z| >= 1 or NaN gives a ring outside every window)
-  const bool in = lon_is_near(x, t) && (unsigned)r < (unsigned)nwin;
+  const bool in = near && (unsigned)r < (unsigned)nwin;
   const unsigned ra = rings + 80u * (in ? (unsigned)r : 0u);
   const double2 fa = lds_d2(ra), fb = lds_d2(ra + 80);
   const double ua = fma(rel, fa.y, fa.x), ub = fma(rel, fb.y, fb.x);
@@ -1448,18 +1476,27 @@ __device__ __forceinline__ bool place_nearest(unsigned rings, int ir_lo, int nwi
   const double la = ea * lds_d1(ra + 56), lb = eb * lds_d1(ra + 136);
   const double2 za = lds_d2(ra + 32), zb = lds_d2(ra + 112);
   const double sin_th = sqrt_near(fma(x, x, y * y));
-  const double ca = fma(sin_th * za.y, cos_small(la), z * za.x);
-  const double cb = fma(sin_th * zb.y, cos_small(lb), z * zb.x);
+  double cla, clb;
+  if constexpr (REGION == kWide) {
+    double sine;
+    sincos_near(la, sine, cla);
+    sincos_near(lb, sine, clb);
+  } else {
+    cla = cos_small(la);
+    clb = cos_small(lb);
+  }
+  const double ca = fma(sin_th * za.y, cla, z * za.x);
+  const double cb = fma(sin_th * zb.y, clb, z * zb.x);
   const bool b = cb > ca;
   o.ring = ra + (b ? 80u : 0u);
   o.j = b ? jb : ja;
   return in && fabs(rf - 0.5) < 0.5 - kEdge && fmax(fabs(ea), fabs(eb)) < 0.5 - kEdge &&
-         fmax(fabs(la), fabs(lb)) <= kCosSmallMax && fabs(ca - cb) > 1e-13;
+         fmax(fabs(la), fabs(lb)) <= (REGION == kWide ? kNearTan : kCosSmallMax) && fabs(ca - cb) > 1e-13;
 }
 
 // A placed pixel's contribution: from the table, or from the map where the
 // launch has no table; false when the table does not hold the pixel.
-template <int PM, bool HAS_QU, typename MapT, int LAYOUT, class Acc>
+template <int REGION, int PM, bool HAS_QU, typename MapT, int LAYOUT, class Acc>
 __device__ __forceinline__ bool add_nearest(const Chan<LAYOUT>& ch, const MapRef& map, const Bore& bo, double bdl,
                                             const ValTable<MapT, LAYOUT>& tab, bool table, const NearPlace& o,
                                             const float* bv, Acc& acc) {
@@ -1477,8 +1514,14 @@ __device__ __forceinline__ bool add_nearest(const Chan<LAYOUT>& ch, const MapRef
     if constexpr (HAS_QU) {
       const double2 zs = lds_d2(o.ring + 32);
       double c2, s2;
-      if (!spin2_small<PM>(zs.x, zs.y, pixel_dphi(bdl, lds_d1(o.ring), o.j, lds_d1(o.ring + 56)), bo, c2, s2))
-        return false;
+      const int j = REGION == kWide ? near_turn(o.j, n) : o.j;
+      const double dphi = pixel_dphi(bdl, lds_d1(o.ring), j, lds_d1(o.ring + 56));
+      if (!spin2_small<PM>(zs.x, zs.y, dphi, bo, c2, s2)) {
+        if constexpr (REGION != kWide) return false;
+        const double2 far = spin2_far(zs.x, zs.y, dphi, bo.z, bo.sth);
+        c2 = far.x;
+        s2 = far.y;
+      }
       v = turned_vals<MapT, LAYOUT>(ch, map, p, c2, s2);
     } else {
       v = raw_vals<MapT, LAYOUT>(ch, map, p);
@@ -1508,14 +1551,14 @@ __device__ __forceinline__ bool add_nearest(const Chan<LAYOUT>& ch, const MapRef
 // (radius rbeam) reaches 2 asin(sqrt((sin^2(rbeam / 2) - sin^2(d / 2)) /
 // (sin theta_u sin theta_q))) in longitude (2% margin), H pixels, and the
 // query's two neighbours lie between -floor(f0 + H) - 1 and floor(f0 + H) + 1.
-// Near the poles the
-// ring table's reservation for any footprint of its reach is taken.  (A
-// pixel outside its ring's slots is still evaluated, directly; only the cost
-// changes.)
+// (A ring that the disc holds whole comes out whole.)  The first rings about a pole
+// take the ring table's reservation for any footprint of its reach.  (A pixel
+// outside its ring's slots is still evaluated, directly; only the cost changes.)
 template <int MODE>
 __device__ __noinline__ void footprint_window(const RingRec* rt0, const SampleBlock* sb, int nside, int tab_cap,
                                               float rbeam, RingWin* rings, int* ring_end, unsigned short* ring_of,
-                                              int4* s_hdr) {
+                                              int4* s_hdr) {  // x first ring, y rings with a next one (0: no window),
+                                                              // z table slots (0: no table)
   const int nr = sb->nr, ir_lo = sb->ir_lo;
   const RingRec* rt = rt0 + ir_lo;
   const double theta_u = sb->theta_u, phi_u = sb->phi_u;
@@ -1536,7 +1579,6 @@ __device__ __noinline__ void footprint_window(const RingRec* rt0, const SampleBl
   }
   const int lane = threadIdx.x;
   const float spacing = 0.9f / (float)nside;  // the widest step between rings
-  const bool disc = theta_u - rbeam > 0.1 && theta_u + rbeam < kPi - 0.1;
   const float hr = __sinf(0.5f * rbeam), inv_su = 1.f / (float)sb->su;
   int carry = 0;
   for (int b0 = 0; b0 < nr; b0 += 32) {
@@ -1551,10 +1593,11 @@ __device__ __noinline__ void footprint_window(const RingRec* rt0, const SampleBl
       rings[t].f0 = f0;
       rings[t].k0 = k0;
       own = __ldg(&r->cap);
-      if (disc) {
+      const float sq = (float)__ldg(&r->sth) - spacing;
+      if (sq > 2.f * spacing) {
         const float d = fmaxf(0.f, fabsf((float)(__ldg(&r->ta) - theta_u)) - spacing);
         const float hd = __sinf(0.5f * d);
-        const float q = fmaxf(0.f, hr * hr - hd * hd) * inv_su / ((float)__ldg(&r->sth) - spacing);
+        const float q = fmaxf(0.f, hr * hr - hd * hd) * inv_su / sq;
         const float H = 2.04f * asinf(fminf(1.f, sqrtf(q))) * (float)inv;
         own = min(own, 2 * (int)((float)f0 + H) + 3);
       }
@@ -1638,7 +1681,7 @@ __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LA
                                                      int ir_lo, int nwin, LoopState<Acc> st) {
   const PixelLoop<MapT, LAYOUT, VecT> p = *sp;
   const unsigned sb = smem_u32(blk);
-  const double cu = blk->cu, su = blk->su, belt_inv = lds_d1(p.rings + 8);
+  const double theta_u = blk->theta_u, cu = blk->cu, su = blk->su, belt_inv = lds_d1(p.rings + 8);
   int s = st.s;
   Acc acc = st.acc;
 #pragma unroll 1
@@ -1654,7 +1697,7 @@ __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LA
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 2; ++k)
-      ok = place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, cu, su, belt_inv, x[k], y[k], z[k], o[k]) && ok;
+      ok = place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, theta_u, cu, su, belt_inv, x[k], y[k], z[k], o[k]) && ok;
     if (!ok) break;
     add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[0], __ldg(p.vals + s), acc);
     add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[1], __ldg(p.vals + s + kSumLanes), acc);
@@ -1664,7 +1707,7 @@ __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LA
     rotate_frame<1>(sb, p.vec, {s * p.ss}, &x, &y, &z);
     if (REGION != kBelt && PM == kParamsRef32 && is_polar(z)) z = polar_z(sb, p.vec, s * p.ss);
     Place o;
-    if (place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, cu, su, belt_inv, x, y, z, o)) {
+    if (place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, theta_u, cu, su, belt_inv, x, y, z, o)) {
       add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o, __ldg(p.vals + s), acc);
       s += kSumLanes;
     }
@@ -1693,8 +1736,8 @@ __device__ __forceinline__ LoopState<Acc> nearest_loop(const PixelLoop<MapT, LAY
     for (int k = 0; k < 2; ++k)
       ok = place_nearest<REGION>(p.rings, ir_lo, nwin, p.nside, x[k], y[k], z[k], o[k]) && ok;
     if (!ok) break;
-    if (!add_nearest<PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o[0], p.vals + s, acc)) break;
-    if (!add_nearest<PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o[1], p.vals + s + kSumLanes,
+    if (!add_nearest<REGION, PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o[0], p.vals + s, acc)) break;
+    if (!add_nearest<REGION, PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o[1], p.vals + s + kSumLanes,
                                                acc)) {
       s += kSumLanes;
       break;
@@ -1705,7 +1748,7 @@ __device__ __forceinline__ LoopState<Acc> nearest_loop(const PixelLoop<MapT, LAY
     rotate_frame<1>(sb, p.vec, {s * p.ss}, &x, &y, &z);
     NearPlace o;
     if (place_nearest<REGION>(p.rings, ir_lo, nwin, p.nside, x, y, z, o) &&
-        add_nearest<PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o, p.vals + s, acc))
+        add_nearest<REGION, PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, bdl, p.tab, table, o, p.vals + s, acc))
       s += kSumLanes;
   }
   st.acc = acc;
@@ -1713,9 +1756,20 @@ __device__ __forceinline__ LoopState<Acc> nearest_loop(const PixelLoop<MapT, LAY
   return st;
 }
 
+// Out of line: the calls inside would spill the other forms' registers.
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+__device__ __noinline__ LoopState<Acc> wide_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
+                                                 int ir_lo, int nwin, bool table, LoopState<Acc> st) {
+  if constexpr (MODE == TODGPU_NEAREST)
+    return nearest_loop<kWide, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, table, st);
+  else
+    return bilinear_loop<kWide, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, st);
+}
+
 template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
 __device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
                                                      const int4& hdr, int nside, const LoopState<Acc>& st) {
+  if (sb->wide) return wide_loop<MODE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, hdr.z > 0, st);
   // the window's rings all in the belt (rings nside to 3 nside)?
   const bool belt = hdr.x >= nside && hdr.x + hdr.y <= 3 * nside;
   if constexpr (MODE == TODGPU_NEAREST) {
