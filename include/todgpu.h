@@ -143,9 +143,15 @@ typedef struct todgpu_gather_args {
  * and tod_nearest._gather_accum_nearest_jit (tod_nearest.py:21-158).
  * vec_orig must be aligned to its element size and beam_vals to 4 bytes;
  * S is at most 2^29.  Beams of more than 16384 pixels run in passes of 1024
- * consecutive pixels, each with its own footprint: order such a beam so that
- * neighbours on the sky follow each other. */
+ * consecutive pixels (4096 without Q and U), each with its own footprint:
+ * order such a beam so that neighbours on the sky follow each other. */
 int todgpu_gather_accum(const todgpu_gather_args *args, void *stream);
+
+/* HOST function: the window rings and table slots (0: no table of pixel values,
+ * the map is read per beam pixel) that a launch reserves for one call's arguments.
+ * Tables and windows decide speed, never results.  No counterpart in the
+ * reference. */
+int todgpu_gather_wants(const todgpu_gather_args *args, int32_t *rings, int32_t *slots);
 
 /* Number of bounded waits of the gather kernels that ran out since the library
  * was loaded: always 0, as they wait on nothing but their own CTA's barriers.

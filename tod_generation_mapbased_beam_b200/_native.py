@@ -127,6 +127,8 @@ def _declare(lib):
     lib.todgpu_spin2.restype = ctypes.c_int
     lib.todgpu_boresight_phi_host.argtypes = [_p, _i64, _p, _i32]
     lib.todgpu_boresight_phi_host.restype = ctypes.c_int
+    lib.todgpu_gather_wants.argtypes = [ctypes.POINTER(GatherArgs), ctypes.POINTER(_i32), ctypes.POINTER(_i32)]
+    lib.todgpu_gather_wants.restype = ctypes.c_int
     lib.todgpu_host_hash.argtypes = [_p, ctypes.c_size_t, ctypes.c_uint64]
     lib.todgpu_host_hash.restype = ctypes.c_uint64
     lib.todgpu_ring_table_bytes.argtypes = [_i64]
@@ -226,6 +228,7 @@ def exported_symbols():
         "todgpu_gather_accum_batched",
         "todgpu_gather_accum_static",
         "todgpu_gather_wait_timeouts",
+        "todgpu_gather_wants",
         "todgpu_bilinear_stencils",
         "todgpu_get_interp_weights",
         "todgpu_ang2pix",

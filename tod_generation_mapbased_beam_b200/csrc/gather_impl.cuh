@@ -13,11 +13,12 @@
 //      ring in the sample's own longitude frame (footprint_window);
 //   3. evaluates the map once per footprint pixel into shared memory: I, and Q
 //      and U turned into the boresight's frame (fill_table; a map pixel is
-//      shared by ~10 (beam pixel, neighbour) pairs of a sample);
+//      shared by ~10 (beam pixel, neighbour) pairs of a sample) -- where that
+//      pays (table_pays); other launches are kernels of their own, without it;
 //   4. strides its threads over the beam pixels: rotation into the frame ->
 //      longitude by a short series -> ring and in-ring position from the window
-//      -> weighted sum of four table entries (bilinear_table) or the nearest
-//      one (nearest_window);
+//      -> weighted sum of four table entries, or of four map pixels
+//      (bilinear_loop), or the nearest one (nearest_loop);
 //   5. reduces the per-lane sums (256 summation lanes in either CTA shape) in a
 //      fixed order and adds them into tod[c, b] (one writer per sample: no
 //      atomics, bit-reproducible runs, the same TOD in every shape).
@@ -48,7 +49,10 @@
 
 namespace todgpu {
 
-constexpr int kRingCap = 192;   // rings per footprint window, at most
+// Rings per footprint window: of a call that names no footprint, of a call's
+// request at most, and of a beam in chunks without a table (three CTAs of 256 threads
+// an SM still hold that window).
+constexpr int kRingCap = 192, kRingMax = 2048, kRingChunk = 448;
 constexpr int kTabCapDefault = 2048;  // table slots per sample when the caller asks for none
 constexpr long long kMaxNside = 16384;
 // Summation lanes of the gather: the beam pixels of a sample are summed in
@@ -431,7 +435,8 @@ struct __align__(16) SampleBlock {
   double oma;                                                // 1 - cos a
   float fkx, fky, fkz, fca, fsa;                             // reference float32 recentring
   int wide;                                                  // the pixel loop's form is kWide
-  float fpad0, fpad1;
+  int far;                                                   // without a table: also where Q and U are turned there
+  float fpad;
   double bz, bsth, bdl;                                      // boresight: z, sin theta, longitude - phi_u in [-pi, pi]
   double phi_u, theta_u;                                     // rotated beam centre
   int ir_lo, nr;                                             // window rings (nr = 0: none)
@@ -512,6 +517,11 @@ __device__ __forceinline__ double lds_d1(unsigned p) {
 __device__ __forceinline__ float4 lds_f4(unsigned p) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 lds_u4(unsigned p) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(p));
   return v;
 }
 __device__ __forceinline__ unsigned lds_u1(unsigned p) {
@@ -666,7 +676,7 @@ __device__ __forceinline__ void rodrigues_matrix(double x, double y, double z, d
   m[8] = fma(oz, z, c);
 }
 
-template <int PM>
+template <int PM, bool TABLE>
 __device__ __noinline__ void prepare_sample(const KArgs& a, long long b, bool has_qu, double cx, double cy, double cz,
                                             double rbeam, bool window, double polar, SampleBlock& sb,
                                             ExactBlock* eb) {
@@ -764,6 +774,7 @@ __device__ __noinline__ void prepare_sample(const KArgs& a, long long b, bool ha
   sb.wide = rbeam > kNearSin - 0.001 || rbeam > (kNearTan - 0.001) * sb.su ||
             (eb != nullptr && nr > 0 && 4 * min(ir_lo, (int)(4 * a.nside) - (ir_lo + nr - 1)) < 158) ||
             (eb != nullptr && a.nside < 40);
+  if (!TABLE) sb.far = sb.wide || (has_qu && fabs(bdl) * sb.su + rbeam > kNearTan * sb.su);
 }
 
 // Two beam pixels (or one) in the sample's frame.  The rotation is read from
@@ -1261,10 +1272,12 @@ __device__ __noinline__ Contrib bilinear_direct(const KArgs& a, const SampleBloc
   return out;
 }
 
-// Where a beam pixel falls in the sample's table: the slots left of it on the
-// ring above and the ring below, and the four weights.
+// Where a beam pixel falls: its left neighbours on the ring above and the ring
+// below -- their slots in the sample's table, or (without a table) the pixels
+// relative to the frame's origin --, the ring above's record and the four weights.
 struct Place {
   int ia, ib;
+  unsigned ra;
   double w[4];
 };
 
@@ -1282,7 +1295,8 @@ constexpr int kAnywhere = 1;
 constexpr int kWide = 2;
 
 // Place of a beam pixel: false when the query is not near the frame's origin
-// in longitude, not between two rings of the window or not among their slots.
+// in longitude, not between two rings of the window or (TABLE) not among their
+// slots.
 // Straight-line code, so that two pixels' chains interleave.
 template <int REGION>
 __device__ __forceinline__ bool frame_position(double x, double y, double& rel) {
@@ -1296,7 +1310,7 @@ __device__ __forceinline__ bool frame_position(double x, double y, double& rel) 
     return lon_is_near(x, t);
   }
 }
-template <int REGION>
+template <int REGION, bool TABLE>
 __device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin, int nside, double theta_u, double cu,
                                             double su, double belt_inv, double x, double y, double z, Place& o) {
   double rel;
@@ -1326,8 +1340,12 @@ __device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin,
   }
   const double ua = fma(rel, f0.y, f0.x), ub = fma(rel, f1.y, f1.x);
   const int ja = __double2int_rd(ua), jb = __double2int_rd(ub);
-  int ia, ib;
-  const bool in_a = slot_of(lds_u1(ra + 64), ja, 2, ia), in_b = slot_of(lds_u1(ra + 144), jb, 2, ib);
+  int ia = ja, ib = jb;
+  bool in_a = true, in_b = true;
+  if constexpr (TABLE) {
+    in_a = slot_of(lds_u1(ra + 64), ja, 2, ia);
+    in_b = slot_of(lds_u1(ra + 144), jb, 2, ib);
+  }
   const double xa = ua - (double)ja, xb = ub - (double)jb;
   double d;
   double rel_th = colat_near(z, cu, su, d);
@@ -1337,6 +1355,7 @@ __device__ __forceinline__ bool place_pixel(unsigned rings, int ir_lo, int nwin,
   const double wa = 1.0 - wb;
   o.ia = ia;
   o.ib = ib;
+  o.ra = ra;
   o.w[0] = wa * (1.0 - xa);
   o.w[1] = wa * xa;
   o.w[2] = wb * (1.0 - xb);
@@ -1358,6 +1377,58 @@ __device__ __forceinline__ void add_placed(const Chan<LAYOUT>& ch, const ValTabl
     if (c >= ch.C) break;
     accumulate<MapT>(acc, c, mix.t[c], bvf);
   }
+}
+
+// A placed pixel's contribution from the map; false when a neighbour is too far
+// from the boresight in longitude for the form.
+template <int REGION, int PM, bool HAS_QU, typename MapT, int LAYOUT, class Acc>
+__device__ __forceinline__ bool add_from_map(const Chan<LAYOUT>& ch, const MapRef& map, const Bore& bo, double bdl,
+                                             const Place& o, float bvf, Acc& acc) {
+  Mix<MapT, LAYOUT, HAS_QU> mix;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const unsigned r = o.ra + 80u * h;
+    const uint4 g = lds_u4(r + 64);  // k0 in y, n in z
+    const double2 fd = lds_d2(r + 48);
+    const long long first = __double_as_longlong(fd.x);
+    const int j = h == 0 ? o.ia : o.ib, n = (int)g.z;
+    int ip = (int)g.y + j;  // (j up to half a turn and two pixels either way)
+    ip += ip < 0 ? n : 0;
+    ip -= ip >= n ? n : 0;
+    ip -= ip >= n ? n : 0;
+    const int in = ip + 1 == n ? 0 : ip + 1;
+    double2 zs = make_double2(0.0, 0.0);
+    double f0 = 0.0;
+    if constexpr (HAS_QU) {
+      zs = lds_d2(r + 32);
+      f0 = lds_d1(r);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const long long p = first + (k == 0 ? ip : in);
+      Vals<ValT<MapT>> v;
+      if constexpr (HAS_QU) {
+        const double dphi = pixel_dphi(bdl, f0, j + k, fd.y);
+        double c2, s2;
+        if (!spin2_small<PM>(zs.x, zs.y, dphi, bo, c2, s2)) {
+          if constexpr (REGION != kWide) return false;
+          const double2 away = spin2_far(zs.x, zs.y, dphi, bo.z, bo.sth);
+          c2 = away.x;
+          s2 = away.y;
+        }
+        v = turned_vals<MapT, LAYOUT>(ch, map, p, c2, s2);
+      } else {
+        v = raw_vals<MapT, LAYOUT>(ch, map, p);
+      }
+      mix.add(ch, h + k == 0, o.w[2 * h + k], v);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c >= ch.C) break;
+    accumulate<MapT>(acc, c, mix.t[c], bvf);
+  }
+  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1540,6 +1611,33 @@ __device__ __forceinline__ bool add_nearest(const Chan<LAYOUT>& ch, const MapRef
 // One sample's window and table.
 // ---------------------------------------------------------------------------
 
+__device__ __forceinline__ void copy_ring(const RingRec* r, double theta_u, RingWin& w) {
+  w.inv_dphi = __ldg(&r->inv_dphi);
+  w.rta = __ldg(&r->ta) - theta_u;
+  w.z = __ldg(&r->z);
+  w.sth = __ldg(&r->sth);
+  w.inv_dta = __ldg(&r->inv_dta);
+  w.first = __ldg(&r->first);
+  w.dphi = __ldg(&r->dphi);
+  w.n = __ldg(&r->n);
+}
+
+// Window of one sample without a table, by the whole CTA.
+static __device__ __noinline__ void plain_window(const RingRec* rt0, const SampleBlock* sb, RingWin* rings,
+                                                 int4* s_hdr) {
+  const int nr = sb->nr;
+  for (int t = threadIdx.x; t < nr; t += blockDim.x) {
+    const RingRec* r = rt0 + sb->ir_lo + t;
+    int k0;
+    double f0;
+    ring_origin(sb->phi_u, __ldg(&r->phi0), __ldg(&r->dphi), __ldg(&r->inv_dphi), k0, f0);
+    rings[t].f0 = f0;
+    rings[t].k0 = k0;
+    copy_ring(r, sb->theta_u, rings[t]);
+  }
+  if (threadIdx.x == 0) *s_hdr = make_int4(sb->ir_lo, nr > 0 ? nr - 1 : 0, 0, 0);
+}
+
 // Window of one sample, by the whole CTA: warp 0 places each ring in the
 // sample's frame, counts its slots and lays them out, the other warps copy the
 // rings' geometry.  ring_end[t] is the first slot past ring t, ring_of[i] the
@@ -1563,18 +1661,7 @@ __device__ __noinline__ void footprint_window(const RingRec* rt0, const SampleBl
   const RingRec* rt = rt0 + ir_lo;
   const double theta_u = sb->theta_u, phi_u = sb->phi_u;
   if (threadIdx.x >= 32) {
-    for (int t = threadIdx.x - 32; t < nr; t += blockDim.x - 32) {
-      const RingRec* r = rt + t;
-      RingWin& w = rings[t];
-      w.inv_dphi = __ldg(&r->inv_dphi);
-      w.rta = __ldg(&r->ta) - theta_u;
-      w.z = __ldg(&r->z);
-      w.sth = __ldg(&r->sth);
-      w.inv_dta = __ldg(&r->inv_dta);
-      w.first = __ldg(&r->first);
-      w.dphi = __ldg(&r->dphi);
-      w.n = __ldg(&r->n);
-    }
+    for (int t = threadIdx.x - 32; t < nr; t += blockDim.x - 32) copy_ring(rt + t, theta_u, rings[t]);
     return;
   }
   const int lane = threadIdx.x;
@@ -1650,7 +1737,7 @@ template <typename MapT, int LAYOUT, typename VecT>
 struct PixelLoop {
   const VecT* vec[3];  // component i of beam pixel s at vec[i][s ss]
   const float* vals;
-  MapRef map;          // nearest without a table
+  MapRef map;          // where there is no table
   unsigned rings;      // shared addresses of the window's rings and the table
   ValTable<MapT, LAYOUT> tab;
   int ss, n, nside;
@@ -1676,7 +1763,11 @@ struct LoopState {
 // table fill is 0.4 and the window 0.1; ~210 instructions an evaluation, 66 of
 // them float64, issue slots 57% and the shared-memory data path 60-70% busy:
 // leaving out 12 of 16 shared loads saved 5%, 22 of 66 float64 operations 13%.
-template <int REGION, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+// TABLE false: the same from the map (bound there: its loads, 12 a pixel with I, Q and
+// U, and L1, see choose_shape).  It stands in for the direct evaluation, one pixel at a
+// time out of line: 1000 pixels of a 45' beam at nside 4096, packed float32, 5000
+// samples 362 us direct, 291 now; 16,000 pixels, I alone, nside 8192, 30' 5090, 1920.
+template <int REGION, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
 __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LAYOUT, VecT>* sp, const SampleBlock* blk,
                                                      int ir_lo, int nwin, LoopState<Acc> st) {
   const PixelLoop<MapT, LAYOUT, VecT> p = *sp;
@@ -1697,19 +1788,35 @@ __device__ __forceinline__ LoopState<Acc> bilinear_loop(const PixelLoop<MapT, LA
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 2; ++k)
-      ok = place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, theta_u, cu, su, belt_inv, x[k], y[k], z[k], o[k]) && ok;
+      ok = place_pixel<REGION, TABLE>(p.rings, ir_lo, nwin, p.nside, theta_u, cu, su, belt_inv, x[k], y[k], z[k], o[k]) && ok;
     if (!ok) break;
-    add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[0], __ldg(p.vals + s), acc);
-    add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[1], __ldg(p.vals + s + kSumLanes), acc);
+    if constexpr (TABLE) {
+      add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[0], __ldg(p.vals + s), acc);
+      add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o[1], __ldg(p.vals + s + kSumLanes), acc);
+    } else {
+      const Bore bo{blk->bz, blk->bsth};
+      if (!add_from_map<REGION, PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, blk->bdl, o[0], __ldg(p.vals + s), acc))
+        break;
+      if (!add_from_map<REGION, PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, bo, blk->bdl, o[1],
+                                                          __ldg(p.vals + s + kSumLanes), acc)) {
+        s += kSumLanes;
+        break;
+      }
+    }
   }
   if (s < p.n) {
     double x, y, z;
     rotate_frame<1>(sb, p.vec, {s * p.ss}, &x, &y, &z);
     if (REGION != kBelt && PM == kParamsRef32 && is_polar(z)) z = polar_z(sb, p.vec, s * p.ss);
     Place o;
-    if (place_pixel<REGION>(p.rings, ir_lo, nwin, p.nside, theta_u, cu, su, belt_inv, x, y, z, o)) {
-      add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o, __ldg(p.vals + s), acc);
-      s += kSumLanes;
+    if (place_pixel<REGION, TABLE>(p.rings, ir_lo, nwin, p.nside, theta_u, cu, su, belt_inv, x, y, z, o)) {
+      if constexpr (TABLE) {
+        add_placed<HAS_QU, MapT, LAYOUT>(p.ch, p.tab, o, __ldg(p.vals + s), acc);
+        s += kSumLanes;
+      } else if (add_from_map<REGION, PM, HAS_QU, MapT, LAYOUT>(p.ch, p.map, Bore{blk->bz, blk->bsth}, blk->bdl, o,
+                                                                __ldg(p.vals + s), acc)) {
+        s += kSumLanes;
+      }
     }
   }
   st.acc = acc;
@@ -1757,28 +1864,31 @@ __device__ __forceinline__ LoopState<Acc> nearest_loop(const PixelLoop<MapT, LAY
 }
 
 // Out of line: the calls inside would spill the other forms' registers.
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
 __device__ __noinline__ LoopState<Acc> wide_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
                                                  int ir_lo, int nwin, bool table, LoopState<Acc> st) {
   if constexpr (MODE == TODGPU_NEAREST)
     return nearest_loop<kWide, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, table, st);
   else
-    return bilinear_loop<kWide, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, st);
+    return bilinear_loop<kWide, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, st);
 }
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
 __device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
                                                      const int4& hdr, int nside, const LoopState<Acc>& st) {
-  if (sb->wide) return wide_loop<MODE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, hdr.z > 0, st);
+  const bool table = TABLE && hdr.z > 0;
+  // (nearest: a launch's sample whose footprint its table does not hold reads the map
+  // there too, so that the loops below have one source of values)
+  if (TABLE ? sb->wide || (MODE == TODGPU_NEAREST && !table) : sb->far)
+    return wide_loop<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, table, st);
   // the window's rings all in the belt (rings nside to 3 nside)?
   const bool belt = hdr.x >= nside && hdr.x + hdr.y <= 3 * nside;
   if constexpr (MODE == TODGPU_NEAREST) {
-    const bool table = hdr.z > 0;
-    if (belt) return nearest_loop<kBelt, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, table, st);
-    return nearest_loop<kAnywhere, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, table, st);
+    if (belt) return nearest_loop<kBelt, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, TABLE, st);
+    return nearest_loop<kAnywhere, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, TABLE, st);
   } else {
-    if (belt) return bilinear_loop<kBelt, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, st);
-    return bilinear_loop<kAnywhere, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, st);
+    if (belt) return bilinear_loop<kBelt, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, st);
+    return bilinear_loop<kAnywhere, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, st);
   }
 }
 
@@ -1786,13 +1896,18 @@ __device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOU
 // The sample loop.
 // ---------------------------------------------------------------------------
 
-// Beams of more than kBeamChunkMin pixels run in chunks of kBeamChunk consecutive
-// pixels, each with its own centre, frame, window and table: a far-sidelobe
-// beam's whole footprint holds 1e5 to 1e6 map pixels, a chunk of a beam in
-// kernels.beam_order a patch that fits shared memory.  (Float64 sums only: the
-// order of the float32 Kahan sums is part of their result.)
+// Beams of more than kBeamChunkMin pixels run in chunks of beam_chunk consecutive
+// pixels, each with its own centre, frame and window: a far-sidelobe beam's whole
+// footprint holds 1e5 to 1e6 map pixels, a chunk of a beam in kernels.beam_order a
+// patch that fits a table.  (Float64 sums only: the order of the float32 Kahan sums is
+// part of their result.)  Without Q and U there is no table to fit, and longer chunks
+// prepare each sample less often (nearest, 100,000 pixels of 1 degree, nside 1024,
+// float32 parameters, 1000 samples: 1024 pixels 2285 us, 4096 1840; with Q and U 2797
+// and 1963, but 3430 and 5230 for an annulus of 3 to 10 degrees, whose map pixels then
+// leave L1).
 constexpr int kBeamChunkMin = 16384;
-constexpr int kBeamChunk = 1024;
+template <bool HAS_QU>
+constexpr int beam_chunk() { return HAS_QU ? 1024 : 4096; }
 
 // What a CTA keeps from sample to sample of a run besides the pixel loop's
 // state, in shared memory: in registers it was spilled, and an L1 that the tables
@@ -1816,7 +1931,7 @@ struct RunState {
 // beam entry over one batch of samples; tile t holds samples [t tile,
 // min(B, (t + 1) tile))), by the whole CTA.  All threads of the CTA must call
 // it together.
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT, bool TILES>
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT, bool TILES>
 __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, long long t_step, long long tile,
                             unsigned char* smem_raw, double* s_red, SampleBlock* s_blk, ExactBlock* s_exact,
                             int4* s_hdr) {
@@ -1843,7 +1958,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
   volatile RunState* run = &run_mem;
   if (tid == 0) run->nerr = 0;
   const int S = (int)a.S;
-  const int step = S > kBeamChunkMin && !MapTraits<MapT>::packed ? kBeamChunk : S;
+  const int step = S > kBeamChunkMin && !MapTraits<MapT>::packed ? beam_chunk<HAS_QU>() : S;
   for (int s0 = 0; s0 < S; s0 += step) {
     const int s1 = min(S, s0 + step);
     double cx, cy, cz, rbeam;
@@ -1853,7 +1968,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
     // a stencil neighbour's centre lies within 1.7/nside rad of its query (one
     // ring spacing plus one pixel width; the opposite pair around a pole
     // within twice the colatitude of ring 1)
-    const bool window = a.ring_table != nullptr && (MODE == TODGPU_NEAREST || a.tab_cap > 0) &&
+    const bool window = a.ring_table != nullptr &&
                         rbeam + 2.0 / (double)a.nside <= __ldg(&static_cast<const RingRec*>(a.ring_table)[0].ta);
     const int n = s1 - s0;
     if (tid == 0) {
@@ -1889,7 +2004,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
       if (tid < nq) {
         const long long b = TILES ? run->sample(q0 + tid) : t_begin + (q0 + tid) * t_step;
         if (TILES) run->b[tid] = b;
-        prepare_sample<PM>(a, b, HAS_QU, run->cx, run->cy, run->cz, run->rbeam, window, polar, s_blk[tid],
+        prepare_sample<PM, TABLE>(a, b, HAS_QU, run->cx, run->cy, run->cz, run->rbeam, window, polar, s_blk[tid],
                            s_exact != nullptr ? s_exact + tid : nullptr);
       }
       __syncthreads();
@@ -1901,11 +2016,14 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
         double* red = s_red + 16 * (i & 1);
         int4 hdr = make_int4(0, 0, 0, 0);
         if (window) {
-          footprint_window<MODE>(static_cast<const RingRec*>(a.ring_table), sb, nside, a.tab_cap, reach, rings,
-                                 ring_end, ring_of, s_hdr);
+          const RingRec* rt = static_cast<const RingRec*>(a.ring_table);
+          if constexpr (TABLE)
+            footprint_window<MODE>(rt, sb, nside, a.tab_cap, reach, rings, ring_end, ring_of, s_hdr);
+          else
+            plain_window(rt, sb, rings, s_hdr);
           __syncthreads();
           hdr = *s_hdr;
-          if (hdr.z > 0) {
+          if (TABLE && hdr.z > 0) {
             fill_table<PM, HAS_QU, MapT, LAYOUT>(ch, MapRef{a.map, a.map_stride}, sb, rings, ring_end, ring_of,
                                                  hdr.z, tab);
             __syncthreads();
@@ -1924,7 +2042,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
           // pixels that the window and table do not hold are evaluated here,
           // each in its place in the sum
           while (st.s < n) {
-            if (hdr.y > 0) st = pixel_loop<MODE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(loop, sb, hdr, nside, st);
+            if (hdr.y > 0) st = pixel_loop<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(loop, sb, hdr, nside, st);
             if (st.s < n) {
               const VecT* v = static_cast<const VecT*>(a.vec) + (s0 + (long long)st.s) * a.vec_ss;
               const float bvf = a.beam[s0 + st.s];
@@ -1990,14 +2108,14 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
   if (tid == 0 && a.err != nullptr && run->nerr) atomicAdd(a.err, run->nerr);
 }
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
 __global__ void __maxnreg__(kRegs) gather_accum_kernel(const __grid_constant__ KArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_red[(kSumLanes / 32) * 4];
   __shared__ SampleBlock s_blk[kPrep];
   __shared__ ExactBlock s_exact[MODE == TODGPU_NEAREST ? kPrep : 1];
   __shared__ int4 s_hdr;
-  run_samples<MODE, HAS_QU, MapT, PM, LAYOUT, false>(a, blockIdx.x, a.B, gridDim.x, 1, smem_raw, s_red, s_blk,
+  run_samples<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT, false>(a, blockIdx.x, a.B, gridDim.x, 1, smem_raw, s_red, s_blk,
                                                      MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
 }
 
@@ -2022,7 +2140,7 @@ struct BatchParams {
   KArgs job[kMaxBatchJobs];
 };
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
 __global__ void __maxnreg__(kRegs) gather_batched_kernel(const __grid_constant__ BatchParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_red[(kSumLanes / 32) * 4];
@@ -2041,7 +2159,7 @@ __global__ void __maxnreg__(kRegs) gather_batched_kernel(const __grid_constant__
         reinterpret_cast<unsigned long long*>(&s_job)[threadIdx.x] =
             reinterpret_cast<const unsigned long long*>(&p.job[j])[threadIdx.x];
       __syncthreads();
-      run_samples<MODE, HAS_QU, MapT, PM, LAYOUT, true>(s_job, t0, ntiles, G, p.tile, smem_raw, s_red, s_blk,
+      run_samples<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT, true>(s_job, t0, ntiles, G, p.tile, smem_raw, s_red, s_blk,
                                                         MODE == TODGPU_NEAREST ? s_exact : nullptr, &s_hdr);
     }
   }
@@ -2073,16 +2191,38 @@ constexpr size_t static_smem() {
   return kPrep * (sizeof(SampleBlock) + (MODE == TODGPU_NEAREST ? sizeof(ExactBlock) : 0)) + 1024;
 }
 
-// Window rings a launch reserves.  A request of N slots is a beam disc of
+// Window rings a launch reserves for a call.  A request of N slots is a beam disc of
 // radius r with at least 3.15 (r nside)^2 slots (kernels.footprint_slots), so r
 // nside <= sqrt(N / 3.15), and such a disc crosses at most 3 r nside + 4 rings
 // of the RING scheme (ring spacing at least 2 / (3 nside) in colatitude, plus
-// the rings either side); the default table reserves kRingCap.
-inline int ring_cap_for(int requested) {
-  if (requested <= 0) return kRingCap;
-  return std::min(kRingCap, (int)std::ceil(3.0 * std::sqrt(requested / 3.15)) + 6);
+// the rings either side); the default table reserves kRingCap.  A request is the
+// whole beam's: a chunk's window has fewer rings (kRingCap with its default table).
+inline int ring_cap_for(int requested, bool chunked, int slots) {
+  if (requested <= 0 || (chunked && slots > 0)) return kRingCap;
+  return std::min(chunked ? kRingChunk : kRingMax, (int)std::ceil(3.0 * std::sqrt(requested / 3.15)) + 6);
 }
 constexpr size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
+
+// Whether a value table of `slots` (`bytes` in all) pays for a pass over `pixels`
+// beam pixels.  Filling a slot costs a map read and a turned (Q, U), more as fewer
+// CTAs share an SM; a pixel read from the table saves four of them.  Bilinear, I, Q
+// and U, 5000 samples unless said, microseconds with the table / without:
+//   nside 2048, 30', 1263 slots (30 KB), 20,000 samples: 200 pixels 479 / 344,
+//     400 pixels 515 / 516, 1600 pixels 673 / 1022;
+//   nside 4096, 30', 4500 slots (108 KB): 1000 pixels 608 / 300, 4000 pixels
+//     802 / 642, 16,000 pixels 1548 / 2072;
+//   packed float32, nside 4096, 45', 9500 slots (114 KB): 4000 pixels 1057 / 668,
+//     16,000 pixels 1685 / 2201;
+//   I alone, nside 4096, 45', 80 KB: 4000 pixels 691 / 544, 16,000 pixels 1315 /
+//     1681; nside 8192, 30', 136 KB: 16,000 pixels 2323 / 1778.
+// So: as many slots a pixel as CTAs with such a table fit an SM, four at most.
+template <int MODE, bool HAS_QU>
+bool table_pays(long long slots, long long pixels, size_t bytes) {
+  // nearest reads one value per beam pixel: a table pays when the footprint
+  // has fewer pixels than the beam (and only for turned Q/U values)
+  if (MODE == TODGPU_NEAREST) return HAS_QU && slots <= pixels;
+  return slots <= (long long)std::min<size_t>(4, kSmemPerSM / (bytes + 8 * 1024)) * pixels;
+}
 
 // Shape of a launch: threads per CTA, window rings, table slots, dynamic
 // shared memory.
@@ -2096,15 +2236,21 @@ inline int ctas_per_sm(int nt, size_t smem) {  // smem: static and dynamic
   return (int)std::min<size_t>(kThreadsSM / nt, kSmemPerSM / per);
 }
 
-// What a launch asks for: the ring window and table request, slot bytes,
+// What a launch asks for: the window's rings and the table's slots, slot bytes,
 // components, samples, beam pixels per pass, the fewest threads per CTA.
 struct Wants {
-  bool window = false;
-  int requested = 0, slots = 0, slot = 0, C = 1;
+  int rings = 1, slots = 0, slot = 0, C = 1;
   long long samples = 0, pixels = 0;
   int min_nt = 128;
   size_t fixed = 0;  // static shared memory
+  bool map_reads = false;  // bilinear with a window
 };
+
+// Shared memory left for a table, and whether one of `slots` fits it.
+inline bool table_fits(int slots, int slot, size_t fixed, int rings) {
+  const size_t used = fixed + window_bytes(rings) + 1024;
+  return used < kSmemPerCTAMax && (size_t)slots <= (kSmemPerCTAMax - used) / (slot + 1);
+}
 
 inline Shape choose_shape(const Wants& w) {
   Shape best;
@@ -2112,14 +2258,17 @@ inline Shape choose_shape(const Wants& w) {
   for (int nt = w.min_nt; nt <= kSumLanes; nt *= 2) {
     Shape s;
     s.nt = nt;
-    s.ring_cap = w.window ? ring_cap_for(w.requested) : 1;
+    s.ring_cap = w.rings;
     const size_t xchg = nt > kMeanLanes ? sizeof(double) * kMeanLanes * (size_t)w.C : 0;
     const size_t head = window_bytes(s.ring_cap);
-    const size_t room = kSmemPerCTAMax - w.fixed - head - 1024;
-    // a table that no CTA can hold is not made (its samples would not fit it)
-    s.tab_cap = (size_t)w.slots <= room / (w.slot + 1) ? (w.slots + 1) & ~1 : 0;
+    s.tab_cap = table_fits(w.slots, w.slot, w.fixed, w.rings) ? (w.slots + 1) & ~1 : 0;
     s.smem = align16(head + ring_of_bytes(s.tab_cap) + std::max(xchg, (size_t)w.slot * s.tab_cap));
     const int threads = nt * ctas_per_sm(nt, s.smem + w.fixed);
+    // without a table bilinear reads the map itself: 256-thread CTAs have fewer
+    // samples in flight on an SM, whose footprints then stay in L1 (16,000 pixels of a
+    // 30' beam at nside 8192, 5000 samples: 5020 us in 128-thread CTAs, 2290; 1000
+    // pixels 297 and 316 at nside 4096)
+    if (w.map_reads && s.tab_cap == 0 && w.pixels >= 2048 && nt < kSumLanes) continue;
     const bool idle = w.samples * nt <= (long long)kThreadsSM * sm_count() && w.pixels >= nt;
     if (threads > best_threads || (threads == best_threads && idle)) {
       best = s;
@@ -2129,33 +2278,45 @@ inline Shape choose_shape(const Wants& w) {
   return best;
 }
 
-// Table slots of a launch (0: no value table): the caller's request, else
-// 32 KiB of the float64 or float32 pairs earlier versions kept.
+// A job's part in its launch: window rings, table slots (0: no value table).  The
+// request is the caller's, else 32 KiB of the float64 or float32 pairs earlier
+// versions kept.  A table that no CTA can hold is not made (no sample would fit it).
+struct JobWants {
+  int rings = 1, slots = 0;
+};
 template <int MODE, bool HAS_QU, typename MapT>
-int wanted_slots(const KArgs& k) {
-  if (k.ring_table == nullptr) return 0;
-  const bool chunked = k.S > kBeamChunkMin && !MapTraits<MapT>::packed;
-  const int req = k.tab_req > 0 && !chunked
-                      ? k.tab_req
-                      : (MapTraits<MapT>::packed ? 2 * kTabCapDefault : kTabCapDefault);
-  if (MODE == TODGPU_BILINEAR) return req;
-  // nearest reads one value per beam pixel: a table pays when the footprint
-  // has fewer pixels than the beam (and only for turned Q/U values)
-  return HAS_QU && req <= (chunked ? kBeamChunk : k.S) ? req : 0;
+JobWants job_wants(const KArgs& k) {
+  JobWants j;
+  if (k.ring_table == nullptr) return j;
+  constexpr bool packed = MapTraits<MapT>::packed;
+  const bool chunked = k.S > kBeamChunkMin && !packed;
+  const long long pixels = chunked ? beam_chunk<HAS_QU>() : k.S;
+  const int slot = slot_bytes(packed, k.C);
+  const int req = k.tab_req > 0 && !chunked ? k.tab_req : (packed ? 2 * kTabCapDefault : kTabCapDefault);
+  const bool holds = !chunked || (HAS_QU && (long long)k.tab_req * pixels <= req * (long long)k.S);
+  if (holds && table_pays<MODE, HAS_QU>(req, pixels, (size_t)req * slot)) j.slots = req;
+  j.rings = ring_cap_for(k.tab_req, chunked, j.slots);
+  if (!table_fits(j.slots, slot, static_smem<MODE>(), j.rings)) {
+    j.slots = 0;
+    j.rings = ring_cap_for(k.tab_req, chunked, 0);
+  }
+  return j;
 }
 
-// One job's part in what its launch asks for (the most any job does).
-template <int MODE, bool HAS_QU, typename MapT, int PM>
-void add_wants(Wants& w, const KArgs& k) {
-  const long long pixels = k.S > kBeamChunkMin && !MapTraits<MapT>::packed ? kBeamChunk : k.S;
-  w.window = w.window || k.ring_table != nullptr;
-  w.requested = std::max(w.requested, k.tab_req);
-  w.slots = std::max(w.slots, wanted_slots<MODE, HAS_QU, MapT>(k));
+// One job's part in what its launch asks for (the most any job does).  `tables`: the
+// launch has tables, and only the jobs with one decide on its window.
+template <int MODE, bool HAS_QU, typename MapT>
+void add_wants(Wants& w, const KArgs& k, bool tables) {
+  const JobWants j = job_wants<MODE, HAS_QU, MapT>(k);
+  if (!tables || j.slots > 0) w.rings = std::max(w.rings, j.rings);
+  w.slots = std::max(w.slots, j.slots);
   w.slot = slot_bytes(MapTraits<MapT>::packed, k.C);
   w.C = k.C;
   w.fixed = static_smem<MODE>();
+  w.map_reads = MODE == TODGPU_BILINEAR && k.ring_table != nullptr;
   w.samples += k.B;
-  w.pixels = std::max(w.pixels, pixels);
+  w.pixels = std::max(w.pixels, k.S > kBeamChunkMin && !MapTraits<MapT>::packed
+                                    ? (long long)beam_chunk<HAS_QU>() : (long long)k.S);
   w.min_nt = std::max(w.min_nt, k.flags_wide ? 256 : 128);
 }
 
@@ -2171,16 +2332,13 @@ int allow_smem(Kern kern, std::once_flag& once, cudaError_t& state) {
   return state == cudaSuccess ? TODGPU_OK : cuda_fail(state, "kernel shared-memory attributes");
 }
 
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
-int launch_gather(KArgs k, cudaStream_t stream) {
-  auto kern = gather_accum_kernel<MODE, HAS_QU, MapT, PM, LAYOUT>;
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_gather(KArgs k, const Wants& w, const Shape& s, cudaStream_t stream) {
+  auto kern = gather_accum_kernel<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT>;
   static std::once_flag once;
   static cudaError_t state = cudaSuccess;
   const int rc = allow_smem(kern, once, state);
   if (rc != TODGPU_OK) return rc;
-  Wants w;
-  add_wants<MODE, HAS_QU, MapT, PM>(w, k);
-  const Shape s = choose_shape(w);
   k.ring_cap = s.ring_cap;
   k.tab_cap = s.tab_cap;
   const long long max_blocks = (long long)sm_count() * ctas_per_sm(s.nt, s.smem + w.fixed);
@@ -2196,33 +2354,34 @@ static_assert(sizeof(KArgs) % 8 == 0 && sizeof(KArgs) / 8 <= 128, "KArgs copied 
 
 // Batched launch: descriptors of up to kMaxBatchJobs jobs per launch, in one
 // CTA shape, sized for the largest table any job asks for.
-template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
-int launch_batched(BatchParams& bp, cudaStream_t stream) {
-  auto kern = gather_batched_kernel<MODE, HAS_QU, MapT, PM, LAYOUT>;
+template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_shape(BatchParams& bp, const Wants& w, const Shape& s, cudaStream_t stream) {
+  auto kern = gather_batched_kernel<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT>;
   static std::once_flag once;
   static cudaError_t state = cudaSuccess;
   const int rc = allow_smem(kern, once, state);
   if (rc != TODGPU_OK) return rc;
-  const long long T = bp.tiles_before[bp.njobs];
-  if (T == 0) return TODGPU_OK;
-  Wants w;
-  bool any_default = false;
-  for (int j = 0; j < bp.njobs; ++j) {
-    add_wants<MODE, HAS_QU, MapT, PM>(w, bp.job[j]);
-    any_default = any_default || bp.job[j].tab_req == 0;
-  }
-  if (any_default) w.requested = 0;
-  const Shape s = choose_shape(w);
   for (int j = 0; j < bp.njobs; ++j) {
     bp.job[j].tab_cap = s.tab_cap;
     bp.job[j].ring_cap = s.ring_cap;
   }
   const long long max_blocks = (long long)sm_count() * ctas_per_sm(s.nt, s.smem + w.fixed);
-  const int grid = (int)std::max(1LL, std::min(T, max_blocks));
+  const int grid = (int)std::max(1LL, std::min(bp.tiles_before[bp.njobs], max_blocks));
   kern<<<grid, s.nt, s.smem, stream>>>(bp);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "gather_batched_kernel launch");
   return TODGPU_OK;
+}
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_batched(BatchParams& bp, cudaStream_t stream) {
+  if (bp.tiles_before[bp.njobs] == 0) return TODGPU_OK;
+  Wants w;
+  bool tables = false;
+  for (int j = 0; j < bp.njobs; ++j) tables = tables || job_wants<MODE, HAS_QU, MapT>(bp.job[j]).slots > 0;
+  for (int j = 0; j < bp.njobs; ++j) add_wants<MODE, HAS_QU, MapT>(w, bp.job[j], tables);
+  const Shape s = choose_shape(w);
+  return s.tab_cap > 0 ? launch_shape<MODE, true, HAS_QU, MapT, PM, LAYOUT>(bp, w, s, stream)
+                       : launch_shape<MODE, false, HAS_QU, MapT, PM, LAYOUT>(bp, w, s, stream);
 }
 
 // A batch in launches of jobs whose own shapes keep equally many threads on an
@@ -2235,12 +2394,12 @@ int launch_batched(BatchParams& bp, cudaStream_t stream) {
 // launch); smaller groups join the next narrower shape's.
 constexpr int kSplitWaves = 16;
 template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
-int launch_grouped(BatchParams& bp, cudaStream_t stream) {
+int launch_alike(BatchParams& bp, cudaStream_t stream) {
   int threads[kMaxBatchJobs], ctas[kMaxBatchJobs];  // threads and CTAs per SM of a job's own shape
   bool alike = true;
   for (int j = 0; j < bp.njobs; ++j) {
     Wants w;
-    add_wants<MODE, HAS_QU, MapT, PM>(w, bp.job[j]);
+    add_wants<MODE, HAS_QU, MapT>(w, bp.job[j], false);
     w.samples = 1LL << 40;
     const Shape s = choose_shape(w);
     ctas[j] = ctas_per_sm(s.nt, s.smem + w.fixed);
@@ -2289,6 +2448,46 @@ int launch_grouped(BatchParams& bp, cudaStream_t stream) {
   return TODGPU_OK;
 }
 
+// The jobs of bp that have a table (or have none), in order.
+template <int MODE, bool HAS_QU, typename MapT>
+void pick_jobs(const BatchParams& bp, bool table, BatchParams& out) {
+  out.njobs = 0;
+  out.tile = bp.tile;
+  out.tiles_before[0] = 0;
+  for (int j = 0; j < bp.njobs; ++j) {
+    if ((job_wants<MODE, HAS_QU, MapT>(bp.job[j]).slots > 0) != table) continue;
+    out.job[out.njobs] = bp.job[j];
+    out.tiles_before[out.njobs + 1] = out.tiles_before[out.njobs] + bp.tiles_before[j + 1] - bp.tiles_before[j];
+    ++out.njobs;
+  }
+}
+
+// Jobs without a table -- sparse beams, footprints beyond one CTA's memory -- have a
+// launch of their own where they are enough work for it, and never decide on the
+// others' table and window: one footprint too large for a table took it from every job
+// of its launch (six beams of 1500 pixels, 30', nside 2048, 20,000 samples each, alone
+// 3.29 ms; with a seventh of 8000 pixels and 2 degrees and 400 samples 9.91, now 4.98,
+// and 20,000 samples 17.7, now 11.0).
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_grouped(BatchParams& bp, cudaStream_t stream) {
+  int with = 0;
+  long long without = 0;  // tiles of the jobs without a table
+  for (int j = 0; j < bp.njobs; ++j) {
+    const bool table = job_wants<MODE, HAS_QU, MapT>(bp.job[j]).slots > 0;
+    with += table;
+    if (!table) without += bp.tiles_before[j + 1] - bp.tiles_before[j];
+  }
+  if (with == 0 || without < (long long)kSplitWaves * sm_count())
+    return launch_alike<MODE, HAS_QU, MapT, PM, LAYOUT>(bp, stream);
+  static thread_local BatchParams part;
+  for (const bool table : {true, false}) {
+    pick_jobs<MODE, HAS_QU, MapT>(bp, table, part);
+    const int rc = launch_alike<MODE, HAS_QU, MapT, PM, LAYOUT>(part, stream);
+    if (rc != TODGPU_OK) return rc;
+  }
+  return TODGPU_OK;
+}
+
 template <int MODE, typename MapT, int PM>
 int dispatch_batched_qu(BatchParams& bp, bool has_qu, bool iqu, cudaStream_t s) {
   if (has_qu && iqu) return launch_grouped<MODE, true, MapT, PM, kLayoutIQU>(bp, s);
@@ -2296,11 +2495,19 @@ int dispatch_batched_qu(BatchParams& bp, bool has_qu, bool iqu, cudaStream_t s) 
                 : launch_grouped<MODE, false, MapT, PM, kLayoutGeneric>(bp, s);
 }
 
+template <int MODE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
+int launch_single(const KArgs& k, cudaStream_t stream) {
+  Wants w;
+  add_wants<MODE, HAS_QU, MapT>(w, k, false);
+  const Shape s = choose_shape(w);
+  return s.tab_cap > 0 ? launch_gather<MODE, true, HAS_QU, MapT, PM, LAYOUT>(k, w, s, stream)
+                       : launch_gather<MODE, false, HAS_QU, MapT, PM, LAYOUT>(k, w, s, stream);
+}
 template <int MODE, typename MapT, int PM>
 int dispatch_qu(const KArgs& k, bool has_qu, cudaStream_t s) {
-  if (has_qu && k.C == 3 && k.c_q == 1 && k.c_u == 2) return launch_gather<MODE, true, MapT, PM, kLayoutIQU>(k, s);
-  return has_qu ? launch_gather<MODE, true, MapT, PM, kLayoutGeneric>(k, s)
-                : launch_gather<MODE, false, MapT, PM, kLayoutGeneric>(k, s);
+  if (has_qu && k.C == 3 && k.c_q == 1 && k.c_u == 2) return launch_single<MODE, true, MapT, PM, kLayoutIQU>(k, s);
+  return has_qu ? launch_single<MODE, true, MapT, PM, kLayoutGeneric>(k, s)
+                : launch_single<MODE, false, MapT, PM, kLayoutGeneric>(k, s);
 }
 
 

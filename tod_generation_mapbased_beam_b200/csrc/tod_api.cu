@@ -481,6 +481,26 @@ extern "C" int todgpu_gather_accum_static(const todgpu_gather_args* a, void* str
   return dispatch_types(k, a->interp, has_qu, a->map_dtype, a->params_dtype, s);
 }
 
+template <typename MapT>
+static JobWants wants_of(const KArgs& k, int interp, bool has_qu) {
+  if (interp == TODGPU_NEAREST)
+    return has_qu ? job_wants<TODGPU_NEAREST, true, MapT>(k) : job_wants<TODGPU_NEAREST, false, MapT>(k);
+  return has_qu ? job_wants<TODGPU_BILINEAR, true, MapT>(k) : job_wants<TODGPU_BILINEAR, false, MapT>(k);
+}
+
+extern "C" int todgpu_gather_wants(const todgpu_gather_args* a, int32_t* rings, int32_t* slots) {
+  const int rc = check_common(a, true);
+  if (rc != TODGPU_OK) return rc;
+  if (!rings || !slots) return fail(TODGPU_EINVAL, "NULL output");
+  const KArgs k = make_kargs(a);
+  const bool has_qu = a->c_q >= 0 && a->c_u >= 0;
+  const bool packed = a->map_dtype == TODGPU_PACKED_F32 || a->map_dtype == TODGPU_PACKED_BF16;
+  const JobWants j = packed ? wants_of<PackF32>(k, a->interp, has_qu) : wants_of<double>(k, a->interp, has_qu);
+  *rings = j.rings;
+  *slots = j.slots;
+  return TODGPU_OK;
+}
+
 extern "C" int64_t todgpu_gather_wait_timeouts(void) {
   // the gather kernels wait on nothing but their own CTA's barriers
   return cudaDeviceSynchronize() == cudaSuccess ? 0 : -1;
