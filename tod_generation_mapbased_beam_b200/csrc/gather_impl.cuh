@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -2320,24 +2321,41 @@ void add_wants(Wants& w, const KArgs& k, bool tables) {
   w.min_nt = std::max(w.min_nt, k.flags_wide ? 256 : 128);
 }
 
+// A kernel's opt-in to more than 48 KB of dynamic shared memory, once per device: the
+// attribute belongs to the current device's copy of the kernel, so a process-wide
+// flag would leave a second GPU's launches failing.
+class SmemOptIn {
+ public:
+  template <typename Bytes>
+  cudaError_t operator()(const void* kern, Bytes bytes) {  // bytes(): asked once per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (e != cudaSuccess || (done_.load() & bit)) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes());
+    if (e == cudaSuccess) done_.fetch_or(bit);
+    return e;
+  }
+
+ private:
+  std::atomic<unsigned long long> done_{0};
+};
+
+// All that the kernel's static shared memory leaves of a CTA's.
 template <typename Kern>
-int allow_smem(Kern kern, std::once_flag& once, cudaError_t& state) {
-  std::call_once(once, [&] {
+int allow_smem(Kern kern, SmemOptIn& opt_in) {
+  const cudaError_t e = opt_in(reinterpret_cast<const void*>(kern), [kern] {
     cudaFuncAttributes fa;
-    state = cudaFuncGetAttributes(&fa, kern);
-    if (state == cudaSuccess)
-      state = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(kSmemPerCTAMax - fa.sharedSizeBytes));
+    return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? (int)(kSmemPerCTAMax - fa.sharedSizeBytes) : -1;
   });
-  return state == cudaSuccess ? TODGPU_OK : cuda_fail(state, "kernel shared-memory attributes");
+  return e == cudaSuccess ? TODGPU_OK : cuda_fail(e, "kernel shared-memory attributes");
 }
 
 template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
 int launch_gather(KArgs k, const Wants& w, const Shape& s, cudaStream_t stream) {
   auto kern = gather_accum_kernel<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT>;
-  static std::once_flag once;
-  static cudaError_t state = cudaSuccess;
-  const int rc = allow_smem(kern, once, state);
+  static SmemOptIn opt_in;
+  const int rc = allow_smem(kern, opt_in);
   if (rc != TODGPU_OK) return rc;
   k.ring_cap = s.ring_cap;
   k.tab_cap = s.tab_cap;
@@ -2357,9 +2375,8 @@ static_assert(sizeof(KArgs) % 8 == 0 && sizeof(KArgs) / 8 <= 128, "KArgs copied 
 template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT>
 int launch_shape(BatchParams& bp, const Wants& w, const Shape& s, cudaStream_t stream) {
   auto kern = gather_batched_kernel<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT>;
-  static std::once_flag once;
-  static cudaError_t state = cudaSuccess;
-  const int rc = allow_smem(kern, once, state);
+  static SmemOptIn opt_in;
+  const int rc = allow_smem(kern, opt_in);
   if (rc != TODGPU_OK) return rc;
   for (int j = 0; j < bp.njobs; ++j) {
     bp.job[j].tab_cap = s.tab_cap;

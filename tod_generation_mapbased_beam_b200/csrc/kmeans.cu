@@ -22,7 +22,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "gather_impl.cuh"
 
@@ -490,12 +489,9 @@ extern "C" int todgpu_kmeans_seed(const double* vec, const double* w, int64_t S,
   double* bsum = dws + 2 * S;
   if (S <= kSeedPixels) {
     const size_t smem = sizeof(double) * kSeedThreads * ((S + kSeedThreads - 1) / kSeedThreads);
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-      attr = cudaFuncSetAttribute(seed_all_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(sizeof(double) * kSeedPixels));
-    });
+    static SmemOptIn opt_in;
+    const cudaError_t attr = opt_in(reinterpret_cast<const void*>(seed_all_kernel),
+                                    [] { return (int)(sizeof(double) * kSeedPixels); });
     if (attr != cudaSuccess) return cuda_fail(attr, "kmeans seeding attributes");
     for (int k0 = 0; k0 < K; k0 += kSeedBatch) {
       SeedDraws d;

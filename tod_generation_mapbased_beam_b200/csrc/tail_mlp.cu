@@ -1186,13 +1186,9 @@ inline bool encode_operand(CUtensorMap* map, const bf16* base, long long rows, i
 
 template <int N>
 bool launch_tc(const GemmArgs& g, cudaStream_t s) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(gemm_tc_fwd_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                TcShape<N>::SMEM);
-  });
-  if (attr != cudaSuccess) return false;
+  static SmemOptIn opt_in;
+  if (opt_in(reinterpret_cast<const void*>(gemm_tc_fwd_kernel<N>), [] { return (int)TcShape<N>::SMEM; }) != cudaSuccess)
+    return false;
   CUtensorMap ta, tw;
   if (!encode_operand(&ta, g.A, g.M, g.K, TC_BM) || !encode_operand(&tw, g.B, g.N, g.K, N)) return false;
   gemm_tc_fwd_kernel<N><<<dim3(g.M / TC_BM, g.N / N), TC_THREADS, TcShape<N>::SMEM, s>>>(ta, tw, g.K, g.bias, g.zout, g.aout,
@@ -1215,13 +1211,10 @@ inline bool forward_tc(const GemmArgs& g, cudaStream_t s) {
 
 template <int N, int O, typename T>
 bool launch_fused(const FusedArgs& f, const PackArgs& k, cudaStream_t s) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(tail_fused_kernel<N, O, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                fused_smem<N>(256));
-  });
-  if (attr != cudaSuccess) return false;
+  static SmemOptIn opt_in;
+  if (opt_in(reinterpret_cast<const void*>(tail_fused_kernel<N, O, T>), [] { return (int)fused_smem<N>(256); }) !=
+      cudaSuccess)
+    return false;
   const long long tiles = (f.B + 127) / 128;
   const int copies = (k.K0 + (k.D - 1) * N) / 8 * N;
   pack_weights_kernel<<<(copies + 255) / 256, 256, 0, s>>>(k);
