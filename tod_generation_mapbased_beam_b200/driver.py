@@ -32,7 +32,7 @@ import torch
 
 from . import _native
 from ._device import require_cuda
-from .kernels import beam_center_angles, gather_accum_angles
+from .kernels import _PIECE_MIN, beam_center_angles, gather_accum_angles, piece_footprints
 from .tod_core import _INTERP, beam_tod_batch, component_slots, device_beam, device_map
 from .tod_rotations import precompute_rotation_vector_batch
 
@@ -135,6 +135,7 @@ class _Entry:
     mp: torch.Tensor
     center: tuple
     rows: tuple | None
+    pieces: object = None  # piece_footprints of a beam wide enough to run in pieces
 
 
 @dataclass
@@ -167,7 +168,10 @@ class DayRunner:
                 vec, bv = device_beam(data["vec_orig"], data["beam_vals"], torch.float64)
                 self._entries.append(_Entry(
                     comps, c_q, c_u, vec, bv, device_map(data, self.mp),
-                    beam_center_angles(data["ra"], data["dec"]), _rows(len(comps), comps)))
+                    beam_center_angles(data["ra"], data["dec"]), _rows(len(comps), comps),
+                    # (found here: it reads the footprints back, which would stop the
+                    # chunks' overlap of upload, kernels and download)
+                    piece_footprints(vec, self.nside) if vec.shape[0] > _PIECE_MIN else None))
 
     # -- reference pointing -------------------------------------------------
     def _run_reference(self, theta, phi, psi):
@@ -201,11 +205,11 @@ class DayRunner:
                 r0, step = e.rows
                 dst = out[r0:r0 + (C - 1) * step + 1:step]
                 gather_accum_angles(interp, e.vec, th, ph, ps, e.center[0], e.center[1], self.nside,
-                                    e.mp, e.beam, dst, e.c_q, e.c_u)
+                                    e.mp, e.beam, dst, e.c_q, e.c_u, pieces=e.pieces)
             else:
                 tmp = torch.zeros((C, out.shape[1]), dtype=torch.float64, device=out.device)
                 gather_accum_angles(interp, e.vec, th, ph, ps, e.center[0], e.center[1], self.nside,
-                                    e.mp, e.beam, tmp, e.c_q, e.c_u)
+                                    e.mp, e.beam, tmp, e.c_q, e.c_u, pieces=e.pieces)
                 out.index_add_(0, torch.tensor(e.comps, device=out.device), tmp)
 
     def _run_device(self, theta, phi, psi):
