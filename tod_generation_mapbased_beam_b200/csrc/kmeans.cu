@@ -40,8 +40,10 @@ __device__ __forceinline__ double dot3(const double* v, double c0, double c1, do
 
 // labels[i] = argmax_k v_i . c_k (first maximum), best[i] = that maximum.  G
 // neighbouring lanes share a pixel, each taking a contiguous part of the
-// centroids (G > 1 where one lane per pixel would leave SMs idle: 5,414 pixels
-// against 200 centroids 50 -> 40 us with its host call).
+// centroids: 8 up to 16384 pixels, where one lane per pixel leaves SMs idle (200 and
+// 1000 centroids, us, one lane / eight: 5414 pixels 8.3 / 5.2, 26.7 / 12.3; 12,288
+// 8.3 / 6.2, 26.7 / 14.7; 30,000 8.3 / 8.3, 26.7 / 28.7; 65,536 10.3 / 14.4, 36.9 /
+// 51.3).
 template <int G>
 __global__ void assign_kernel(const double* vec, long long S, const double* cent, int K, int* labels, double* best) {
   __shared__ double sc[kCentTile * 3];
@@ -517,7 +519,7 @@ extern "C" int todgpu_kmeans_assign(const double* vec, int64_t S, const double* 
   if (!vec || !centroids || !labels || !best) return fail(TODGPU_EINVAL, "NULL pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* lab = reinterpret_cast<int*>(labels);
-  if (S <= (1 << 16))
+  if (S <= (1 << 14))
     assign_kernel<8><<<blocks_for(8 * S, kThreads), kThreads, 0, s>>>(vec, S, centroids, K, lab, best);
   else
     assign_kernel<1><<<blocks_for(S, kThreads), kThreads, 0, s>>>(vec, S, centroids, K, lab, best);
