@@ -1868,9 +1868,11 @@ __device__ __forceinline__ LoopState<Acc> nearest_loop(const PixelLoop<MapT, LAY
 template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT, class Acc, typename VecT>
 __device__ __noinline__ LoopState<Acc> wide_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
                                                  int ir_lo, int nwin, bool table, LoopState<Acc> st) {
-  if constexpr (MODE == TODGPU_NEAREST)
+  if constexpr (MODE == TODGPU_NEAREST) {
+    if (TABLE && !sb->wide)
+      return nearest_loop<kAnywhere, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, false, st);
     return nearest_loop<kWide, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, table, st);
-  else
+  } else
     return bilinear_loop<kWide, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, ir_lo, nwin, st);
 }
 
@@ -1878,8 +1880,8 @@ template <int MODE, bool TABLE, bool HAS_QU, typename MapT, int PM, int LAYOUT, 
 __device__ __forceinline__ LoopState<Acc> pixel_loop(const PixelLoop<MapT, LAYOUT, VecT>* p, const SampleBlock* sb,
                                                      const int4& hdr, int nside, const LoopState<Acc>& st) {
   const bool table = TABLE && hdr.z > 0;
-  // (nearest: a launch's sample whose footprint its table does not hold reads the map
-  // there too, so that the loops below have one source of values)
+  // (nearest: a sample whose footprint the launch's table does not hold reads the map
+  // there too, so that the loops below have one source of values: 1% of a nearest call)
   if (TABLE ? sb->wide || (MODE == TODGPU_NEAREST && !table) : sb->far)
     return wide_loop<MODE, TABLE, HAS_QU, MapT, PM, LAYOUT, Acc, VecT>(p, sb, hdr.x, hdr.y, table, st);
   // the window's rings all in the belt (rings nside to 3 nside)?
@@ -2199,7 +2201,8 @@ constexpr size_t static_smem() {
 // the rings either side); the default table reserves kRingCap.  A request is the
 // whole beam's: a chunk's window has fewer rings (kRingCap with its default table).
 inline int ring_cap_for(int requested, bool chunked, int slots) {
-  if (requested <= 0 || (chunked && slots > 0)) return kRingCap;
+  if (chunked ? slots > 0 : requested <= 0) return kRingCap;
+  if (requested <= 0) return kRingChunk;
   return std::min(chunked ? kRingChunk : kRingMax, (int)std::ceil(3.0 * std::sqrt(requested / 3.15)) + 6);
 }
 constexpr size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
