@@ -12,9 +12,12 @@ A step is one pass of the fused kernel over the whole batch.
 * ``value``: samples/s with the kernel inputs (float32 rotation parameters,
   boresight longitudes, beam, map) resident in HBM; the step zeroes the
   float64 (3, B) accumulator and runs the kernel.  Inputs (~1 GB) exceed L2.
-* ``roofline``: the gather view of the kernel -- S x K stencil pixels of R =
-  32-byte float64 records per sample -- against the L2 read bandwidth
-  measured live by ``todgpu_l2_probe``.
+* ``roofline``: the float64 arithmetic that an evaluation cannot do without
+  against the FP64 peak measured live (instruction issue bounds the kernel).
+  ``gather_frac``, there and in the other sections, is the gather view that
+  earlier versions were bound by -- S x K stencil pixels of R-byte records per
+  sample against the L2 read bandwidth measured live by ``todgpu_l2_probe`` --
+  of data that is no longer read from L2; it compares versions.
 * ``parity``: both modes of the timed configuration (same beam order, same
   map records, same float32 parameters) against the CPU oracle on a subset of
   samples spread over the day; nearest-pixel identity by an index map.
@@ -56,6 +59,10 @@ sys.path.insert(0, ROOT)
 
 METRIC = "TOD samples/s, 1 B200: FP64 plain vs mixed/learned-tail at fixed RMS error"
 
+# Float64 flops that a (sample, beam pixel) evaluation cannot do without: rotation,
+# place between the rings and on them, weights, four (value, weight) sums of I, Q, U.
+FLOPS_PER_EVAL = 71
+
 # FP64 flops per (sample, beam pixel) evaluation of the reference algorithm,
 # counted by ncu (dadd + dmul + 2 * dfma) on the direct-evaluation path
 # (TODGPU_FLAG_NO_TABLES) of the config-2 workload.  The timed kernel takes
@@ -92,7 +99,7 @@ def parse_args():
     p.add_argument("--no-tables", action="store_true",
                    help="evaluate ring data and spin-2 angles directly (A/B comparison)")
     p.add_argument("--no-beam-stage", action="store_true",
-                   help="read the beam from global memory instead of shared memory (A/B comparison)")
+                   help="no effect (the beam is never staged); kept for callers")
     p.add_argument("--cpu-seconds", type=float, default=10.0,
                    help="target CPU time of the bounded CPU-baseline sample")
     return p.parse_args()
@@ -496,22 +503,21 @@ def run_ours(args, dist):
     kernel_ms = dist.max(statistics.mean(kern_ms))
     value = B * dist.world * args.steps / (total_ms / 1e3)
 
-    # roofline: the gather view of the kernel -- S x K stencil pixels of R = 32
-    # byte float64 records per sample -- against the L2 read bandwidth measured
-    # now.  Beside it: the reference-equivalent FP64 rate (ncu-counted flops of
-    # the reference algorithm on this GPU) against the FP64 FMA peak measured
-    # now, and the compulsory HBM bytes against the measured HBM peak.
+    # roofline: the compulsory float64 arithmetic of an evaluation against the FP64
+    # FMA peak measured now.  Beside it: the reference-equivalent FP64 rate
+    # (ncu-counted flops of the reference algorithm on this GPU), the gather view and
+    # the compulsory HBM bytes against the measured HBM peak.
     peaks, peak_src = measured_peaks()
     l2_peak = l2_peak_gbs()
-    g_gbs, g_frac = gather_frac(B, S, args.mode, 32, kernel_ms, l2_peak)
+    _, g_frac = gather_frac(B, S, args.mode, 32, kernel_ms, l2_peak)
     fp64_peak = fp64_peak_tflops()
     ref_tflops = float(B) * S * REF_FLOPS_PER_EVAL[args.mode] / (kernel_ms / 1e3) / 1e12
     hbm_bytes = B * (4 * 11 + 8 * 3 * 2) + S * 16
-    roofline = {"bound": "l2", "achieved": g4(g_gbs), "peak": g4(l2_peak), "unit": "GB/s", "frac": g4(g_frac),
-                "traffic": None, "kernel": "gather_accum_kernel", "kernel_ms": g4(kernel_ms),
-                "bytes_per_sample": S * STENCIL[args.mode] * 32,
-                "peak_source": "todgpu_l2_probe, this run",
-                "fp64_peak_tflops": g4(fp64_peak),
+    own_tflops = float(B) * S * FLOPS_PER_EVAL / (kernel_ms / 1e3) / 1e12
+    roofline = {"bound": "issue", "achieved": g4(own_tflops), "peak": g4(fp64_peak), "unit": "TFLOP/s",
+                "frac": g4(own_tflops / fp64_peak), "traffic": None, "kernel": "gather_accum_kernel",
+                "kernel_ms": g4(kernel_ms), "flops_per_eval": FLOPS_PER_EVAL,
+                "peak_source": "todgpu_fp64_probe, this run", "gather_frac": g4(g_frac),
                 "ref_equiv_fp64_frac": g4(ref_tflops / fp64_peak),
                 "hbm_frac": g4(hbm_bytes / (kernel_ms / 1e3) / 1e9 / peaks["hbm_gbs"])}
     result = {"value": value, "ms_per_step": total_ms / args.steps, "roofline": roofline, "clocks": clk,

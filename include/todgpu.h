@@ -124,9 +124,11 @@ typedef struct todgpu_gather_args {
                             footprint's worth (about 1.03 (3.06 x^2 + 13.2 x + 12) + 8 for
                             a beam of radius x / nside) also sizes the window's rings, and
                             the smaller the table the more samples an SM works on.  A
-                            request beyond shared memory makes no table.  A sample whose
-                            footprint needs more than the table evaluates its pixels
-                            directly (same results).  Must be >= 0. */
+                            request beyond shared memory, or beyond what so few beam
+                            pixels would read, makes no table: the pixel loop reads the
+                            map (todgpu_gather_wants).  A sample whose footprint needs
+                            more than the table evaluates its pixels directly.  The
+                            results are the same.  Must be >= 0. */
   const void *ring_table;/* optional: table built by todgpu_ring_table_build for this
                             nside; NULL evaluates ring data and spin-2 angles directly */
   const void *theta;     /* (B,) boresight colatitude (TODGPU_ANGLES) */

@@ -372,7 +372,7 @@ struct __align__(16) RingRec {
   double dphi;      // pixel spacing
   double ta;        // acos(z)
   double inv_dta;   // 1 / (ta(ir + 1) - ta), correctly rounded (0 for the last ring)
-  int first32;      // first pixel index in 32 bits (exact while 12 nside^2 < 2^31)
+  int unused0;
   int n;            // pixels in the ring
   double inv_dphi;  // 1 / dphi, correctly rounded
   long long first;  // first pixel index
@@ -380,7 +380,7 @@ struct __align__(16) RingRec {
   int unused;
 };
 static_assert(sizeof(RingRec) == 80, "RingRec must be 80 bytes");
-static_assert(offsetof(RingRec, phi0) == 16 && offsetof(RingRec, ta) == 32 && offsetof(RingRec, first32) == 48,
+static_assert(offsetof(RingRec, phi0) == 16 && offsetof(RingRec, ta) == 32 && offsetof(RingRec, unused0) == 48,
               "RingRec pairs must sit on 16-byte boundaries");
 
 // The geometry of ring ir (all fields but cap), the values the ring table holds.
@@ -393,7 +393,7 @@ __device__ __forceinline__ RingRec make_ring(long long nside, long long ir) {
   r.phi0 = ri.phi0;
   r.dphi = ri.dphi;
   r.first = ri.first;
-  r.first32 = (int)ri.first;
+  r.unused0 = 0;
   r.n = (int)ri.n;
   r.inv_dphi = 1.0 / ri.dphi;
   r.inv_dta = ir < 4 * nside - 1 ? 1.0 / (acos(hp_ring_z(nside, ir + 1)) - r.ta) : 0.0;
@@ -573,8 +573,8 @@ __device__ __forceinline__ double atan_near(double t) {
   return fma(t * w, p, t);
 }
 
-// sin and cos of |x| <= kNearTan by their Taylor series (terms left out below
-// 2e-17 relative).
+// sin and cos of |x| <= kNearTan by their Taylor series (the first terms left out
+// are below 2.4e-17 of the sine and 3e-20).
 __device__ __forceinline__ void sincos_near(double x, double& s, double& c) {
   const double w = x * x;
   double p = fma(w, 1.0 / 362880.0, -1.0 / 5040.0);
@@ -588,12 +588,12 @@ __device__ __forceinline__ void sincos_near(double x, double& s, double& c) {
   c = fma(w, q, 1.0);
 }
 
-// Longitude of (x, y) in the sample's frame.
 // x > 0 and |t| < kNearTan for t = y / x by div_near, on the high words (a t
 // that is not finite -- x zero, denormal, infinite or NaN -- fails).
 __device__ __forceinline__ bool lon_is_near(double x, double t) {
   return __double2hiint(x) >= 0 && (__double2hiint(t) & 0x7fffffff) < 0x3fc00000;
 }
+// Longitude of (x, y) in the sample's frame.
 __device__ __forceinline__ double frame_lon(double x, double y) {
   const double t = div_near(y, x);
   return lon_is_near(x, t) ? atan_near(t) : atan2(y, x);
@@ -1761,8 +1761,8 @@ struct LoopState {
 // Bound (30' beam, S = 1512, nside 1024, 120k samples, float64 records): 5.30 ms
 // with the map gathered and the spin-2 angle looked up per neighbour (677
 // thread instructions an evaluation, L1 at 79%), 2.52 ms now, of which the
-// table fill is 0.4 and the window 0.1; ~210 instructions an evaluation, 66 of
-// them float64, issue slots 57% and the shared-memory data path 60-70% busy:
+// table fill is 0.4 and the window 0.1; 294 instructions an evaluation, all parts of a
+// sample counted, 66 float64 ones in this loop, issue slots 57% and the shared-memory data path 60-70% busy:
 // leaving out 12 of 16 shared loads saved 5%, 22 of 66 float64 operations 13%.
 // TABLE false: the same from the map (bound there: its loads, 12 a pixel with I, Q and
 // U, and L1, see choose_shape).  It stands in for the direct evaluation, one pixel at a
@@ -1996,7 +1996,7 @@ __device__ void run_samples(const KArgs& a, long long t_begin, long long t_end, 
       loop->nside = nside;
       loop->ch = ch;
     }
-    // the nearest rule's margin on ring boundaries (nearest_window) holds away
+    // the nearest rule's margin on ring boundaries (place_nearest) holds away
     // from the poles, where a ring's width in z vanishes
     const float reach = (float)rbeam;
     const double polar = MODE == TODGPU_NEAREST ? 0.01 : -4.0;

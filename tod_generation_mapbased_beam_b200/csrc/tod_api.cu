@@ -41,7 +41,7 @@ __global__ void ring_table_kernel(long long nside, double reach, RingRec* t, boo
     h.first = 0;
     h.n = 0;
     h.cap = 0;
-    h.first32 = 0;
+    h.unused0 = 0;
     h.unused = 0;
     h.inv_dphi = 0.0;
     h.inv_dta = 0.0;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) static_reach_kernel(const KArgs a, RingRe
     h.first = 0;
     h.n = 0;
     h.cap = 0;
-    h.first32 = 0;
+    h.unused0 = 0;
     h.unused = 0;
     h.inv_dphi = 0.0;
     h.inv_dta = 0.0;
