@@ -39,6 +39,10 @@ def uniform_pointings(n, seed):
     return (np.arccos(rng.uniform(-1.0, 1.0, n)), rng.uniform(0.0, 2 * np.pi, n), rng.uniform(0.0, 2 * np.pi, n))
 
 
+# Evaluations (samples x tail pixels) from which the plain tail reads records.
+_RECORD_EVALS = 5_000_000
+
+
 class LearnedTailTOD:
     """I/Q/U TOD of one beam entry (components [I, Q, U], spin-2 on) with the
     tail learned.
@@ -61,9 +65,7 @@ class LearnedTailTOD:
         # The float64 forms read the map itself in every call: a float64 CUDA tensor is
         # the caller's own, and a sky refilled in place (by alm2map, say, which no
         # modification counter shows) is the one the next call sees.  Records packed
-        # here would be the old sky's; they gain nothing at nside 1024 (301 pointings of
-        # a 284,000-pixel tail: 4.81 ms planar, 4.82 in records) and 12% below (nside 256
-        # and 512), about what packing them in each call would cost.
+        # here would be the old sky's (see _tail_sky).
         self.sky = sky
         self.sky_main = None if main_map == "f64" else pack_map(sky, main_map)
         self.main_map = main_map
@@ -86,6 +88,17 @@ class LearnedTailTOD:
         gather_accum_angles(self.interp, vec, theta, phi, psi, self.center[0], self.center[1], self.nside, mp, bv,
                             tod, c_q=1, c_u=2, pieces=pieces)
 
+    def _tail_sky(self, n):
+        """The map as the plain tail of ``n`` samples reads it: the caller's, or a copy
+        of it in records made for this call -- a third of the reads, the same values --
+        where that pays.  Microseconds planar / in records / packing them: nside 256,
+        17,604 pixels, 100 samples 635 / 581 / 40, 2000 samples 2713 / 2289 / 40; nside
+        512, 70,632 pixels, 40 samples 625 / 614 / 73, 301 samples 1550 / 1340 / 73;
+        nside 128, 2000 samples 631 / 635 / 31; nside 1024, 301 samples 4721 / 4646 / 238."""
+        if 256 <= self.nside <= 512 and n * self.tail_vec.shape[0] >= _RECORD_EVALS:
+            return pack_map(self.sky, "f64")
+        return self.sky
+
     @staticmethod
     def _dev(a, dev):
         t = torch.as_tensor(a, device=dev)
@@ -99,10 +112,11 @@ class LearnedTailTOD:
         B = th.numel()
         if tod is None:
             tod = torch.zeros((3, B), dtype=torch.float64, device=self.device)
+        sky = self._tail_sky(B)
         for b0 in range(0, B, self.tail_chunk):
             b1 = min(B, b0 + self.tail_chunk)
             part = torch.zeros((3, b1 - b0), dtype=torch.float64, device=self.device)
-            self._gather(self.tail_vec, self.tail_bv, self.sky, th[b0:b1], ph[b0:b1], ps[b0:b1], part,
+            self._gather(self.tail_vec, self.tail_bv, sky, th[b0:b1], ph[b0:b1], ps[b0:b1], part,
                          self.tail_pieces)
             tod[:, b0:b1] += part
         return tod
