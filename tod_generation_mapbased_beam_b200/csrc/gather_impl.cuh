@@ -2207,6 +2207,10 @@ inline int ring_cap_for(int requested, bool chunked, int slots) {
 }
 constexpr size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
+// (Nearest: only for turned Q and U values.)
+template <int MODE, bool HAS_QU>
+constexpr bool may_have_table() { return MODE == TODGPU_BILINEAR || HAS_QU; }
+
 // Whether a value table of `slots` (`bytes` in all) pays for a pass over `pixels`
 // beam pixels.  Filling a slot costs a map read and a turned (Q, U), more as fewer
 // CTAs share an SM; a pixel read from the table saves four of them.  Bilinear, I, Q
@@ -2222,9 +2226,10 @@ constexpr size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 // So: as many slots a pixel as CTAs with such a table fit an SM, four at most.
 template <int MODE, bool HAS_QU>
 bool table_pays(long long slots, long long pixels, size_t bytes) {
+  if (!may_have_table<MODE, HAS_QU>()) return false;
   // nearest reads one value per beam pixel: a table pays when the footprint
-  // has fewer pixels than the beam (and only for turned Q/U values)
-  if (MODE == TODGPU_NEAREST) return HAS_QU && slots <= pixels;
+  // has fewer pixels than the beam
+  if (MODE == TODGPU_NEAREST) return slots <= pixels;
   return slots <= (long long)std::min<size_t>(4, kSmemPerSM / (bytes + 8 * 1024)) * pixels;
 }
 
@@ -2400,8 +2405,9 @@ int launch_batched(BatchParams& bp, cudaStream_t stream) {
   for (int j = 0; j < bp.njobs; ++j) tables = tables || job_wants<MODE, HAS_QU, MapT>(bp.job[j]).slots > 0;
   for (int j = 0; j < bp.njobs; ++j) add_wants<MODE, HAS_QU, MapT>(w, bp.job[j], tables);
   const Shape s = choose_shape(w);
-  return s.tab_cap > 0 ? launch_shape<MODE, true, HAS_QU, MapT, PM, LAYOUT>(bp, w, s, stream)
-                       : launch_shape<MODE, false, HAS_QU, MapT, PM, LAYOUT>(bp, w, s, stream);
+  if constexpr (may_have_table<MODE, HAS_QU>())
+    if (s.tab_cap > 0) return launch_shape<MODE, true, HAS_QU, MapT, PM, LAYOUT>(bp, w, s, stream);
+  return launch_shape<MODE, false, HAS_QU, MapT, PM, LAYOUT>(bp, w, s, stream);
 }
 
 // A batch in launches of jobs whose own shapes keep equally many threads on an
@@ -2520,8 +2526,9 @@ int launch_single(const KArgs& k, cudaStream_t stream) {
   Wants w;
   add_wants<MODE, HAS_QU, MapT>(w, k, false);
   const Shape s = choose_shape(w);
-  return s.tab_cap > 0 ? launch_gather<MODE, true, HAS_QU, MapT, PM, LAYOUT>(k, w, s, stream)
-                       : launch_gather<MODE, false, HAS_QU, MapT, PM, LAYOUT>(k, w, s, stream);
+  if constexpr (may_have_table<MODE, HAS_QU>())
+    if (s.tab_cap > 0) return launch_gather<MODE, true, HAS_QU, MapT, PM, LAYOUT>(k, w, s, stream);
+  return launch_gather<MODE, false, HAS_QU, MapT, PM, LAYOUT>(k, w, s, stream);
 }
 template <int MODE, typename MapT, int PM>
 int dispatch_qu(const KArgs& k, bool has_qu, cudaStream_t s) {
