@@ -519,6 +519,16 @@ _PIECE = 1024
 # to there (284k pixels of an annulus, 301 samples: 4.72 ms; 5.06 at 3000, 5.11 at
 # 4400, 6.8 at 8192, where one CTA has the SM; pieces of 512 or 2048 pixels 5.9, 6.7).
 _PIECE_SLOTS = 2600
+# Wider pieces ask for a window without a table, as the gather's rule gives it: for more
+# slots than four times their pixels.  (With neither, every pixel went through the direct
+# evaluation: 60,000 pixels of 3 to 12 degrees, nside 1024, 8000 samples, I alone, nearest
+# 17.7 ms, now 7.4.)  Up to the slots of 700 window rings, which three CTAs of 256 threads
+# hold, and where they are tiles enough for the launch of their own that the library then
+# makes (16 an SM): fewer share the others' launch, where a window gains them nothing
+# (71,000 pixels, nside 512, 80 samples: 512 us, 560 with the windows).
+_PIECE_NO_TABLE = 4 * _PIECE + 1
+_PIECE_WINDOW = 170_000
+_PIECE_OWN_LAUNCH = 16 * 148
 _PIECE_TILE = 16  # samples per work tile of a piece's job
 _PIECE_SCRATCH = 1 << 28  # bytes of the pieces' own outputs: 116,000 samples of 96 pieces, I, Q and U
 
@@ -526,10 +536,11 @@ _PIECE_SCRATCH = 1 << 28  # bytes of the pieces' own outputs: 116,000 samples of
 class PiecePlan(NamedTuple):
     """:func:`piece_footprints` of a beam of S pixels over a map of one nside."""
 
-    slots: np.ndarray  # table slots of every piece
-    reach: float       # the pieces' largest footprint [rad]
+    slots: np.ndarray  # requested slots of every piece
+    reach: float       # the largest footprint with a table [rad]
     S: int
     nside: int
+    window_reach: float  # the largest with a window [rad]
 
 
 def _check_plan(plan, S, nside):
@@ -542,7 +553,8 @@ def _check_plan(plan, S, nside):
 def piece_footprints(vec, nside):
     """:class:`PiecePlan` of a wide beam, a CUDA (S, 3) tensor: the angle from a
     piece's mean direction to its farthest pixel, found on the device; pieces too
-    wide for a table ask for 2 slots.  A plan that a program keeps with its beam
+    wide for a table ask for more slots than one may have (a window alone), and those too
+    wide for that for 2.  A plan that a program keeps with its beam
     (``gather_accum_angles(pieces=...)``)."""
     S = vec.shape[0]
     n = (S + _PIECE - 1) // _PIECE
@@ -553,9 +565,10 @@ def piece_footprints(vec, nside):
     r = np.arccos(np.clip(low.cpu().numpy(), -1.0, 1.0))
     r = np.where(np.isfinite(r), r, np.pi) + 3.0 / float(nside) + 2e-5
     slots = footprint_slots(nside, r)
-    fits = slots <= _PIECE_SLOTS
-    return PiecePlan(np.where(fits, slots, 2).astype(np.int32), float(r[fits].max()) if fits.any() else 0.0, S,
-                     int(nside))
+    tabled, window = slots <= _PIECE_SLOTS, slots <= _PIECE_WINDOW
+    slots = np.where(tabled, slots, np.where(window, np.maximum(slots, _PIECE_NO_TABLE), 2))
+    most = lambda which: float(r[which].max()) if which.any() else 0.0
+    return PiecePlan(slots.astype(np.int32), most(tabled), S, int(nside), most(window))
 
 
 def _gather_pieces(args, vec, beam, nside, tod, pieces):
@@ -568,16 +581,19 @@ def _gather_pieces(args, vec, beam, nside, tod, pieces):
     run in blocks of samples, so the pieces' outputs stay within _PIECE_SCRATCH (the
     sums are a sample's own: the same in any block)."""
     S = vec.shape[0]
-    slots, reach = (pieces if pieces is not None else piece_footprints(vec, nside))[:2]
+    plan = pieces if pieces is not None else piece_footprints(vec, nside)
+    C, B = tod.shape
+    most = min(96, len(plan.slots))
+    block = min(B, max(_PIECE_TILE, _PIECE_SCRATCH // (most * C * 8) // _PIECE_TILE * _PIECE_TILE))
+    wide = plan.slots >= _PIECE_NO_TABLE
+    own = min(96, int(wide.sum())) * -(-block // _PIECE_TILE) >= _PIECE_OWN_LAUNCH
+    slots, reach = (plan.slots, plan.window_reach) if own else (np.where(wide, 2, plan.slots), plan.reach)
     flat = vec.contiguous()  # (pieces of a planar beam are not planar beams)
     args.flags &= ~_native.FLAG_BEAM_PLANAR
     if not args.flags & _native.FLAG_NO_TABLES and reach > 0.0:
         args.ring_table = ring_table(nside, reach, vec.device).data_ptr()
     elif not args.flags & _native.FLAG_NO_TABLES:
         args.ring_table = ring_table(nside, 3.0 / float(nside), vec.device).data_ptr()
-    C, B = tod.shape
-    most = min(96, len(slots))
-    block = min(B, max(_PIECE_TILE, _PIECE_SCRATCH // (most * C * 8) // _PIECE_TILE * _PIECE_TILE))
     part = torch.empty((most, C, block), dtype=torch.float64, device=vec.device)
     size = ctypes.sizeof(_native.GatherArgs)
     jobs = np.tile(np.frombuffer(bytes(args), np.uint8), (len(slots), 1))
@@ -587,7 +603,8 @@ def _gather_pieces(args, vec, beam, nside, tod, pieces):
     field("beam_vals", np.uint64)[:] = beam.data_ptr() + first * 4
     field("S", np.int64)[:] = np.minimum(_PIECE, S - first)
     field("tab_slots", np.int32)[:] = slots
-    jobs = np.ascontiguousarray(jobs[np.argsort(slots, kind="stable")])
+    # (those without a table first: the longest)
+    jobs = np.ascontiguousarray(jobs[np.argsort(np.where(slots <= _PIECE_SLOTS, slots, 0), kind="stable")])
     for b0 in range(0, B, block):
         nb = min(block, B - b0)
         for name in ("axes", "cos_a", "sin_a", "ax_pts", "cos_p", "sin_p"):
